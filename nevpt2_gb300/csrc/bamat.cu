@@ -15,7 +15,7 @@ namespace nvpt {
 #define FF(i, j) f[tri_index((i) + ncore, (j) + ncore) - 1]
 
 __global__ void __launch_bounds__(128) k_bamat_direct(Rdm r, const double *atwo, const double *f, int ncore,
-                                                      double *amat, double *atmat) {
+                                                      double *amat, double *atmat, const int *flag) {
     const int n = r.n, M = r.M;
     ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
     ll n6 = (ll)n * n * n * n * n * n;
@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(128) k_bamat_direct(Rdm r, const double *atwo,
     const int b = (int)(x % n) + 1; x /= n;
     const int c = (int)(x % n) + 1;
     for (int s = 1; s <= M; ++s) {
+        if (flag && !flag[s - 1]) continue;
         double A = 0.0, At = 0.0;
         for (int d = 1; d <= n; ++d) {
             double fda = FF(d, a), fcd = FF(c, d), fbd = FF(b, d);
@@ -77,9 +78,9 @@ __global__ void __launch_bounds__(128) k_bamat_direct(Rdm r, const double *atwo,
 }
 
 void launch_bamat_direct(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
-                         cudaStream_t st) {
+                         cudaStream_t st, const int *flag) {
     ll n6 = (ll)r.n * r.n * r.n * r.n * r.n * r.n;
-    k_bamat_direct<<<(unsigned)((n6 + 127) / 128), 128, 0, st>>>(r, atwo, f, ncore, amat, atmat);
+    k_bamat_direct<<<(unsigned)((n6 + 127) / 128), 128, 0, st>>>(r, atwo, f, ncore, amat, atmat, flag);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 

@@ -19,15 +19,13 @@
 // sums (bamat_rest below).
 // The slabs are materialised from the packed 4-RDM (ord8 gathers, delta
 // corrections of eeee) in the four K-major layouts the GEMMs read.
+#include "bamat_sym.cuh"
 #include "nvpt2_internal.h"
 #include "ozaki.cuh"
-#include "tuner.h"
-
-#include <cublas_v2.h>
 
 #include <algorithm>
-#include <cstdlib>
 #include <atomic>
+#include <cstdlib>
 #include <vector>
 
 namespace nvpt {
@@ -74,7 +72,8 @@ __global__ void __launch_bounds__(256) k_bamat_slabs(Rdm r, int s, const int *sl
 constexpr int kSlabTileMax = 16 * (16 * 17 + 1);
 __global__ void __launch_bounds__(256) k_bamat_slabs_t(Rdm r, int s, const int *slab_cp, const int *slab_ap,
                                                        int nslab, double *X1, double *X2, double *X3, double *X4,
-                                                       unsigned long long *rmax) {
+                                                       unsigned long long *rmax, const int *flag) {
+    if (flag && !*flag) return;
     __shared__ double tile[kSlabTileMax];
     __shared__ double mwz[256];
     const int n = r.n, sw = n + 1, sf = n * (n + 1) + 1;
@@ -181,7 +180,9 @@ __global__ void k_bamat_ints(const double *atwo, int n, double *A1, double *A2, 
 // 0-based row-major offset of X[x3,x4,x5,x6,cp,ap] ("cp,ap last" layout).
 #define RX6(x3, x4, x5, x6) (((((ll)(x3) * n + (x4)) * n + (x5)) * n + (x6)) * n2 + cpap)
 
-__global__ void __launch_bounds__(256) k_rest_dense(Rdm r, int s, double *E2, double *E2t, double *EE2) {
+__global__ void __launch_bounds__(256) k_rest_dense(Rdm r, int s, double *E2, double *E2t, double *EE2,
+                                                    const int *flag) {
+    if (flag && !*flag) return;
     const int n = r.n;
     const ll n4 = (ll)n * n * n * n, n6 = n4 * n * n;
     ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
@@ -228,7 +229,8 @@ __global__ void k_rest_ints(const double *atwo, const double *f, int ncore, int 
 
 // D[c,a,cp,ap] (n^4 outputs, ap fastest).  U = the EE2 x atwo GEMM, same layout.
 __global__ void __launch_bounds__(256) k_rest_delta(int n, const double *atwo, const double *Fs, const double *E2,
-                                                    const double *EE2, const double *U, double *D) {
+                                                    const double *EE2, const double *U, double *D, const int *flag) {
+    if (flag && !*flag) return;
     const ll n2 = (ll)n * n, n4 = n2 * n2;
     ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n4) return;
@@ -250,7 +252,8 @@ __global__ void __launch_bounds__(256) k_rest_delta(int n, const double *atwo, c
 // Writes amat/atmat(s, ap,bp,cp,a,b,c) (=, not +=) with the lower-order terms.
 __global__ void __launch_bounds__(256) k_rest_out(int n, int M, int s, const double *Fs, const double *E2,
                                                   const double *E2t, const double *T, const double *V,
-                                                  const double *D, double *amat, double *atmat) {
+                                                  const double *D, double *amat, double *atmat, const int *flag) {
+    if (flag && !*flag) return;
     __shared__ double sF[4 * 16 * 16];
     const ll n2 = (ll)n * n, n4 = n2 * n2;
     for (int i = threadIdx.x; i < 4 * n2; i += blockDim.x) sF[i] = Fs[i];
@@ -284,47 +287,36 @@ __global__ void __launch_bounds__(256) k_rest_out(int n, int M, int s, const dou
 }
 #undef RX6
 
-// row-major C[m,nn] = A^T B with A [k,m] and B [k,nn] row-major (batched over
-// B and C with the given strides; A shared).
-static int dgemm_rm_tA(cublasHandle_t h, long long m, long long nn, long long k, const double *A, const double *B,
-                       long long strideB, double *C, long long strideC, int batch) {
-    const double one = 1.0, zero = 0.0;
-    if (batch == 1)
-        return (int)cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, (int)nn, (int)m, (int)k, &one, B, (int)nn, A, (int)m,
-                                &zero, C, (int)nn);
-    return (int)cublasDgemmStridedBatched(h, CUBLAS_OP_N, CUBLAS_OP_T, (int)nn, (int)m, (int)k, &one, B, (int)nn,
-                                          strideB, A, (int)m, 0, &zero, C, (int)nn, strideC, batch);
-}
+static void dgemm_small(cudaStream_t st, ll m, ll nn, ll k, bool ta, const double *A, ll sA, const double *B, ll sB,
+                        double *C, ll sC, int batch, const int *flag);
 
 // Lower-order part of bamat for state s into amat/atmat; scratch holds
 // 4 n^6 + 5 n^4 + 4 n^2 doubles.
-static int bamat_rest(cublasHandle_t h, const Rdm &r, int s, const double *atwo, const double *f, int ncore,
-                      double *amat, double *atmat, double *scratch, cudaStream_t st) {
+static void bamat_rest(const Rdm &r, int s, const double *atwo, const double *f, int ncore, double *amat,
+                       double *atmat, double *scratch, cudaStream_t st, const int *flag) {
     const int n = r.n, M = r.M;
     const ll n2 = (ll)n * n, n4 = n2 * n2, n6 = n4 * n2;
     double *E2 = scratch, *E2t = E2 + n6, *T = E2t + n6, *V = T + n6;
     double *EE2 = V + n6, *U = EE2 + n4, *D = U + n4, *G = D + n4, *H = G + n4, *Fs = H + n4;
-    k_rest_dense<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(r, s, E2, E2t, EE2);
+    k_rest_dense<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(r, s, E2, E2t, EE2, flag);
     k_rest_ints<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(atwo, f, ncore, n, Fs, G, H);
     g_launches.fetch_add(2, std::memory_order_relaxed);
-    int rc = 0;
     // T[(bp,b)][(c,a),(cp,ap)] = G^T E2[(bp,b)][(d,e),(cp,ap)]
-    rc |= dgemm_rm_tA(h, n2, n2, n2, G, E2, n4, T, n4, (int)n2);
+    dgemm_small(st, n2, n2, n2, true, G, 0, E2, n4, T, n4, (int)n2, flag);
     // V[(b,bp),(a,c,cp,ap)] = H^T E2[(d,e),(a,c,cp,ap)]
-    rc |= dgemm_rm_tA(h, n2, n4, n2, H, E2, 0, V, 0, 1);
+    dgemm_small(st, n2, n4, n2, true, H, 0, E2, 0, V, 0, 1, flag);
     // U[(c,a),(cp,ap)] = G^T EE2[(d,e),(cp,ap)]
-    rc |= dgemm_rm_tA(h, n2, n2, n2, G, EE2, 0, U, 0, 1);
-    if (rc) return rc;
-    k_rest_delta<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(n, atwo, Fs, E2, EE2, U, D);
-    k_rest_out<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(n, M, s, Fs, E2, E2t, T, V, D, amat, atmat);
+    dgemm_small(st, n2, n2, n2, true, G, 0, EE2, 0, U, 0, 1, flag);
+    k_rest_delta<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(n, atwo, Fs, E2, EE2, U, D, flag);
+    k_rest_out<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(n, M, s, Fs, E2, E2t, T, V, D, amat, atmat, flag);
     g_launches.fetch_add(2, std::memory_order_relaxed);
-    return 0;
 }
 
 // Add the GEMM results: Tk are [(cp,ap) slab][rows][n] with the row layouts
 // of the GEMMs above (slab index = cp*n + ap).
 __global__ void k_bamat_assemble(int n, int M, int s, const double *T1, const double *T2, const double *T3,
-                                 const double *T4, double *amat, double *atmat) {
+                                 const double *T4, double *amat, double *atmat, const int *flag) {
+    if (flag && !*flag) return;
     ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
     const ll n3 = (ll)n * n * n, n4 = n3 * n;
     ll n6 = n3 * n3;
@@ -366,10 +358,12 @@ struct SkinnyJobs {
     const double *X[4];
     const double *B[4];
     double *C[4];
+    const int *flag;  // null, or the launch does nothing while *flag is zero
 };
 
 template <int RPT>
 __global__ void __launch_bounds__(256, 2) k_dgemm_skinny(SkinnyJobs jobs, ll rows, int N, int K) {
+    if (jobs.flag && !*jobs.flag) return;
     constexpr int BM = 32 * RPT, LD = BM + 1, NX = BM / 8;
     __shared__ double Xs[kSkBK * LD];
     __shared__ __align__(16) double Bs[kSkBK * 16];
@@ -437,6 +431,7 @@ __global__ void __launch_bounds__(256, 2) k_dgemm_skinny(SkinnyJobs jobs, ll row
 // .f64): A a0 = A[lane/4][lane%4], B b0 = B[lane%4][lane/4], C c0,c1 =
 // C[lane/4][2(lane%4) + {0,1}].
 __global__ void __launch_bounds__(256, 2) k_dgemm_skinny_dmma(SkinnyJobs jobs, ll rows, int N, int K) {
+    if (jobs.flag && !*jobs.flag) return;
     constexpr int BM = 128, LD = BM + 1, NX = BM / 8;
     __shared__ double Xs[kSkBK * LD];
     __shared__ __align__(16) double Bs[kSkBK * 16];
@@ -519,50 +514,28 @@ static void launch_skinny(int rpt, cudaStream_t st, const SkinnyJobs &j, ll rows
 }
 
 static int dgemm_skinny4(cudaStream_t st, ll rows, int N, int K, const double *const X[4], const double *const B[4],
-                         double *const C[4]) {
+                         double *const C[4], const int *flag) {
     SkinnyJobs j;
+    j.flag = flag;
     for (int i = 0; i < 4; ++i) {
         j.X[i] = X[i];
         j.B[i] = B[i];
         j.C[i] = C[i];
     }
-    // rows per thread (tile height 32 RPT), tuned per shape
-    // variant, tuned per shape: DFMA with 2 or 4 rows per thread, or DMMA;
-    // NVPT_SKINNY_VARIANT (1, 2, 4) fixes it (tests of each variant)
-    static const int kRpt[] = {2, 4, 1};
+    // Four rows per thread while there are few row tiles, two at the largest
+    // shapes (65536 x 4096 x 16: 27.6 ms with two, 28.6 with four, 32.5 on the
+    // FP64 tensor cores); NVPT_SKINNY_VARIANT (1, 2, 4) fixes the variant
+    // (tests of each).
     static const int forced = [] {
         const char *e = std::getenv("NVPT_SKINNY_VARIANT");
         const int v = e ? std::atoi(e) : 0;
         return (v == 1 || v == 2 || v == 4) ? v : 0;
     }();
-    if (forced) {
-        launch_skinny(forced, st, j, rows, N, K);
-        return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
-    }
-    const std::string key = "bamat_skinny.rows_per_thread/" + std::to_string(rows) + "x" + std::to_string(K) + "x" +
-                            std::to_string(N);
-    int used = -1;
-    const int rpt = tune::choose(key, kRpt, 3, 4, st, [&](int c) { launch_skinny(c, st, j, rows, N, K); used = c; });
-    if (used < 0) launch_skinny(rpt, st, j, rows, N, K);
+    launch_skinny(forced ? forced : rows >= 65536 ? 2 : 4, st, j, rows, N, K);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
 }
 
 // ---------------------------------------------------------------------------
-struct BamatGemm {
-    cublasHandle_t h = nullptr;
-    ~BamatGemm() {
-        if (h) cublasDestroy(h);
-    }
-};
-
-static int dgemm_rm(cublasHandle_t h, long long m, long long nn, long long k, const double *A, const double *B,
-                    double *C) {
-    // row-major C[m,nn] = A[m,k] B[k,nn]  <=>  column-major C^T = B^T A^T
-    const double one = 1.0, zero = 0.0;
-    return (int)cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, (int)nn, (int)m, (int)k, &one, B, (int)nn, A, (int)k,
-                            &zero, C, (int)nn);
-}
-
 // Device buffers of one launch_bamat_gemm call, released on every return path
 // (stream-ordered frees on the call's stream).
 struct AsyncBuffers {
@@ -584,117 +557,80 @@ struct AsyncBuffers {
 
 __global__ void k_slab_list(int n, int *cp, int *ap);
 
-// Returns 0 on success, else a CUDA / cuBLAS error code (nonzero).
-int launch_bamat_gemm(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
-                      cudaStream_t st, int slabs_per_batch, bool split) {
+// Returns 0 on success, 2 on a failed allocation, 5 if a split-precision
+// product timed out, else a launch failure.
+int launch_bamat(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
+                 cudaStream_t st, bool split) {
     const int n = r.n, M = r.M;
-    const ll n3 = (ll)n * n * n, n4 = n3 * n, n6 = n3 * n3;
-    static thread_local BamatGemm handle;
-    if (!handle.h && cublasCreate(&handle.h) != CUBLAS_STATUS_SUCCESS) return 1;
-    if (cublasSetStream(handle.h, st) != CUBLAS_STATUS_SUCCESS) return 1;
-    cublasSetMathMode(handle.h, CUBLAS_DEFAULT_MATH);
-    // lower-order part first (writes amat/atmat), then add the GEMM terms
-    {
-        AsyncBuffers rest(st);
-        double *scr;
-        const ll n2 = (ll)n * n;
-        if (!rest.get(&scr, sizeof(double) * (4 * n6 + 5 * n4 + 4 * n2))) return 2;
-        int rrc = 0;
-        for (int s = 0; s < M && !rrc; ++s) rrc = bamat_rest(handle.h, r, s, atwo, f, ncore, amat, atmat, scr, st);
-        if (rrc) return 3;
-    }
+    const ll n2 = (ll)n * n, n3 = n2 * n, n4 = n3 * n, n6 = n3 * n3;
     AsyncBuffers buf(st);
-    double *A1, *A2, *A3, *T, *X[2];
-    const int B = slabs_per_batch;
+    // Slabs of the general route: a few at a time, or all of them where they are small.
+    const bool direct = n <= 5;
+    const int B = direct ? 0 : n <= 8 ? (int)n2 : 16;
+    const size_t xd = std::max<size_t>(4 * (size_t)B * n6, split ? 0 : (size_t)SymScratch::doubles(n));
+    double *X;
+    int *flag = nullptr;
+    if (!buf.get(&X, sizeof(double) * xd)) return 2;
+    // FP64: one contraction per state whose inputs have their physical
+    // symmetries (bamat_sym.cu); it raises flag[s] where they have not, and the
+    // general route below does the flagged states.  Its scratch is the slab
+    // buffer: each state's general route follows in stream order.
+    auto flag_of = [&](int s) { return flag ? flag + s : nullptr; };
+    if (!split) {
+        if (!buf.get(&flag, sizeof(int) * M)) return 2;
+        cudaMemsetAsync(flag, 0, sizeof(int) * M, st);
+        const SymScratch S(n, X);
+        launch_sym_ops(atwo, f, ncore, n, S, M, flag, st);
+        for (int s = 0; s < M; ++s)
+            if (launch_sym_state(r, s, atwo, S, amat, atmat, flag, st)) return 3;
+        if (direct) {
+            launch_bamat_direct(r, atwo, f, ncore, amat, atmat, st, flag);
+            return 0;
+        }
+    } else if (direct) {
+        launch_bamat_direct(r, atwo, f, ncore, amat, atmat, st, nullptr);
+        return 0;
+    }
+    double *A1, *A2, *A3, *T;
     int *slabs;
-    if (!buf.get(&A1, sizeof(double) * 3 * n4) || !buf.get(&T, sizeof(double) * 4 * n6) ||
-        !buf.get(&X[0], sizeof(double) * 4 * (size_t)B * n6) || !buf.get(&X[1], sizeof(double) * 4 * (size_t)B * n6) ||
-        !buf.get(&slabs, sizeof(int) * 2 * n * n))
+    if (!buf.get(&A1, sizeof(double) * 3 * n4) || !buf.get(&T, sizeof(double) * (4 * n6 + 5 * n4 + 4 * n2)) ||
+        !buf.get(&slabs, sizeof(int) * 2 * n2))
         return 2;
     A2 = A1 + n4;
     A3 = A2 + n4;
+    // lower-order part first (writes amat/atmat, scratch T), then add the GEMM terms
+    for (int s = 0; s < M; ++s) bamat_rest(r, s, atwo, f, ncore, amat, atmat, T, st, flag_of(s));
     k_bamat_ints<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(atwo, n, A1, A2, A3);
-    k_slab_list<<<(unsigned)((n * n + 255) / 256), 256, 0, st>>>(n, slabs, slabs + n * n);
+    k_slab_list<<<(unsigned)((n2 + 255) / 256), 256, 0, st>>>(n, slabs, slabs + n2);
     g_launches.fetch_add(2, std::memory_order_relaxed);
     int rc = 0;
     // split precision: digit workspace for a full batch of slabs
     void *ozw = nullptr;
-    unsigned long long *rmax[2] = {nullptr, nullptr};  // row maxima of the four slab layouts (split digits)
+    unsigned long long *rmax = nullptr;  // row maxima of the four slab layouts (split digits)
     if (split) {
         oz::OzPlan pl(4, (ll)B * n3, (int)n3, n);
-        if (!buf.get(&ozw, pl.bytes()) || !buf.get(&rmax[0], sizeof(unsigned long long) * 4 * (size_t)B * n3) ||
-            !buf.get(&rmax[1], sizeof(unsigned long long) * 4 * (size_t)B * n3))
-            return 2;
+        if (!buf.get(&ozw, pl.bytes()) || !buf.get(&rmax, sizeof(unsigned long long) * 4 * (size_t)B * n3)) return 2;
     }
-    // Slab production (gather-bound on the packed 4-RDM) runs one batch ahead
-    // on a stream of its own into the other of two slab buffers, so that it
-    // overlaps the products of the current batch (FP64 pipe, or HBM-bound
-    // digit streams in split mode).  Events order buffer reuse; the guard
-    // joins the producer stream into st before the buffers are released
-    // (it is destroyed before `buf`).
-    struct Producer {
-        cudaStream_t st, g = nullptr;
-        cudaEvent_t in = nullptr, gen[2] = {nullptr, nullptr}, use[2] = {nullptr, nullptr}, end = nullptr;
-        bool ok = false;
-        explicit Producer(cudaStream_t s) : st(s) {
-            ok = cudaStreamCreateWithFlags(&g, cudaStreamNonBlocking) == cudaSuccess;
-            for (cudaEvent_t *e : {&in, &gen[0], &gen[1], &use[0], &use[1], &end})
-                ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
-            ok = ok && cudaEventRecord(in, st) == cudaSuccess && cudaStreamWaitEvent(g, in, 0) == cudaSuccess;
-        }
-        ~Producer() {
-            if (g && end) {
-                cudaEventRecord(end, g);
-                cudaStreamWaitEvent(st, end, 0);
+    for (int s = 0; s < M && !rc; ++s) {
+        for (int s0 = 0; s0 < n2 && !rc; s0 += B) {
+            const int nb = std::min(B, (int)n2 - s0);
+            const ll rows = (ll)nb * n3;
+            const double *Xs[4] = {X, X + (ll)B * n6, X + 2 * (ll)B * n6, X + 3 * (ll)B * n6}, *As[4] = {A1, A2, A3, A3};
+            if (rmax) cudaMemsetAsync(rmax, 0, sizeof(unsigned long long) * 4 * (size_t)rows, st);
+            k_bamat_slabs_t<<<(unsigned)rows, 256, 0, st>>>(r, s, slabs + s0, slabs + n2 + s0, nb, X, X + (ll)B * n6,
+                                                            X + 2 * (ll)B * n6, X + 3 * (ll)B * n6, rmax, flag_of(s));
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+            double *Ts[4] = {T + (ll)s0 * n4, T + n6 + (ll)s0 * n4, T + 2 * n6 + (ll)s0 * n4, T + 3 * n6 + (ll)s0 * n4};
+            if (split) {
+                const unsigned long long *Rm[4] = {rmax, rmax + rows, rmax + 2 * rows, rmax + 3 * rows};
+                rc |= oz::oz_gemm_skinny(oz::OzPlan(4, rows, (int)n3, n), Xs, As, Ts, n, n, ozw, st, Rm);
+            } else {
+                rc |= dgemm_skinny4(st, rows, n, (int)n3, Xs, As, Ts, flag_of(s));
             }
-            for (cudaEvent_t e : {in, gen[0], gen[1], use[0], use[1], end})
-                if (e) cudaEventDestroy(e);
-            if (g) cudaStreamDestroy(g);
         }
-    } prod(st);
-    if (!prod.ok) return 1;
-    const int per_state = (n * n + B - 1) / B, nbatch = M * per_state;
-    auto batch = [&](int gb, int &s, int &s0, int &nb) {
-        s = gb / per_state;
-        s0 = (gb % per_state) * B;
-        nb = std::min(B, n * n - s0);
-    };
-    auto produce = [&](int gb) {
-        int s, s0, nb;
-        batch(gb, s, s0, nb);
-        const int q = gb & 1;
-        if (gb >= 2) cudaStreamWaitEvent(prod.g, prod.use[q], 0);
-        const ll rows = (ll)nb * n3;
-        double *X1 = X[q], *X2 = X1 + (ll)B * n6, *X3 = X2 + (ll)B * n6, *X4 = X3 + (ll)B * n6;
-        if (rmax[q]) cudaMemsetAsync(rmax[q], 0, sizeof(unsigned long long) * 4 * (size_t)rows, prod.g);
-        k_bamat_slabs_t<<<(unsigned)rows, 256, 0, prod.g>>>(r, s, slabs + s0, slabs + n * n + s0, nb, X1, X2, X3, X4,
-                                                             rmax[q]);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        cudaEventRecord(prod.gen[q], prod.g);
-    };
-    produce(0);
-    for (int gb = 0; gb < nbatch && !rc; ++gb) {
-        if (gb + 1 < nbatch) produce(gb + 1);
-        int s, s0, nb;
-        batch(gb, s, s0, nb);
-        const int q = gb & 1;
-        cudaStreamWaitEvent(st, prod.gen[q], 0);
-        const ll rows = (ll)nb * n3;
-        double *X1 = X[q], *X2 = X1 + (ll)B * n6, *X3 = X2 + (ll)B * n6, *X4 = X3 + (ll)B * n6;
-        double *T1 = T + (ll)s0 * n4, *T2 = T + n6 + (ll)s0 * n4, *T3 = T + 2 * n6 + (ll)s0 * n4,
-               *T4 = T + 3 * n6 + (ll)s0 * n4;
-        const double *Xs[4] = {X1, X2, X3, X4}, *As[4] = {A1, A2, A3, A3};
-        double *Ts[4] = {T1, T2, T3, T4};
-        if (split) {
-            const unsigned long long *Rm[4] = {rmax[q], rmax[q] + rows, rmax[q] + 2 * rows, rmax[q] + 3 * rows};
-            rc |= oz::oz_gemm_skinny(oz::OzPlan(4, rows, (int)n3, n), Xs, As, Ts, n, n, ozw, st, Rm);
-        } else {
-            rc |= dgemm_skinny4(st, rows, n, (int)n3, Xs, As, Ts);
-        }
-        cudaEventRecord(prod.use[q], st);
-        if (!rc && s0 + nb == n * n) {  // last batch of state s
+        if (!rc) {
             k_bamat_assemble<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(n, M, s, T, T + n6, T + 2 * n6, T + 3 * n6,
-                                                                        amat, atmat);
+                                                                        amat, atmat, flag_of(s));
             g_launches.fetch_add(1, std::memory_order_relaxed);
         }
     }
@@ -720,7 +656,8 @@ static __device__ __align__(256) double g_bamat_scratch[kBamatStaticDoubles];
 // Row-major C[m,nn] = op(A) B, op(A) = A [m,k] or, with ta, A^T for A [k,m];
 // B [k,nn].  blockIdx.z selects the batch (strides sA, sB, sC).
 __global__ void __launch_bounds__(256) k_dgemm_small(int m, int nn, int k, int ta, const double *A, ll sA,
-                                                     const double *B, ll sB, double *C, ll sC) {
+                                                     const double *B, ll sB, double *C, ll sC, const int *flag) {
+    if (flag && !*flag) return;
     __shared__ double As[16][17], Bs[16][17];
     const int tx = threadIdx.x, ty = threadIdx.y;
     A += (ll)blockIdx.z * sA;
@@ -741,9 +678,9 @@ __global__ void __launch_bounds__(256) k_dgemm_small(int m, int nn, int k, int t
 }
 
 static void dgemm_small(cudaStream_t st, ll m, ll nn, ll k, bool ta, const double *A, ll sA, const double *B, ll sB,
-                        double *C, ll sC, int batch) {
+                        double *C, ll sC, int batch, const int *flag) {
     dim3 grid((unsigned)((nn + 15) / 16), (unsigned)((m + 15) / 16), (unsigned)batch);
-    k_dgemm_small<<<grid, dim3(16, 16), 0, st>>>((int)m, (int)nn, (int)k, ta ? 1 : 0, A, sA, B, sB, C, sC);
+    k_dgemm_small<<<grid, dim3(16, 16), 0, st>>>((int)m, (int)nn, (int)k, ta ? 1 : 0, A, sA, B, sB, C, sC, flag);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
@@ -808,14 +745,14 @@ int launch_bamat_static(const Rdm &r, const double *atwo, const double *f, int n
         // lower-order terms (bamat_rest with the small GEMM kernel)
         double *E2 = scratch, *E2t = E2 + n6, *T = E2t + n6, *V = T + n6;
         double *EE2 = V + n6, *U = EE2 + n4, *D = U + n4, *G = D + n4, *H = G + n4, *Fs = H + n4;
-        k_rest_dense<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(r, s, E2, E2t, EE2);
+        k_rest_dense<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(r, s, E2, E2t, EE2, nullptr);
         k_rest_ints<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(atwo, f, ncore, n, Fs, G, H);
         g_launches.fetch_add(2, std::memory_order_relaxed);
-        dgemm_small(st, n2, n2, n2, true, G, 0, E2, n4, T, n4, (int)n2);
-        dgemm_small(st, n2, n4, n2, true, H, 0, E2, 0, V, 0, 1);
-        dgemm_small(st, n2, n2, n2, true, G, 0, EE2, 0, U, 0, 1);
-        k_rest_delta<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(n, atwo, Fs, E2, EE2, U, D);
-        k_rest_out<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(n, M, s, Fs, E2, E2t, T, V, D, amat, atmat);
+        dgemm_small(st, n2, n2, n2, true, G, 0, E2, n4, T, n4, (int)n2, nullptr);
+        dgemm_small(st, n2, n4, n2, true, H, 0, E2, 0, V, 0, 1, nullptr);
+        dgemm_small(st, n2, n2, n2, true, G, 0, EE2, 0, U, 0, 1, nullptr);
+        k_rest_delta<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(n, atwo, Fs, E2, EE2, U, D, nullptr);
+        k_rest_out<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(n, M, s, Fs, E2, E2t, T, V, D, amat, atmat, nullptr);
         g_launches.fetch_add(2, std::memory_order_relaxed);
         // n^9 part, one slab at a time (the same scratch, reused in stream order)
         double *A1 = scratch, *A2 = A1 + n4, *A3 = A2 + n4;
@@ -828,10 +765,10 @@ int launch_bamat_static(const Rdm &r, const double *atwo, const double *f, int n
         for (int sl = 0; sl < n2; ++sl) {
             k_bamat_slabs<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(r, s, cpl + sl, apl + sl, 1, X1, X2, X3, X4);
             g_launches.fetch_add(1, std::memory_order_relaxed);
-            dgemm_small(st, n3, n, n3, false, X1, 0, A1, 0, T1, 0, 1);
-            dgemm_small(st, n3, n, n3, false, X2, 0, A2, 0, T2, 0, 1);
-            dgemm_small(st, n3, n, n3, false, X3, 0, A3, 0, T3, 0, 1);
-            dgemm_small(st, n3, n, n3, false, X4, 0, A3, 0, T4, 0, 1);
+            dgemm_small(st, n3, n, n3, false, X1, 0, A1, 0, T1, 0, 1, nullptr);
+            dgemm_small(st, n3, n, n3, false, X2, 0, A2, 0, T2, 0, 1, nullptr);
+            dgemm_small(st, n3, n, n3, false, X3, 0, A3, 0, T3, 0, 1, nullptr);
+            dgemm_small(st, n3, n, n3, false, X4, 0, A3, 0, T4, 0, 1, nullptr);
             k_bamat_assemble_slab<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(n, M, s, sl / n, sl % n, T1, T2, T3,
                                                                                 T4, amat, atmat);
             g_launches.fetch_add(1, std::memory_order_relaxed);

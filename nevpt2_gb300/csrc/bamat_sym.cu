@@ -1,0 +1,595 @@
+// A-matrices of the (+-1') classes (src/koopro4QD.F90:3974-4104) from one n^9
+// contraction.
+//
+// The reference's loop needs four contractions of the four-operator products
+// with the active integrals.  For RDMs with their physical symmetries
+//   Gamma_k[P1 .. Pk] invariant under permutations of the pairs P = (creator,
+//   annihilator) and under exchange of all creators with all annihilators,
+// and integrals with (ij|kl) = (ji|kl) = (kl|ij), the Gamma4 part of each is
+// the same tensor with other arguments,
+//   F[A,B;c,a] = sum_{d,f,e} Gamma4[A, B, (d,f), (e,c)] (df|ea),
+// F is symmetric under A <-> B, and (df| is symmetric, so n^9 flops take the
+// place of 8 n^9.  What normal ordering adds is of order n^8 in Gamma3,
+//   J[P1,P2;x,y]     = sum_{d,f} Gamma3[P1, P2, (d,f)] (df|xy)
+//   Kx[P1,P2;x,y]    = sum_{d,e} Gamma3[P1, P2, (d,e)] (xd|ye)
+//   Wca[p,(q,r),s;x,y] = sum_{f,e} Gamma3[(p,f), (q,r), (e,s)] (xf|ye)
+//   Waa[p,(q,r),t;x,y] = sum_{f,e} Gamma3[(p,f), (q,r), (t,e)] (xf|ye)
+// each with a two-fold symmetry in its row labels, and n^7 and below.  With
+// A = (cp,ap), B = (bp,b), B' = (b,bp), P^T = (annihilator, creator), E3, E2
+// the three- and two-operator products, g = f + K/2, K(x,y) = sum_z (xz|zy):
+//   amat  = sum_d [E3[A,B,(d,c)] g(d,a) - E3[A,B,(a,d)] g(c,d) - E3[A,(bp,d),(a,c)] g(b,d)]
+//         + F[A,B;c,a] - F[A^T,B^T;a,c] - F[A^T,(c,a);bp,b]
+//         + Wca[cp,B,c;ap,a] + J[(cp,c),B;ap,a] - Waa[cp,B,a;ap,c] - Waa[bp,A,a;b,c]
+//         - Waa[cp,(a,c),bp;ap,b] + Kronecker-delta terms (k_sym_out)
+// and likewise atmat.  tests/test_bamat_sym.py evaluates these sums in numpy
+// against the reference's loop.
+//
+// Which inputs take this route is decided on the device, for each state,
+// without a host synchronisation: k_sym_unpack checks every symmetry that is
+// used, to 2^-45 of the largest element of Gamma1 (and of the largest (ii|ii)
+// for the integrals) -- the rounding of an RDM builder is below, anything else
+// is not -- and raises the state's flag.  Every kernel here returns at once for
+// a flagged state, and every kernel of the general route (bamat_gemm.cu)
+// returns at once for the others.
+#include <algorithm>
+
+#include "bamat_sym.cuh"
+
+namespace nvpt {
+namespace {
+
+constexpr double kSymTol = 0x1p-45;
+
+__host__ __device__ __forceinline__ int pidx(int i, int j) { return i * (i + 1) / 2 + j; }  // i >= j
+__device__ __forceinline__ int pmx(int i, int j) { return i > j ? pidx(i, j) : pidx(j, i); }
+
+// Packed rank (0-based) of a descending quadruple of 0-based indices.
+__device__ __forceinline__ int rank4(const int v[4]) { return lindice4(v[0] + 1, v[1] + 1, v[2] + 1, v[3] + 1) - 1; }
+
+// Sorts v descending; o[j] = original position of the j-th largest.
+__device__ __forceinline__ void sort4(int v[4], int o[4]) {
+    o[0] = 0; o[1] = 1; o[2] = 2; o[3] = 3;
+#define NV_CE(i, j)                       \
+    if (v[i] < v[j]) {                    \
+        int t = v[i]; v[i] = v[j]; v[j] = t; \
+        t = o[i]; o[i] = o[j]; o[j] = t;  \
+    }
+    NV_CE(0, 1) NV_CE(2, 3) NV_CE(0, 2) NV_CE(1, 3) NV_CE(1, 2)
+#undef NV_CE
+}
+
+#define AT(i, j, k, l) atwo[(i) + (ll)n * ((j) + (ll)n * ((k) + (ll)n * (l)))]
+
+// Integral operands, key table and the symmetry check of the integrals (n^4
+// threads, once per call).
+__global__ void __launch_bounds__(256) k_sym_ops(const double *atwo, const double *f, int ncore, int n, SymScratch S,
+                                                 int M, int *flag) {
+    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+    const ll n2 = (ll)n * n, n4 = n2 * n2;
+    if (t >= n4) return;
+    const int l = (int)(t % n), k = (int)((t / n) % n), j = (int)((t / n2) % n), i = (int)(t / (n2 * n));
+    double scale = 0.0;
+    for (int q = 0; q < n; ++q) scale = fmax(scale, fabs(AT(q, q, q, q)));
+    const double v = AT(i, j, k, l), tol = kSymTol * scale;
+    if (!(fabs(v - AT(j, i, k, l)) <= tol) || !(fabs(v - AT(k, l, i, j)) <= tol))
+        for (int s = 0; s < M; ++s) flag[s] = 1;
+    const int np = n * (n + 1) / 2;
+    if (i >= j && j >= k && k >= l) {
+        const int key[4] = {i, j, k, l};
+        S.key[rank4(key)] = i | j << 4 | k << 8 | l << 12;
+    }
+    if (i >= j) S.Bf[((ll)k * np + pidx(i, j)) * n + l] = v;  // [(e, df), a] = (df|ea)
+    S.I4[((ll)j * n + l) * n2 + (ll)i * n + k] = v;           // [(f, e), (x, y)] = (xf|ye)
+    if (k >= l) S.IJ[((ll)j * n + i) * np + pidx(k, l)] = v;  // [(f, d), (x y)] = (df|xy)
+    if (t < n2) {                                             // (x, y) = (k, l)
+        double kk = 0.0;
+        for (int z = 0; z < n; ++z) kk += AT(k, z, z, l);
+        const double fkl = f[tri_index(k + 1 + ncore, l + 1 + ncore) - 1];
+        S.fm[t] = fkl;
+        S.K[t] = kk;
+        S.g[t] = fkl + 0.5 * kk;
+    }
+}
+
+// Largest |Gamma1| of the state: the scale of its symmetry checks.
+__device__ double rdm_scale(const Rdm &r, int s) {
+    __shared__ double red[8];
+    double m = 0.0;
+    for (int i = threadIdx.x; i < r.n * r.n; i += blockDim.x) m = fmax(m, fabs(r.d1[s + (ll)r.M * i]));
+    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
+    return m;
+}
+
+// H[K][l1 + n l2 + n^2 l3 + n^3 l4] = Gamma4 with creators the key K and any
+// annihilators: the transpose of the packed 4-RDM, completed over the
+// annihilators of higher rank than K (where the packed form keeps the
+// exchanged element).  Reads are coalesced along K, writes along l1.  The
+// blocks from nub on check Gamma1..3.  Bound by HBM: 16 W n^4 bytes.
+__global__ void __launch_bounds__(256) k_sym_unpack(Rdm r, int s, const int *key, unsigned nub, double *H, int *flag) {
+    const int n = r.n, M = r.M;
+    const ll n2 = (ll)n * n, n3 = n2 * n, n4 = n2 * n2, W = r.W;
+    const double tol = kSymTol * rdm_scale(r, s);
+    auto differ = [tol](double x, double y) { return !(fabs(x - y) <= tol); };
+    bool bad = false;
+    if (blockIdx.x >= nub) {
+        const ll t = (ll)(blockIdx.x - nub) * blockDim.x + threadIdx.x;
+        if (t < n3 * n3) {
+            ll x = t;
+            int q[6];
+            for (int i = 0; i < 6; ++i) { q[i] = (int)(x % n); x /= n; }
+            auto d3 = [&](int a, int b, int c, int d, int e, int f) {
+                return r.d3[s + (ll)M * (a + n * (b + n * (c + (ll)n * (d + n * (e + (ll)n * f)))))];
+            };
+            const double v = r.d3[s + (ll)M * t];
+            bad = differ(v, d3(q[1], q[0], q[2], q[4], q[3], q[5])) || differ(v, d3(q[0], q[2], q[1], q[3], q[5], q[4])) ||
+                  differ(v, d3(q[3], q[4], q[5], q[0], q[1], q[2]));
+            if (t < n4) {
+                auto d2 = [&](int a, int b, int c, int d) { return r.d2[s + (ll)M * (a + n * (b + n * (c + (ll)n * d)))]; };
+                const double w = r.d2[s + (ll)M * t];
+                bad = bad || differ(w, d2(q[1], q[0], q[3], q[2])) || differ(w, d2(q[2], q[3], q[0], q[1]));
+            }
+            if (t < n2) bad = bad || differ(r.d1[s + (ll)M * t], r.d1[s + (ll)M * (q[1] + n * q[0])]);
+        }
+        if (bad) flag[s] = 1;
+        return;
+    }
+    __shared__ double tile[32][33];
+    const double *ro4 = r.ro4 + W * n4 * s;
+    const unsigned kb = (unsigned)((W + 31) / 32);
+    const ll K0 = (ll)(blockIdx.x % kb) * 32, L0 = (ll)(blockIdx.x / kb) * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const ll K = K0 + tx;
+    const int pk = K < W ? key[K] : 0;
+    const int k[4] = {pk & 15, pk >> 4 & 15, pk >> 8 & 15, pk >> 12 & 15};
+    const ll pw[4] = {1, n, n2, n3};
+    for (int y = ty; y < 32; y += 8) {
+        const ll L = L0 + y;
+        double v = 0.0;
+        if (L < n4 && K < W) {
+            const int l[4] = {(int)(L % n), (int)((L / n) % n), (int)((L / n2) % n), (int)(L / n3)};
+            int q[4] = {l[0], l[1], l[2], l[3]}, o[4];
+            sort4(q, o);
+            const int rl = rank4(q);
+            ll mate = 0;  // the annihilators of the exchanged element
+#pragma unroll
+            for (int j = 0; j < 4; ++j) mate += pw[j] * (o[j] == 0 ? k[0] : o[j] == 1 ? k[1] : o[j] == 2 ? k[2] : k[3]);
+            if (rl > K) {
+                v = ro4[rl + W * mate];
+            } else {
+                v = ro4[K + W * L];
+                if (rl == K) bad = bad || differ(v, ro4[K + W * mate]);
+#pragma unroll
+                for (int j = 0; j < 3; ++j)  // equal creators: their annihilators may be exchanged
+                    if (k[j] == k[j + 1] && l[j] < l[j + 1])
+                        bad = bad || differ(v, ro4[K + W * (L + (l[j + 1] - l[j]) * (pw[j] - pw[j + 1]))]);
+            }
+        }
+        tile[tx][y] = v;
+    }
+    if (bad) flag[s] = 1;
+    __syncthreads();
+    for (int y = ty; y < 32; y += 8)
+        if (K0 + y < W && L0 + tx < n4) H[(K0 + y) * n4 + L0 + tx] = tile[y][tx];
+}
+
+// F for the creators (cp >= bp): rows ((cp,bp), ap, b, c), columns a,
+//   F = sum_e sum_{d >= f} X_e[(b,c), df] (df|ea),
+//   X_e[(b,c), df] = Gamma4[cp,bp,d,e; ap,b,f,c] + (d > f) Gamma4[cp,bp,f,e; ap,b,d,c].
+// One CTA owns (cp,bp), ap and bc values of b.  For each e it gathers X_e from
+// H into shared memory -- the sort of the four creators is done once per d and
+// turns the annihilators' offsets into four strides -- and multiplies: threads
+// are (row group, column), RPT rows each.  Bound by the FP64 pipe (2 FMA per
+// clock and SM): the gathers (two loads per n FMAs) run under the products of
+// the SM's other CTA.
+template <int RPT>
+__global__ void __launch_bounds__(256) k_sym_f(int n, int bc, const double *__restrict__ H,
+                                               const double *__restrict__ Bf, double *__restrict__ F,
+                                               const int *flag) {
+    if (*flag) return;
+    extern __shared__ double sm[];
+    __shared__ ll s_base[16];
+    __shared__ int s_w[16][3];
+    const int np = n * (n + 1) / 2, tid = threadIdx.x;
+    const int n2 = n * n, n4 = n2 * n2;
+    const int nchunk = (n + bc - 1) / bc;
+    int blk = blockIdx.x;
+    const int b0 = (blk % nchunk) * bc; blk /= nchunk;
+    const int ap = blk % n, pr = blk / n;
+    int cp = (int)((sqrtf(8.0f * pr + 1.0f) - 1.0f) * 0.5f);
+    while (pidx(cp + 1, 0) <= pr) ++cp;
+    while (pidx(cp, 0) > pr) --cp;
+    const int bp = pr - pidx(cp, 0);
+    const int nb = min(bc, n - b0), R = nb * n, ldx = np | 1;  // odd: no bank conflicts down a column
+    double *X = sm, *B = sm + bc * n * ldx;                    // [row][df], [df][a]
+    const int groups = 256 / n, col = tid % n, grp = tid / n;
+    const bool live = grp < groups;
+    double acc[RPT];
+    int ro[RPT];
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        acc[i] = 0.0;
+        ro[i] = min(grp + i * groups, R - 1) * ldx;
+    }
+    for (int e = 0; e < n; ++e) {
+        if (tid < n) {
+            int v[4] = {cp, bp, tid, e}, o[4];
+            sort4(v, o);
+            int w[4], p = 1;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (o[j] == i) w[i] = p;
+                p *= n;
+            }
+            s_base[tid] = (ll)rank4(v) * n4 + ap * w[0] + b0 * w[1];
+            s_w[tid][0] = w[1];
+            s_w[tid][1] = w[2];
+            s_w[tid][2] = w[3];
+        }
+        for (int i = tid; i < np * n; i += 256) B[i] = Bf[(ll)e * np * n + i];
+        __syncthreads();
+        for (int i = tid; i < R * np; i += 256) {
+            const int row = i % R, df = i / R;
+            const int c = row % n, b = row / n;
+            int d = (int)((sqrtf(8.0f * df + 1.0f) - 1.0f) * 0.5f);
+            if (pidx(d + 1, 0) <= df) ++d;
+            if (pidx(d, 0) > df) --d;
+            const int f = df - pidx(d, 0);
+            double x = H[s_base[d] + b * s_w[d][0] + f * s_w[d][1] + c * s_w[d][2]];
+            if (d != f) x += H[s_base[f] + b * s_w[f][0] + d * s_w[f][1] + c * s_w[f][2]];
+            X[row * ldx + df] = x;
+        }
+        __syncthreads();
+        if (live) {
+#pragma unroll 4
+            for (int k = 0; k < np; ++k) {
+                const double y = B[k * n + col];
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) acc[i] = fma(X[ro[i] + k], y, acc[i]);
+            }
+        }
+        __syncthreads();
+    }
+    if (!live) return;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        const int row = grp + i * groups;
+        if (row < R) F[(((ll)pr * n + ap) * n2 + b0 * n + row) * n + col] = acc[i];
+    }
+}
+
+// The n^8 contractions, blockIdx.z: 0 Wca, 1 Waa, 2 Kx, 3 J.  Rows ((p >= p'),
+// q, r): Wca and Waa have p' their second creator (s or t) and (q,r) the free
+// pair, Kx and J the pairs (p,q), (p',r).  The rows of Gamma3 are affine in the
+// two summed indices, lo the one with stride M, so the tile loads need no
+// intermediate matrix.  64 x 64 tiles, 4 x 4 per thread; bound by the FP64 pipe.
+constexpr int kN8 = 64, kN8K = 16;
+__global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__restrict__ I4,
+                                                const double *__restrict__ IJ, double *out, const int *flag) {
+    if (*flag) return;
+    __shared__ double As[kN8K][kN8 + 1], Bs[kN8K][kN8];
+    const int n = r.n, np = n * (n + 1) / 2, kind = blockIdx.z;
+    const ll M = r.M, n1 = n, n2 = n1 * n, n3 = n2 * n, n4 = n2 * n2, n5 = n4 * n;
+    const ll rows = np * n2;
+    const int N = kind == 3 ? np : (int)n2;
+    const int c0 = blockIdx.y * kN8;
+    if (c0 >= N) return;
+    const ll r0 = (ll)blockIdx.x * kN8;
+    const double *Bm = kind == 3 ? IJ : I4;
+    double *C = out + kind * rows * n2;
+    const ll hi = M * (kind == 0 ? n4 : kind == 1 ? n1 : n3);
+    const int tid = threadIdx.x, lk = tid & 15, lr = tid >> 4;
+    const double *base[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const ll row = min(r0 + lr + 16 * i, rows - 1);
+        const int q2 = (int)(row % n), q1 = (int)((row / n) % n), pr = (int)(row / n2);
+        int p = (int)((sqrtf(8.0f * pr + 1.0f) - 1.0f) * 0.5f);
+        if (pidx(p + 1, 0) <= pr) ++p;
+        if (pidx(p, 0) > pr) --p;
+        const int p2 = pr - pidx(p, 0);
+        ll o;
+        if (kind == 0) o = n1 * p + n2 * q1 + n3 * p2 + n5 * q2;        // (e,s), (p,f), (q,r)
+        else if (kind == 1) o = n2 * q2 + n3 * p2 + n4 * p + n5 * q1;   // (e,t), (f,p), (r,q): exchanged
+        else if (kind == 2) o = n1 * q1 + n2 * q2 + n4 * p + n5 * p2;   // (e,d), (q,p), (r,p'): exchanged
+        else o = n1 * p + n2 * p2 + n4 * q1 + n5 * q2;                  // (d,f), (p,q), (p',r)
+        base[i] = r.d3 + s + M * o;
+    }
+    double acc[4][4] = {};
+    const int tc = (tid & 15) * 4, tr = (tid >> 4) * 4;
+    const int K = (int)n2;
+    for (int k0 = 0; k0 < K; k0 += kN8K) {
+        const int k = k0 + lk;
+        const ll ko = (k / n) * hi + (k % n) * M;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) As[lk][lr + 16 * i] = k < K ? base[i][ko] : 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int kk = (tid >> 6) + 4 * i, c = tid & 63;
+            Bs[kk][c] = (k0 + kk < K && c0 + c < N) ? Bm[(ll)(k0 + kk) * N + c0 + c] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < kN8K; ++kk) {
+            double a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                a[i] = As[kk][tr + i];
+                b[i] = Bs[kk][tc + i];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (r0 + tr + i < rows && c0 + tc + j < N) C[(r0 + tr + i) * N + c0 + tc + j] = acc[i][j];
+}
+
+// Accessors of the intermediates (0-based labels).
+struct SymView {
+    Rdm r;
+    int s, n;
+    ll n2, rows;  // rows of one n^8 block
+    const double *F, *N8, *G1, *G3, *Q1, *W2, *J2, *Y2, *atwo, *fm, *K, *g;
+
+    __device__ __forceinline__ double d1(int a, int b) const { return r.d1[s + (ll)r.M * (a + n * b)]; }
+    __device__ __forceinline__ double d2(int a, int b, int c, int d) const {
+        return r.d2[s + (ll)r.M * (a + n * (b + n * (c + n * d)))];
+    }
+    // Gamma3 with the annihilators fastest (the exchanged element)
+    __device__ __forceinline__ double d3(int a, int b, int c, int d, int e, int f) const {
+        return r.d3[s + (ll)r.M * (d + n * (e + n * (f + n * (a + (ll)n * (b + n * c)))))];
+    }
+    __device__ __forceinline__ double e2(int a, int b, int c, int d) const {  // <E_ab E_cd>
+        double v = d2(a, c, b, d);
+        if (b == c) v += d1(a, d);
+        return v;
+    }
+    __device__ __forceinline__ double e3(int a, int b, int c, int d, int e, int f) const {  // <E_ab E_cd E_ef>
+        double v = d3(a, c, e, b, d, f);
+        if (e == d) v += d2(a, c, b, f);
+        if (e == b) v += d2(a, c, f, d);
+        if (b == c) {
+            v += d2(a, e, d, f);
+            if (e == d) v += d1(a, f);
+        }
+        return v;
+    }
+    __device__ __forceinline__ double ai(int i, int j, int k, int l) const {
+        return atwo[i + n * (j + n * (k + n * l))];
+    }
+    // F[(p,q), (p2,q2); c, a]
+    __device__ __forceinline__ double f4(int p, int q, int p2, int q2, int c, int a) const {
+        const ll row = p >= p2 ? (ll)(pidx(p, p2) * n + q) * n + q2 : (ll)(pidx(p2, p) * n + q2) * n + q;
+        return F[(row * n + c) * n + a];
+    }
+    __device__ __forceinline__ ll row3(int p, int p2, int q, int q2) const {
+        return (ll)(pidx(p, p2) * n + q) * n + q2;
+    }
+    __device__ __forceinline__ double wca(int p, int q, int q2, int t, int x, int y) const {
+        return p >= t ? N8[row3(p, t, q, q2) * n2 + x * n + y] : N8[row3(t, p, q2, q) * n2 + y * n + x];
+    }
+    __device__ __forceinline__ double waa(int p, int q, int q2, int t, int x, int y) const {
+        const double *A = N8 + rows * n2;
+        return p >= t ? A[row3(p, t, q, q2) * n2 + x * n + y] : A[row3(t, p, q, q2) * n2 + y * n + x];
+    }
+    __device__ __forceinline__ double kx(int p, int q, int p2, int q2, int x, int y) const {
+        const double *A = N8 + 2 * rows * n2;
+        return p >= p2 ? A[row3(p, p2, q, q2) * n2 + x * n + y] : A[row3(p2, p, q2, q) * n2 + x * n + y];
+    }
+    __device__ __forceinline__ double jj(int p, int q, int p2, int q2, int x, int y) const {
+        const double *A = N8 + 3 * rows * n2;
+        const int np = n * (n + 1) / 2;
+        return p >= p2 ? A[row3(p, p2, q, q2) * np + pmx(x, y)] : A[row3(p2, p, q2, q) * np + pmx(x, y)];
+    }
+    __device__ __forceinline__ ll i4(int a, int b, int c, int d) const { return ((ll)(a * n + b) * n + c) * n + d; }
+};
+
+// n^6 sums over two indices, one thread per n^4 element:
+//   G1[p,q,c,a] = sum_e J[(p,q),(e,c);e,a]        G3[p,q,r,x] = sum_e J[(p,e),(q,r);x,e]
+//   Q1[p,t;x,y] = sum Gamma2[(p,f),(t,e)] (xf|ye)  W2[p,s;x,y] = sum Gamma2[(p,f),(e,s)] (xf|ye)
+//   J2[p,q;x,y] = sum Gamma2[(p,q),(d,f)] (df|xy)  Y2[p,c;q,b] = sum Gamma2[(p,c),(e,f)] (qf|be)
+__global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double *G3, double *Q1, double *W2,
+                                                  double *J2, double *Y2, const int *flag) {
+    if (*flag) return;
+    const int n = v.n;
+    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= v.n2 * v.n2) return;
+    const int d = (int)(t % n), c = (int)((t / n) % n), b = (int)((t / v.n2) % n), a = (int)(t / (v.n2 * n));
+    double g1 = 0.0, g3 = 0.0, q1 = 0.0, w2 = 0.0, j2 = 0.0, y2 = 0.0;
+    for (int e = 0; e < n; ++e) {
+        g1 += v.jj(a, b, e, c, e, d);
+        g3 += v.jj(a, e, b, c, d, e);
+        for (int f = 0; f < n; ++f) {
+            const double x = v.ai(c, f, d, e);
+            q1 = fma(v.d2(a, b, f, e), x, q1);
+            w2 = fma(v.d2(a, e, f, b), x, w2);
+            y2 = fma(v.d2(a, e, b, f), x, y2);
+            j2 = fma(v.d2(a, e, b, f), v.ai(e, f, c, d), j2);
+        }
+    }
+    G1[t] = g1; G3[t] = g3; Q1[t] = q1; W2[t] = w2; J2[t] = j2; Y2[t] = y2;
+}
+
+// amat/atmat(s, ap,bp,cp,a,b,c), one thread per element, ap fastest.
+__global__ void __launch_bounds__(256) k_sym_out(SymView v, double *amat, double *atmat, const int *flag) {
+    if (*flag) return;
+    const int n = v.n;
+    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= v.n2 * v.n2 * v.n2) return;
+    ll x = t;
+    const int ap = (int)(x % n); x /= n;
+    const int bp = (int)(x % n); x /= n;
+    const int cp = (int)(x % n); x /= n;
+    const int a = (int)(x % n); x /= n;
+    const int b = (int)(x % n); x /= n;
+    const int c = (int)x;
+    double A = v.f4(cp, ap, bp, b, c, a) - v.f4(ap, cp, b, bp, a, c) - v.f4(ap, cp, c, a, bp, b);
+    double T = v.f4(ap, cp, bp, b, a, c) - v.f4(cp, ap, b, bp, c, a) - v.f4(cp, ap, a, c, bp, b);
+    A += v.wca(cp, bp, b, c, ap, a) + v.jj(cp, c, bp, b, ap, a) - v.waa(cp, bp, b, a, ap, c) -
+         v.waa(bp, cp, ap, a, b, c) - v.waa(cp, a, c, bp, ap, b);
+    T += v.waa(cp, b, bp, a, ap, c) + v.waa(b, cp, ap, a, bp, c) - v.waa(c, ap, cp, bp, a, b) -
+         v.wca(cp, b, bp, c, ap, a) - v.wca(b, cp, ap, c, bp, a) - v.wca(cp, a, c, bp, ap, b);
+    T += 2.0 * v.jj(cp, ap, a, c, b, bp) - v.jj(cp, c, b, bp, ap, a) - v.jj(cp, ap, b, c, bp, a) -
+         v.jj(cp, bp, a, c, ap, b) - v.kx(cp, ap, a, c, b, bp);
+    double s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    for (int d = 0; d < n; ++d) {
+        const double gda = v.g[d * n + a], gcd = v.g[c * n + d], gbd = v.g[b * n + d];
+        s1 += v.e3(cp, ap, bp, b, d, c) * gda - v.e3(cp, ap, bp, b, a, d) * gcd - v.e3(cp, ap, bp, d, a, c) * gbd;
+        s2 += v.e3(cp, ap, b, bp, a, d) * gcd - v.e3(cp, ap, b, bp, d, c) * gda - v.e3(cp, ap, d, bp, a, c) * gbd;
+        // two-operator sums of atmat
+        s3 += 2.0 * (v.d2(cp, d, ap, c) * v.ai(d, a, b, bp) + v.d2(cp, a, d, c) * v.ai(ap, d, b, bp));
+        s3 -= v.d2(cp, b, d, c) * v.ai(ap, d, bp, a) + v.d2(cp, b, c, d) * v.ai(bp, d, ap, a);
+        s3 -= v.d2(cp, a, d, c) * v.ai(bp, d, b, ap) + v.d2(cp, d, bp, c) * v.ai(d, a, b, ap);
+        s3 -= v.d2(cp, d, c, bp) * v.ai(ap, a, b, d) + v.d2(cp, d, ap, c) * v.ai(bp, a, b, d);
+    }
+    A += s1;
+    T += s2 + s3 + 2.0 * v.e2(cp, ap, a, c) * v.g[b * n + bp];
+    T += v.d1(cp, c) * (2.0 * v.ai(ap, a, b, bp) - v.ai(bp, a, b, ap));
+    // Kronecker deltas
+    auto q2 = [&](int p, int y) {  // sum Gamma2[(p,e),(d,f)] (df|ye)
+        double q = 0.0;
+        for (int e = 0; e < n; ++e) q += v.J2[v.i4(p, e, y, e)];
+        return q;
+    };
+    if (ap == bp) {
+        A += v.G1[v.i4(cp, b, c, a)] - v.G1[v.i4(b, cp, a, c)] - v.G3[v.i4(cp, a, c, b)] - v.Q1[v.i4(cp, a, b, c)];
+        if (a == b) A -= q2(cp, c);
+    }
+    if (ap == a) A -= v.G3[v.i4(cp, bp, b, c)] + v.G3[v.i4(bp, cp, c, b)] + v.Q1[v.i4(bp, cp, b, c)];
+    if (a == b) A -= v.G3[v.i4(bp, cp, ap, c)] + v.Q1[v.i4(cp, bp, ap, c)];
+    if (ap == b) {
+        T += v.G1[v.i4(bp, cp, a, c)] - v.G1[v.i4(cp, bp, c, a)] - v.W2[v.i4(cp, c, bp, a)] -
+             v.J2[v.i4(cp, c, bp, a)] + v.Q1[v.i4(cp, a, bp, c)];
+        if (bp == a) T += q2(cp, c);
+    }
+    if (ap == a)
+        T += v.G3[v.i4(cp, b, bp, c)] + v.Q1[v.i4(b, cp, bp, c)] - v.G1[v.i4(cp, c, bp, b)] -
+             v.Y2[v.i4(cp, c, bp, b)] + 2.0 * v.J2[v.i4(cp, c, b, bp)];
+    if (bp == a)
+        T += v.G3[v.i4(b, cp, ap, c)] + v.Q1[v.i4(cp, b, ap, c)] - v.G1[v.i4(cp, ap, c, b)] -
+             v.J2[v.i4(cp, c, b, ap)] - v.W2[v.i4(cp, c, ap, b)];
+    if (b == bp) {
+        double D = 2.0 * (v.G1[v.i4(cp, ap, c, a)] + v.J2[v.i4(cp, c, ap, a)] + v.W2[v.i4(cp, c, ap, a)] -
+                          v.G3[v.i4(a, cp, ap, c)] - v.Q1[v.i4(cp, a, ap, c)]) +
+                   v.d1(cp, c) * v.K[ap * n + a];
+        for (int d = 0; d < n; ++d)
+            D += v.d2(cp, d, ap, c) * v.K[d * n + a] - v.d2(cp, a, ap, d) * v.K[c * n + d] +
+                 2.0 * (v.e2(cp, ap, d, c) * v.fm[d * n + a] - v.e2(cp, ap, a, d) * v.fm[c * n + d]);
+        if (a == ap) {
+            D -= 2.0 * q2(cp, c);
+            for (int d = 0; d < n; ++d) D -= v.d1(cp, d) * v.K[c * n + d];
+        }
+        T += D;
+    }
+    const ll o = v.s + (ll)v.r.M * t;
+    amat[o] = A;
+    atmat[o] = T;
+}
+#undef AT
+
+// Values of b per CTA of k_sym_f and rows per thread: the split with the least
+// idle row slots whose tile leaves two CTAs per SM (at most 72 KB of X).
+struct FShape {
+    int bc = 1, rpt = 1;
+};
+FShape f_shape(int n) {
+    const int np = n * (n + 1) / 2, groups = 256 / n;
+    FShape best;
+    double eff = 0.0;
+    for (int bc = 1; bc <= n; ++bc) {
+        const int R = bc * n, rpt = (R + groups - 1) / groups;
+        if (rpt > kSymMaxRpt || (ll)R * (np | 1) * 8 > 72 * 1024) break;
+        const int chunks = (n + bc - 1) / bc;
+        const double e = (double)(n * n) / ((double)chunks * rpt * groups);
+        if (e > eff * 1.02) {
+            eff = e;
+            best.bc = bc;
+            best.rpt = rpt;
+        }
+    }
+    return best;
+}
+
+using FKernel = void (*)(int, int, const double *, const double *, double *, const int *);
+FKernel f_kernel(int rpt) {
+    switch (rpt) {
+        case 1: return k_sym_f<1>;
+        case 2: return k_sym_f<2>;
+        case 3: return k_sym_f<3>;
+        case 4: return k_sym_f<4>;
+        case 5: return k_sym_f<5>;
+        default: return k_sym_f<6>;
+    }
+}
+
+}  // namespace
+
+ll SymScratch::doubles(int n) {
+    const ll n2 = (ll)n * n, n4 = n2 * n2, np = n * (n + 1) / 2;
+    const ll W = (ll)n * (n + 1) * (n + 2) * (n + 3) / 24;
+    return W * n4 + 4 * np * n4 + np * np * n2 + 7 * n4 + 2 * np * n2 + 3 * n2 + W / 2 + 1;
+}
+
+SymScratch::SymScratch(int n, double *w) {
+    const ll n2 = (ll)n * n, n4 = n2 * n2, np = n * (n + 1) / 2;
+    const ll W = (ll)n * (n + 1) * (n + 2) * (n + 3) / 24;
+    auto take = [&w](ll k) {
+        double *p = w;
+        w += k;
+        return p;
+    };
+    H = take(W * n4);
+    F = take(np * n4);
+    N8 = take(3 * np * n4 + np * np * n2);
+    for (double **p : {&G1, &G3, &Q1, &W2, &J2, &Y2}) *p = take(n4);
+    Bf = take(np * n2);
+    I4 = take(n4);
+    IJ = take(n2 * np);
+    fm = take(n2);
+    K = take(n2);
+    g = take(n2);
+    key = (int *)take(W / 2 + 1);
+}
+
+void launch_sym_ops(const double *atwo, const double *f, int ncore, int n, const SymScratch &S, int M, int *flag,
+                    cudaStream_t st) {
+    const ll n4 = (ll)n * n * n * n;
+    k_sym_ops<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(atwo, f, ncore, n, S, M, flag);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+}
+
+int launch_sym_state(const Rdm &r, int s, const double *atwo, const SymScratch &S, double *amat, double *atmat,
+                     int *flag, cudaStream_t st) {
+    const int n = r.n, np = n * (n + 1) / 2;
+    const ll n2 = (ll)n * n, n4 = n2 * n2, n6 = n4 * n2, rows = np * n2;
+    const ll ub = ((r.W + 31) / 32) * ((n4 + 31) / 32), cb = (n6 + 255) / 256;
+    k_sym_unpack<<<(unsigned)(ub + cb), 256, 0, st>>>(r, s, S.key, (unsigned)ub, S.H, flag);
+    const int *fl = flag + s;
+    const dim3 g8((unsigned)((rows + kN8 - 1) / kN8), (unsigned)((n2 + kN8 - 1) / kN8), 4);
+    k_sym_n8<<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
+    const FShape fs = f_shape(n);
+    const FKernel fk = f_kernel(fs.rpt);
+    const int smem = (fs.bc * n * (np | 1) + np * n) * (int)sizeof(double);
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute((const void *)fk, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
+        return 1;
+    fk<<<(unsigned)(np * n * ((n + fs.bc - 1) / fs.bc)), 256, smem, st>>>(n, fs.bc, S.H, S.Bf, S.F, fl);
+    SymView v{r, s, n, n2, rows, S.F, S.N8, S.G1, S.G3, S.Q1, S.W2, S.J2, S.Y2, atwo, S.fm, S.K, S.g};
+    k_sym_small<<<(unsigned)((n4 + 63) / 64), 64, 0, st>>>(v, S.G1, S.G3, S.Q1, S.W2, S.J2, S.Y2, fl);
+    k_sym_out<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(v, amat, atmat, fl);
+    g_launches.fetch_add(5, std::memory_order_relaxed);
+    return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
+}
+
+}  // namespace nvpt

@@ -1,0 +1,29 @@
+// The A-matrices from one n^9 contraction (bamat_sym.cu): scratch layout and
+// launchers.
+#pragma once
+#include "nvpt2_internal.h"
+
+namespace nvpt {
+
+constexpr int kSymMaxRpt = 6;  // rows per thread of the n^9 product
+
+// Views into one scratch block of doubles(n) doubles, reused for every state.
+struct SymScratch {
+    double *H, *F, *N8;                       // unpacked 4-RDM [W][n^4]; F; the four n^8 tensors
+    double *G1, *G3, *Q1, *W2, *J2, *Y2;      // n^4 sums
+    double *Bf, *I4, *IJ, *fm, *K, *g;        // integral operands, f, K and f + K/2
+    int *key;                                 // packed key quadruples [W]
+    SymScratch(int n, double *w);
+    static ll doubles(int n);
+};
+
+// Integral operands and the check of the integrals' symmetry: sets flag[0..M)
+// (zeroed by the caller) where it fails.
+void launch_sym_ops(const double *atwo, const double *f, int ncore, int n, const SymScratch &S, int M, int *flag,
+                    cudaStream_t st);
+// One state: the check of its RDMs (flag[s]) and, unless flagged, its
+// A-matrices.  0, or 1 on a launch failure.
+int launch_sym_state(const Rdm &r, int s, const double *atwo, const SymScratch &S, double *amat, double *atmat,
+                     int *flag, cudaStream_t st);
+
+}  // namespace nvpt

@@ -608,19 +608,11 @@ int nvpt_bamat_d(nvpt_context *ctx, double *amat, double *atmat, const double *a
     cudaStream_t st = pick(ctx, stream);
     Rdm r = make_rdm(nact, metat, dal, taa, daaa, ro4);
     launch_build_f(f, aj, atwo, (int)nact, (int)ncore, 1, st);
-    // Tiny active spaces: one thread per element evaluates the reference's
-    // loop directly.  Otherwise the n^9 part runs as dense GEMMs over
-    // materialised four-operator slabs (bamat_gemm.cu).  With symmetry the
-    // dense contractions are the same (the integrals the reference's branch
-    // skips vanish by symmetry) and its output screen follows.
-    if (nact <= 5) {
-        launch_bamat_direct(r, atwo, f, (int)ncore, amat, atmat, st);
-        if (irr) launch_sym_screen(amat, atmat, (int)metat, (int)nact, 6, irr, st);
-        return after_launch(ctx, "bamat");
-    }
+    // With symmetry the dense contractions are the same (the integrals the
+    // reference's branch skips vanish by symmetry) and its output screen
+    // follows.
     const bool split = ctx->precision == NVPT_PRECISION_SPLIT;
-    const int slabs = 16;
-    int rc = launch_bamat_gemm(r, atwo, f, (int)ncore, amat, atmat, st, slabs, split);
+    int rc = launch_bamat(r, atwo, f, (int)ncore, amat, atmat, st, split);
     if (rc == 2) return fail(ctx, NVPT_ENOMEM, "bamat: device allocation failed");
     if (rc == 5) return fail(ctx, NVPT_ETIMEDOUT, "bamat: a split-precision product timed out waiting on its pipeline");
     if (rc) return fail(ctx, NVPT_ECUDA, split ? "bamat: split-precision product failed" : "bamat: GEMM failed");

@@ -31,14 +31,15 @@ void launch_bcmat(const Rdm &r, const double *atwo, const double *f, int ncore, 
                   cudaStream_t st);
 void launch_bdmat(const Rdm &r, const double *atwo, const double *f, const double *aj, int ncore, double *d,
                   double *dt, cudaStream_t st);
+// One thread per element (bamat.cu); with flag, only the states s with flag[s] set.
 void launch_bamat_direct(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
-                         cudaStream_t st);
-// Dense-contraction A-matrix builder (bamat_gemm.cu); 0 on success, 2 on a
-// failed allocation, 5 if a split-precision product timed out, else a
-// cuBLAS / launch failure.  split: the n^9 slab products run as Ozaki digit
-// products on the tensor cores (ozaki.cu) instead of FP64 DGEMMs.
-int launch_bamat_gemm(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
-                      cudaStream_t st, int slabs_per_batch, bool split = false);
+                         cudaStream_t st, const int *flag);
+// A-matrix builder (bamat_gemm.cu, bamat_sym.cu); 0 on success, 2 on a
+// failed allocation, 5 if a split-precision product timed out, else a launch
+// failure.  split: the n^9 slab products run as Ozaki digit products on the
+// tensor cores (ozaki.cu) instead of FP64.
+int launch_bamat(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
+                 cudaStream_t st, bool split = false);
 // No-allocation A-matrix builder (bamat_gemm.cu): scratch in a static device
 // array sized for kBamatStaticNactMax active orbitals; 0 on success, 1 if
 // nact exceeds the limit.

@@ -14,11 +14,14 @@
 //   Kx[P1,P2;x,y]    = sum_{d,e} Gamma3[P1, P2, (d,e)] (xd|ye)
 //   Wca[p,(q,r),s;x,y] = sum_{f,e} Gamma3[(p,f), (q,r), (e,s)] (xf|ye)
 //   Waa[p,(q,r),t;x,y] = sum_{f,e} Gamma3[(p,f), (q,r), (t,e)] (xf|ye)
-// each with a two-fold symmetry in its row labels, and n^7 and below.  With
-// A = (cp,ap), B = (bp,b), B' = (b,bp), P^T = (annihilator, creator), E3, E2
-// the three- and two-operator products, g = f + K/2, K(x,y) = sum_z (xz|zy):
-//   amat  = sum_d [E3[A,B,(d,c)] g(d,a) - E3[A,B,(a,d)] g(c,d) - E3[A,(bp,d),(a,c)] g(b,d)]
-//         + F[A,B;c,a] - F[A^T,B^T;a,c] - F[A^T,(c,a);bp,b]
+// each with a two-fold symmetry in its row labels, and n^7 and below.  The
+// one-electron operator g = f + K/2, K(x,y) = sum_z (xz|zy), goes into F, J and
+// the two-operator J2 as
+//   F += sum_d Gamma3[A, B, (d,c)] g(d,a),  J += Gamma2[P1, P2] g(x,y),
+//   J2[p,q;x,y] = sum_{d,f} Gamma2[(p,q), (d,f)] (df|xy) + Gamma1[p,q] g(x,y)
+// and appears nowhere else.  With A = (cp,ap), B = (bp,b), B' = (b,bp),
+// P^T = (annihilator, creator):
+//   amat  = F[A,B;c,a] - F[A^T,B^T;a,c] - F[A^T,(c,a);bp,b]
 //         + Wca[cp,B,c;ap,a] + J[(cp,c),B;ap,a] - Waa[cp,B,a;ap,c] - Waa[bp,A,a;b,c]
 //         - Waa[cp,(a,c),bp;ap,b] + Kronecker-delta terms (k_sym_out)
 // and likewise atmat.  tests/test_bamat_sym.py evaluates these sums in numpy
@@ -81,13 +84,11 @@ __global__ void __launch_bounds__(256) k_sym_ops(const double *atwo, const doubl
     if (i >= j) S.Bf[((ll)k * np + pidx(i, j)) * n + l] = v;  // [(e, df), a] = (df|ea)
     S.I4[((ll)j * n + l) * n2 + (ll)i * n + k] = v;           // [(f, e), (x, y)] = (xf|ye)
     if (k >= l) S.IJ[((ll)j * n + i) * np + pidx(k, l)] = v;  // [(f, d), (x y)] = (df|xy)
+    S.Lb[t] = 2.0 * AT(l, k, j, i) - AT(i, k, j, l);          // [i][j][k][l] = 2 (lk|ji) - (ik|jl)
     if (t < n2) {                                             // (x, y) = (k, l)
         double kk = 0.0;
         for (int z = 0; z < n; ++z) kk += AT(k, z, z, l);
-        const double fkl = f[tri_index(k + 1 + ncore, l + 1 + ncore) - 1];
-        S.fm[t] = fkl;
-        S.K[t] = kk;
-        S.g[t] = fkl + 0.5 * kk;
+        S.g[t] = f[tri_index(k + 1 + ncore, l + 1 + ncore) - 1] + 0.5 * kk;
     }
 }
 
@@ -177,7 +178,8 @@ __global__ void __launch_bounds__(256) k_sym_unpack(Rdm r, int s, const int *key
 
 // F for the creators (cp >= bp): rows ((cp,bp), ap, b, c), columns a,
 //   F = sum_e sum_{d >= f} X_e[(b,c), df] (df|ea),
-//   X_e[(b,c), df] = Gamma4[cp,bp,d,e; ap,b,f,c] + (d > f) Gamma4[cp,bp,f,e; ap,b,d,c].
+//   X_e[(b,c), df] = Gamma4[cp,bp,d,e; ap,b,f,c] + (d > f) Gamma4[cp,bp,f,e; ap,b,d,c]
+// plus sum_d Gamma3[(cp,ap),(bp,b),(d,c)] g(d,a) as one more K chunk (e = n).
 // One CTA owns (cp,bp), ap and bc values of b.  For each e it gathers X_e from
 // H into shared memory -- the sort of the four creators is done once per d and
 // turns the annihilators' offsets into four strides -- and multiplies: threads
@@ -185,14 +187,14 @@ __global__ void __launch_bounds__(256) k_sym_unpack(Rdm r, int s, const int *key
 // clock and SM): the gathers (two loads per n FMAs) run under the products of
 // the SM's other CTA.
 template <int RPT>
-__global__ void __launch_bounds__(256) k_sym_f(int n, int bc, const double *__restrict__ H,
-                                               const double *__restrict__ Bf, double *__restrict__ F,
-                                               const int *flag) {
+__global__ void __launch_bounds__(256) k_sym_f(Rdm r, int s, int bc, const double *__restrict__ H,
+                                               const double *__restrict__ Bf, const double *__restrict__ g,
+                                               double *__restrict__ F, const int *flag) {
     if (*flag) return;
     extern __shared__ double sm[];
     __shared__ ll s_base[16];
     __shared__ int s_w[16][3];
-    const int np = n * (n + 1) / 2, tid = threadIdx.x;
+    const int n = r.n, np = n * (n + 1) / 2, tid = threadIdx.x;
     const int n2 = n * n, n4 = n2 * n2;
     const int nchunk = (n + bc - 1) / bc;
     int blk = blockIdx.x;
@@ -213,8 +215,9 @@ __global__ void __launch_bounds__(256) k_sym_f(int n, int bc, const double *__re
         acc[i] = 0.0;
         ro[i] = min(grp + i * groups, R - 1) * ldx;
     }
-    for (int e = 0; e < n; ++e) {
-        if (tid < n) {
+    for (int e = 0; e <= n; ++e) {
+        const int nk = e < n ? np : n;
+        if (e < n && tid < n) {
             int v[4] = {cp, bp, tid, e}, o[4];
             sort4(v, o);
             int w[4], p = 1;
@@ -230,11 +233,17 @@ __global__ void __launch_bounds__(256) k_sym_f(int n, int bc, const double *__re
             s_w[tid][1] = w[2];
             s_w[tid][2] = w[3];
         }
-        for (int i = tid; i < np * n; i += 256) B[i] = Bf[(ll)e * np * n + i];
+        const double *Be = e < n ? Bf + (ll)e * np * n : g;
+        for (int i = tid; i < nk * n; i += 256) B[i] = Be[i];
         __syncthreads();
-        for (int i = tid; i < R * np; i += 256) {
+        for (int i = tid; i < R * nk; i += 256) {
             const int row = i % R, df = i / R;
             const int c = row % n, b = row / n;
+            if (e == n) {  // Gamma3 with its annihilators as the first pair index: d = df
+                X[row * ldx + df] =
+                    r.d3[s + (ll)r.M * (df + n * cp + n2 * bp + (ll)(n2 * n) * c + (ll)n4 * ap + (ll)n4 * n * (b0 + b))];
+                continue;
+            }
             int d = (int)((sqrtf(8.0f * df + 1.0f) - 1.0f) * 0.5f);
             if (pidx(d + 1, 0) <= df) ++d;
             if (pidx(d, 0) > df) --d;
@@ -246,7 +255,7 @@ __global__ void __launch_bounds__(256) k_sym_f(int n, int bc, const double *__re
         __syncthreads();
         if (live) {
 #pragma unroll 4
-            for (int k = 0; k < np; ++k) {
+            for (int k = 0; k < nk; ++k) {
                 const double y = B[k * n + col];
 #pragma unroll
                 for (int i = 0; i < RPT; ++i) acc[i] = fma(X[ro[i] + k], y, acc[i]);
@@ -269,7 +278,8 @@ __global__ void __launch_bounds__(256) k_sym_f(int n, int bc, const double *__re
 // intermediate matrix.  64 x 64 tiles, 4 x 4 per thread; bound by the FP64 pipe.
 constexpr int kN8 = 64, kN8K = 16;
 __global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__restrict__ I4,
-                                                const double *__restrict__ IJ, double *out, const int *flag) {
+                                                const double *__restrict__ IJ, const double *g, double *out,
+                                                const int *flag) {
     if (*flag) return;
     __shared__ double As[kN8K][kN8 + 1], Bs[kN8K][kN8];
     const int n = r.n, np = n * (n + 1) / 2, kind = blockIdx.z;
@@ -329,10 +339,31 @@ __global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__re
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
+        const ll row = r0 + tr + i;
+        if (row >= rows) break;
+        double w = 0.0;  // J += Gamma2[(p,q), (p',r)] g(x,y)
+        if (kind == 3) {
+            const int pr = (int)(row / n2);
+            int p = (int)((sqrtf(8.0f * pr + 1.0f) - 1.0f) * 0.5f);
+            if (pidx(p + 1, 0) <= pr) ++p;
+            if (pidx(p, 0) > pr) --p;
+            w = r.d2[s + M * (p + n1 * (pr - pidx(p, 0)) + n2 * ((row / n) % n) + n3 * (row % n))];
+        }
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (r0 + tr + i < rows && c0 + tc + j < N) C[(r0 + tr + i) * N + c0 + tc + j] = acc[i][j];
+        for (int j = 0; j < 4; ++j) {
+            const int col = c0 + tc + j;
+            if (col >= N) break;
+            double v = acc[i][j];
+            if (kind == 3) {
+                int x = (int)((sqrtf(8.0f * col + 1.0f) - 1.0f) * 0.5f);
+                if (pidx(x + 1, 0) <= col) ++x;
+                if (pidx(x, 0) > col) --x;
+                v = fma(w, g[x * n + col - pidx(x, 0)], v);
+            }
+            C[row * N + col] = v;
+        }
+    }
 }
 
 // Accessors of the intermediates (0-based labels).
@@ -340,30 +371,11 @@ struct SymView {
     Rdm r;
     int s, n;
     ll n2, rows;  // rows of one n^8 block
-    const double *F, *N8, *G1, *G3, *Q1, *W2, *J2, *Y2, *atwo, *fm, *K, *g;
+    const double *F, *N8, *G1, *G3, *Q1, *JW, *J2, *Z, *atwo, *Lb, *g;
 
     __device__ __forceinline__ double d1(int a, int b) const { return r.d1[s + (ll)r.M * (a + n * b)]; }
     __device__ __forceinline__ double d2(int a, int b, int c, int d) const {
         return r.d2[s + (ll)r.M * (a + n * (b + n * (c + n * d)))];
-    }
-    // Gamma3 with the annihilators fastest (the exchanged element)
-    __device__ __forceinline__ double d3(int a, int b, int c, int d, int e, int f) const {
-        return r.d3[s + (ll)r.M * (d + n * (e + n * (f + n * (a + (ll)n * (b + n * c)))))];
-    }
-    __device__ __forceinline__ double e2(int a, int b, int c, int d) const {  // <E_ab E_cd>
-        double v = d2(a, c, b, d);
-        if (b == c) v += d1(a, d);
-        return v;
-    }
-    __device__ __forceinline__ double e3(int a, int b, int c, int d, int e, int f) const {  // <E_ab E_cd E_ef>
-        double v = d3(a, c, e, b, d, f);
-        if (e == d) v += d2(a, c, b, f);
-        if (e == b) v += d2(a, c, f, d);
-        if (b == c) {
-            v += d2(a, e, d, f);
-            if (e == d) v += d1(a, f);
-        }
-        return v;
     }
     __device__ __forceinline__ double ai(int i, int j, int k, int l) const {
         return atwo[i + n * (j + n * (k + n * l))];
@@ -396,17 +408,17 @@ struct SymView {
 };
 
 // n^6 sums over two indices, one thread per n^4 element:
-//   G1[p,q,c,a] = sum_e J[(p,q),(e,c);e,a]        G3[p,q,r,x] = sum_e J[(p,e),(q,r);x,e]
-//   Q1[p,t;x,y] = sum Gamma2[(p,f),(t,e)] (xf|ye)  W2[p,s;x,y] = sum Gamma2[(p,f),(e,s)] (xf|ye)
-//   J2[p,q;x,y] = sum Gamma2[(p,q),(d,f)] (df|xy)  Y2[p,c;q,b] = sum Gamma2[(p,c),(e,f)] (qf|be)
-__global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double *G3, double *Q1, double *W2,
-                                                  double *J2, double *Y2, const int *flag) {
+//   G1[p,q,c,a] = sum_e J[(p,q),(e,c);e,a]         G3[p,q,r,x] = sum_e J[(p,e),(q,r);x,e]
+//   Q1[p,t,x,y] = sum Gamma2[(p,f),(t,e)] (xf|ye)  J2 as above
+//   JW = J2 + sum Gamma2[(p,f),(e,q)] (xf|ey)      Z[p,c,q,b] = 2 J2 - sum Gamma2[(p,c),(e,f)] (qf|be)
+__global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double *G3, double *Q1, double *JW,
+                                                  double *J2, double *Z, const int *flag) {
     if (*flag) return;
     const int n = v.n;
     const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= v.n2 * v.n2) return;
     const int d = (int)(t % n), c = (int)((t / n) % n), b = (int)((t / v.n2) % n), a = (int)(t / (v.n2 * n));
-    double g1 = 0.0, g3 = 0.0, q1 = 0.0, w2 = 0.0, j2 = 0.0, y2 = 0.0;
+    double g1 = 0.0, g3 = 0.0, q1 = 0.0, w2 = 0.0, j2 = v.d1(a, b) * v.g[c * n + d], y2 = 0.0;
     for (int e = 0; e < n; ++e) {
         g1 += v.jj(a, b, e, c, e, d);
         g3 += v.jj(a, e, b, c, d, e);
@@ -418,83 +430,88 @@ __global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double 
             j2 = fma(v.d2(a, e, b, f), v.ai(e, f, c, d), j2);
         }
     }
-    G1[t] = g1; G3[t] = g3; Q1[t] = q1; W2[t] = w2; J2[t] = j2; Y2[t] = y2;
+    G1[t] = g1; G3[t] = g3; Q1[t] = q1; JW[t] = j2 + w2; J2[t] = j2; Z[t] = 2.0 * j2 - y2;
 }
 
-// amat/atmat(s, ap,bp,cp,a,b,c), one thread per element, ap fastest.
+// amat/atmat(s, ap,bp,cp,a,b,c): a thread owns (a, c, b, bp, cp), a fastest,
+// and kOutAp values of ap.  With a and c across a warp most gathers of F and the
+// n^8 tensors (whose last indices are a, c or b) use whole sectors.  The sums
+// over one index (Gamma2 with the integrals: the FP64 work, 6 n FMAs per
+// element) keep ap in registers, so that five of their six factors are loaded
+// once for all of them.
+constexpr int kOutAp = 4;
 __global__ void __launch_bounds__(256) k_sym_out(SymView v, double *amat, double *atmat, const int *flag) {
     if (*flag) return;
     const int n = v.n;
+    const ll n5 = v.n2 * v.n2 * n;
     const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= v.n2 * v.n2 * v.n2) return;
+    if (t >= n5) return;
     ll x = t;
-    const int ap = (int)(x % n); x /= n;
-    const int bp = (int)(x % n); x /= n;
-    const int cp = (int)(x % n); x /= n;
     const int a = (int)(x % n); x /= n;
+    const int c = (int)(x % n); x /= n;
     const int b = (int)(x % n); x /= n;
-    const int c = (int)x;
-    double A = v.f4(cp, ap, bp, b, c, a) - v.f4(ap, cp, b, bp, a, c) - v.f4(ap, cp, c, a, bp, b);
-    double T = v.f4(ap, cp, bp, b, a, c) - v.f4(cp, ap, b, bp, c, a) - v.f4(cp, ap, a, c, bp, b);
-    A += v.wca(cp, bp, b, c, ap, a) + v.jj(cp, c, bp, b, ap, a) - v.waa(cp, bp, b, a, ap, c) -
-         v.waa(bp, cp, ap, a, b, c) - v.waa(cp, a, c, bp, ap, b);
-    T += v.waa(cp, b, bp, a, ap, c) + v.waa(b, cp, ap, a, bp, c) - v.waa(c, ap, cp, bp, a, b) -
-         v.wca(cp, b, bp, c, ap, a) - v.wca(b, cp, ap, c, bp, a) - v.wca(cp, a, c, bp, ap, b);
-    T += 2.0 * v.jj(cp, ap, a, c, b, bp) - v.jj(cp, c, b, bp, ap, a) - v.jj(cp, ap, b, c, bp, a) -
-         v.jj(cp, bp, a, c, ap, b) - v.kx(cp, ap, a, c, b, bp);
-    double s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    const int bp = (int)(x % n); x /= n;
+    const int cp = (int)x;
+    const int ap0 = blockIdx.y * kOutAp;
+    double sum[kOutAp] = {};
     for (int d = 0; d < n; ++d) {
-        const double gda = v.g[d * n + a], gcd = v.g[c * n + d], gbd = v.g[b * n + d];
-        s1 += v.e3(cp, ap, bp, b, d, c) * gda - v.e3(cp, ap, bp, b, a, d) * gcd - v.e3(cp, ap, bp, d, a, c) * gbd;
-        s2 += v.e3(cp, ap, b, bp, a, d) * gcd - v.e3(cp, ap, b, bp, d, c) * gda - v.e3(cp, ap, d, bp, a, c) * gbd;
-        // two-operator sums of atmat
-        s3 += 2.0 * (v.d2(cp, d, ap, c) * v.ai(d, a, b, bp) + v.d2(cp, a, d, c) * v.ai(ap, d, b, bp));
-        s3 -= v.d2(cp, b, d, c) * v.ai(ap, d, bp, a) + v.d2(cp, b, c, d) * v.ai(bp, d, ap, a);
-        s3 -= v.d2(cp, a, d, c) * v.ai(bp, d, b, ap) + v.d2(cp, d, bp, c) * v.ai(d, a, b, ap);
-        s3 -= v.d2(cp, d, c, bp) * v.ai(ap, a, b, d) + v.d2(cp, d, ap, c) * v.ai(bp, a, b, d);
-    }
-    A += s1;
-    T += s2 + s3 + 2.0 * v.e2(cp, ap, a, c) * v.g[b * n + bp];
-    T += v.d1(cp, c) * (2.0 * v.ai(ap, a, b, bp) - v.ai(bp, a, b, ap));
-    // Kronecker deltas
-    auto q2 = [&](int p, int y) {  // sum Gamma2[(p,e),(d,f)] (df|ye)
-        double q = 0.0;
-        for (int e = 0; e < n; ++e) q += v.J2[v.i4(p, e, y, e)];
-        return q;
-    };
-    if (ap == bp) {
-        A += v.G1[v.i4(cp, b, c, a)] - v.G1[v.i4(b, cp, a, c)] - v.G3[v.i4(cp, a, c, b)] - v.Q1[v.i4(cp, a, b, c)];
-        if (a == b) A -= q2(cp, c);
-    }
-    if (ap == a) A -= v.G3[v.i4(cp, bp, b, c)] + v.G3[v.i4(bp, cp, c, b)] + v.Q1[v.i4(bp, cp, b, c)];
-    if (a == b) A -= v.G3[v.i4(bp, cp, ap, c)] + v.Q1[v.i4(cp, bp, ap, c)];
-    if (ap == b) {
-        T += v.G1[v.i4(bp, cp, a, c)] - v.G1[v.i4(cp, bp, c, a)] - v.W2[v.i4(cp, c, bp, a)] -
-             v.J2[v.i4(cp, c, bp, a)] + v.Q1[v.i4(cp, a, bp, c)];
-        if (bp == a) T += q2(cp, c);
-    }
-    if (ap == a)
-        T += v.G3[v.i4(cp, b, bp, c)] + v.Q1[v.i4(b, cp, bp, c)] - v.G1[v.i4(cp, c, bp, b)] -
-             v.Y2[v.i4(cp, c, bp, b)] + 2.0 * v.J2[v.i4(cp, c, b, bp)];
-    if (bp == a)
-        T += v.G3[v.i4(b, cp, ap, c)] + v.Q1[v.i4(cp, b, ap, c)] - v.G1[v.i4(cp, ap, c, b)] -
-             v.J2[v.i4(cp, c, b, ap)] - v.W2[v.i4(cp, c, ap, b)];
-    if (b == bp) {
-        double D = 2.0 * (v.G1[v.i4(cp, ap, c, a)] + v.J2[v.i4(cp, c, ap, a)] + v.W2[v.i4(cp, c, ap, a)] -
-                          v.G3[v.i4(a, cp, ap, c)] - v.Q1[v.i4(cp, a, ap, c)]) +
-                   v.d1(cp, c) * v.K[ap * n + a];
-        for (int d = 0; d < n; ++d)
-            D += v.d2(cp, d, ap, c) * v.K[d * n + a] - v.d2(cp, a, ap, d) * v.K[c * n + d] +
-                 2.0 * (v.e2(cp, ap, d, c) * v.fm[d * n + a] - v.e2(cp, ap, a, d) * v.fm[c * n + d]);
-        if (a == ap) {
-            D -= 2.0 * q2(cp, c);
-            for (int d = 0; d < n; ++d) D -= v.d1(cp, d) * v.K[c * n + d];
+        const double m1 = 2.0 * v.ai(d, a, b, bp) - v.ai(bp, a, b, d), m2 = v.d2(d, c, cp, a), m3 = v.d2(d, c, cp, b);
+        const double m4 = v.d2(d, c, b, cp), m5 = v.d2(d, cp, c, bp), m6 = v.d2(d, cp, bp, c);
+#pragma unroll
+        for (int i = 0; i < kOutAp; ++i) {
+            const int ap = min(ap0 + i, n - 1);
+            double y = fma(m1, v.d2(ap, c, cp, d), sum[i]);                     // Gamma2[(cp,ap),(d,c)] [2 (da|b bp) - (bp a|bd)]
+            y = fma(m2, v.Lb[ap + n * (d + n * (b + n * bp))], y);              // Gamma2[(cp,d),(a,c)] [2 (ap d|b bp) - (bp d|b ap)]
+            y = fma(-m3, v.ai(ap, d, bp, a), y);                                // Gamma2[(cp,d),(b,c)] (ap d|bp a)
+            y = fma(-m4, v.ai(ap, a, bp, d), y);                                // Gamma2[(cp,c),(b,d)] (bp d|ap a)
+            y = fma(-m5, v.ai(ap, b, a, d), y);                                 // Gamma2[(cp,bp),(d,c)] (da|b ap)
+            sum[i] = fma(-m6, v.ai(ap, a, b, d), y);                            // Gamma2[(cp,c),(d,bp)] (ap a|bd)
         }
-        T += D;
     }
-    const ll o = v.s + (ll)v.r.M * t;
-    amat[o] = A;
-    atmat[o] = T;
+    const double d1 = v.d1(cp, c);
+#pragma unroll
+    for (int i = 0; i < kOutAp; ++i) {
+        const int ap = ap0 + i;
+        if (ap >= n) break;
+        double A = v.f4(cp, ap, bp, b, c, a) - v.f4(ap, cp, b, bp, a, c) - v.f4(ap, cp, c, a, bp, b);
+        double T = v.f4(ap, cp, bp, b, a, c) - v.f4(cp, ap, b, bp, c, a) - v.f4(cp, ap, a, c, bp, b);
+        A += v.wca(cp, bp, b, c, ap, a) + v.jj(cp, c, bp, b, ap, a) - v.waa(cp, bp, b, a, ap, c) -
+             v.waa(bp, cp, ap, a, b, c) - v.waa(cp, a, c, bp, ap, b);
+        T += v.waa(cp, b, bp, a, ap, c) + v.waa(b, cp, ap, a, bp, c) - v.waa(c, ap, cp, bp, a, b) -
+             v.wca(cp, b, bp, c, ap, a) - v.wca(b, cp, ap, c, bp, a) - v.wca(cp, a, c, bp, ap, b);
+        T += 2.0 * v.jj(cp, ap, a, c, b, bp) - v.jj(cp, c, b, bp, ap, a) - v.jj(cp, ap, b, c, bp, a) -
+             v.jj(cp, bp, a, c, ap, b) - v.kx(cp, ap, a, c, b, bp);
+        T += sum[i] + d1 * (2.0 * v.ai(ap, a, b, bp) - v.ai(bp, a, b, ap));
+        // Kronecker deltas
+        auto q2 = [&]() {  // sum_e J2[cp,e;c,e]
+            double q = 0.0;
+            for (int e = 0; e < n; ++e) q += v.J2[v.i4(cp, e, c, e)];
+            return q;
+        };
+        if (ap == bp) {
+            A += v.G1[v.i4(cp, b, c, a)] - v.G1[v.i4(b, cp, a, c)] - v.G3[v.i4(cp, a, c, b)] - v.Q1[v.i4(cp, a, b, c)];
+            if (a == b) A -= q2();
+        }
+        if (ap == a) {
+            A -= v.G3[v.i4(cp, bp, b, c)] + v.G3[v.i4(bp, cp, c, b)] + v.Q1[v.i4(bp, cp, b, c)];
+            T += v.G3[v.i4(cp, b, bp, c)] + v.Q1[v.i4(b, cp, bp, c)] - v.G1[v.i4(cp, c, bp, b)] + v.Z[v.i4(cp, c, bp, b)];
+        }
+        if (a == b) A -= v.G3[v.i4(bp, cp, ap, c)] + v.Q1[v.i4(cp, bp, ap, c)];
+        if (ap == b) {
+            T += v.G1[v.i4(bp, cp, a, c)] - v.G1[v.i4(cp, bp, c, a)] - v.JW[v.i4(cp, c, bp, a)] + v.Q1[v.i4(cp, a, bp, c)];
+            if (bp == a) T += q2();
+        }
+        if (bp == a)
+            T += v.G3[v.i4(b, cp, ap, c)] + v.Q1[v.i4(cp, b, ap, c)] - v.G1[v.i4(cp, ap, c, b)] - v.JW[v.i4(cp, c, ap, b)];
+        if (b == bp) {
+            T += 2.0 * (v.G1[v.i4(cp, ap, c, a)] + v.JW[v.i4(cp, c, ap, a)] - v.G3[v.i4(a, cp, ap, c)] -
+                        v.Q1[v.i4(cp, a, ap, c)]);
+            if (a == ap) T -= 2.0 * q2();
+        }
+        const ll o = v.s + (ll)v.r.M * (ap + n * (bp + n * (cp + n * (a + (ll)n * (b + n * c)))));
+        amat[o] = A;
+        atmat[o] = T;
+    }
 }
 #undef AT
 
@@ -521,7 +538,7 @@ FShape f_shape(int n) {
     return best;
 }
 
-using FKernel = void (*)(int, int, const double *, const double *, double *, const int *);
+using FKernel = void (*)(Rdm, int, int, const double *, const double *, const double *, double *, const int *);
 FKernel f_kernel(int rpt) {
     switch (rpt) {
         case 1: return k_sym_f<1>;
@@ -538,7 +555,7 @@ FKernel f_kernel(int rpt) {
 ll SymScratch::doubles(int n) {
     const ll n2 = (ll)n * n, n4 = n2 * n2, np = n * (n + 1) / 2;
     const ll W = (ll)n * (n + 1) * (n + 2) * (n + 3) / 24;
-    return W * n4 + 4 * np * n4 + np * np * n2 + 7 * n4 + 2 * np * n2 + 3 * n2 + W / 2 + 1;
+    return W * n4 + 4 * np * n4 + np * np * n2 + 8 * n4 + 2 * np * n2 + n2 + W / 2 + 1;
 }
 
 SymScratch::SymScratch(int n, double *w) {
@@ -552,12 +569,11 @@ SymScratch::SymScratch(int n, double *w) {
     H = take(W * n4);
     F = take(np * n4);
     N8 = take(3 * np * n4 + np * np * n2);
-    for (double **p : {&G1, &G3, &Q1, &W2, &J2, &Y2}) *p = take(n4);
+    for (double **p : {&G1, &G3, &Q1, &JW, &J2, &Z}) *p = take(n4);
     Bf = take(np * n2);
     I4 = take(n4);
     IJ = take(n2 * np);
-    fm = take(n2);
-    K = take(n2);
+    Lb = take(n4);
     g = take(n2);
     key = (int *)take(W / 2 + 1);
 }
@@ -577,17 +593,19 @@ int launch_sym_state(const Rdm &r, int s, const double *atwo, const SymScratch &
     k_sym_unpack<<<(unsigned)(ub + cb), 256, 0, st>>>(r, s, S.key, (unsigned)ub, S.H, flag);
     const int *fl = flag + s;
     const dim3 g8((unsigned)((rows + kN8 - 1) / kN8), (unsigned)((n2 + kN8 - 1) / kN8), 4);
-    k_sym_n8<<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
+    k_sym_n8<<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.g, S.N8, fl);
     const FShape fs = f_shape(n);
     const FKernel fk = f_kernel(fs.rpt);
     const int smem = (fs.bc * n * (np | 1) + np * n) * (int)sizeof(double);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute((const void *)fk, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
         return 1;
-    fk<<<(unsigned)(np * n * ((n + fs.bc - 1) / fs.bc)), 256, smem, st>>>(n, fs.bc, S.H, S.Bf, S.F, fl);
-    SymView v{r, s, n, n2, rows, S.F, S.N8, S.G1, S.G3, S.Q1, S.W2, S.J2, S.Y2, atwo, S.fm, S.K, S.g};
-    k_sym_small<<<(unsigned)((n4 + 63) / 64), 64, 0, st>>>(v, S.G1, S.G3, S.Q1, S.W2, S.J2, S.Y2, fl);
-    k_sym_out<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(v, amat, atmat, fl);
+    fk<<<(unsigned)(np * n * ((n + fs.bc - 1) / fs.bc)), 256, smem, st>>>(r, s, fs.bc, S.H, S.Bf, S.g,
+                                                                                       S.F, fl);
+    SymView v{r, s, n, n2, rows, S.F, S.N8, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, atwo, S.Lb, S.g};
+    k_sym_small<<<(unsigned)((n4 + 63) / 64), 64, 0, st>>>(v, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, fl);
+    const dim3 go((unsigned)((n4 * n + 255) / 256), (unsigned)((n + kOutAp - 1) / kOutAp));
+    k_sym_out<<<go, 256, 0, st>>>(v, amat, atmat, fl);
     g_launches.fetch_add(5, std::memory_order_relaxed);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
 }

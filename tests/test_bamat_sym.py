@@ -49,45 +49,38 @@ def test_one_contraction_equals_the_loop(n, ne):
     A0, At0 = (np.asarray(x)[0] for x in _oracle(p, T, aj))
     D1, D2, D3, D4 = p.dal[0], p.taa[0], p.daaa[0], _dense4(p, 0)
     d = np.eye(n)
-    h = np.array([[aj[synth.tri(i + 3, j + 3) - 1] for j in range(n)] for i in range(n)])
-    K = es("deea->da", T)
-    f, g = h - 0.5 * K, h
-    EE = D2.transpose(0, 2, 1, 3) + es("bc,ad->abcd", d, D1)
-    E3 = D3.transpose(0, 3, 1, 4, 2, 5) + es("ed,acbf->abcdef", d, D2) + es("eb,acfd->abcdef", d, D2)
-    E3 = E3 + es("bc,aedf->abcdef", d, D2) + es("bc,ed,af->abcdef", d, d, D1)
-    F = es("pqdersfc,dfea->prqsca", D4, T, optimize=True)  # [A, B, c, a]
-    J, Kx = es("pqdrsf,dfxy->prqsxy", D3, T), es("pqdrse,dxye->prqsxy", D3, T)
+    h = np.array([[aj[synth.tri(i + 3, j + 3) - 1] for j in range(n)] for i in range(n)])  # f + K/2 = aj
+    F = es("pqdersfc,dfea->prqsca", D4, T, optimize=True) + es("pqdrsc,da->prqsca", D3, h)  # [A, B, c, a]
+    J = es("pqdrsf,dfxy->prqsxy", D3, T) + es("pqrs,xy->prqsxy", D2, h)
+    Kx = es("pqdrse,dxye->prqsxy", D3, T)
     Wca, Waa = es("pqefrs,xfey->pqrsxy", D3, T), es("pqtfre,xfye->pqrtxy", D3, T)
     G1, G3 = es("pqecea->pqca", J), es("peqrxe->pqrx", J)
-    Q1, W2 = es("ptfe,xfye->ptxy", D2, T), es("pefs,xfey->psxy", D2, T)
-    J2, Y2, Q2 = es("pdqf,dfxy->pqxy", D2, T), es("pecf,qfbe->pcqb", D2, T), es("pdef,dfce->pc", D2, T)
+    Q1 = es("ptfe,xfye->ptxy", D2, T)
+    J2 = es("pdqf,dfxy->pqxy", D2, T) + es("pq,xy->pqxy", D1, h)
+    JW = J2 + es("pefs,xfey->psxy", D2, T)
+    Z = 2 * J2 - es("pecf,qfbe->pcqb", D2, T)
+    Q2 = es("pece->pc", J2)
     o = "->jkialc"  # i, j, k, l = cp, ap, bp, b
-    A = es("ijkldc,da" + o, E3, g) - es("ijklad,cd" + o, E3, g) - es("ijkdac,ld" + o, E3, g)
-    A = A + es("ijklca" + o, F) - es("jilkac" + o, F) - es("jicakl" + o, F)
+    A = es("ijklca" + o, F) - es("jilkac" + o, F) - es("jicakl" + o, F)
     A += es("iklcja" + o, Wca) + es("icklja" + o, J) - es("iklajc" + o, Waa) - es("kijalc" + o, Waa)
+    A -= es("iackjl" + o, Waa) + es("la,kijc" + o, d, G3) + es("la,ikjc" + o, d, Q1)
     A += es("jk,ilca" + o, d, G1) - es("jk,liac" + o, d, G1) - es("jk,iacl" + o, d, G3) - es("jk,ialc" + o, d, Q1)
-    A -= es("iackjl" + o, Waa) + es("ja,iklc" + o, d, G3) + es("ja,kicl" + o, d, G3) + es("ja,kilc" + o, d, Q1)
-    A -= es("la,kijc" + o, d, G3) + es("la,ikjc" + o, d, Q1) + es("jk,la,ic" + o, d, d, Q2)
+    A -= es("ja,iklc" + o, d, G3) + es("ja,kicl" + o, d, G3) + es("ja,kilc" + o, d, Q1) + es("jk,la,ic" + o, d, d, Q2)
     assert rel_err(A, A0) < 1e-12
-    B = es("ijlkad,cd" + o, E3, g) - es("ijlkdc,da" + o, E3, g) - es("ijdkac,ld" + o, E3, g)
-    B = B + 2 * es("ijac,lk" + o, EE, g) - es("ijlkca" + o, F) + es("jiklac" + o, F) - es("ijackl" + o, F)
-    B -= es("ilkcja" + o, Wca) + es("iclkja" + o, J) + es("lijcka" + o, Wca) + es("ijlcka" + o, J)
-    B -= es("jl,ikca" + o, d, G1) + es("jl,icka" + o, d, W2) + es("jl,icka" + o, d, J2)
-    B -= es("ilfc,jfka" + o, D2, T) + es("ilcf,kfja" + o, D2, T)
-    B += es("jl,kiac" + o, d, G1) + es("ilkajc" + o, Waa) + es("ja,ilkc" + o, d, G3) + es("lijakc" + o, Waa)
-    B += es("ka,lijc" + o, d, G3) + es("jl,iakc" + o, d, Q1) + es("jl,ka,ic" + o, d, d, Q2)
-    B += es("ka,iljc" + o, d, Q1) + es("ja,likc" + o, d, Q1)
-    B -= es("ikacjl" + o, J) + es("iackjl" + o, Wca) + es("ja,ickl" + o, d, G1) + es("ja,ickl" + o, d, Y2)
-    B -= es("ijaclk" + o, Kx) + es("ka,ijcl" + o, d, G1) + es("ka,iclj" + o, d, J2) + es("ka,icjl" + o, d, W2)
-    B -= es("cjikal" + o, Waa) + es("iafc,kflj" + o, D2, T) + es("idkc,dalj" + o, D2, T)
-    B -= es("ieck,jale" + o, D2, T) + es("iejc,kale" + o, D2, T) + es("ic,kalj" + o, D1, T)
-    B += 2 * (es("ijaclk" + o, J) + es("idjc,dalk" + o, D2, T) + es("ja,iclk" + o, d, J2) + es("iaec,jelk" + o, D2, T))
-    B += 2 * es("ic,jalk" + o, D1, T)
-    D = 2 * (G1 + es("icja->ijca", J2) + es("icja->ijca", W2) - es("aijc->ijca", G3) - es("iajc->ijca", Q1))
-    D = D + es("idjc,da->ijca", D2, K) + es("ic,ja->ijca", D1, K) - 2 * es("ja,ic->ijca", d, Q2)
-    D = D - es("iajd,cd->ijca", D2, K) - es("ja,id,cd->ijca", d, D1, K)
-    D = D + 2 * es("ijdc,da->ijca", EE, f) - 2 * es("ijad,cd->ijca", EE, f)
-    B += es("lk,ijca" + o, d, D)
+    B = es("jiklac" + o, F) - es("ijlkca" + o, F) - es("ijackl" + o, F)
+    B = B + es("ilkajc" + o, Waa) + es("lijakc" + o, Waa) - es("cjikal" + o, Waa)
+    B -= es("ilkcja" + o, Wca) + es("lijcka" + o, Wca) + es("iackjl" + o, Wca)
+    B += 2 * es("ijaclk" + o, J) - es("iclkja" + o, J) - es("ijlcka" + o, J) - es("ikacjl" + o, J) - es("ijaclk" + o, Kx)
+    B += 2 * es("idjc,dalk" + o, D2, T) - es("iejc,kale" + o, D2, T)
+    B += 2 * es("iaec,jelk" + o, D2, T) - es("iafc,kflj" + o, D2, T)
+    B -= es("ilfc,jfka" + o, D2, T) + es("ilcf,kfja" + o, D2, T) + es("idkc,dalj" + o, D2, T) + es("ieck,jale" + o, D2, T)
+    B += 2 * es("ic,jalk" + o, D1, T) - es("ic,kalj" + o, D1, T)
+    B += es("ja,ilkc" + o, d, G3) + es("ja,likc" + o, d, Q1) - es("ja,ickl" + o, d, G1) + es("ja,ickl" + o, d, Z)
+    B += es("jl,kiac" + o, d, G1) - es("jl,ikca" + o, d, G1) - es("jl,icka" + o, d, JW) + es("jl,iakc" + o, d, Q1)
+    B += es("jl,ka,ic" + o, d, d, Q2) + es("ka,lijc" + o, d, G3) + es("ka,iljc" + o, d, Q1)
+    B -= es("ka,ijcl" + o, d, G1) + es("ka,icjl" + o, d, JW)
+    D = G1 + es("icja->ijca", JW) - es("aijc->ijca", G3) - es("iajc->ijca", Q1) - es("ja,ic->ijca", d, Q2)
+    B += 2 * es("lk,ijca" + o, d, D)
     assert rel_err(B, At0) < 1e-12
 
 

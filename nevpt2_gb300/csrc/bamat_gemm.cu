@@ -78,61 +78,64 @@ __global__ void __launch_bounds__(256) k_bamat_slabs_t(Rdm r, int s, const int *
     __shared__ double mwz[256];
     const int n = r.n, sw = n + 1, sf = n * (n + 1) + 1;
     const ll n2 = (ll)n * n, n3 = n2 * n, n6 = n3 * n3;
-    ll b = blockIdx.x;
-    const int d = (int)(b % n); b /= n;
-    const int v = (int)(b % n); b /= n;
-    const int u = (int)(b % n); b /= n;
-    const int sl = (int)b;
-    const int cp = slab_cp[sl], ap = slab_ap[sl];
-    for (int i = threadIdx.x; i < n3; i += blockDim.x) {
-        const int z = i % n, w = (i / n) % n, f = i / (int)n2;
-        tile[f * sf + w * sw + z] = r.eeee(cp + 1, ap + 1, u + 1, v + 1, d + 1, f + 1, w + 1, z + 1, s + 1);
-    }
-    __syncthreads();
-    const ll base = (ll)sl * n6;
-    for (int i = threadIdx.x; i < n3; i += blockDim.x) {
-        // X1 rows (u,v,z) cols (d,f,w): i = (z, f, w)
-        {
-            const int w = i % n, f = (i / n) % n, z = i / (int)n2;
-            X1[base + (((ll)u * n + v) * n + z) * n3 + ((ll)d * n + f) * n + w] = tile[f * sf + w * sw + z];
+    for (ll blk = blockIdx.x; blk < nslab * n3; blk += gridDim.x) {
+        __syncthreads();
+        ll b = blk;
+        const int d = (int)(b % n); b /= n;
+        const int v = (int)(b % n); b /= n;
+        const int u = (int)(b % n); b /= n;
+        const int sl = (int)b;
+        const int cp = slab_cp[sl], ap = slab_ap[sl];
+        for (int i = threadIdx.x; i < n3; i += blockDim.x) {
+            const int z = i % n, w = (i / n) % n, f = i / (int)n2;
+            tile[f * sf + w * sw + z] = r.eeee(cp + 1, ap + 1, u + 1, v + 1, d + 1, f + 1, w + 1, z + 1, s + 1);
         }
-        // X2 rows (u,v,w) cols (d,f,z): i = (w, f, z)
-        {
-            const int z = i % n, f = (i / n) % n, w = i / (int)n2;
-            X2[base + (((ll)u * n + v) * n + w) * n3 + ((ll)d * n + f) * n + z] = tile[f * sf + w * sw + z];
+        __syncthreads();
+        const ll base = (ll)sl * n6;
+        for (int i = threadIdx.x; i < n3; i += blockDim.x) {
+            // X1 rows (u,v,z) cols (d,f,w): i = (z, f, w)
+            {
+                const int w = i % n, f = (i / n) % n, z = i / (int)n2;
+                X1[base + (((ll)u * n + v) * n + z) * n3 + ((ll)d * n + f) * n + w] = tile[f * sf + w * sw + z];
+            }
+            // X2 rows (u,v,w) cols (d,f,z): i = (w, f, z)
+            {
+                const int z = i % n, f = (i / n) % n, w = i / (int)n2;
+                X2[base + (((ll)u * n + v) * n + w) * n3 + ((ll)d * n + f) * n + z] = tile[f * sf + w * sw + z];
+            }
+            // X3 rows (u,w,z) cols (v,d,f), X4 rows (v,w,z) cols (u,d,f): i = (w, z, f)
+            {
+                const int f = i % n, z = (i / n) % n, w = i / (int)n2;
+                const double x = tile[f * sf + w * sw + z];
+                X3[base + (((ll)u * n + w) * n + z) * n3 + ((ll)v * n + d) * n + f] = x;
+                X4[base + (((ll)v * n + w) * n + z) * n3 + ((ll)u * n + d) * n + f] = x;
+            }
         }
-        // X3 rows (u,w,z) cols (v,d,f), X4 rows (v,w,z) cols (u,d,f): i = (w, z, f)
-        {
-            const int f = i % n, z = (i / n) % n, w = i / (int)n2;
-            const double x = tile[f * sf + w * sw + z];
-            X3[base + (((ll)u * n + w) * n + z) * n3 + ((ll)v * n + d) * n + f] = x;
-            X4[base + (((ll)v * n + w) * n + z) * n3 + ((ll)u * n + d) * n + f] = x;
+        if (!rmax) continue;
+        // m(w,z) = max_f |x|: the X3 / X4 partials; X1 (row z) = max_w, X2 (row w) = max_z
+        for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+            const int z = i % n, w = i / n;
+            double m = 0.0;
+            for (int f = 0; f < n; ++f) m = fmax(m, fabs(tile[f * sf + w * sw + z]));
+            mwz[i] = m;
         }
-    }
-    if (!rmax) return;
-    // m(w,z) = max_f |x|: the X3 / X4 partials; X1 (row z) = max_w, X2 (row w) = max_z
-    for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-        const int z = i % n, w = i / n;
-        double m = 0.0;
-        for (int f = 0; f < n; ++f) m = fmax(m, fabs(tile[f * sf + w * sw + z]));
-        mwz[i] = m;
-    }
-    __syncthreads();
-    const ll rows = (ll)nslab * n3, r0 = (ll)sl * n3;
-    for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-        const int z = i % n, w = i / n;
-        const unsigned long long m = (unsigned long long)__double_as_longlong(mwz[i]);
-        atomicMax(rmax + 2 * rows + r0 + ((ll)u * n + w) * n + z, m);
-        atomicMax(rmax + 3 * rows + r0 + ((ll)v * n + w) * n + z, m);
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double m1 = 0.0, m2 = 0.0;
-        for (int j = 0; j < n; ++j) {
-            m1 = fmax(m1, mwz[j * n + i]);  // row z = i: over w
-            m2 = fmax(m2, mwz[i * n + j]);  // row w = i: over z
+        __syncthreads();
+        const ll rows = (ll)nslab * n3, r0 = (ll)sl * n3;
+        for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+            const int z = i % n, w = i / n;
+            const unsigned long long m = (unsigned long long)__double_as_longlong(mwz[i]);
+            atomicMax(rmax + 2 * rows + r0 + ((ll)u * n + w) * n + z, m);
+            atomicMax(rmax + 3 * rows + r0 + ((ll)v * n + w) * n + z, m);
         }
-        atomicMax(rmax + 0 * rows + r0 + ((ll)u * n + v) * n + i, (unsigned long long)__double_as_longlong(m1));
-        atomicMax(rmax + 1 * rows + r0 + ((ll)u * n + v) * n + i, (unsigned long long)__double_as_longlong(m2));
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            double m1 = 0.0, m2 = 0.0;
+            for (int j = 0; j < n; ++j) {
+                m1 = fmax(m1, mwz[j * n + i]);  // row z = i: over w
+                m2 = fmax(m2, mwz[i * n + j]);  // row w = i: over z
+            }
+            atomicMax(rmax + 0 * rows + r0 + ((ll)u * n + v) * n + i, (unsigned long long)__double_as_longlong(m1));
+            atomicMax(rmax + 1 * rows + r0 + ((ll)u * n + v) * n + i, (unsigned long long)__double_as_longlong(m2));
+        }
     }
 }
 
@@ -557,6 +560,12 @@ struct AsyncBuffers {
 
 __global__ void k_slab_list(int n, int *cp, int *ap);
 
+// Split mode takes the digit products from this many active orbitals on; the
+// FP64 products are the faster and the more exact below (one state, FP64 / digits:
+// n = 10 1.68 / 1.81 ms, n = 11 3.32 / 3.07, n = 14 22.6 / 14.4, n = 16 60.4 / 37.3).
+constexpr int kSplitMinNact = 11;
+constexpr unsigned kSlabCtas = 152 * 16;  // CTAs of a slab launch: one wave or so, looping
+
 // Returns 0 on success, 2 on a failed allocation, 5 if a split-precision
 // product timed out, else a launch failure.
 int launch_bamat(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
@@ -564,34 +573,39 @@ int launch_bamat(const Rdm &r, const double *atwo, const double *f, int ncore, d
     const int n = r.n, M = r.M;
     const ll n2 = (ll)n * n, n3 = n2 * n, n4 = n3 * n, n6 = n3 * n3;
     AsyncBuffers buf(st);
-    // Slabs of the general route: a few at a time, or all of them where they are small.
-    const bool direct = n <= 5;
-    const int B = direct ? 0 : n <= 8 ? (int)n2 : 16;
-    const size_t xd = std::max<size_t>(4 * (size_t)B * n6, split ? 0 : (size_t)SymScratch::doubles(n));
-    double *X;
-    int *flag = nullptr;
-    if (!buf.get(&X, sizeof(double) * xd)) return 2;
-    // FP64: one contraction per state whose inputs have their physical
-    // symmetries (bamat_sym.cu); it raises flag[s] where they have not, and the
-    // general route below does the flagged states.  Its scratch is the slab
-    // buffer: each state's general route follows in stream order.
-    auto flag_of = [&](int s) { return flag ? flag + s : nullptr; };
-    if (!split) {
-        if (!buf.get(&flag, sizeof(int) * M)) return 2;
-        cudaMemsetAsync(flag, 0, sizeof(int) * M, st);
-        const SymScratch S(n, X);
-        launch_sym_ops(atwo, f, ncore, n, S, M, flag, st);
-        for (int s = 0; s < M; ++s)
-            if (launch_sym_state(r, s, atwo, S, amat, atmat, flag, st)) return 3;
-        if (direct) {
-            launch_bamat_direct(r, atwo, f, ncore, amat, atmat, st, flag);
-            return 0;
-        }
-    } else if (direct) {
-        launch_bamat_direct(r, atwo, f, ncore, amat, atmat, st, nullptr);
+    // One contraction per state whose inputs have their physical symmetries
+    // (bamat_sym.cu); it raises flag[s] where they have not, and the general
+    // route below does the flagged states.  The two share their scratch: each
+    // state's general route follows in stream order.
+    const bool direct = n <= 5;                           // general route: one thread per element
+    const int B = direct ? 0 : n <= 8 && !split ? (int)n2 : 16;  // else slabs at a time
+    const bool digits = split && n >= kSplitMinNact;
+    const size_t sd = (size_t)SymScratch::doubles(n);
+    double *X, *T = nullptr;
+    int *flag, *oz_err;
+    void *ozw = nullptr;
+    if (!buf.get(&X, sizeof(double) * std::max(4 * (size_t)B * n6, sd + (digits ? sym_split_rows_doubles(n) : 0))) ||
+        !buf.get(&flag, sizeof(int) * (M + 1)))
+        return 2;
+    oz_err = flag + M;
+    if (split && !direct) {
+        size_t wb = oz::OzPlan(4, (ll)B * n3, (int)n3, n).bytes();
+        if (digits) wb = std::max(wb, sym_split_oz_bytes(n));
+        if (!buf.get(&ozw, wb)) return 2;
+    }
+    cudaMemsetAsync(flag, 0, sizeof(int) * (M + 1), st);
+    const SymScratch S(n, X);
+    launch_sym_ops(atwo, f, ncore, n, S, M, flag, st);
+    for (int s = 0; s < M; ++s)
+        if (digits ? launch_sym_state_split(r, s, atwo, S, X + sd, ozw, oz_err, amat, atmat, flag, st)
+                   : launch_sym_state(r, s, atwo, S, amat, atmat, flag, st))
+            return 3;
+    if (direct) {
+        launch_bamat_direct(r, atwo, f, ncore, amat, atmat, st, flag);
         return 0;
     }
-    double *A1, *A2, *A3, *T;
+    // ---- the general route, for the flagged states
+    double *A1, *A2, *A3;
     int *slabs;
     if (!buf.get(&A1, sizeof(double) * 3 * n4) || !buf.get(&T, sizeof(double) * (4 * n6 + 5 * n4 + 4 * n2)) ||
         !buf.get(&slabs, sizeof(int) * 2 * n2))
@@ -599,44 +613,38 @@ int launch_bamat(const Rdm &r, const double *atwo, const double *f, int ncore, d
     A2 = A1 + n4;
     A3 = A2 + n4;
     // lower-order part first (writes amat/atmat, scratch T), then add the GEMM terms
-    for (int s = 0; s < M; ++s) bamat_rest(r, s, atwo, f, ncore, amat, atmat, T, st, flag_of(s));
+    for (int s = 0; s < M; ++s) bamat_rest(r, s, atwo, f, ncore, amat, atmat, T, st, flag + s);
     k_bamat_ints<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(atwo, n, A1, A2, A3);
     k_slab_list<<<(unsigned)((n2 + 255) / 256), 256, 0, st>>>(n, slabs, slabs + n2);
     g_launches.fetch_add(2, std::memory_order_relaxed);
-    int rc = 0;
-    // split precision: digit workspace for a full batch of slabs
-    void *ozw = nullptr;
     unsigned long long *rmax = nullptr;  // row maxima of the four slab layouts (split digits)
-    if (split) {
-        oz::OzPlan pl(4, (ll)B * n3, (int)n3, n);
-        if (!buf.get(&ozw, pl.bytes()) || !buf.get(&rmax, sizeof(unsigned long long) * 4 * (size_t)B * n3)) return 2;
-    }
-    for (int s = 0; s < M && !rc; ++s) {
-        for (int s0 = 0; s0 < n2 && !rc; s0 += B) {
+    if (split && !buf.get(&rmax, sizeof(unsigned long long) * 4 * (size_t)B * n3)) return 2;
+    for (int s = 0; s < M; ++s) {
+        for (int s0 = 0; s0 < n2; s0 += B) {
             const int nb = std::min(B, (int)n2 - s0);
             const ll rows = (ll)nb * n3;
             const double *Xs[4] = {X, X + (ll)B * n6, X + 2 * (ll)B * n6, X + 3 * (ll)B * n6}, *As[4] = {A1, A2, A3, A3};
             if (rmax) cudaMemsetAsync(rmax, 0, sizeof(unsigned long long) * 4 * (size_t)rows, st);
-            k_bamat_slabs_t<<<(unsigned)rows, 256, 0, st>>>(r, s, slabs + s0, slabs + n2 + s0, nb, X, X + (ll)B * n6,
-                                                            X + 2 * (ll)B * n6, X + 3 * (ll)B * n6, rmax, flag_of(s));
+            k_bamat_slabs_t<<<(unsigned)std::min<ll>(rows, kSlabCtas), 256, 0, st>>>(
+                r, s, slabs + s0, slabs + n2 + s0, nb, X, X + (ll)B * n6, X + 2 * (ll)B * n6, X + 3 * (ll)B * n6, rmax,
+                flag + s);
             g_launches.fetch_add(1, std::memory_order_relaxed);
             double *Ts[4] = {T + (ll)s0 * n4, T + n6 + (ll)s0 * n4, T + 2 * n6 + (ll)s0 * n4, T + 3 * n6 + (ll)s0 * n4};
             if (split) {
                 const unsigned long long *Rm[4] = {rmax, rmax + rows, rmax + 2 * rows, rmax + 3 * rows};
-                rc |= oz::oz_gemm_skinny(oz::OzPlan(4, rows, (int)n3, n), Xs, As, Ts, n, n, ozw, st, Rm);
-            } else {
-                rc |= dgemm_skinny4(st, rows, n, (int)n3, Xs, As, Ts, flag_of(s));
+                if (oz::oz_gemm_skinny(oz::OzPlan(4, rows, (int)n3, n), Xs, As, Ts, n, n, ozw, st, Rm,
+                                       oz::Gate{flag + s, true}, oz_err))
+                    return 3;
+            } else if (dgemm_skinny4(st, rows, n, (int)n3, Xs, As, Ts, flag + s)) {
+                return 3;
             }
         }
-        if (!rc) {
-            k_bamat_assemble<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(n, M, s, T, T + n6, T + 2 * n6, T + 3 * n6,
-                                                                        amat, atmat, flag_of(s));
-            g_launches.fetch_add(1, std::memory_order_relaxed);
-        }
+        k_bamat_assemble<<<(unsigned)((n6 + 255) / 256), 256, 0, st>>>(n, M, s, T, T + n6, T + 2 * n6, T + 3 * n6,
+                                                                    amat, atmat, flag + s);
+        g_launches.fetch_add(1, std::memory_order_relaxed);
     }
-    // the product kernels share one error flag (a wait that timed out)
-    if (ozw && !rc && oz::oz_check_error(ozw, st) != 0) rc = 5;
-    return rc == 5 ? 5 : (rc ? 3 : 0);
+    // the digit products share one error flag (a wait that timed out)
+    return split && oz::oz_check_error(oz_err, st) != 0 ? 5 : 0;
 }
 
 // ===========================================================================

@@ -37,14 +37,22 @@
 #include <algorithm>
 
 #include "bamat_sym.cuh"
+#include "ozaki.cuh"
 
 namespace nvpt {
 namespace {
 
 constexpr double kSymTol = 0x1p-45;
+constexpr int kSymXRows = 4;  // rows per warp of k_sym_x
 
 __host__ __device__ __forceinline__ int pidx(int i, int j) { return i * (i + 1) / 2 + j; }  // i >= j
 __device__ __forceinline__ int pmx(int i, int j) { return i > j ? pidx(i, j) : pidx(j, i); }
+__device__ __forceinline__ void unpair(int p, int &i, int &j) {  // p = pidx(i, j)
+    i = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
+    if (pidx(i + 1, 0) <= p) ++i;
+    if (pidx(i, 0) > p) --i;
+    j = p - pidx(i, 0);
+}
 
 // Packed rank (0-based) of a descending quadruple of 0-based indices.
 __device__ __forceinline__ int rank4(const int v[4]) { return lindice4(v[0] + 1, v[1] + 1, v[2] + 1, v[3] + 1) - 1; }
@@ -88,7 +96,10 @@ __global__ void __launch_bounds__(256) k_sym_ops(const double *atwo, const doubl
     if (t < n2) {                                             // (x, y) = (k, l)
         double kk = 0.0;
         for (int z = 0; z < n; ++z) kk += AT(k, z, z, l);
-        S.g[t] = f[tri_index(k + 1 + ncore, l + 1 + ncore) - 1] + 0.5 * kk;
+        const double g = f[tri_index(k + 1 + ncore, l + 1 + ncore) - 1] + 0.5 * kk;
+        S.g[t] = g;
+        S.Bf[(ll)n * np * n + t] = g;  // the last K chunk of F
+        if (k >= l) S.IJ[n2 * np + pidx(k, l)] = g;
     }
 }
 
@@ -108,7 +119,8 @@ __device__ double rdm_scale(const Rdm &r, int s) {
 // annihilators: the transpose of the packed 4-RDM, completed over the
 // annihilators of higher rank than K (where the packed form keeps the
 // exchanged element).  Reads are coalesced along K, writes along l1.  The
-// blocks from nub on check Gamma1..3.  Bound by HBM: 16 W n^4 bytes.
+// blocks from nub on check Gamma1..3.  Bound by HBM (16 W n^4 bytes) and by the
+// gathers of the completed half; n = 16: 3.9 ms.
 __global__ void __launch_bounds__(256) k_sym_unpack(Rdm r, int s, const int *key, unsigned nub, double *H, int *flag) {
     const int n = r.n, M = r.M;
     const ll n2 = (ll)n * n, n3 = n2 * n, n4 = n2 * n2, W = r.W;
@@ -185,75 +197,87 @@ __global__ void __launch_bounds__(256) k_sym_unpack(Rdm r, int s, const int *key
 // turns the annihilators' offsets into four strides -- and multiplies: threads
 // are (row group, column), RPT rows each.  Bound by the FP64 pipe (2 FMA per
 // clock and SM): the gathers (two loads per n FMAs) run under the products of
-// the SM's other CTA.
-template <int RPT>
-__global__ void __launch_bounds__(256) k_sym_f(Rdm r, int s, int bc, const double *__restrict__ H,
-                                               const double *__restrict__ Bf, const double *__restrict__ g,
-                                               double *__restrict__ F, const int *flag) {
-    if (*flag) return;
-    extern __shared__ double sm[];
+// the SM's other CTAs.  n = 16: 36.3 ms for 3.9e10 flops, 1.07 TFLOP/s (the four
+// products it replaced took 459 ms at 1.20); n = 11: 1.5 ms.
+struct FBlock {  // what one CTA owns: (cp >= bp) = pair pr, ap, rows (b0 .. b0 + R / n, c)
+    int pr, cp, bp, ap, b0, R;
+};
+__device__ __forceinline__ FBlock f_block(int n, int bc, int blk) {
+    FBlock f;
+    const int nchunk = (n + bc - 1) / bc;
+    f.b0 = (blk % nchunk) * bc;
+    blk /= nchunk;
+    f.ap = blk % n;
+    f.pr = blk / n;
+    unpair(f.pr, f.cp, f.bp);
+    f.R = min(bc, n - f.b0) * n;
+    return f;
+}
+// X_e of the block into shared memory, X[row * ldx + k]: k = df for e < n, k = d
+// (Gamma3) for e = n.  Starts and ends with all threads of the CTA together.
+__device__ __forceinline__ void f_gather(const Rdm &r, int s, const FBlock &f, int e, const double *__restrict__ H,
+                                         double *X, int ldx) {
     __shared__ ll s_base[16];
     __shared__ int s_w[16][3];
-    const int n = r.n, np = n * (n + 1) / 2, tid = threadIdx.x;
-    const int n2 = n * n, n4 = n2 * n2;
-    const int nchunk = (n + bc - 1) / bc;
-    int blk = blockIdx.x;
-    const int b0 = (blk % nchunk) * bc; blk /= nchunk;
-    const int ap = blk % n, pr = blk / n;
-    int cp = (int)((sqrtf(8.0f * pr + 1.0f) - 1.0f) * 0.5f);
-    while (pidx(cp + 1, 0) <= pr) ++cp;
-    while (pidx(cp, 0) > pr) --cp;
-    const int bp = pr - pidx(cp, 0);
-    const int nb = min(bc, n - b0), R = nb * n, ldx = np | 1;  // odd: no bank conflicts down a column
-    double *X = sm, *B = sm + bc * n * ldx;                    // [row][df], [df][a]
+    const int n = r.n, n2 = n * n, n4 = n2 * n2, np = n * (n + 1) / 2, tid = threadIdx.x, R = f.R;
+    if (e < n && tid < n) {
+        int v[4] = {f.cp, f.bp, tid, e}, o[4], w[4], p = 1;
+        sort4(v, o);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (o[j] == i) w[i] = p;
+            p *= n;
+        }
+        s_base[tid] = (ll)rank4(v) * n4 + f.ap * w[0] + f.b0 * w[1];
+        s_w[tid][0] = w[1];
+        s_w[tid][1] = w[2];
+        s_w[tid][2] = w[3];
+    }
+    __syncthreads();
+    if (e == n) {  // Gamma3 with its annihilators exchanged, d the fastest index
+        const double *d3 = r.d3 + s + (ll)r.M * (n * f.cp + n2 * f.bp + (ll)n4 * (f.ap + n * f.b0));
+        for (int i = tid; i < R * n; i += 256) {
+            const int row = i % R, d = i / R;
+            X[row * ldx + d] = d3[(ll)r.M * (d + n2 * n * (row % n) + (ll)n4 * n * (row / n))];
+        }
+    } else {
+        for (int i = tid; i < R * np; i += 256) {
+            const int row = i % R, df = i / R;
+            const int c = row % n, b = row / n;
+            int d, g;
+            unpair(df, d, g);
+            double x = H[s_base[d] + b * s_w[d][0] + g * s_w[d][1] + c * s_w[d][2]];
+            if (d != g) x += H[s_base[g] + b * s_w[g][0] + d * s_w[g][1] + c * s_w[g][2]];
+            X[row * ldx + df] = x;
+        }
+    }
+    __syncthreads();
+}
+
+template <int RPT>
+__global__ void __launch_bounds__(256) k_sym_f(Rdm r, int s, int bc, const double *__restrict__ H,
+                                               const double *__restrict__ Bf, double *__restrict__ F,
+                                               const int *flag) {
+    if (*flag) return;
+    extern __shared__ double sm[];
+    const int n = r.n, np = n * (n + 1) / 2, tid = threadIdx.x, ldx = np | 1;  // odd: no bank conflicts down a column
+    const FBlock f = f_block(n, bc, blockIdx.x);
+    double *X = sm, *B = sm + bc * n * ldx;
     const int groups = 256 / n, col = tid % n, grp = tid / n;
-    const bool live = grp < groups;
     double acc[RPT];
     int ro[RPT];
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
         acc[i] = 0.0;
-        ro[i] = min(grp + i * groups, R - 1) * ldx;
+        ro[i] = min(grp + i * groups, f.R - 1) * ldx;
     }
     for (int e = 0; e <= n; ++e) {
         const int nk = e < n ? np : n;
-        if (e < n && tid < n) {
-            int v[4] = {cp, bp, tid, e}, o[4];
-            sort4(v, o);
-            int w[4], p = 1;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (o[j] == i) w[i] = p;
-                p *= n;
-            }
-            s_base[tid] = (ll)rank4(v) * n4 + ap * w[0] + b0 * w[1];
-            s_w[tid][0] = w[1];
-            s_w[tid][1] = w[2];
-            s_w[tid][2] = w[3];
-        }
-        const double *Be = e < n ? Bf + (ll)e * np * n : g;
-        for (int i = tid; i < nk * n; i += 256) B[i] = Be[i];
-        __syncthreads();
-        for (int i = tid; i < R * nk; i += 256) {
-            const int row = i % R, df = i / R;
-            const int c = row % n, b = row / n;
-            if (e == n) {  // Gamma3 with its annihilators as the first pair index: d = df
-                X[row * ldx + df] =
-                    r.d3[s + (ll)r.M * (df + n * cp + n2 * bp + (ll)(n2 * n) * c + (ll)n4 * ap + (ll)n4 * n * (b0 + b))];
-                continue;
-            }
-            int d = (int)((sqrtf(8.0f * df + 1.0f) - 1.0f) * 0.5f);
-            if (pidx(d + 1, 0) <= df) ++d;
-            if (pidx(d, 0) > df) --d;
-            const int f = df - pidx(d, 0);
-            double x = H[s_base[d] + b * s_w[d][0] + f * s_w[d][1] + c * s_w[d][2]];
-            if (d != f) x += H[s_base[f] + b * s_w[f][0] + d * s_w[f][1] + c * s_w[f][2]];
-            X[row * ldx + df] = x;
-        }
-        __syncthreads();
-        if (live) {
+        for (int i = tid; i < nk * n; i += 256) B[i] = Bf[(ll)e * np * n + i];
+        f_gather(r, s, f, e, H, X, ldx);
+        if (grp < groups) {
 #pragma unroll 4
             for (int k = 0; k < nk; ++k) {
                 const double y = B[k * n + col];
@@ -263,11 +287,51 @@ __global__ void __launch_bounds__(256) k_sym_f(Rdm r, int s, int bc, const doubl
         }
         __syncthreads();
     }
-    if (!live) return;
+    if (grp >= groups) return;
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
         const int row = grp + i * groups;
-        if (row < R) F[(((ll)pr * n + ap) * n2 + b0 * n + row) * n + col] = acc[i];
+        if (row < f.R) F[(((ll)f.pr * n + f.ap) * n * n + f.b0 * n + row) * n + col] = acc[i];
+    }
+}
+
+// The operand of F as rows in memory, for the digit product: rows ((cp,bp) from
+// pr0, ap, b, c), K = n (np + 1) columns (e, df) and d, with each row's largest
+// magnitude.  A CTA gathers as above; its warps write whole rows (n = 14: 4.2 ms
+// for 3.4 GB, bound by the gathers).
+__global__ void __launch_bounds__(256) k_sym_x(Rdm r, int s, int bc, int pr0, const double *__restrict__ H,
+                                               double *__restrict__ X, unsigned long long *__restrict__ rmax,
+                                               const int *flag) {
+    if (*flag) return;
+    extern __shared__ double sm[];
+    const int n = r.n, np = n * (n + 1) / 2, ldx = np | 1, K = n * (np + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    FBlock f = f_block(n, bc, blockIdx.x + pr0 * n * ((n + bc - 1) / bc));
+    const ll row0 = ((ll)(f.pr - pr0) * n + f.ap) * n * n + f.b0 * n;
+    double mx[kSymXRows];
+#pragma unroll
+    for (int i = 0; i < kSymXRows; ++i) mx[i] = 0.0;
+    for (int e = 0; e <= n; ++e) {
+        const int nk = e < n ? np : n;
+        f_gather(r, s, f, e, H, sm, ldx);
+#pragma unroll
+        for (int i = 0; i < kSymXRows; ++i) {
+            const int row = warp + 8 * i;
+            if (row >= f.R) break;
+            for (int k = lane; k < nk; k += 32) {
+                const double x = sm[row * ldx + k];
+                mx[i] = fmax(mx[i], fabs(x));
+                X[(row0 + row) * K + e * np + k] = x;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < kSymXRows; ++i) {
+        const int row = warp + 8 * i;
+        if (row >= f.R) break;
+        for (int o = 16; o; o >>= 1) mx[i] = fmax(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], o));
+        if (lane == 0) rmax[row0 + row] = (unsigned long long)__double_as_longlong(mx[i]);
     }
 }
 
@@ -275,39 +339,49 @@ __global__ void __launch_bounds__(256) k_sym_f(Rdm r, int s, int bc, const doubl
 // q, r): Wca and Waa have p' their second creator (s or t) and (q,r) the free
 // pair, Kx and J the pairs (p,q), (p',r).  The rows of Gamma3 are affine in the
 // two summed indices, lo the one with stride M, so the tile loads need no
-// intermediate matrix.  64 x 64 tiles, 4 x 4 per thread; bound by the FP64 pipe.
+// intermediate matrix.  64 x 64 tiles, 4 x 4 per thread; bound by the FP64 pipe
+// (n = 16: 13.8 ms for 1.6e10 flops, 1.14 TFLOP/s).
 constexpr int kN8 = 64, kN8K = 16;
+// Offset of a row of Gamma3 (in units of M) and the stride of its slow summed index.
+__device__ __forceinline__ ll n8_row(int n, int kind, ll row) {
+    const ll n1 = n, n2 = n1 * n, n3 = n2 * n, n4 = n2 * n2, n5 = n4 * n;
+    const int q2 = (int)(row % n), q1 = (int)((row / n) % n);
+    int p, p2;
+    unpair((int)(row / n2), p, p2);
+    if (kind == 0) return n1 * p + n2 * q1 + n3 * p2 + n5 * q2;       // (e,s), (p,f), (q,r)
+    if (kind == 1) return n2 * q2 + n3 * p2 + n4 * p + n5 * q1;       // (e,t), (f,p), (r,q): exchanged
+    if (kind == 2) return n1 * q1 + n2 * q2 + n4 * p + n5 * p2;       // (e,d), (q,p), (r,p'): exchanged
+    return n1 * p + n2 * p2 + n4 * q1 + n5 * q2;                      // (d,f), (p,q), (p',r)
+}
+__device__ __forceinline__ ll n8_hi(int n, int kind) {
+    return kind == 0 ? (ll)n * n * n * n : kind == 1 ? (ll)n : (ll)n * n * n;
+}
+// Gamma2 factor of row ((p >= p'), q, r) of J
+__device__ __forceinline__ double n8_pair2(const Rdm &r, int s, ll row) {
+    const int n = r.n;
+    int p, p2;
+    unpair((int)(row / (n * n)), p, p2);
+    return r.d2[s + (ll)r.M * (p + n * (p2 + n * ((row / n) % n + n * (row % n))))];
+}
 __global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__restrict__ I4,
-                                                const double *__restrict__ IJ, const double *g, double *out,
-                                                const int *flag) {
+                                                const double *__restrict__ IJ, double *out, const int *flag) {
     if (*flag) return;
     __shared__ double As[kN8K][kN8 + 1], Bs[kN8K][kN8];
     const int n = r.n, np = n * (n + 1) / 2, kind = blockIdx.z;
-    const ll M = r.M, n1 = n, n2 = n1 * n, n3 = n2 * n, n4 = n2 * n2, n5 = n4 * n;
-    const ll rows = np * n2;
+    const ll M = r.M, n2 = (ll)n * n, rows = np * n2;
     const int N = kind == 3 ? np : (int)n2;
     const int c0 = blockIdx.y * kN8;
     if (c0 >= N) return;
     const ll r0 = (ll)blockIdx.x * kN8;
     const double *Bm = kind == 3 ? IJ : I4;
     double *C = out + kind * rows * n2;
-    const ll hi = M * (kind == 0 ? n4 : kind == 1 ? n1 : n3);
+    const ll hi = M * n8_hi(n, kind);
     const int tid = threadIdx.x, lk = tid & 15, lr = tid >> 4;
     const double *base[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const ll row = min(r0 + lr + 16 * i, rows - 1);
-        const int q2 = (int)(row % n), q1 = (int)((row / n) % n), pr = (int)(row / n2);
-        int p = (int)((sqrtf(8.0f * pr + 1.0f) - 1.0f) * 0.5f);
-        if (pidx(p + 1, 0) <= pr) ++p;
-        if (pidx(p, 0) > pr) --p;
-        const int p2 = pr - pidx(p, 0);
-        ll o;
-        if (kind == 0) o = n1 * p + n2 * q1 + n3 * p2 + n5 * q2;        // (e,s), (p,f), (q,r)
-        else if (kind == 1) o = n2 * q2 + n3 * p2 + n4 * p + n5 * q1;   // (e,t), (f,p), (r,q): exchanged
-        else if (kind == 2) o = n1 * q1 + n2 * q2 + n4 * p + n5 * p2;   // (e,d), (q,p), (r,p'): exchanged
-        else o = n1 * p + n2 * p2 + n4 * q1 + n5 * q2;                  // (d,f), (p,q), (p',r)
-        base[i] = r.d3 + s + M * o;
+        base[i] = r.d3 + s + M * n8_row(n, kind, row);
     }
     double acc[4][4] = {};
     const int tc = (tid & 15) * 4, tr = (tid >> 4) * 4;
@@ -342,28 +416,30 @@ __global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__re
     for (int i = 0; i < 4; ++i) {
         const ll row = r0 + tr + i;
         if (row >= rows) break;
-        double w = 0.0;  // J += Gamma2[(p,q), (p',r)] g(x,y)
-        if (kind == 3) {
-            const int pr = (int)(row / n2);
-            int p = (int)((sqrtf(8.0f * pr + 1.0f) - 1.0f) * 0.5f);
-            if (pidx(p + 1, 0) <= pr) ++p;
-            if (pidx(p, 0) > pr) --p;
-            w = r.d2[s + M * (p + n1 * (pr - pidx(p, 0)) + n2 * ((row / n) % n) + n3 * (row % n))];
-        }
+        const double w = kind == 3 ? n8_pair2(r, s, row) : 0.0;  // J += Gamma2[(p,q), (p',r)] g(x,y)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int col = c0 + tc + j;
             if (col >= N) break;
             double v = acc[i][j];
-            if (kind == 3) {
-                int x = (int)((sqrtf(8.0f * col + 1.0f) - 1.0f) * 0.5f);
-                if (pidx(x + 1, 0) <= col) ++x;
-                if (pidx(x, 0) > col) --x;
-                v = fma(w, g[x * n + col - pidx(x, 0)], v);
-            }
+            if (kind == 3) v = fma(w, IJ[n2 * np + col], v);
             C[row * N + col] = v;
         }
     }
+}
+
+// The operands of the n^8 contractions as rows in memory, for the digit
+// products: kinds 0-2 [row][n^2], J [row][n^2 + 1] with its Gamma2 factor last.
+__global__ void __launch_bounds__(256) k_sym_rows(Rdm r, int s, double *__restrict__ R, const int *flag) {
+    if (*flag) return;
+    const int n = r.n, kind = blockIdx.y, n2 = n * n, K = kind == 3 ? n2 + 1 : n2;
+    const ll rows = (ll)(n * (n + 1) / 2) * n2;
+    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= rows * K) return;
+    const ll row = t / K;
+    const int k = (int)(t % K);
+    R[kind * rows * n2 + t] = k == n2 ? n8_pair2(r, s, row)
+                                      : r.d3[s + (ll)r.M * (n8_row(n, kind, row) + (k / n) * n8_hi(n, kind) + k % n)];
 }
 
 // Accessors of the intermediates (0-based labels).
@@ -438,7 +514,8 @@ __global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double 
 // n^8 tensors (whose last indices are a, c or b) use whole sectors.  The sums
 // over one index (Gamma2 with the integrals: the FP64 work, 6 n FMAs per
 // element) keep ap in registers, so that five of their six factors are loaded
-// once for all of them.
+// once for all of them.  n = 16: 5.8 ms (one element per thread, ap across the
+// warp: 24.7 ms).
 constexpr int kOutAp = 4;
 __global__ void __launch_bounds__(256) k_sym_out(SymView v, double *amat, double *atmat, const int *flag) {
     if (*flag) return;
@@ -538,7 +615,7 @@ FShape f_shape(int n) {
     return best;
 }
 
-using FKernel = void (*)(Rdm, int, int, const double *, const double *, const double *, double *, const int *);
+using FKernel = void (*)(Rdm, int, int, const double *, const double *, double *, const int *);
 FKernel f_kernel(int rpt) {
     switch (rpt) {
         case 1: return k_sym_f<1>;
@@ -555,7 +632,7 @@ FKernel f_kernel(int rpt) {
 ll SymScratch::doubles(int n) {
     const ll n2 = (ll)n * n, n4 = n2 * n2, np = n * (n + 1) / 2;
     const ll W = (ll)n * (n + 1) * (n + 2) * (n + 3) / 24;
-    return W * n4 + 4 * np * n4 + np * np * n2 + 8 * n4 + 2 * np * n2 + n2 + W / 2 + 1;
+    return W * n4 + 4 * np * n4 + np * np * n2 + 8 * n4 + 2 * np * n2 + np + 2 * n2 + W / 2 + 1;
 }
 
 SymScratch::SymScratch(int n, double *w) {
@@ -570,9 +647,9 @@ SymScratch::SymScratch(int n, double *w) {
     F = take(np * n4);
     N8 = take(3 * np * n4 + np * np * n2);
     for (double **p : {&G1, &G3, &Q1, &JW, &J2, &Z}) *p = take(n4);
-    Bf = take(np * n2);
+    Bf = take((np + 1) * n2);
     I4 = take(n4);
-    IJ = take(n2 * np);
+    IJ = take((n2 + 1) * np);
     Lb = take(n4);
     g = take(n2);
     key = (int *)take(W / 2 + 1);
@@ -585,29 +662,97 @@ void launch_sym_ops(const double *atwo, const double *f, int ncore, int n, const
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
+namespace {
+void sym_finish(const SymView &v, const SymScratch &S, double *amat, double *atmat, const int *fl, cudaStream_t st) {
+    const ll n = v.n, n4 = n * n * n * n;
+    k_sym_small<<<(unsigned)((n4 + 63) / 64), 64, 0, st>>>(v, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, fl);
+    const dim3 go((unsigned)((n4 * n + 255) / 256), (unsigned)((n + kOutAp - 1) / kOutAp));
+    k_sym_out<<<go, 256, 0, st>>>(v, amat, atmat, fl);
+    g_launches.fetch_add(2, std::memory_order_relaxed);
+}
+void sym_unpack(const Rdm &r, int s, const SymScratch &S, int *flag, cudaStream_t st) {
+    const ll n = r.n, n4 = n * n * n * n;
+    const ll ub = ((r.W + 31) / 32) * ((n4 + 31) / 32), cb = (n4 * n * n + 255) / 256;
+    k_sym_unpack<<<(unsigned)(ub + cb), 256, 0, st>>>(r, s, S.key, (unsigned)ub, S.H, flag);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+}
+SymView sym_view(const Rdm &r, int s, const double *atwo, const SymScratch &S) {
+    const ll n2 = (ll)r.n * r.n;
+    return SymView{r, s, r.n, n2, r.n * (r.n + 1) / 2 * n2, S.F, S.N8, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, atwo, S.Lb, S.g};
+}
+}  // namespace
+
 int launch_sym_state(const Rdm &r, int s, const double *atwo, const SymScratch &S, double *amat, double *atmat,
                      int *flag, cudaStream_t st) {
-    const int n = r.n, np = n * (n + 1) / 2;
-    const ll n2 = (ll)n * n, n4 = n2 * n2, n6 = n4 * n2, rows = np * n2;
-    const ll ub = ((r.W + 31) / 32) * ((n4 + 31) / 32), cb = (n6 + 255) / 256;
-    k_sym_unpack<<<(unsigned)(ub + cb), 256, 0, st>>>(r, s, S.key, (unsigned)ub, S.H, flag);
-    const int *fl = flag + s;
+    const int n = r.n, np = n * (n + 1) / 2, *fl = flag + s;
+    const ll n2 = (ll)n * n, rows = np * n2;
+    sym_unpack(r, s, S, flag, st);
     const dim3 g8((unsigned)((rows + kN8 - 1) / kN8), (unsigned)((n2 + kN8 - 1) / kN8), 4);
-    k_sym_n8<<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.g, S.N8, fl);
+    k_sym_n8<<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
     const FShape fs = f_shape(n);
     const FKernel fk = f_kernel(fs.rpt);
     const int smem = (fs.bc * n * (np | 1) + np * n) * (int)sizeof(double);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute((const void *)fk, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
         return 1;
-    fk<<<(unsigned)(np * n * ((n + fs.bc - 1) / fs.bc)), 256, smem, st>>>(r, s, fs.bc, S.H, S.Bf, S.g,
-                                                                                       S.F, fl);
-    SymView v{r, s, n, n2, rows, S.F, S.N8, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, atwo, S.Lb, S.g};
-    k_sym_small<<<(unsigned)((n4 + 63) / 64), 64, 0, st>>>(v, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, fl);
-    const dim3 go((unsigned)((n4 * n + 255) / 256), (unsigned)((n + kOutAp - 1) / kOutAp));
-    k_sym_out<<<go, 256, 0, st>>>(v, amat, atmat, fl);
-    g_launches.fetch_add(5, std::memory_order_relaxed);
+    fk<<<(unsigned)(np * n * ((n + fs.bc - 1) / fs.bc)), 256, smem, st>>>(r, s, fs.bc, S.H, S.Bf, S.F, fl);
+    g_launches.fetch_add(2, std::memory_order_relaxed);
+    sym_finish(sym_view(r, s, atwo, S), S, amat, atmat, fl, st);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
+}
+
+int launch_sym_state_split(const Rdm &r, int s, const double *atwo, const SymScratch &S, double *rows_buf,
+                           void *oz_work, int *oz_err, double *amat, double *atmat, int *flag, cudaStream_t st) {
+    const int n = r.n, np = n * (n + 1) / 2, *fl = flag + s;
+    const ll n2 = (ll)n * n, n3 = n2 * n, rows = np * n2;
+    const oz::Gate gate{fl, false};
+    sym_unpack(r, s, S, flag, st);
+    // F: the operand rows of some creator pairs at a time, then their digit product
+    const int bc = std::max(1, kSymXRows * 8 / n), K = n * (np + 1), prs = sym_split_pairs(n);
+    const int smem = bc * n * (np | 1) * (int)sizeof(double);
+    if (smem > 48 * 1024 && cudaFuncSetAttribute((const void *)k_sym_x, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 100 * 1024) != cudaSuccess)
+        return 1;
+    for (int p0 = 0; p0 < np; p0 += prs) {
+        const int p = std::min(prs, np - p0);
+        unsigned long long *rmax = (unsigned long long *)(rows_buf + p * n3 * K);
+        k_sym_x<<<(unsigned)(p * n * ((n + bc - 1) / bc)), 256, smem, st>>>(r, s, bc, p0, S.H, rows_buf, rmax, fl);
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        const double *X[1] = {rows_buf}, *B[1] = {S.Bf};
+        double *F[1] = {S.F + p0 * n3 * n};
+        const unsigned long long *rm[1] = {rmax};
+        if (oz::oz_gemm_skinny(oz::OzPlan(1, p * n3, K, n), X, B, F, n, n, oz_work, st, rm, gate, oz_err)) return 1;
+    }
+    // the n^8 tensors: Wca, Waa and Kx share their right-hand operand
+    const dim3 gr((unsigned)((rows * (n2 + 1) + 255) / 256), 4);
+    k_sym_rows<<<gr, 256, 0, st>>>(r, s, rows_buf, fl);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    oz::WideGemm g;
+    g.m = 3 * rows; g.n = n2; g.K = (int)n2;
+    g.A = rows_buf; g.a_r = n2; g.a_k = 1;
+    g.B = S.I4; g.b_c = 1; g.b_k = n2;
+    g.C = S.N8; g.ldc = n2;
+    if (oz::oz_gemm_wide(g, oz_work, oz_err, st)) return 1;
+    g.m = rows; g.n = np; g.K = (int)n2 + 1;
+    g.A = rows_buf + 3 * rows * n2; g.a_r = n2 + 1;
+    g.B = S.IJ; g.b_k = np;
+    g.C = S.N8 + 3 * rows * n2; g.ldc = np;
+    if (oz::oz_gemm_wide(g, oz_work, oz_err, st)) return 1;
+    sym_finish(sym_view(r, s, atwo, S), S, amat, atmat, fl, st);
+    return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
+}
+
+int sym_split_pairs(int n) { return std::max(1, std::min(n * (n + 1) / 2, 65536 / (n * n * n))); }
+
+ll sym_split_rows_doubles(int n) {
+    const ll n2 = (ll)n * n, np = n * (n + 1) / 2, xr = sym_split_pairs(n) * n2 * n;
+    return std::max(xr * (n * (np + 1) + 1), np * n2 * (4 * n2 + 1));
+}
+
+size_t sym_split_oz_bytes(int n) {
+    const ll n2 = (ll)n * n, np = n * (n + 1) / 2;
+    return std::max({oz::OzPlan(1, sym_split_pairs(n) * n2 * n, n * (int)(np + 1), n).bytes(),
+                     oz::oz_wide_bytes(3 * np * n2, n2, (int)n2), oz::oz_wide_bytes(np * n2, np, (int)n2 + 1)});
 }
 
 }  // namespace nvpt

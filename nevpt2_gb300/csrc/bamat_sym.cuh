@@ -1,6 +1,8 @@
 // The A-matrices from one n^9 contraction (bamat_sym.cu): scratch layout and
 // launchers.
 #pragma once
+#include <cstddef>
+
 #include "nvpt2_internal.h"
 
 namespace nvpt {
@@ -25,5 +27,15 @@ void launch_sym_ops(const double *atwo, const double *f, int ncore, int n, const
 // A-matrices.  0, or 1 on a launch failure.
 int launch_sym_state(const Rdm &r, int s, const double *atwo, const SymScratch &S, double *amat, double *atmat,
                      int *flag, cudaStream_t st);
+
+// The same with the n^9 and n^8 contractions as digit products on the tensor
+// cores: rows_buf holds sym_split_rows_doubles(n) doubles (operand rows, of
+// sym_split_pairs(n) creator pairs at a time for F), oz_work
+// sym_split_oz_bytes(n) bytes; a wait that timed out sets *oz_err.
+int launch_sym_state_split(const Rdm &r, int s, const double *atwo, const SymScratch &S, double *rows_buf,
+                           void *oz_work, int *oz_err, double *amat, double *atmat, int *flag, cudaStream_t st);
+int sym_split_pairs(int n);
+ll sym_split_rows_doubles(int n);
+size_t sym_split_oz_bytes(int n);
 
 }  // namespace nvpt

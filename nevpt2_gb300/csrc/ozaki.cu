@@ -102,7 +102,8 @@ __device__ __forceinline__ void issue_pass(uint64_t dA, uint64_t dB, uint32_t tm
 // integers, so the order over K does not change the result.
 __device__ __forceinline__ int kc_start(long long tile, int nkc) { return (int)((tile * 13) % nkc); }
 
-__global__ void __launch_bounds__(THREADS, 1) k_oz_gemm(OzBatch b, int *err) {
+__global__ void __launch_bounds__(THREADS, 1) k_oz_gemm(OzBatch b, int *err, Gate gate) {
+    if (gate.closed()) return;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_tfull, bar_tempty, bar_done;
     __shared__ uint32_t s_tmem;
@@ -319,8 +320,20 @@ __device__ __forceinline__ void digits(double x, int E, uint16_t (&d)[NSL]) {
 // the 8 warps take every 8th group of four K octets; each lane stores the
 // 16-byte chunk (8 digits) of one row and octet per slice.  nrt * 128 rows
 // are written (zeros past `rows`).
-__global__ void __launch_bounds__(256) k_oz_split_rows(const double *X, long long rows, int K, int nkc, int nrt,
-                                                       uint8_t *ad, int *rexp, const unsigned long long *rmax) {
+// blockIdx.y is the product.
+struct SplitSrc {
+    const double *X[4], *A[4];
+    const unsigned long long *rmax[4];
+};
+__global__ void __launch_bounds__(256) k_oz_split_rows(SplitSrc src, OzBatch b, int K, Gate gate) {
+    if (gate.closed()) return;
+    const OzJob &J = b.job[blockIdx.y];
+    const double *__restrict__ X = src.X[blockIdx.y];
+    const unsigned long long *rmax = src.rmax[blockIdx.y];
+    const long long rows = J.rows;
+    const int nkc = b.nkc, nrt = J.nrt;
+    uint8_t *ad = const_cast<uint8_t *>(J.ad);
+    int *rexp = const_cast<int *>(J.rexp);
     __shared__ double smax[8][8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rr = lane & 7, ph = lane >> 3;
     const long long row = (long long)blockIdx.x * 8 + rr;
@@ -367,12 +380,19 @@ __global__ void __launch_bounds__(256) k_oz_split_rows(const double *X, long lon
     }
 }
 
-// Columns of A ([K, ncols] row-major, ld = lda) -> digit tiles (one block).
-__global__ void __launch_bounds__(256) k_oz_split_cols(const double *A, int K, int ncols, int lda, int nkc,
-                                                       uint8_t *bd, int *cexp) {
+// Columns of A ([K, ncols] row-major, ld = lda) -> digit tiles, one block per
+// K chunk.  Every block takes the column maxima over all of A itself (K x 16
+// doubles from L2, 0.5 MB at most): one block doing everything took 160 us at
+// K = 2744, a serial tail before every product.
+__global__ void __launch_bounds__(256) k_oz_split_cols(SplitSrc src, OzBatch b, int K, int lda, Gate gate) {
+    if (gate.closed()) return;
+    const double *__restrict__ A = src.A[blockIdx.y];
+    uint8_t *bd = const_cast<uint8_t *>(b.job[blockIdx.y].bd);
+    int *cexp = const_cast<int *>(b.job[blockIdx.y].cexp);
+    const int ncols = b.ncols;
     __shared__ double smax[256];
     __shared__ int sE[NB];
-    const int tid = threadIdx.x, c = tid % NB;
+    const int tid = threadIdx.x, c = tid % NB, kc = blockIdx.x;
     double mx = 0.0;
     if (c < ncols)
         for (int k = tid / NB; k < K; k += 256 / NB) mx = fmax(mx, fabs(A[(long long)k * lda + c]));
@@ -382,19 +402,17 @@ __global__ void __launch_bounds__(256) k_oz_split_cols(const double *A, int K, i
         double m = 0.0;
         for (int i = tid; i < 256; i += NB) m = fmax(m, smax[i]);
         sE[tid] = exp_above(m);
-        cexp[tid] = sE[tid];
+        if (kc == 0) cexp[tid] = sE[tid];
     }
     __syncthreads();
-    for (long long i = tid; i < (long long)nkc * KC * NB; i += 256) {
-        const int k = (int)(i / NB), col = (int)(i % NB);
+    for (int i = tid; i < KC * NB; i += 256) {
+        const int kl = i / NB, k = kc * KC + kl, col = i % NB;
         const double x = (col < ncols && k < K) ? A[(long long)k * lda + col] : 0.0;
         uint16_t d[NSL];
         digits(x, sE[col], d);
-        const int kc = k / KC;
-        for (int q = 0; q < NSL; ++q) {
-            const int row = q * NB + col;
-            *(uint16_t *)(bd + (size_t)kc * B_STAGE + sw128_off(row, k % KC)) = d[q];
-        }
+#pragma unroll
+        for (int q = 0; q < NSL; ++q)
+            *(uint16_t *)(bd + (size_t)kc * B_STAGE + sw128_off(q * NB + col, kl)) = d[q];
     }
 }
 
@@ -406,7 +424,7 @@ size_t OzPlan::bytes() const {
 }
 
 int oz_gemm_skinny(const OzPlan &pl, const double *const *X, const double *const *A, double *const *T, int lda,
-                   int ldt, void *work, cudaStream_t st, const unsigned long long *const *rowmax) {
+                   int ldt, void *work, cudaStream_t st, const unsigned long long *const *rowmax, Gate gate, int *err) {
     if (pl.njob < 1 || pl.njob > 4 || pl.K < 1 || pl.K > kMaxK || pl.ncols < 1 || pl.ncols > NB) return 1;
     static bool attr_set = false;
     if (!attr_set) {
@@ -415,14 +433,17 @@ int oz_gemm_skinny(const OzPlan &pl, const double *const *X, const double *const
         attr_set = true;
     }
     uint8_t *w = (uint8_t *)work;
-    int *err = (int *)w;
+    if (!err) {
+        err = (int *)w;
+        cudaMemsetAsync(err, 0, sizeof(int), st);
+    }
     w += 256;
+    SplitSrc src{};
     OzBatch b{};
     b.njob = pl.njob;
     b.nkc = pl.nkc;
     b.ncols = pl.ncols;
     b.ldo = ldt;
-    cudaMemsetAsync(err, 0, sizeof(int), st);
     for (int j = 0; j < pl.njob; ++j) {
         uint8_t *ad = w;
         w += (size_t)pl.nrt * pl.nkc * A_ROW;
@@ -432,12 +453,14 @@ int oz_gemm_skinny(const OzPlan &pl, const double *const *X, const double *const
         w += (size_t)pl.nkc * B_STAGE;
         int *cexp = (int *)w;
         w += 256;
-        k_oz_split_rows<<<(unsigned)((long long)pl.nrt * BM / 8), 256, 0, st>>>(X[j], pl.rows, pl.K, pl.nkc, pl.nrt,
-                                                                              ad, rexp, rowmax ? rowmax[j] : nullptr);
-        k_oz_split_cols<<<1, 256, 0, st>>>(A[j], pl.K, pl.ncols, lda, pl.nkc, bd, cexp);
-        g_launches.fetch_add(2, std::memory_order_relaxed);
+        src.X[j] = X[j];
+        src.A[j] = A[j];
+        src.rmax[j] = rowmax ? rowmax[j] : nullptr;
         b.job[j] = OzJob{ad, rexp, bd, cexp, T[j], pl.rows, pl.nrt};
     }
+    k_oz_split_rows<<<dim3((unsigned)((long long)pl.nrt * BM / 8), pl.njob), 256, 0, st>>>(src, b, pl.K, gate);
+    k_oz_split_cols<<<dim3(pl.nkc, pl.njob), 256, 0, st>>>(src, b, pl.K, lda, gate);
+    g_launches.fetch_add(2, std::memory_order_relaxed);
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -447,8 +470,8 @@ int oz_gemm_skinny(const OzPlan &pl, const double *const *X, const double *const
     const long long abytes = (long long)pl.njob * ((long long)pl.nrt * pl.nkc * A_ROW + (long long)pl.nkc * B_STAGE +
                                                    pl.rows * pl.ncols * (long long)sizeof(double));
     ProfSpan span;
-    span.begin("oz_gemm", st, abytes);
-    k_oz_gemm<<<grid, THREADS, SMEM_BYTES, st>>>(b, err);
+    if (!gate.flag || !gate.run) span.begin("oz_gemm", st, abytes);
+    k_oz_gemm<<<grid, THREADS, SMEM_BYTES, st>>>(b, err, gate);
     span.end();
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;

@@ -64,14 +64,25 @@ struct OzPlan {
     size_t bytes() const;  // device workspace
 };
 
+// A launch that a device flag decides on: null runs always, otherwise the
+// kernels return at once unless (*flag != 0) == run.
+struct Gate {
+    const int *flag = nullptr;
+    bool run = true;
+    __device__ __forceinline__ bool closed() const { return flag && (*flag != 0) != run; }
+};
+
 // Enqueue digit splits + the tensor-core product on `st`.  work: bytes()
 // of device memory (16-byte aligned).  0 on success; nonzero for bad shapes
-// or launch failure.  The kernel's own error flag (a wait that timed out) is
-// read back by oz_check_error (synchronises `st`; 0 = fine, 4 = timeout).
+// or launch failure.  A wait that timed out sets *err (device memory, zeroed by
+// the caller; null: the first word of work, zeroed by each call), which
+// oz_check_error reads back (synchronises `st`; 0 = fine, 4 = timeout).
 // rowmax (optional): per product, max_k |X[i,k]| of every row as the bit
-// pattern of the double (the split then skips its own pass over X).
+// pattern of the double (the split then skips its own pass over X).  Launches
+// behind a gate that waits for a raised flag are not profiled.
 int oz_gemm_skinny(const OzPlan &pl, const double *const *X, const double *const *A, double *const *T, int lda,
-                   int ldt, void *work, cudaStream_t st, const unsigned long long *const *rowmax = nullptr);
+                   int ldt, void *work, cudaStream_t st, const unsigned long long *const *rowmax = nullptr,
+                   Gate gate = Gate(), int *err = nullptr);
 int oz_check_error(const void *work, cudaStream_t st);
 
 // General products (ozaki_wide.cu): C[m, n] (row-major, ldc) =

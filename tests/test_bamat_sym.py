@@ -131,3 +131,19 @@ def test_inputs_without_a_symmetry_take_the_general_route(gpu_ctx, n, ne, what):
             keep = np.isfinite(ref[s])
             if keep.any():
                 assert abs(got[s][keep] - ref[s][keep]).max() < 1e-10 * abs(ref[s][keep]).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [6, 10, 11, 12])
+def test_split_route_matches_fp64(gpu_ctx, n):
+    """Both sides of the size from which split mode takes the digit products, the second state without the
+    symmetry of its 4-RDM.  Digit products keep 2^-59 of the row and column maxima: 1e-12 of the largest element."""
+    from nevpt2_gb300 import koopro
+    p, atwo, aj = _inputs(n, 6, 2, 90 + n, ndet=200)
+    p.ro4[10, 0, 1, 2, 0, 1] += 1e-3 * abs(p.ro4).max()
+    ref = _gpu(p, atwo, aj)
+    with koopro.precision(koopro.SPLIT):
+        got = _gpu(p, atwo, aj)
+    for g, r in zip(got, ref):
+        for s in range(2):
+            assert rel_err(g[s], r[s]) < 1e-12

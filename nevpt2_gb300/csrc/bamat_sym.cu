@@ -38,21 +38,12 @@
 
 #include "bamat_sym.cuh"
 #include "ozaki.cuh"
+#include "sym_check.cuh"
 
 namespace nvpt {
 namespace {
 
-constexpr double kSymTol = 0x1p-45;
 constexpr int kSymXRows = 4;  // rows per warp of k_sym_x
-
-__host__ __device__ __forceinline__ int pidx(int i, int j) { return i * (i + 1) / 2 + j; }  // i >= j
-__device__ __forceinline__ int pmx(int i, int j) { return i > j ? pidx(i, j) : pidx(j, i); }
-__device__ __forceinline__ void unpair(int p, int &i, int &j) {  // p = pidx(i, j)
-    i = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
-    if (pidx(i + 1, 0) <= p) ++i;
-    if (pidx(i, 0) > p) --i;
-    j = p - pidx(i, 0);
-}
 
 // Packed rank (0-based) of a descending quadruple of 0-based indices.
 __device__ __forceinline__ int rank4(const int v[4]) { return lindice4(v[0] + 1, v[1] + 1, v[2] + 1, v[3] + 1) - 1; }
@@ -79,10 +70,8 @@ __global__ void __launch_bounds__(256) k_sym_ops(const double *atwo, const doubl
     const ll n2 = (ll)n * n, n4 = n2 * n2;
     if (t >= n4) return;
     const int l = (int)(t % n), k = (int)((t / n) % n), j = (int)((t / n2) % n), i = (int)(t / (n2 * n));
-    double scale = 0.0;
-    for (int q = 0; q < n; ++q) scale = fmax(scale, fabs(AT(q, q, q, q)));
-    const double v = AT(i, j, k, l), tol = kSymTol * scale;
-    if (!(fabs(v - AT(j, i, k, l)) <= tol) || !(fabs(v - AT(k, l, i, j)) <= tol))
+    const double v = AT(i, j, k, l);
+    if (integral_asymmetric(atwo, n, i, j, k, l))
         for (int s = 0; s < M; ++s) flag[s] = 1;
     const int np = n * (n + 1) / 2;
     if (i >= j && j >= k && k >= l) {
@@ -103,18 +92,6 @@ __global__ void __launch_bounds__(256) k_sym_ops(const double *atwo, const doubl
     }
 }
 
-// Largest |Gamma1| of the state: the scale of its symmetry checks.
-__device__ double rdm_scale(const Rdm &r, int s) {
-    __shared__ double red[8];
-    double m = 0.0;
-    for (int i = threadIdx.x; i < r.n * r.n; i += blockDim.x) m = fmax(m, fabs(r.d1[s + (ll)r.M * i]));
-    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    __syncthreads();
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-    return m;
-}
-
 // H[K][l1 + n l2 + n^2 l3 + n^3 l4] = Gamma4 with creators the key K and any
 // annihilators: the transpose of the packed 4-RDM, completed over the
 // annihilators of higher rank than K (where the packed form keeps the
@@ -122,33 +99,16 @@ __device__ double rdm_scale(const Rdm &r, int s) {
 // blocks from nub on check Gamma1..3.  Bound by HBM (16 W n^4 bytes) and by the
 // gathers of the completed half; n = 16: 3.9 ms.
 __global__ void __launch_bounds__(256) k_sym_unpack(Rdm r, int s, const int *key, unsigned nub, double *H, int *flag) {
-    const int n = r.n, M = r.M;
+    const int n = r.n;
     const ll n2 = (ll)n * n, n3 = n2 * n, n4 = n2 * n2, W = r.W;
-    const double tol = kSymTol * rdm_scale(r, s);
-    auto differ = [tol](double x, double y) { return !(fabs(x - y) <= tol); };
-    bool bad = false;
+    const double tol = rdm_tolerance(r, s);
     if (blockIdx.x >= nub) {
         const ll t = (ll)(blockIdx.x - nub) * blockDim.x + threadIdx.x;
-        if (t < n3 * n3) {
-            ll x = t;
-            int q[6];
-            for (int i = 0; i < 6; ++i) { q[i] = (int)(x % n); x /= n; }
-            auto d3 = [&](int a, int b, int c, int d, int e, int f) {
-                return r.d3[s + (ll)M * (a + n * (b + n * (c + (ll)n * (d + n * (e + (ll)n * f)))))];
-            };
-            const double v = r.d3[s + (ll)M * t];
-            bad = differ(v, d3(q[1], q[0], q[2], q[4], q[3], q[5])) || differ(v, d3(q[0], q[2], q[1], q[3], q[5], q[4])) ||
-                  differ(v, d3(q[3], q[4], q[5], q[0], q[1], q[2]));
-            if (t < n4) {
-                auto d2 = [&](int a, int b, int c, int d) { return r.d2[s + (ll)M * (a + n * (b + n * (c + (ll)n * d)))]; };
-                const double w = r.d2[s + (ll)M * t];
-                bad = bad || differ(w, d2(q[1], q[0], q[3], q[2])) || differ(w, d2(q[2], q[3], q[0], q[1]));
-            }
-            if (t < n2) bad = bad || differ(r.d1[s + (ll)M * t], r.d1[s + (ll)M * (q[1] + n * q[0])]);
-        }
-        if (bad) flag[s] = 1;
+        if (t < n3 * n3 && rdm_asymmetric(r, s, t, tol)) flag[s] = 1;
         return;
     }
+    bool bad = false;
+    auto differ = [tol](double x, double y) { return sym_differ(x, y, tol); };
     __shared__ double tile[32][33];
     const double *ro4 = r.ro4 + W * n4 * s;
     const unsigned kb = (unsigned)((W + 31) / 32);

@@ -579,15 +579,11 @@ int nvpt_koop_matrices_ctl_d(nvpt_context *ctx, int64_t metat, int64_t nact, int
     cudaStream_t st = pick(ctx, stream);
     Rdm r = make_rdm(nact, metat, dal, taa, daaa, nullptr);
     int n = (int)nact, nc = (int)ncore;
-    launch_build_f(f, aj, atwo, n, nc, 0, st);
-    launch_koopE(r, atwo, f, nc, ipko1, eako1, st);
-    launch_hrdm(r, hrdm2, st);
-    launch_build_f(f, aj, atwo, n, nc, 1, st);
-    launch_koop2E(r, atwo, f, nc, ipko2, eako2, st);
+    double *const out[8] = {ipko1, eako1, hrdm2, ipko2, eako2, gk0pa, gk0pd, gk0pf};
+    launch_koop_ctl(r, atwo, aj, nc, f, out, st);
     // koop2E's its() screen with the context's symmetry tables (none: C1)
     if (ctx->ijkl.ni4 >= 0 && ctx->ijkl.nsym > 1 && ctx->ijkl.norb >= ncore + nact)
         launch_sym_screen(ipko2, eako2, (int)metat, n, 4, ctx->ijkl.itsym() + ncore, st);
-    launch_koop0p(r, atwo, f, nc, gk0pa, gk0pd, gk0pf, st);
     return after_launch(ctx, "koop_matrices_ctl");
 }
 
@@ -793,8 +789,7 @@ int nvpt_bbmat_d(nvpt_context *ctx, const double *atwo, double *bmat, double *bt
     NV_TRY(check_nact(ctx, nact, metat));
     cudaStream_t st = pick(ctx, stream);
     Rdm r = make_rdm(nact, metat, dal, taa, daaa, nullptr);
-    launch_build_f(f, aj, atwo, (int)nact, (int)ncore, 2, st);
-    launch_bbmat(r, atwo, f, aj, (int)ncore, bmat, btmat, st);
+    launch_bbmat(r, atwo, aj, (int)ncore, f, bmat, btmat, st);
     return after_launch(ctx, "bbmat");
 }
 
@@ -804,8 +799,7 @@ int nvpt_bcmat_d(nvpt_context *ctx, const double *atwo, double *cmat, double *ct
     NV_TRY(check_nact(ctx, nact, metat));
     cudaStream_t st = pick(ctx, stream);
     Rdm r = make_rdm(nact, metat, dal, taa, daaa, nullptr);
-    launch_build_f(f, aj, atwo, (int)nact, (int)ncore, 1, st);
-    launch_bcmat(r, atwo, f, (int)ncore, cmat, ctmat, st);
+    launch_bcmat(r, atwo, aj, (int)ncore, f, cmat, ctmat, st);
     return after_launch(ctx, "bcmat");
 }
 
@@ -815,8 +809,7 @@ int nvpt_bdmat_d(nvpt_context *ctx, const double *atwo, double *dmat, double *dt
     NV_TRY(check_nact(ctx, nact, metat));
     cudaStream_t st = pick(ctx, stream);
     Rdm r = make_rdm(nact, metat, dal, taa, nullptr, nullptr);
-    launch_build_f(f, aj, atwo, (int)nact, (int)ncore, 2, st);
-    launch_bdmat(r, atwo, f, aj, (int)ncore, dmat, dtmat, st);
+    launch_bdmat(r, atwo, aj, (int)ncore, f, dmat, dtmat, st);
     return after_launch(ctx, "bdmat");
 }
 

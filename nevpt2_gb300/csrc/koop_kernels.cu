@@ -1,17 +1,13 @@
 // Stage-1 kernels: partial traces of the packed 4-RDM, active integrals and
 // the generalised Koopmans matrices, FP64.
 //
-// One thread owns one output element and performs the reference's reduction
-// for it in the reference's summation order, so no atomics are needed and
-// results are deterministic.  The reference loop nests each kernel restates
-// are cited on the kernel.  The n^9 A-matrix builder has its own file
-// (bamat.cu); this file holds the n^5..n^7 work.
+// No atomics: results are deterministic.  The reference loop nests each kernel
+// restates are cited on the kernel.  The n^9 A-matrix builder has its own files
+// (bamat*.cu); this file holds the n^5..n^7 work.
+#include "koop_sym.cuh"
 #include "nvpt2_internal.h"
 
-#include <cublas_v2.h>
-
 #include <algorithm>
-#include <vector>
 
 namespace nvpt {
 
@@ -60,12 +56,20 @@ __global__ void k_build_f(double *f, const double *aj, const double *atwo, int n
 // transpose-add.  Summation order per element: the case-A terms in l order,
 // then the others in l order (the reference adds all in l order).
 constexpr int kBro3States = 8;  // states per pass of the first kernel
-__global__ void __launch_bounds__(256) k_bro3_case_a(Rdm r, const int *col_order, int s0, int ns, double *P,
-                                                     double *Q) {
+__global__ void __launch_bounds__(256) k_bro3_case_a(Rdm r, int s0, int ns, double *P, double *Q) {
     const int n = r.n, M = r.M;
     const ll n3 = (ll)n * n * n;
-    const int c = col_order[blockIdx.x];
-    const int ii = c % n + 1, jj = (c / n) % n + 1, kk = c / (n * n) + 1;
+    // block = 6 multiset + permutation; a permutation equal to an earlier one has nothing to do
+    int m = blockIdx.x / 6, v[3] = {0, 0, 0};
+    while ((v[2] + 1) * (v[2] + 2) * (v[2] + 3) / 6 <= m) ++v[2];
+    m -= v[2] * (v[2] + 1) * (v[2] + 2) / 6;
+    while ((v[1] + 1) * (v[1] + 2) / 2 <= m) ++v[1];
+    v[0] = m - v[1] * (v[1] + 1) / 2;  // v[0] <= v[1] <= v[2]
+    const int pm = blockIdx.x % 6;
+    const unsigned distinct = v[0] == v[1] ? (v[1] == v[2] ? 0x01 : 0x13) : (v[1] == v[2] ? 0x0d : 0x3f);
+    if (!(distinct >> pm & 1)) return;
+    const int i0 = pm >> 1, ii = v[i0] + 1, jj = v[(i0 + 1 + (pm & 1)) % 3] + 1, kk = v[(i0 + 2 - (pm & 1)) % 3] + 1;
+    const int c = ii - 1 + n * (jj - 1 + n * (kk - 1));
     __shared__ int s_n2[16];  // normind(ii,jj,kk,l) per l
     if (threadIdx.x < n) s_n2[threadIdx.x] = normind4(ii, jj, kk, threadIdx.x + 1);
     __syncthreads();
@@ -169,259 +173,83 @@ __global__ void k_bro1(Rdm r, double *dal, double inv) {
 // ---------------------------------------------------------------------------
 // src/koopro4QD.F90:3900-3971 get_aj_atwo with the Cholesky integrals of
 // src/ijkl_utils.F90:637-688: (ij|kl) = sum_Q L(Q,indice(i,j)) L(Q,indice(k,l)).
-__device__ __forceinline__ double chol_ai(const double *L, int Q, int i, int j, int k, int l) {
-    const double *x = L + (ll)Q * (tri_index(i, j) - 1);
-    const double *y = L + (ll)Q * (tri_index(k, l) - 1);
-    double s = 0.0;
-    for (int q = 0; q < Q; ++q) s += x[q] * y[q];
-    return s;
-}
-
-__global__ void k_atwo(const double *L, int Q, int n, int ncore, double *atwo) {
-    ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    int x[4];
-    decode(t, n, 4, x);
-    atwo[t] = chol_ai(L, Q, x[0] + ncore, x[1] + ncore, x[2] + ncore, x[3] + ncore);
-}
-
-// aj(active upper triangle) = oneint + sum_{j<=ncore} [2(ab|jj) - (aj|jb)]; the
-// rest of aj is a copy of oneint (made by the caller).
-__global__ void k_aj(const double *oneint, const double *L, int Q, int n, int ncore, double *aj) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * n) return;
-    int a = t % n + 1, b = t / n + 1;
-    if (b < a) return;
-    int ac = a + ncore, bc = b + ncore;
-    ll jab = tri_index(ac, bc) - 1;
-    double v = oneint[jab];
-    for (int j = 1; j <= ncore; ++j) v = v + 2.0 * chol_ai(L, Q, ac, bc, j, j) - chol_ai(L, Q, ac, j, j, bc);
-    aj[jab] = v;
+//
+// Columns L(.,pair) are contiguous and a CTA owns one active pair, a warp a dot
+// product: blocks [0, np): atwo for the pairs up to its own, written to the
+// eight equal positions; [np, 2 np): aj = oneint + sum_j [2 (ab|jj) - (aj|jb)];
+// the rest copy oneint to the other elements of aj.
+__global__ void __launch_bounds__(256) k_aj_atwo(const double *__restrict__ oneint, const double *__restrict__ L, int Q,
+                                                 int n, int ncore, ll npair, double *atwo, double *aj) {
+    __shared__ double red[8];
+    const int np = n * (n + 1) / 2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int pr = blockIdx.x;
+    if (pr >= 2 * np) {
+        for (ll i = (ll)(pr - 2 * np) * 256 + threadIdx.x; i < npair; i += (ll)(gridDim.x - 2 * np) * 256) {
+            // row of the triangle holding i: the active block is rows and columns ncore + 1 .. ncore + n
+            ll row = (ll)((sqrt(8.0 * (double)i + 1.0) - 1.0) * 0.5);
+            while ((row + 1) * (row + 2) / 2 <= i) ++row;
+            while (row * (row + 1) / 2 > i) --row;
+            const ll c = i - row * (row + 1) / 2;
+            if (!(row >= ncore && row < ncore + n && c >= ncore)) aj[i] = oneint[i];
+        }
+        return;
+    }
+    const bool one = pr >= np;
+    if (one) pr -= np;
+    int a = 0;
+    while ((a + 1) * (a + 2) / 2 <= pr) ++a;
+    const int b = pr - a * (a + 1) / 2;  // a >= b
+    const ll pab = tri_index(a + 1 + ncore, b + 1 + ncore) - 1;
+    const double *x = L + (ll)Q * pab;
+    if (!one) {
+        for (int p2 = warp; p2 <= pr; p2 += 8) {
+            int c = 0;
+            while ((c + 1) * (c + 2) / 2 <= p2) ++c;
+            const int d = p2 - c * (c + 1) / 2;
+            const double *y = L + (ll)Q * (tri_index(c + 1 + ncore, d + 1 + ncore) - 1);
+            double v = 0.0;
+            for (int q = lane; q < Q; q += 32) v = fma(x[q], y[q], v);
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane < 8) {  // (ab|cd) at its eight places
+                const int i = lane & 1 ? b : a, j = lane & 1 ? a : b, k = lane & 2 ? d : c, l = lane & 2 ? c : d;
+                if (lane & 4) ATWO(k + 1, l + 1, i + 1, j + 1) = v;
+                else ATWO(i + 1, j + 1, k + 1, l + 1) = v;
+            }
+        }
+        return;
+    }
+    double v = 0.0;
+    for (int j = warp; j < ncore; j += 8) {
+        const double *jj = L + (ll)Q * (tri_index(j + 1, j + 1) - 1);
+        const double *aj_ = L + (ll)Q * (tri_index(a + 1 + ncore, j + 1) - 1);
+        const double *jb = L + (ll)Q * (tri_index(b + 1 + ncore, j + 1) - 1);
+        for (int q = lane; q < Q; q += 32) v += 2.0 * x[q] * jj[q] - aj_[q] * jb[q];
+    }
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) v += red[w];
+        aj[pab] = oneint[pab] + v;
+    }
 }
 
 // ---------------------------------------------------------------------------
-// src/koop_matrices.F90:165-250 koopE.  Thread per (ap, a).
-__global__ void k_koopE(Rdm r, const double *atwo, const double *f, int ncore, double *koopipa, double *koopeaa) {
-    const int n = r.n, M = r.M;
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * n) return;
-    int ap = t % n + 1, a = t / n + 1;
-    for (int s = 1; s <= M; ++s) {
-        double ip = 0.0;
-        for (int c = 1; c <= n; ++c) {
-            ip -= FF(a, c) * r.D1(s, ap, c);
-            for (int d = 1; d <= n; ++d)
-                for (int ie = 1; ie <= n; ++ie) ip -= ATWO(c, ie, a, d) * r.D2(s, ap, c, d, ie);
-        }
-        ip = 2.0 * ip;
-        double dumm = 2.0 * FF(ap, a);
-        for (int d = 1; d <= n; ++d)
-            for (int ie = 1; ie <= n; ++ie) dumm += (2.0 * ATWO(d, ie, ap, a) - ATWO(ap, ie, d, a)) * r.D1(s, d, ie);
-        O3(koopipa, s, ap, a) = ip;
-        O3(koopeaa, s, ap, a) = ip + 2.0 * dumm;
-    }
-}
+// The generalised Koopmans matrices: koopE, koop2E, koopman0pE
+// (src/koop_matrices.F90:165-591), bbmat, bcmat, bdmat (src/koopro4QD.F90:4231-4459).
+//
+// Their n^7 sums are contractions of an operand G(r1,r2,z; k1,k2,k3), a few
+// accessors of one state's RDMs, with the active integrals over (k1,k2,k3):
+// P[(r1,r2,z), x] = sum_k G T(k; x).  A CTA owns some pairs (r1,r2) with all z
+// and x, evaluates G into shared memory 32 k at a time -- rows r1 first, which
+// is the index that most of the 3-RDM loads have fastest -- and multiplies.
+// What the reference adds to an output element are P's of the same pair with z
+// and x exchanged, so the CTA finishes its elements itself: nothing is
+// materialised, and koop_matrices_ctl is one launch.  Small spaces are bound by
+// latency (CTAs of one pair, the k range split over the threads left), large
+// ones by the FP64 pipe and the accessors.
+enum KoopOp { IP1, IP2, EA1, EA2, A1, A2, D1, D2, B1, BT, C1, C2, C3, CT1, CT2, CT3 };
 
-// src/koop_matrices.F90:78-88 (2-HRDM through ro2t)
-__global__ void k_hrdm(Rdm r, double *hrdm) {
-    const int n = r.n, M = r.M;
-    ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    int x[4];
-    decode(t, n, 4, x);
-    for (int s = 1; s <= M; ++s) hrdm[(s - 1) + (ll)M * t] = r.ro2t(x[0], x[1], x[2], x[3], s);
-}
-
-// src/koop_matrices.F90:297-335 koop2E, 2-IP part.  Thread per (ap,bp,a,b).
-__global__ void k_koop2E_ip(Rdm r, const double *atwo, const double *f, int ncore, double *koopaa) {
-    const int n = r.n, M = r.M;
-    ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    int x[4];
-    decode(t, n, 4, x);
-    const int ap = x[0], bp = x[1], a = x[2], b = x[3];
-    for (int s = 1; s <= M; ++s) {
-        double acc = 0.0;
-        for (int d = 1; d <= n; ++d) {
-            acc = acc - FF(a, d) * r.D2(s, ap, bp, d, b) - FF(b, d) * r.D2(s, ap, bp, a, d);
-            for (int ie = 1; ie <= n; ++ie)
-                for (int ief = 1; ief <= n; ++ief) {
-                    double dint = ATWO(d, ie, a, ief), dint2 = ATWO(d, ie, b, ief);
-                    double dum = r.D3(s, ap, bp, d, ief, b, ie);
-                    if (d == ief) dum += 0.5 * r.D2(s, ap, bp, ie, b);
-                    if (d == b) dum += 0.5 * r.D2(s, ap, bp, ief, ie);
-                    acc -= dint * dum;
-                    dum = r.D3(s, ap, bp, d, a, ief, ie);
-                    if (d == a) dum += 0.5 * r.D2(s, ap, bp, ie, ief);
-                    if (d == ief) dum += 0.5 * r.D2(s, ap, bp, a, ie);
-                    acc -= dint2 * dum;
-                }
-        }
-        O5(koopaa, s, ap, bp, a, b) = acc;
-    }
-}
-
-// src/koop_matrices.F90:336-384 koop2E, 2-EA part.  Thread per (ap,bp,a,b).
-__global__ void k_koop2E_ea(Rdm r, const double *atwo, const double *f, int ncore, double *koopeaa) {
-    const int n = r.n, M = r.M;
-    ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    int x[4];
-    decode(t, n, 4, x);
-    const int ap = x[0], bp = x[1], a = x[2], b = x[3];
-    for (int s = 1; s <= M; ++s) {
-        double acc = 0.0;
-        for (int c = 1; c <= n; ++c) {
-            acc += FF(a, c) * r.ro2t(ap, bp, c, b, s) + FF(b, c) * r.ro2t(ap, bp, a, c, s);
-            for (int d = 1; d <= n; ++d)
-                for (int ie = 1; ie <= n; ++ie) {
-                    double dint = ATWO(c, ie, d, a);
-                    double dum = -r.ro3t(ap, bp, ie, d, b, c, s);
-                    if (c == ie) dum += 2.0 * r.ro2t(ap, bp, d, b, s);
-                    if (d == ie) dum -= 0.5 * r.ro2t(ap, bp, c, b, s);
-                    if (b == ie) dum -= 0.5 * r.ro2t(ap, bp, d, c, s);
-                    acc += dint * dum;
-                    dint = ATWO(c, ie, d, b);
-                    dum = -r.ro3t(ap, bp, ie, a, d, c, s);
-                    if (c == ie) dum += 2.0 * r.ro2t(ap, bp, a, d, s);
-                    if (a == ie) dum -= 0.5 * r.ro2t(ap, bp, c, d, s);
-                    if (d == ie) dum -= 0.5 * r.ro2t(ap, bp, a, c, s);
-                    acc += dint * dum;
-                }
-        }
-        O5(koopeaa, s, ap, bp, a, b) = acc;
-    }
-}
-
-// The same 2-EA matrix as products.  Per state, the bracketed operands of
-// the reference's inner sum over (c, d, ie) are materialised as two n^3 x n^3
-// row blocks,
-//   G[(ap,bp,b), (c,d,ie)]       = -ro3t(ap,bp,ie,d,b,c) + 2[c=ie] ro2t(ap,bp,d,b)
-//                                  - 1/2 [d=ie] ro2t(ap,bp,c,b) - 1/2 [b=ie] ro2t(ap,bp,d,c)
-//   G[n^3 + (ap,bp,a), (c,d,ie)] = -ro3t(ap,bp,ie,a,d,c) + 2[c=ie] ro2t(ap,bp,a,d)
-//                                  - 1/2 [a=ie] ro2t(ap,bp,c,d) - 1/2 [d=ie] ro2t(ap,bp,a,c)
-// and one GEMM with A1[(c,d,ie), x] = atwo(c,ie,d,x) gives both contractions;
-// k_koop2E_ea_out adds the one-electron terms.  Indices 0-based, last fastest.
-__global__ void k_koop2E_ea_ops(Rdm r, int s, double *G) {
-    const int n = r.n;
-    const ll n3 = (ll)n * n * n, n6 = n3 * n3;
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 2 * n6) return;
-    const int half = (int)(t / n6);
-    const ll x = t % n6, col = x % n3, row = x / n3;
-    const int ie = (int)(col % n) + 1, d = (int)((col / n) % n) + 1, c = (int)(col / ((ll)n * n)) + 1;
-    const int z = (int)(row % n) + 1, bp = (int)((row / n) % n) + 1, ap = (int)(row / ((ll)n * n)) + 1;
-    double dum;
-    if (half == 0) {
-        const int b = z;
-        dum = -r.ro3t(ap, bp, ie, d, b, c, s);
-        if (c == ie) dum += 2.0 * r.ro2t(ap, bp, d, b, s);
-        if (d == ie) dum -= 0.5 * r.ro2t(ap, bp, c, b, s);
-        if (b == ie) dum -= 0.5 * r.ro2t(ap, bp, d, c, s);
-    } else {
-        const int a = z;
-        dum = -r.ro3t(ap, bp, ie, a, d, c, s);
-        if (c == ie) dum += 2.0 * r.ro2t(ap, bp, a, d, s);
-        if (a == ie) dum -= 0.5 * r.ro2t(ap, bp, c, d, s);
-        if (d == ie) dum -= 0.5 * r.ro2t(ap, bp, a, c, s);
-    }
-    G[t] = dum;
-}
-__global__ void k_koop2E_ea_ints(const double *atwo, int n, double *A1) {
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    const int x = (int)(t % n) + 1;
-    const ll k = t / n;
-    const int ie = (int)(k % n) + 1, d = (int)((k / n) % n) + 1, c = (int)(k / ((ll)n * n)) + 1;
-    A1[t] = ATWO(c, ie, d, x);
-}
-__global__ void k_koop2E_ea_out(Rdm r, int s, const double *f, int ncore, const double *P, double *koopeaa) {
-    const int n = r.n, M = r.M;
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    const ll n4 = (ll)n * n * n * n;
-    if (t >= n4) return;
-    int x[4];
-    decode(t, n, 4, x);
-    const int ap = x[0], bp = x[1], a = x[2], b = x[3];
-    double acc = 0.0;
-    for (int c = 1; c <= n; ++c) acc += FF(a, c) * r.ro2t(ap, bp, c, b, s) + FF(b, c) * r.ro2t(ap, bp, a, c, s);
-    const ll pre = ((ll)(ap - 1) * n + (bp - 1)) * n;
-    acc += P[(pre + (b - 1)) * n + (a - 1)] + P[n4 + (pre + (a - 1)) * n + (b - 1)];
-    O5(koopeaa, s, ap, bp, a, b) = acc;
-}
-
-// src/koop_matrices.F90:433-541 koopman0pE, A (koopaa) and D (koopbb) of the
-// 0' class.  Thread per (bp,ap,a,b).
-__global__ void k_koop0p_ad(Rdm r, const double *atwo, const double *f, int ncore, double *koopaa,
-                            double *koopbb) {
-    const int n = r.n, M = r.M;
-    ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    int x[4];
-    decode(t, n, 4, x);
-    const int bp = x[0], ap = x[1], a = x[2], b = x[3];
-    for (int s = 1; s <= M; ++s) {
-        double A = 0.0, Dm = 0.0;
-        for (int c = 1; c <= n; ++c) {
-            double fca = FF(c, a), fbc = FF(b, c);
-            A += 2.0 * (fca * r.ee2(bp, ap, c, b, s) - fbc * r.ee2(bp, ap, a, c, s));
-            for (int d = 1; d <= n; ++d)
-                for (int ie = 1; ie <= n; ++ie) {
-                    double dum1 = r.eee2(bp, ap, c, ie, d, b, s) + r.eee2(bp, ap, d, b, c, ie, s);
-                    double dum2 = r.eee2(bp, ap, a, ie, c, d, s) + r.eee2(bp, ap, c, d, a, ie, s);
-                    A += ATWO(c, ie, d, a) * dum1 - ATWO(b, ie, c, d) * dum2;
-                }
-        }
-        for (int c = 1; c <= n; ++c) {
-            double fca = FF(c, a), fbc = FF(b, c);
-            double dum1 = -r.ee2(a, ap, bp, c, s);
-            if (a == ap) dum1 += 2.0 * r.D1(s, bp, c);
-            if (bp == ap) dum1 += r.D1(s, a, c);
-            double dum2 = -r.ee2(c, ap, bp, b, s);
-            if (ap == c) dum2 += 2.0 * r.D1(s, bp, b);
-            if (bp == ap) dum2 += r.D1(s, c, b);
-            Dm += -fbc * dum1 + fca * dum2;
-            for (int d = 1; d <= n; ++d)
-                for (int ie = 1; ie <= n; ++ie) {
-                    double e1 = -r.eee2(c, ie, a, ap, bp, d, s) - r.eee2(a, ap, bp, d, c, ie, s);
-                    if (ap == a) e1 += 2.0 * (r.ee2(c, ie, bp, d, s) + r.ee2(bp, d, c, ie, s));
-                    if (bp == ap) e1 += r.ee2(c, ie, a, d, s) + r.ee2(a, d, c, ie, s);
-                    if (ap == c) {
-                        e1 -= r.ee2(a, ie, bp, d, s);
-                        if (ie == a) e1 += 2.0 * r.D1(s, bp, d);
-                    }
-                    if (bp == ie) {
-                        e1 += r.ee2(a, ap, c, d, s);
-                        if (ap == a) e1 -= 2.0 * r.D1(s, c, d);
-                    }
-                    double e2 = -r.eee2(c, ie, d, ap, bp, b, s) - r.eee2(d, ap, bp, b, c, ie, s);
-                    if (ap == d) e2 += 2.0 * (r.ee2(c, ie, bp, b, s) + r.ee2(bp, b, c, ie, s));
-                    if (bp == ap) e2 += r.ee2(c, ie, d, b, s) + r.ee2(d, b, c, ie, s);
-                    if (ap == c) {
-                        e2 -= r.ee2(d, ie, bp, b, s);
-                        if (d == ie) e2 += 2.0 * r.D1(s, bp, b);
-                    }
-                    if (bp == ie) {
-                        e2 += r.ee2(d, ap, c, b, s);
-                        if (d == ap) e2 -= 2.0 * r.D1(s, c, b);
-                    }
-                    Dm += -0.5 * ATWO(c, ie, b, d) * e1 + 0.5 * ATWO(c, ie, d, a) * e2;
-                }
-        }
-        O5(koopaa, s, bp, ap, a, b) = A;
-        O5(koopbb, s, bp, ap, a, b) = Dm;
-    }
-}
-
-// The same A and D of the 0' class as products.  Per state, the operands of
-// the reference's sums over (c, d, ie) are materialised as four n^3 x n^3
-// blocks (rows (bp,ap,z), columns (c,d,ie), ie fastest):
-//   0: eee2(bp,ap,c,ie,d,z) + eee2(bp,ap,d,z,c,ie)             (A, z = b) x atwo(c,ie,d,a)
-//   1: the D operand of the atwo(c,ie,d,a) term               (D, z = b) x atwo(c,ie,d,a)
-//   2: eee2(bp,ap,z,ie,c,d) + eee2(bp,ap,c,d,z,ie)             (A, z = a) x atwo(b,ie,c,d)
-//   3: the D operand of the atwo(c,ie,b,d) term               (D, z = a) x atwo(c,ie,b,d)
-// and three GEMMs give the n^7 sums; k_koop0p_out adds the n^5 one-electron
-// terms, with the signs and halves of the reference.
 __device__ __forceinline__ double koop0p_e1(const Rdm &r, int c, int d, int ie, int bp, int ap, int a, int s) {
     double e1 = -r.eee2(c, ie, a, ap, bp, d, s) - r.eee2(a, ap, bp, d, c, ie, s);
     if (ap == a) e1 += 2.0 * (r.ee2(c, ie, bp, d, s) + r.ee2(bp, d, c, ie, s));
@@ -450,246 +278,355 @@ __device__ __forceinline__ double koop0p_e2(const Rdm &r, int c, int d, int ie, 
     }
     return e2;
 }
-__global__ void k_koop0p_ops(Rdm r, int s, double *G) {
-    const int n = r.n;
-    const ll n3 = (ll)n * n * n, n6 = n3 * n3;
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 4 * n6) return;
-    const int blk = (int)(t / n6);
-    const ll x = t % n6, col = x % n3, row = x / n3;
-    const int ie = (int)(col % n) + 1, d = (int)((col / n) % n) + 1, c = (int)(col / ((ll)n * n)) + 1;
-    const int z = (int)(row % n) + 1, ap = (int)((row / n) % n) + 1, bp = (int)(row / ((ll)n * n)) + 1;
-    double v;
-    if (blk == 0) v = r.eee2(bp, ap, c, ie, d, z, s) + r.eee2(bp, ap, d, z, c, ie, s);
-    else if (blk == 1) v = koop0p_e2(r, c, d, ie, bp, ap, z, s);
-    else if (blk == 2) v = r.eee2(bp, ap, z, ie, c, d, s) + r.eee2(bp, ap, c, d, z, ie, s);
-    else v = koop0p_e1(r, c, d, ie, bp, ap, z, s);
-    G[t] = v;
-}
-// A2[(c,d,ie), x] = atwo(x,ie,c,d), A3[(c,d,ie), x] = atwo(c,ie,x,d)
-__global__ void k_koop0p_ints(const double *atwo, int n, double *A2, double *A3) {
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    const int x = (int)(t % n) + 1;
-    const ll k = t / n;
-    const int ie = (int)(k % n) + 1, d = (int)((k / n) % n) + 1, c = (int)(k / ((ll)n * n)) + 1;
-    A2[t] = ATWO(x, ie, c, d);
-    A3[t] = ATWO(c, ie, x, d);
-}
-__global__ void k_koop0p_out(Rdm r, int s, const double *f, int ncore, const double *P01, const double *P2,
-                             const double *P3, double *koopaa, double *koopbb) {
-    const int n = r.n, M = r.M;
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    const ll n3 = (ll)n * n * n, n4 = n3 * n;
-    if (t >= n4) return;
-    int x[4];
-    decode(t, n, 4, x);
-    const int bp = x[0], ap = x[1], a = x[2], b = x[3];
-    double A = 0.0, Dm = 0.0;
-    for (int c = 1; c <= n; ++c) {
-        const double fca = FF(c, a), fbc = FF(b, c);
-        A += 2.0 * (fca * r.ee2(bp, ap, c, b, s) - fbc * r.ee2(bp, ap, a, c, s));
-    }
-    for (int c = 1; c <= n; ++c) {
-        const double fca = FF(c, a), fbc = FF(b, c);
-        double dum1 = -r.ee2(a, ap, bp, c, s);
-        if (a == ap) dum1 += 2.0 * r.D1(s, bp, c);
-        if (bp == ap) dum1 += r.D1(s, a, c);
-        double dum2 = -r.ee2(c, ap, bp, b, s);
-        if (ap == c) dum2 += 2.0 * r.D1(s, bp, b);
-        if (bp == ap) dum2 += r.D1(s, c, b);
-        Dm += -fbc * dum1 + fca * dum2;
-    }
-    const ll rb = ((ll)(bp - 1) * n + (ap - 1)) * n + (b - 1), ra = ((ll)(bp - 1) * n + (ap - 1)) * n + (a - 1);
-    A += P01[rb * n + (a - 1)] - P2[ra * n + (b - 1)];
-    Dm += -0.5 * P3[ra * n + (b - 1)] + 0.5 * P01[(n3 + rb) * n + (a - 1)];
-    O5(koopaa, s, bp, ap, a, b) = A;
-    O5(koopbb, s, bp, ap, a, b) = Dm;
-}
 
-// src/koop_matrices.F90:546-571 koopman0pE, F (koopab).  Thread per (a,b).
-__global__ void k_koop0p_f(Rdm r, const double *atwo, const double *f, int ncore, double *koopab) {
-    const int n = r.n, M = r.M;
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * n) return;
-    int a = t % n + 1, b = t / n + 1;
-    for (int s = 1; s <= M; ++s) {
-        double acc = 0.0;
-        for (int c = 1; c <= n; ++c) {
-            acc += 2.0 * (FF(c, a) * r.D1(s, c, b) - FF(b, c) * r.D1(s, a, c));
-            for (int d = 1; d <= n; ++d)
-                for (int ie = 1; ie <= n; ++ie) {
-                    double dum1 = r.ee2(c, ie, d, b, s) + r.ee2(d, b, c, ie, s);
-                    double dum2 = r.ee2(a, ie, c, d, s) + r.ee2(c, d, a, ie, s);
-                    acc += ATWO(c, ie, d, a) * dum1 - ATWO(b, ie, c, d) * dum2;
-                }
+// G of one operation at 1-based labels.
+template <int OP>
+__device__ __forceinline__ double koop_operand(const Rdm &r, int s, int r1, int r2, int z, int k1, int k2, int k3) {
+    if constexpr (OP == IP1 || OP == IP2) {  // (ap,bp,b) / (ap,bp,a); (d,ie,ief)
+        const int ap = r1, bp = r2, d = k1, ie = k2, ief = k3;
+        double v;
+        if constexpr (OP == IP1) {
+            v = r.D3(s, ap, bp, d, ief, z, ie);
+            if (d == ief) v += 0.5 * r.D2(s, ap, bp, ie, z);
+            if (d == z) v += 0.5 * r.D2(s, ap, bp, ief, ie);
+        } else {
+            v = r.D3(s, ap, bp, d, z, ief, ie);
+            if (d == z) v += 0.5 * r.D2(s, ap, bp, ie, ief);
+            if (d == ief) v += 0.5 * r.D2(s, ap, bp, z, ie);
         }
-        O3(koopab, s, a, b) = acc;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// src/koopro4QD.F90:4231-4299 bbmat.  Thread per (ap,bp,cp,a).  The EA part
-// multiplies by aj, not by the modified f (reference quirk kept).
-__global__ void k_bbmat(Rdm r, const double *atwo, const double *f, const double *aj, int ncore, double *bmat,
-                        double *btmat) {
-    const int n = r.n, M = r.M;
-    ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    int x[4];
-    decode(t, n, 4, x);
-    const int ap = x[0], bp = x[1], cp = x[2], a = x[3];
-    for (int s = 1; s <= M; ++s) {
-        double B = 0.0, Bt = 0.0;
-        for (int c = 1; c <= n; ++c) {
-            B -= FF(c, a) * r.ee2(cp, ap, bp, c, s);
-            Bt += AJ(c, a) * r.ee2tr(cp, ap, bp, c, s);
-            for (int ie = 1; ie <= n; ++ie)
-                for (int ief = 1; ief <= n; ++ief) {
-                    double dint = ATWO(a, ie, c, ief);
-                    B -= r.eee2(cp, ap, bp, ie, c, ief, s) * dint;
-                    Bt += r.eee2t(cp, ap, bp, ie, c, ief, s) * dint;
-                }
+        return v;
+    } else if constexpr (OP == EA1 || OP == EA2) {  // (ap,bp,b) / (ap,bp,a); (c,d,ie)
+        const int ap = r1, bp = r2, c = k1, d = k2, ie = k3;
+        double v;
+        if constexpr (OP == EA1) {
+            v = -r.ro3t(ap, bp, ie, d, z, c, s);
+            if (c == ie) v += 2.0 * r.ro2t(ap, bp, d, z, s);
+            if (d == ie) v -= 0.5 * r.ro2t(ap, bp, c, z, s);
+            if (z == ie) v -= 0.5 * r.ro2t(ap, bp, d, c, s);
+        } else {
+            v = -r.ro3t(ap, bp, ie, z, d, c, s);
+            if (c == ie) v += 2.0 * r.ro2t(ap, bp, z, d, s);
+            if (z == ie) v -= 0.5 * r.ro2t(ap, bp, c, d, s);
+            if (d == ie) v -= 0.5 * r.ro2t(ap, bp, z, c, s);
         }
-        O5(bmat, s, ap, bp, cp, a) = B;
-        O5(btmat, s, ap, bp, cp, a) = Bt;
+        return v;
+    } else if constexpr (OP == A1) {  // (bp,ap,b); (c,d,ie)
+        return r.eee2(r1, r2, k1, k3, k2, z, s) + r.eee2(r1, r2, k2, z, k1, k3, s);
+    } else if constexpr (OP == A2) {  // (bp,ap,a); (c,d,ie)
+        return r.eee2(r1, r2, z, k3, k1, k2, s) + r.eee2(r1, r2, k1, k2, z, k3, s);
+    } else if constexpr (OP == D1) {
+        return koop0p_e2(r, k1, k2, k3, r1, r2, z, s);
+    } else if constexpr (OP == D2) {
+        return koop0p_e1(r, k1, k2, k3, r1, r2, z, s);
+    } else if constexpr (OP == B1) {  // (cp,ap,bp); (ie,c,ief)
+        return r.eee2(r1, r2, z, k1, k2, k3, s);
+    } else if constexpr (OP == BT) {
+        return r.eee2t(r1, r2, z, k1, k2, k3, s);
+    } else if constexpr (OP == C1) {  // (ap,b,c); (d,ief,ie)
+        return r.eee2(r1, r2, k1, k2, k3, z, s);
+    } else if constexpr (OP == C2) {  // (ap,b,a)
+        return r.eee2(r1, r2, k1, k2, z, k3, s);
+    } else if constexpr (OP == C3) {  // (ap,a,c)
+        return r.eee2(r1, k3, k1, k2, r2, z, s);
+    } else if constexpr (OP == CT1) {
+        return r.eee2tl(r1, r2, k1, k2, k3, z, s);
+    } else if constexpr (OP == CT2) {
+        return r.eee2tl(r1, r2, k1, k2, z, k3, s);
+    } else {
+        return r.eee2tl(r1, k3, k1, k2, r2, z, s);
     }
 }
 
-// src/koopro4QD.F90:4301-4397 bcmat.  Thread per (ap,a,b,c); the reference's
-// d loop is the reduction.
-__global__ void k_bcmat(Rdm r, const double *atwo, const double *f, int ncore, double *cmat, double *ctmat) {
-    const int n = r.n, M = r.M;
-    ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    int x[4];
-    decode(t, n, 4, x);
-    const int ap = x[0], a = x[1], b = x[2], c = x[3];
-    for (int s = 1; s <= M; ++s) {
-        double C = 0.0, Ct = 0.0;
-        for (int d = 1; d <= n; ++d) {
-            double fda = FF(d, a), fcd = FF(c, d), fbd = FF(b, d);
-            C += fda * r.ee2(ap, b, d, c, s) - fcd * r.ee2(ap, b, a, d, s) - fbd * r.ee2(ap, d, a, c, s);
-            Ct += fda * r.ee2t(ap, b, d, c, s) - fcd * r.ee2t(ap, b, a, d, s) + fbd * r.ee2t(ap, d, a, c, s);
-            for (int ie = 1; ie <= n; ++ie) {
-                double dint1 = ATWO(c, ie, d, a), dint2 = ATWO(d, ie, ie, a);
-                double dint3 = ATWO(c, d, d, ie), dint4 = ATWO(b, d, d, ie);
-                C += r.ee2(ap, b, d, ie, s) * dint1 -
-                     0.5 * (r.ee2(ap, b, d, c, s) * dint2 + r.ee2(ap, b, a, ie, s) * dint3 - r.ee2(ap, ie, a, c, s) * dint4);
-                Ct += r.ee2t(ap, b, d, ie, s) * dint1 -
-                      0.5 * (r.ee2t(ap, b, d, c, s) * dint2 + r.ee2t(ap, b, a, ie, s) * dint3 -
-                             r.ee2t(ap, ie, a, c, s) * dint4);
-                for (int ief = 1; ief <= n; ++ief) {
-                    double di1 = ATWO(d, ief, ie, a), di2 = ATWO(d, ief, c, ie), di3 = ATWO(d, ief, b, ie);
-                    C += r.eee2(ap, b, d, ief, ie, c, s) * di1 - r.eee2(ap, b, d, ief, a, ie, s) * di2 -
-                         r.eee2(ap, ie, d, ief, a, c, s) * di3;
-                    Ct += r.eee2tl(ap, b, d, ief, ie, c, s) * di1 - r.eee2tl(ap, b, d, ief, a, ie, s) * di2 +
-                          r.eee2tl(ap, ie, d, ief, a, c, s) * di3;
+// Strides of the integral T(k; x) in k1, k2, k3, x.
+template <int OP>
+__device__ __forceinline__ void koop_strides(int n, int &s1, int &s2, int &s3, int &sx) {
+    const int p1 = n, p2 = n * n, p3 = n * n * n;
+    if constexpr (OP == IP1 || OP == IP2) { s1 = 1; s2 = p1; s3 = p3; sx = p2; }                 // (d,ie,x,ief)
+    else if constexpr (OP == EA1 || OP == EA2 || OP == A1 || OP == D1) { s1 = 1; s2 = p2; s3 = p1; sx = p3; }  // (c,ie,d,x)
+    else if constexpr (OP == A2) { s1 = p2; s2 = p3; s3 = p1; sx = 1; }                           // (x,ie,c,d)
+    else if constexpr (OP == D2) { s1 = 1; s2 = p3; s3 = p1; sx = p2; }                           // (c,ie,x,d)
+    else if constexpr (OP == B1 || OP == BT) { s1 = p1; s2 = p2; s3 = p3; sx = 1; }               // (x,ie,c,ief)
+    else if constexpr (OP == C1 || OP == CT1) { s1 = 1; s2 = p1; s3 = p2; sx = p3; }              // (d,ief,ie,x)
+    else { s1 = 1; s2 = p1; s3 = p3; sx = p2; }                                                   // (d,ief,x,ie)
+}
+
+constexpr int kKoopRpt = 4;     // most rows per thread
+struct KoopTile {
+    int n, pair0, npair, R;     // pairs of the CTA, rows R = npair n (row = z npair + pair)
+    int kc;                     // k per shared-memory chunk
+    double *A, *B, *P;          // [kc][R + 1], [kc][n], results [2][R][n]
+};
+// k per chunk: about 2048 operand elements, so that a small CTA does not
+// synchronise more often than it computes
+__host__ __device__ __forceinline__ int koop_chunk(int n, int G) { return max(32, min(256, 2048 / (G * n))); }
+
+// P[slot][row][x] of one operation; all threads of the CTA.
+template <int OP>
+__device__ __forceinline__ void koop_contract(const Rdm &r, int s, const double *__restrict__ atwo, const KoopTile &t,
+                                              int slot) {
+    const int n = t.n, R = t.R, lda = R + 1, tid = threadIdx.x, K = n * n * n;
+    int s1, s2, s3, sx;
+    koop_strides<OP>(n, s1, s2, s3, sx);
+    // threads: column, row group, and -- when one row per thread leaves room -- a share of the k's
+    const int groups = 256 / n, rpt = (R + groups - 1) / groups;
+    const int slices = rpt == 1 ? 256 / (R * n) : 1, per = rpt == 1 ? R * n : 256;
+    const int slice = tid / per, q = tid % per, col = q % n, grp = q / n;
+    const bool live = slice < slices && grp < groups && (rpt > 1 || grp < R);
+    double acc[kKoopRpt] = {};
+    for (int k0 = 0; k0 < K; k0 += t.kc) {
+        const int nk = min(t.kc, K - k0);
+        for (int i = tid; i < nk * R; i += 256) {
+            const int row = i % R, kk = i / R, k = k0 + kk;
+            const int pair = t.pair0 + row % t.npair, z = row / t.npair;
+            t.A[kk * lda + row] =
+                koop_operand<OP>(r, s, pair % n + 1, pair / n + 1, z + 1, k % n + 1, (k / n) % n + 1, k / (n * n) + 1);
+        }
+        for (int i = tid; i < nk * n; i += 256) {
+            const int x = i % n, k = k0 + i / n;
+            t.B[i] = atwo[(k % n) * s1 + ((k / n) % n) * s2 + (k / (n * n)) * s3 + x * sx];
+        }
+        __syncthreads();
+        if (live) {
+            if (rpt == 1) {
+                for (int kk = slice; kk < nk; kk += slices) acc[0] = fma(t.A[kk * lda + grp], t.B[kk * n + col], acc[0]);
+            } else {
+                for (int kk = 0; kk < nk; ++kk) {
+                    const double b = t.B[kk * n + col];
+#pragma unroll
+                    for (int i = 0; i < kKoopRpt; ++i)
+                        if (i < rpt) acc[i] = fma(t.A[kk * lda + min(grp + i * groups, R - 1)], b, acc[i]);
                 }
             }
         }
-        O5(cmat, s, ap, a, b, c) = C;
-        O5(ctmat, s, ap, a, b, c) = Ct;
+        __syncthreads();
     }
-}
-
-// The same C / C~ matrices as products.  Per state, the operands of the n^7
-// sums over (d, ief, ie) are materialised as six n^3 x n^3 blocks (rows
-// (ap,u,w), columns (d,ief,ie), ie fastest), eee2 for C and eee2tl for C~:
-//   0/1: e(ap,u,d,ief,ie,w), u = b, w = c     x atwo(d,ief,ie,a)
-//   2/3: e(ap,u,d,ief,w,ie), u = b, w = a     x atwo(d,ief,c,ie)
-//   4/5: e(ap,ie,d,ief,u,w), u = a, w = c     x atwo(d,ief,b,ie)
-// three GEMMs (the C and C~ blocks stacked) give them; k_bcmat_out adds the
-// one-electron and n^6 terms in the reference's form.
-__global__ void k_bcmat_ops(Rdm r, int s, double *G) {
-    const int n = r.n;
-    const ll n3 = (ll)n * n * n, n6 = n3 * n3;
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 6 * n6) return;
-    const int blk = (int)(t / n6);
-    const ll x = t % n6, col = x % n3, row = x / n3;
-    const int ie = (int)(col % n) + 1, ief = (int)((col / n) % n) + 1, d = (int)(col / ((ll)n * n)) + 1;
-    const int w = (int)(row % n) + 1, u = (int)((row / n) % n) + 1, ap = (int)(row / ((ll)n * n)) + 1;
-    double v;
-    switch (blk) {
-    case 0: v = r.eee2(ap, u, d, ief, ie, w, s); break;
-    case 1: v = r.eee2tl(ap, u, d, ief, ie, w, s); break;
-    case 2: v = r.eee2(ap, u, d, ief, w, ie, s); break;
-    case 3: v = r.eee2tl(ap, u, d, ief, w, ie, s); break;
-    case 4: v = r.eee2(ap, ie, d, ief, u, w, s); break;
-    default: v = r.eee2tl(ap, ie, d, ief, u, w, s); break;
-    }
-    G[t] = v;
-}
-// B1[(d,ief,ie), x] = atwo(d,ief,ie,x), B2[(d,ief,ie), x] = atwo(d,ief,x,ie)
-__global__ void k_bcmat_ints(const double *atwo, int n, double *B1, double *B2) {
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (ll)n * n * n * n) return;
-    const int x = (int)(t % n) + 1;
-    const ll k = t / n;
-    const int ie = (int)(k % n) + 1, ief = (int)((k / n) % n) + 1, d = (int)(k / ((ll)n * n)) + 1;
-    B1[t] = ATWO(d, ief, ie, x);
-    B2[t] = ATWO(d, ief, x, ie);
-}
-__global__ void k_bcmat_out(Rdm r, int s, const double *atwo, const double *f, int ncore, const double *P,
-                            double *cmat, double *ctmat) {
-    const int n = r.n, M = r.M;
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    const ll n3 = (ll)n * n * n, n4 = n3 * n;
-    if (t >= n4) return;
-    int x[4];
-    decode(t, n, 4, x);
-    const int ap = x[0], a = x[1], b = x[2], c = x[3];
-    double C = 0.0, Ct = 0.0;
-    for (int d = 1; d <= n; ++d) {
-        const double fda = FF(d, a), fcd = FF(c, d), fbd = FF(b, d);
-        C += fda * r.ee2(ap, b, d, c, s) - fcd * r.ee2(ap, b, a, d, s) - fbd * r.ee2(ap, d, a, c, s);
-        Ct += fda * r.ee2t(ap, b, d, c, s) - fcd * r.ee2t(ap, b, a, d, s) + fbd * r.ee2t(ap, d, a, c, s);
-        for (int ie = 1; ie <= n; ++ie) {
-            const double dint1 = ATWO(c, ie, d, a), dint2 = ATWO(d, ie, ie, a);
-            const double dint3 = ATWO(c, d, d, ie), dint4 = ATWO(b, d, d, ie);
-            C += r.ee2(ap, b, d, ie, s) * dint1 -
-                 0.5 * (r.ee2(ap, b, d, c, s) * dint2 + r.ee2(ap, b, a, ie, s) * dint3 - r.ee2(ap, ie, a, c, s) * dint4);
-            Ct += r.ee2t(ap, b, d, ie, s) * dint1 -
-                  0.5 * (r.ee2t(ap, b, d, c, s) * dint2 + r.ee2t(ap, b, a, ie, s) * dint3 -
-                         r.ee2t(ap, ie, a, c, s) * dint4);
+    double *P = t.P + slot * R * n;
+    if (rpt == 1) {
+        for (int sl = 0; sl < slices; ++sl) {  // slices in order: a fixed sum
+            if (live && slice == sl) P[grp * n + col] = sl ? P[grp * n + col] + acc[0] : acc[0];
+            __syncthreads();
         }
+    } else {
+        if (live)
+#pragma unroll
+            for (int i = 0; i < kKoopRpt; ++i)
+                if (i < rpt && grp + i * groups < R) P[(grp + i * groups) * n + col] = acc[i];
+        __syncthreads();
     }
-    // P: [3 GEMMs][2 n^3 rows (C block, C~ block)][n]
-    const ll rbc = ((ll)(ap - 1) * n + (b - 1)) * n + (c - 1), rba = ((ll)(ap - 1) * n + (b - 1)) * n + (a - 1);
-    const ll rac = ((ll)(ap - 1) * n + (a - 1)) * n + (c - 1);
-    const double *P1 = P, *P2 = P + 2 * n4, *P3 = P + 4 * n4;
-    C += P1[rbc * n + (a - 1)] - P2[rba * n + (c - 1)] - P3[rac * n + (b - 1)];
-    Ct += P1[(n3 + rbc) * n + (a - 1)] - P2[(n3 + rba) * n + (c - 1)] + P3[(n3 + rac) * n + (b - 1)];
-    O5(cmat, s, ap, a, b, c) = C;
-    O5(ctmat, s, ap, a, b, c) = Ct;
 }
 
-// src/koopro4QD.F90:4399-4459 bdmat.  Thread per (ap,a); EA part uses aj.
-__global__ void k_bdmat(Rdm r, const double *atwo, const double *f, const double *aj, int ncore, double *dmat,
-                        double *dtmat) {
-    const int n = r.n, M = r.M;
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * n) return;
-    int ap = t % n + 1, a = t / n + 1;
-    for (int s = 1; s <= M; ++s) {
-        double D = 0.0, Dt = 0.0;
-        for (int c = 1; c <= n; ++c) {
-            D -= FF(c, a) * r.D1(s, ap, c);
-            double dum = -r.D1(s, ap, c);
-            if (ap == c) dum += 2.0;
-            Dt += AJ(c, a) * dum;
-            for (int ie = 1; ie <= n; ++ie)
-                for (int ief = 1; ief <= n; ++ief) {
-                    double dint = ATWO(a, ie, c, ief);
-                    D -= r.ee2(ap, ie, c, ief, s) * dint;
-                    Dt += r.ee2t(ap, ie, c, ief, s) * dint;
+// The builder's one-electron operator on the active block (mode 0: aj, 1: aj -
+// K/2, 2: aj - K with K(a,b) = sum_c (ac|cb)) in shared memory, and, by one CTA
+// of the launch, in the upper triangle of f(*).
+__device__ __forceinline__ void koop_operator(double *ff, const double *aj, const double *atwo, int n, int ncore,
+                                              int mode, double *f) {
+    for (int i = threadIdx.x; i < n * n; i += blockDim.x) {
+        const int x = i % n + 1, y = i / n + 1, a = min(x, y), b = max(x, y);
+        double v = AJ(a, b);
+        if (mode != 0)
+            for (int c = 1; c <= n; ++c) v -= (mode == 1 ? 0.5 : 1.0) * ATWO(a, c, c, b);
+        ff[i] = v;
+        if (f && x <= y) FF(x, y) = v;
+    }
+    __syncthreads();
+}
+#define FS(i, j) ff[((j)-1) * n + (i)-1]
+
+__device__ __forceinline__ double block_reduce(double v, double *red) {
+    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += red[w];
+    return t;
+}
+
+struct KoopOut {
+    double *p[8];
+};
+
+// koop_matrices_ctl.  blockIdx.y: 0 2-IP, 1 2-EA and the 2-HRDM, 2 A and 3 D of
+// the 0' class, 4 koopE and the 0' F (a CTA per element); blockIdx.z: state.
+// out: ipko1, eako1, hrdm2, ipko2, eako2, gk0pa, gk0pd, gk0pf.
+__global__ void __launch_bounds__(256) k_koop_ctl(Rdm r, const double *__restrict__ atwo, const double *__restrict__ aj,
+                                                  int ncore, int G, double *f, KoopOut out, const int *flag) {
+    const int part = blockIdx.y;
+    if (part != 4 && flag && !flag[blockIdx.z]) return;
+    extern __shared__ double sm[];
+    const int n = r.n, M = r.M, s = blockIdx.z + 1, tid = threadIdx.x;
+    double *ff = sm;
+    KoopTile t;
+    t.n = n;
+    t.kc = koop_chunk(n, G);
+    t.A = ff + n * n;
+    t.B = t.A + t.kc * (G * n + 1);
+    t.P = t.B + t.kc * n;
+    koop_operator(ff, aj, atwo, n, ncore, 1, part == 4 && blockIdx.x == 0 && blockIdx.z == 0 ? f : nullptr);
+    if (part == 4) {
+        for (int it = blockIdx.x; it < n * n; it += gridDim.x) {
+            const int x = it % n + 1, y = it / n + 1;  // koopE (ap, a); F (a, b)
+            double ip = 0.0, ea = 0.0, fv = 0.0;
+            for (int k = tid; k < n * n * n; k += 256) {
+                const int c = k % n + 1, d = (k / n) % n + 1, ie = k / (n * n) + 1;
+                ip -= ATWO(c, ie, y, d) * r.D2(s, x, c, d, ie);
+                fv += ATWO(c, ie, d, x) * (r.ee2(c, ie, d, y, s) + r.ee2(d, y, c, ie, s)) -
+                      ATWO(y, ie, c, d) * (r.ee2(x, ie, c, d, s) + r.ee2(c, d, x, ie, s));
+                if (ie == 1) ea += (2.0 * ATWO(c, d, x, y) - ATWO(x, d, c, y)) * r.D1(s, c, d);
+            }
+            for (int c = tid + 1; c <= n; c += 256) {
+                ip -= AJ(y, c) * r.D1(s, x, c);
+                fv += 2.0 * (FS(c, x) * r.D1(s, c, y) - FS(y, c) * r.D1(s, x, c));
+            }
+            double *red = t.A;
+            ip = block_reduce(ip, red);
+            ea = block_reduce(ea, red);
+            fv = block_reduce(fv, red);
+            if (tid == 0) {
+                O3(out.p[0], s, x, y) = 2.0 * ip;
+                O3(out.p[1], s, x, y) = 2.0 * ip + 2.0 * (2.0 * AJ(x, y) + ea);
+                O3(out.p[7], s, x, y) = fv;
+            }
+        }
+        return;
+    }
+    t.pair0 = blockIdx.x * G;
+    t.npair = min(G, n * n - t.pair0);
+    t.R = t.npair * n;
+    switch (part) {
+    case 0: koop_contract<IP1>(r, s, atwo, t, 0); koop_contract<IP2>(r, s, atwo, t, 1); break;
+    case 1: koop_contract<EA1>(r, s, atwo, t, 0); koop_contract<EA2>(r, s, atwo, t, 1); break;
+    case 2: koop_contract<A1>(r, s, atwo, t, 0); koop_contract<A2>(r, s, atwo, t, 1); break;
+    default: koop_contract<D1>(r, s, atwo, t, 0); koop_contract<D2>(r, s, atwo, t, 1); break;
+    }
+    const double *P0 = t.P, *P1 = t.P + t.R * n;  // [z npair + pair][x]
+    for (int i = tid; i < t.R * n; i += 256) {
+        const int g = i % t.npair, a0 = (i / t.npair) % n, b0 = i / (t.npair * n), a = a0 + 1, b = b0 + 1;
+        const int p = (t.pair0 + g) % n + 1, q = (t.pair0 + g) / n + 1;
+        const double x0 = P0[(b0 * t.npair + g) * n + a0], x1 = P1[(a0 * t.npair + g) * n + b0];
+        double v = 0.0;
+        if (part == 0) {  // (ap,bp) = (p,q)
+            for (int d = 1; d <= n; ++d) v -= FS(a, d) * r.D2(s, p, q, d, b) + FS(b, d) * r.D2(s, p, q, a, d);
+            O5(out.p[3], s, p, q, a, b) = v - x0 - x1;
+        } else if (part == 1) {
+            for (int c = 1; c <= n; ++c) v += FS(a, c) * r.ro2t(p, q, c, b, s) + FS(b, c) * r.ro2t(p, q, a, c, s);
+            O5(out.p[4], s, p, q, a, b) = v + x0 + x1;
+            O5(out.p[2], s, p, q, a, b) = r.ro2t(p, q, a, b, s);
+        } else if (part == 2) {  // (bp,ap) = (p,q)
+            for (int c = 1; c <= n; ++c) v += 2.0 * (FS(c, a) * r.ee2(p, q, c, b, s) - FS(b, c) * r.ee2(p, q, a, c, s));
+            O5(out.p[5], s, p, q, a, b) = v + x0 - x1;
+        } else {
+            for (int c = 1; c <= n; ++c) {
+                double d1 = -r.ee2(a, q, p, c, s), d2 = -r.ee2(c, q, p, b, s);
+                if (a == q) d1 += 2.0 * r.D1(s, p, c);
+                if (c == q) d2 += 2.0 * r.D1(s, p, b);
+                if (p == q) {
+                    d1 += r.D1(s, a, c);
+                    d2 += r.D1(s, c, b);
                 }
+                v += FS(c, a) * d2 - FS(b, c) * d1;
+            }
+            O5(out.p[6], s, p, q, a, b) = v + 0.5 * x0 - 0.5 * x1;
         }
+    }
+}
+
+// bbmat (blockIdx.y 0 B, 1 B~; rows (cp,ap,bp)) and the two passes of bcmat
+// (kind 1: the first two contractions and all lower terms of C / C~, rows
+// (ap,b,.); kind 2: the third, rows (ap,a,c), added to it).  B~ multiplies the
+// one-electron part by aj, not by the modified f (reference quirk kept).
+__global__ void __launch_bounds__(256) k_koop_bc(Rdm r, const double *__restrict__ atwo, const double *__restrict__ aj,
+                                                 int ncore, int G, int kind, double *f, double *x0, double *x1,
+                                                 const int *flag) {
+    const bool first = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0, skip = flag && !flag[blockIdx.z];
+    if (skip && !first) return;
+    extern __shared__ double sm[];
+    const int n = r.n, M = r.M, s = blockIdx.z + 1, part = blockIdx.y, tid = threadIdx.x;
+    double *ff = sm;
+    KoopTile t;
+    t.n = n;
+    t.kc = koop_chunk(n, G);
+    t.A = ff + n * n;
+    t.B = t.A + t.kc * (G * n + 1);
+    t.P = t.B + t.kc * n;
+    t.pair0 = blockIdx.x * G;
+    t.npair = min(G, n * n - t.pair0);
+    t.R = t.npair * n;
+    koop_operator(ff, aj, atwo, n, ncore, kind == 0 ? 2 : 1, first && kind != 2 ? f : nullptr);
+    if (skip) return;
+    if (kind == 0) {
+        if (part == 0) koop_contract<B1>(r, s, atwo, t, 0);
+        else koop_contract<BT>(r, s, atwo, t, 0);
+    } else if (kind == 1) {
+        if (part == 0) { koop_contract<C1>(r, s, atwo, t, 0); koop_contract<C2>(r, s, atwo, t, 1); }
+        else { koop_contract<CT1>(r, s, atwo, t, 0); koop_contract<CT2>(r, s, atwo, t, 1); }
+    } else {
+        if (part == 0) koop_contract<C3>(r, s, atwo, t, 0);
+        else koop_contract<CT3>(r, s, atwo, t, 0);
+    }
+    const double *P0 = t.P, *P1 = t.P + t.R * n;
+    double *out = part == 0 ? x0 : x1;
+    for (int i = tid; i < t.R * n; i += 256) {
+        const int g = i % t.npair, z0 = (i / t.npair) % n, w0 = i / (t.npair * n);
+        const int p = (t.pair0 + g) % n + 1, q = (t.pair0 + g) / n + 1, z = z0 + 1, w = w0 + 1;
+        double v = 0.0;
+        if (kind == 0) {  // (cp,ap) = (p,q), bp = z, a = w
+            const double x = P0[(z0 * t.npair + g) * n + w0];
+            if (part == 0)
+                for (int c = 1; c <= n; ++c) v -= FS(c, w) * r.ee2(p, q, z, c, s);
+            else
+                for (int c = 1; c <= n; ++c) v += AJ(c, w) * r.ee2tr(p, q, z, c, s);
+            O5(out, s, q, z, p, w) = part == 0 ? v - x : v + x;
+        } else if (kind == 1) {  // (ap,b) = (p,q), a = z, c = w
+            const int ap = p, b = q, a = z, c = w;
+            auto e = [&](int i1, int i2, int i3, int i4) {
+                return part == 0 ? r.ee2(i1, i2, i3, i4, s) : r.ee2t(i1, i2, i3, i4, s);
+            };
+            const double sg = part == 0 ? -1.0 : 1.0;
+            for (int d = 1; d <= n; ++d) {
+                v += FS(d, a) * e(ap, b, d, c) - FS(c, d) * e(ap, b, a, d) + sg * FS(b, d) * e(ap, d, a, c);
+                for (int ie = 1; ie <= n; ++ie) {
+                    const double dint1 = ATWO(c, ie, d, a), dint2 = ATWO(d, ie, ie, a);
+                    const double dint3 = ATWO(c, d, d, ie), dint4 = ATWO(b, d, d, ie);
+                    v += e(ap, b, d, ie) * dint1 -
+                         0.5 * (e(ap, b, d, c) * dint2 + e(ap, b, a, ie) * dint3 - e(ap, ie, a, c) * dint4);
+                }
+            }
+            O5(out, s, ap, a, b, c) = v + P0[(w0 * t.npair + g) * n + z0] - P1[(z0 * t.npair + g) * n + w0];
+        } else {  // (ap,a) = (p,q), c = z, b = w
+            const double x = P0[(z0 * t.npair + g) * n + w0];
+            O5(out, s, p, q, w, z) += part == 0 ? -x : x;
+        }
+    }
+}
+
+// bdmat: a CTA per (ap,a) and state; the EA part uses aj.
+__global__ void __launch_bounds__(256) k_koop_d(Rdm r, const double *atwo, const double *aj, int ncore, double *f,
+                                                double *dmat, double *dtmat) {
+    __shared__ double ff[256], red[8];
+    const int n = r.n, M = r.M, s = blockIdx.y + 1;
+    koop_operator(ff, aj, atwo, n, ncore, 2, blockIdx.x == 0 && blockIdx.y == 0 ? f : nullptr);
+    const int ap = blockIdx.x % n + 1, a = blockIdx.x / n + 1;
+    double D = 0.0, Dt = 0.0;
+    for (int k = threadIdx.x; k < n * n * n; k += 256) {
+        const int ie = k % n + 1, c = (k / n) % n + 1, ief = k / (n * n) + 1;
+        const double dint = ATWO(a, ie, c, ief);
+        D -= r.ee2(ap, ie, c, ief, s) * dint;
+        Dt += r.ee2t(ap, ie, c, ief, s) * dint;
+    }
+    for (int c = threadIdx.x + 1; c <= n; c += 256) {
+        const double g = r.D1(s, ap, c);
+        D -= FS(c, a) * g;
+        Dt += AJ(c, a) * ((ap == c ? 2.0 : 0.0) - g);
+    }
+    D = block_reduce(D, red);
+    Dt = block_reduce(Dt, red);
+    if (threadIdx.x == 0) {
         O3(dmat, s, ap, a) = D;
         O3(dtmat, s, ap, a) = Dt;
     }
 }
+#undef FS
 
 // ---------------------------------------------------------------------------
 // Host launchers.
@@ -700,53 +637,22 @@ void launch_build_f(double *f, const double *aj, const double *atwo, int n, int 
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-// Column groups in an order that puts the permutations of one multiset
-// {ii,jj,kk} next to each other (they read the same ro4 columns).
-static void bro3_column_order(int n, std::vector<int> &ord) {
-    ord.clear();
-    for (int a = 0; a < n; ++a)
-        for (int b = a; b < n; ++b)
-            for (int c = b; c < n; ++c) {
-                const int v[3] = {a, b, c};
-                static const int P[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
-                int seen[6], ns = 0;
-                for (auto &pp : P) {
-                    const int code = v[pp[0]] + n * (v[pp[1]] + n * v[pp[2]]);
-                    bool dup = false;
-                    for (int q = 0; q < ns; ++q) dup |= seen[q] == code;
-                    if (!dup) {
-                        seen[ns++] = code;
-                        ord.push_back(code);
-                    }
-                }
-            }
-}
-
 int launch_bro3(const Rdm &r, double *daaa, int nele, cudaStream_t st) {
     const int n = r.n, M = r.M;
     const ll n3 = (ll)n * n * n, n6 = n3 * n3;
-    std::vector<int> ord;
-    bro3_column_order(n, ord);
     double *P = nullptr;
-    int *d_ord = nullptr;
     if (cudaMallocAsync((void **)&P, sizeof(double) * 2 * (size_t)(M * n6), st) != cudaSuccess) return 2;
-    if (cudaMallocAsync((void **)&d_ord, sizeof(int) * ord.size(), st) != cudaSuccess) {
-        cudaFreeAsync(P, st);
-        return 2;
-    }
     double *Q = P + (size_t)M * n6;
-    cudaMemcpyAsync(d_ord, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice, st);
     ProfSpan span;
     span.begin("bro3", st, 0);
     for (int s0 = 0; s0 < M; s0 += kBro3States) {
-        k_bro3_case_a<<<(unsigned)n3, 256, 0, st>>>(r, d_ord, s0, std::min(kBro3States, M - s0), P, Q);
+        k_bro3_case_a<<<(unsigned)(n * (n + 1) * (n + 2)), 256, 0, st>>>(r, s0, std::min(kBro3States, M - s0), P, Q);
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
     dim3 g((unsigned)((n3 + 31) / 32), (unsigned)((n3 + 31) / 32));
     k_bro3_combine<<<g, 256, 0, st>>>(P, Q, daaa, n3, M, 1.0 / (double)(nele - 3));
     span.end();
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    cudaFreeAsync(d_ord, st);
     cudaFreeAsync(P, st);
     return 0;
 }
@@ -762,153 +668,94 @@ void launch_bro1(const Rdm &r, double *dal, int nele, cudaStream_t st) {
 
 void launch_aj_atwo(const double *oneint, const double *L, int Q, int n, int ncore, int norb, double *atwo,
                     double *aj, cudaStream_t st) {
-    cudaMemcpyAsync(aj, oneint, sizeof(double) * (size_t)norb * (norb + 1) / 2, cudaMemcpyDeviceToDevice, st);
-    k_aj<<<blocks_for((ll)n * n, 64), 64, 0, st>>>(oneint, L, Q, n, ncore, aj);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    ll n4 = (ll)n * n * n * n;
-    k_atwo<<<blocks_for(n4, 128), 128, 0, st>>>(L, Q, n, ncore, atwo);
+    const ll npair = (ll)norb * (norb + 1) / 2;
+    const unsigned np = n * (n + 1) / 2, copy = (unsigned)std::min<ll>((npair + 255) / 256, 304);
+    k_aj_atwo<<<2 * np + copy, 256, 0, st>>>(oneint, L, Q, n, ncore, npair, atwo, aj);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-void launch_koopE(const Rdm &r, const double *atwo, const double *f, int ncore, double *ip, double *ea,
-                  cudaStream_t st) {
-    k_koopE<<<blocks_for((ll)r.n * r.n, 64), 64, 0, st>>>(r, atwo, f, ncore, ip, ea);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+// Pairs per CTA: few idle rows, and enough CTAs for the chip.
+static int koop_pairs(int n, int parts) {
+    const int groups = 256 / n;
+    int best = 1;
+    double top = 0.0;
+    for (int G = 1; G * n <= kKoopRpt * groups && G <= 6; ++G) {
+        const int rpt = (G * n + groups - 1) / groups;
+        const double fill = rpt == 1 ? 1.0 : (double)(G * n) / (rpt * groups);
+        const double ctas = (double)((n * n + G - 1) / G) * parts;
+        // a CTA evaluates each operand once for n products: more rows only fill the threads
+        const double score = fill * std::min(1.0, ctas / 304.0) * (rpt == 1 && G > 1 ? 0.99 : 1.0);
+        if (score > top) {
+            top = score;
+            best = G;
+        }
+    }
+    return best;
 }
-void launch_hrdm(const Rdm &r, double *hrdm, cudaStream_t st) {
-    ll n4 = (ll)r.n * r.n * r.n * r.n;
-    k_hrdm<<<blocks_for(n4, 256), 256, 0, st>>>(r, hrdm);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+static size_t koop_smem(int n, int G) {
+    const int kc = koop_chunk(n, G);
+    return sizeof(double) * (size_t)(n * n + kc * (G * n + 1) + kc * n + 2 * G * n * n);
 }
+
+// The one-contraction route (koop_sym.cu) with the direct kernels behind its
+// flags, from kKoopSymMin active orbitals on; below, the direct kernels alone
+// have fewer launches.  Without room for the route's scratch: the direct kernels.
+constexpr int kKoopSymMin = 6;
 namespace {
-struct KoopBlas {
-    cublasHandle_t h = nullptr;
-    ~KoopBlas() {
-        if (h) cublasDestroy(h);
+struct SymFlags {
+    int *p = nullptr;
+    cudaStream_t st;
+    SymFlags(const Rdm &r, const double *atwo, const double *aj, int ncore, int kind, double *const out[5],
+             cudaStream_t s)
+        : st(s) {
+        if (r.n < kKoopSymMin || cudaMallocAsync((void **)&p, sizeof(int) * r.M, st) != cudaSuccess) {
+            p = nullptr;
+            return;
+        }
+        cudaMemsetAsync(p, 0, sizeof(int) * r.M, st);
+        if (launch_koop_sym(r, atwo, aj, ncore, kind, out, p, st)) {
+            cudaFreeAsync(p, st);
+            p = nullptr;
+        }
+    }
+    ~SymFlags() {
+        if (p) cudaFreeAsync(p, st);
     }
 };
 }  // namespace
 
-void launch_koop2E(const Rdm &r, const double *atwo, const double *f, int ncore, double *ip2, double *ea2,
-                   cudaStream_t st) {
-    const int n = r.n;
-    const ll n3 = (ll)n * n * n, n4 = n3 * n, n6 = n3 * n3;
-    k_koop2E_ip<<<blocks_for(n4, 64), 64, 0, st>>>(r, atwo, f, ncore, ip2);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    // 2-EA: operand blocks + one GEMM per state
-    static thread_local KoopBlas blas;
-    double *G = nullptr, *A1 = nullptr, *P = nullptr;
-    bool ok = (blas.h || cublasCreate(&blas.h) == CUBLAS_STATUS_SUCCESS) &&
-              cublasSetStream(blas.h, st) == CUBLAS_STATUS_SUCCESS &&
-              cudaMallocAsync((void **)&G, sizeof(double) * 2 * (size_t)n6, st) == cudaSuccess &&
-              cudaMallocAsync((void **)&A1, sizeof(double) * (size_t)n4, st) == cudaSuccess &&
-              cudaMallocAsync((void **)&P, sizeof(double) * 2 * (size_t)n4, st) == cudaSuccess;
-    if (!ok) {  // no room for the operand blocks: the per-element kernel
-        if (G) cudaFreeAsync(G, st);
-        if (A1) cudaFreeAsync(A1, st);
-        k_koop2E_ea<<<blocks_for(n4, 64), 64, 0, st>>>(r, atwo, f, ncore, ea2);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        return;
-    }
-    k_koop2E_ea_ints<<<blocks_for(n4, 256), 256, 0, st>>>(atwo, n, A1);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    const double one = 1.0, zero = 0.0;
-    for (int s = 1; s <= r.M; ++s) {
-        k_koop2E_ea_ops<<<blocks_for(2 * n6, 256), 256, 0, st>>>(r, s, G);
-        // row-major P[2 n^3, n] = G[2 n^3, n^3] A1[n^3, n]
-        cublasDgemm(blas.h, CUBLAS_OP_N, CUBLAS_OP_N, n, (int)(2 * n3), (int)n3, &one, A1, n, G, (int)n3, &zero, P, n);
-        k_koop2E_ea_out<<<blocks_for(n4, 256), 256, 0, st>>>(r, s, f, ncore, P, ea2);
-        g_launches.fetch_add(2, std::memory_order_relaxed);
-    }
-    cudaFreeAsync(G, st);
-    cudaFreeAsync(A1, st);
-    cudaFreeAsync(P, st);
-}
-void launch_koop0p(const Rdm &r, const double *atwo, const double *f, int ncore, double *gk0pa, double *gk0pd,
-                   double *gk0pf, cudaStream_t st) {
-    const int n = r.n;
-    const ll n3 = (ll)n * n * n, n4 = n3 * n, n6 = n3 * n3;
-    static thread_local KoopBlas blas;
-    double *G = nullptr, *Ai = nullptr, *P = nullptr;
-    const bool ok = (blas.h || cublasCreate(&blas.h) == CUBLAS_STATUS_SUCCESS) &&
-                    cublasSetStream(blas.h, st) == CUBLAS_STATUS_SUCCESS &&
-                    cudaMallocAsync((void **)&G, sizeof(double) * 4 * (size_t)n6, st) == cudaSuccess &&
-                    cudaMallocAsync((void **)&Ai, sizeof(double) * 3 * (size_t)n4, st) == cudaSuccess &&
-                    cudaMallocAsync((void **)&P, sizeof(double) * 4 * (size_t)n4, st) == cudaSuccess;
-    if (ok) {
-        double *A1 = Ai, *A2 = Ai + n4, *A3 = Ai + 2 * n4;
-        k_koop2E_ea_ints<<<blocks_for(n4, 256), 256, 0, st>>>(atwo, n, A1);
-        k_koop0p_ints<<<blocks_for(n4, 256), 256, 0, st>>>(atwo, n, A2, A3);
-        g_launches.fetch_add(2, std::memory_order_relaxed);
-        const double one = 1.0, zero = 0.0;
-        for (int s = 1; s <= r.M; ++s) {
-            k_koop0p_ops<<<blocks_for(4 * n6, 256), 256, 0, st>>>(r, s, G);
-            // row-major P01[2 n^3, n] = G[0:2 n^3] A1; P2 = G[2 n^3:3 n^3] A2; P3 = G[3 n^3:] A3
-            cublasDgemm(blas.h, CUBLAS_OP_N, CUBLAS_OP_N, n, (int)(2 * n3), (int)n3, &one, A1, n, G, (int)n3, &zero,
-                        P, n);
-            cublasDgemm(blas.h, CUBLAS_OP_N, CUBLAS_OP_N, n, (int)n3, (int)n3, &one, A2, n, G + 2 * n6, (int)n3, &zero,
-                        P + 2 * n4, n);
-            cublasDgemm(blas.h, CUBLAS_OP_N, CUBLAS_OP_N, n, (int)n3, (int)n3, &one, A3, n, G + 3 * n6, (int)n3, &zero,
-                        P + 3 * n4, n);
-            k_koop0p_out<<<blocks_for(n4, 256), 256, 0, st>>>(r, s, f, ncore, P, P + 2 * n4, P + 3 * n4, gk0pa, gk0pd);
-            g_launches.fetch_add(2, std::memory_order_relaxed);
-        }
-        cudaFreeAsync(G, st);
-        cudaFreeAsync(Ai, st);
-        cudaFreeAsync(P, st);
-    } else {  // no room for the operand blocks: the per-element kernel
-        if (G) cudaFreeAsync(G, st);
-        if (Ai) cudaFreeAsync(Ai, st);
-        k_koop0p_ad<<<blocks_for(n4, 64), 64, 0, st>>>(r, atwo, f, ncore, gk0pa, gk0pd);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-    }
-    k_koop0p_f<<<blocks_for((ll)r.n * r.n, 64), 64, 0, st>>>(r, atwo, f, ncore, gk0pf);
+void launch_koop_ctl(const Rdm &r, const double *atwo, const double *aj, int ncore, double *f, double *const out[8],
+                     cudaStream_t st) {
+    const int n = r.n, G = koop_pairs(n, 4 * r.M);
+    double *const so[5] = {out[3], out[4], out[5], out[6], out[2]};
+    const SymFlags flag(r, atwo, aj, ncore, 0, so, st);
+    KoopOut o;
+    for (int i = 0; i < 8; ++i) o.p[i] = out[i];
+    k_koop_ctl<<<dim3((n * n + G - 1) / G, 5, r.M), 256, koop_smem(n, G), st>>>(r, atwo, aj, ncore, G, f, o, flag.p);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
-void launch_bbmat(const Rdm &r, const double *atwo, const double *f, const double *aj, int ncore, double *b,
-                  double *bt, cudaStream_t st) {
-    ll n4 = (ll)r.n * r.n * r.n * r.n;
-    k_bbmat<<<blocks_for(n4, 64), 64, 0, st>>>(r, atwo, f, aj, ncore, b, bt);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-}
-void launch_bcmat(const Rdm &r, const double *atwo, const double *f, int ncore, double *c, double *ct,
+void launch_bbmat(const Rdm &r, const double *atwo, const double *aj, int ncore, double *f, double *b, double *bt,
                   cudaStream_t st) {
-    const int n = r.n;
-    const ll n3 = (ll)n * n * n, n4 = n3 * n, n6 = n3 * n3;
-    static thread_local KoopBlas blas;
-    double *G = nullptr, *Bi = nullptr, *P = nullptr;
-    const bool ok = (blas.h || cublasCreate(&blas.h) == CUBLAS_STATUS_SUCCESS) &&
-                    cublasSetStream(blas.h, st) == CUBLAS_STATUS_SUCCESS &&
-                    cudaMallocAsync((void **)&G, sizeof(double) * 6 * (size_t)n6, st) == cudaSuccess &&
-                    cudaMallocAsync((void **)&Bi, sizeof(double) * 2 * (size_t)n4, st) == cudaSuccess &&
-                    cudaMallocAsync((void **)&P, sizeof(double) * 6 * (size_t)n4, st) == cudaSuccess;
-    if (!ok) {  // no room for the operand blocks: the per-element kernel
-        if (G) cudaFreeAsync(G, st);
-        if (Bi) cudaFreeAsync(Bi, st);
-        k_bcmat<<<blocks_for(n4, 64), 64, 0, st>>>(r, atwo, f, ncore, c, ct);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        return;
-    }
-    double *B1 = Bi, *B2 = Bi + n4;
-    k_bcmat_ints<<<blocks_for(n4, 256), 256, 0, st>>>(atwo, n, B1, B2);
+    const int n = r.n, G = koop_pairs(n, 2 * r.M);
+    double *const so[5] = {b, bt};
+    const SymFlags flag(r, atwo, aj, ncore, 1, so, st);
+    k_koop_bc<<<dim3((n * n + G - 1) / G, 2, r.M), 256, koop_smem(n, G), st>>>(r, atwo, aj, ncore, G, 0, f, b, bt,
+                                                                              flag.p);
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    const double one = 1.0, zero = 0.0;
-    const double *Bs[3] = {B1, B2, B2};
-    for (int s = 1; s <= r.M; ++s) {
-        k_bcmat_ops<<<blocks_for(6 * n6, 256), 256, 0, st>>>(r, s, G);
-        for (int g = 0; g < 3; ++g)  // row-major P_g[2 n^3, n] = G[blocks 2g, 2g+1] B_g
-            cublasDgemm(blas.h, CUBLAS_OP_N, CUBLAS_OP_N, n, (int)(2 * n3), (int)n3, &one, Bs[g], n, G + 2 * g * n6,
-                        (int)n3, &zero, P + 2 * g * n4, n);
-        k_bcmat_out<<<blocks_for(n4, 256), 256, 0, st>>>(r, s, atwo, f, ncore, P, c, ct);
-        g_launches.fetch_add(2, std::memory_order_relaxed);
-    }
-    cudaFreeAsync(G, st);
-    cudaFreeAsync(Bi, st);
-    cudaFreeAsync(P, st);
 }
-void launch_bdmat(const Rdm &r, const double *atwo, const double *f, const double *aj, int ncore, double *d,
-                  double *dt, cudaStream_t st) {
-    k_bdmat<<<blocks_for((ll)r.n * r.n, 64), 64, 0, st>>>(r, atwo, f, aj, ncore, d, dt);
+void launch_bcmat(const Rdm &r, const double *atwo, const double *aj, int ncore, double *f, double *c, double *ct,
+                  cudaStream_t st) {
+    const int n = r.n, G = koop_pairs(n, 2 * r.M);
+    double *const so[5] = {c, ct};
+    const SymFlags flag(r, atwo, aj, ncore, 2, so, st);
+    for (int kind = 1; kind <= 2; ++kind)
+        k_koop_bc<<<dim3((n * n + G - 1) / G, 2, r.M), 256, koop_smem(n, G), st>>>(r, atwo, aj, ncore, G, kind, f, c, ct,
+                                                                                  flag.p);
+    g_launches.fetch_add(2, std::memory_order_relaxed);
+}
+void launch_bdmat(const Rdm &r, const double *atwo, const double *aj, int ncore, double *f, double *d, double *dt,
+                  cudaStream_t st) {
+    k_koop_d<<<dim3(r.n * r.n, r.M), 256, 0, st>>>(r, atwo, aj, ncore, f, d, dt);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 

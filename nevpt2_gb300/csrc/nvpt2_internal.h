@@ -18,19 +18,16 @@ void launch_bro2(const Rdm &r, double *taa, int nele, cudaStream_t st);
 void launch_bro1(const Rdm &r, double *dal, int nele, cudaStream_t st);
 void launch_aj_atwo(const double *oneint, const double *L, int Q, int n, int ncore, int norb, double *atwo,
                     double *aj, cudaStream_t st);
-void launch_koopE(const Rdm &r, const double *atwo, const double *f, int ncore, double *ip, double *ea,
+// The Koopmans builders; f receives the builder's operator on the active
+// triangle.  out: ipko1, eako1, hrdm2, ipko2, eako2, gk0pa, gk0pd, gk0pf.
+void launch_koop_ctl(const Rdm &r, const double *atwo, const double *aj, int ncore, double *f, double *const out[8],
+                     cudaStream_t st);
+void launch_bbmat(const Rdm &r, const double *atwo, const double *aj, int ncore, double *f, double *b, double *bt,
                   cudaStream_t st);
-void launch_hrdm(const Rdm &r, double *hrdm, cudaStream_t st);
-void launch_koop2E(const Rdm &r, const double *atwo, const double *f, int ncore, double *ip2, double *ea2,
-                   cudaStream_t st);
-void launch_koop0p(const Rdm &r, const double *atwo, const double *f, int ncore, double *gk0pa, double *gk0pd,
-                   double *gk0pf, cudaStream_t st);
-void launch_bbmat(const Rdm &r, const double *atwo, const double *f, const double *aj, int ncore, double *b,
-                  double *bt, cudaStream_t st);
-void launch_bcmat(const Rdm &r, const double *atwo, const double *f, int ncore, double *c, double *ct,
+void launch_bcmat(const Rdm &r, const double *atwo, const double *aj, int ncore, double *f, double *c, double *ct,
                   cudaStream_t st);
-void launch_bdmat(const Rdm &r, const double *atwo, const double *f, const double *aj, int ncore, double *d,
-                  double *dt, cudaStream_t st);
+void launch_bdmat(const Rdm &r, const double *atwo, const double *aj, int ncore, double *f, double *d, double *dt,
+                  cudaStream_t st);
 // One thread per element (bamat.cu); with flag, only the states s with flag[s] set.
 void launch_bamat_direct(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
                          cudaStream_t st, const int *flag);

@@ -625,7 +625,7 @@ class PencilFork {
         th_ = std::thread([this, Sp, Kp, n, thr]() {
             try {
                 ck(cudaSetDevice(dev_), "cudaSetDevice");
-                ok_ = metric_above(aux_[0], Sp, n, thr) && pencil_tridiag(aux_[0], Kp, Sp, n, pt_);
+                ok_ = pencil_tridiag(aux_[0], Kp, Sp, n, thr, pt_);
             } catch (...) {
                 err_ = std::current_exception();
             }
@@ -652,7 +652,7 @@ class PencilFork {
         } else {
             cudaStreamSynchronize(a.st);
         }
-        for (T *t : {&pt_.U, &pt_.A, &pt_.d, &pt_.e, &pt_.tau}) t->st = c_.st;
+        for (T *t : {&pt_.U, &pt_.A, &pt_.d, &pt_.e, &pt_.tau, &pt_.N}) t->st = c_.st;
         a.split = false;
         a.oz_err = nullptr;
         a.sm_share = 1;
@@ -899,8 +899,8 @@ class Runner {
                       const std::function<void(double *)> &fill) {
         if (nd == 0 || L == 0 || !c.all_pc_resolvent) return false;
         PencilTridiag PT;
-        if (!(metric_above(c, S.p, nd, thr) && pencil_tridiag(c, K.p, S.p, nd, PT))) return false;
-        acc.nnew[nnew_slot + 10 * s] = (int)nd;
+        if (!pencil_tridiag(c, K.p, S.p, nd, thr, PT)) return false;
+        acc.nnew[nnew_slot + 10 * s] = (int)(nd - PT.k);
         const long long rows = (long long)M * L;
         T Z = alloc(c, {rows, nd}, false);
         fill(Z.p);
@@ -1512,12 +1512,12 @@ class Runner {
                 for (int r = 0; r < nv; ++r) acc.rhoir[i + (size_t)nc * (r + (size_t)nv * s)] += rl[(size_t)i * nv + r];
         };
         PencilTridiag PT;
-        if (c.all_pc_resolvent && metric_above(c, S.p, n2, thr) && pencil_tridiag(c, K.p, S.p, n2, PT)) {
+        if (c.all_pc_resolvent && pencil_tridiag(c, K.p, S.p, n2, thr, PT)) {
             // every metric eigenvalue is kept: resolvents of the pencil (as in
             // the (+-1') classes) on the numerators before the PC basis change,
             //   z = [di A1 + 2 h g1 | -dj A1 + dk A2 - h g1]   (R = z C),
             // and for the density the vector g = [2 da | -da] (vaux = g C)
-            acc.nnew[8 + 10 * s] = (int)n2;
+            acc.nnew[8 + 10 * s] = (int)(n2 - PT.k);
             const long long rows = (long long)M * L + nrho;
             T Z = alloc(c, {rows, n2}, false);
             auto zrows = [&](const T &A1, const T &A2, const double *g1, double *out) {
@@ -1796,11 +1796,11 @@ class Runner {
                 }
         };
         if (fork && fork->join()) {
-            // Every metric eigenvalue is kept (nnew = n3): the PC sums over
+            // Every metric eigenvalue but exact zeros is kept: the PC sums over
             // the eigenpairs of K v = w S v are resolvents of the pencil,
             //   sum_mu r_mu^2 / (w_mu + s) = z^T (K + s S)^-1 z,
             // evaluated in the pencil's tridiagonal form (no eigenvectors).
-            acc.nnew[(minus ? 7 : 6) + 10 * s] = (int)n3;
+            acc.nnew[(minus ? 7 : 6) + 10 * s] = (int)(n3 - PT.k);
             // The QD cross terms and the densities need z_j^T x and g_d^T x
             // with x = (K + s S)^-1 z.  Mapping every z_j and g_d into the
             // tridiagonal basis costs M L + nd vector transforms; mapping the L

@@ -467,17 +467,102 @@ void reduce_to_standard(Ctx &c, double *A, const double *U, long long n) {
     }
 }
 
-bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, PencilTridiag &P) {
+namespace {
+// Deterministic start vectors of the inverse iteration, in [-0.5, 0.5).
+__global__ void k_start_block(double *X, long long count) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count) return;
+    unsigned long long z = (unsigned long long)(t + 1) * 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    X[t] = (double)((z ^ (z >> 31)) >> 11) * 0x1p-53 - 0.5;
+}
+
+// The null vectors of the positive semidefinite S (full storage), if its
+// eigenvalues below thr are all null: N [k, n] orthonormal rows.  Block inverse
+// iteration on S + delta, delta = 1e-9 of the largest diagonal element: a null
+// vector gains a factor w / delta on the kept ones in each of the three steps.
+// False if the metric is not of this kind.
+bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long long &k) {
+    const long long b = std::min<long long>(64, n);
+    k = 0;
+    T L = alloc(c, {n, n}, false), X = alloc(c, {b, n}, false), Y = alloc(c, {b, n}, false);
+    T w = alloc(c, {b}, false), H = alloc(c, {b, b}, false), V = alloc(c, {b, b}, false);
+    ck(cudaMemcpyAsync(L.p, S, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.st), "copy");
+    std::vector<double> dg(n);
+    ck(cudaMemcpy2DAsync(dg.data(), sizeof(double), S, sizeof(double) * (n + 1), sizeof(double), n,
+                         cudaMemcpyDeviceToHost, c.st), "diagonal");
+    ck(cudaStreamSynchronize(c.st), "sync");
+    double top = 0.0;
+    for (double x : dg) top = std::max(top, x);
+    if (!(top > 0.0)) return false;
+    k_add_diag<<<nblk(n), TPB, 0, c.st>>>(L.p, n, 1e-9 * top);
+    k_start_block<<<nblk(b * n), TPB, 0, c.st>>>(X.p, b * n);
+    g_launches.fetch_add(2, std::memory_order_relaxed);
+    const int Ni = (int)n, bi = (int)b;
+    int lw = 0;
+    ck(cusolverDnDpotrf_bufferSize(c.sol, CUBLAS_FILL_MODE_UPPER, Ni, L.p, Ni, &lw), "potrf_bufferSize");
+    SolverWork sw(c, lw);
+    ck(cusolverDnDpotrf(c.sol, CUBLAS_FILL_MODE_UPPER, Ni, L.p, Ni, sw.w, lw, sw.info), "potrf");
+    if (sw.status() != 0) return false;
+    // rows of X are the columns of a column-major [n, b]: solve, then orthonormalise by QR
+    T tau = alloc(c, {b}, false);
+    int lq = 0, lg = 0;
+    ck(cusolverDnDgeqrf_bufferSize(c.sol, Ni, bi, X.p, Ni, &lq), "geqrf_bufferSize");
+    ck(cusolverDnDorgqr_bufferSize(c.sol, Ni, bi, bi, X.p, Ni, tau.p, &lg), "orgqr_bufferSize");
+    SolverWork qw(c, std::max(lq, lg));
+    for (int it = 0; it < 3; ++it) {
+        ck(cusolverDnDpotrs(c.sol, CUBLAS_FILL_MODE_UPPER, Ni, bi, L.p, Ni, X.p, Ni, sw.info), "potrs");
+        ck(cusolverDnDgeqrf(c.sol, Ni, bi, X.p, Ni, tau.p, qw.w, lq, qw.info), "geqrf");
+        ck(cusolverDnDorgqr(c.sol, Ni, bi, bi, X.p, Ni, tau.p, qw.w, lg, qw.info), "orgqr");
+    }
+    std::vector<double> wh(b);
+    // Rayleigh-Ritz in the block
+    gemm(c, false, false, b, n, n, 1.0, X.p, n, S, n, 0.0, Y.p, n);
+    gemm(c, false, true, b, b, n, 1.0, Y.p, n, X.p, n, 0.0, H.p, b);
+    eigh_upper(c, H.p, b, w.p, V.p);
+    ck(cudaMemcpyAsync(wh.data(), w.p, sizeof(double) * b, cudaMemcpyDeviceToHost, c.st), "w copy");
+    ck(cudaStreamSynchronize(c.st), "sync");
+    while (k < b && !(wh[k] >= thr)) {
+        if (!(std::fabs(wh[k]) <= 1e-12 * top)) return false;
+        ++k;
+    }
+    if (k == 0 || k > 48) return false;
+    N = alloc(c, {k, n}, false);
+    gemm(c, false, false, k, n, b, 1.0, V.p, b, X.p, n, 0.0, N.p, n);
+    return true;
+}
+}  // namespace
+
+bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, double thr, PencilTridiag &P) {
     P.n = n;
+    P.k = 0;
     if (n == 0) return true;
     const int N = (int)n;
     P.U = alloc(c, {n, n}, false);
     P.A = alloc(c, {n, n}, false);
+    symmetrize_upper(c, S, n, P.U.p);
+    symmetrize_upper(c, K, n, P.A.p);
+    if (!metric_above(c, S, n, thr)) {
+        if (!metric_null(c, P.U.p, n, thr, P.N, P.k)) return false;
+        const long long k = P.k;
+        // S + N^T N, then every eigenvalue has to be above the threshold
+        gemm(c, true, false, n, n, k, 1.0, P.N.p, n, P.N.p, n, 1.0, P.U.p, n);
+        if (!metric_above(c, P.U.p, n, thr)) return false;
+        // P K P + N^T N = K - N^T G - G^T N + N^T (1 + G N^T) N with G = N K
+        T G = alloc(c, {k, n}, false), M = alloc(c, {k, k}, false), Q = alloc(c, {k, n}, false);
+        gemm(c, false, false, k, n, n, 1.0, P.N.p, n, P.A.p, n, 0.0, G.p, n);
+        gemm(c, false, true, k, k, n, 1.0, G.p, n, P.N.p, n, 0.0, M.p, k);
+        k_add_diag<<<nblk(k), TPB, 0, c.st>>>(M.p, k, 1.0);
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        gemm(c, false, false, k, n, k, 0.5, M.p, k, P.N.p, n, 0.0, Q.p, n);
+        axpby(c, k * n, 1.0, Q.p, -1.0, G.p, Q.p);  // Q = (1 + G N^T) N / 2 - G
+        gemm(c, true, false, n, n, k, 1.0, P.N.p, n, Q.p, n, 1.0, P.A.p, n);
+        gemm(c, true, false, n, n, k, 1.0, Q.p, n, P.N.p, n, 1.0, P.A.p, n);
+    }
     P.d = alloc(c, {n}, false);
     P.e = alloc(c, {n}, true);
     P.tau = alloc(c, {n}, true);
-    symmetrize_upper(c, S, n, P.U.p);
-    symmetrize_upper(c, K, n, P.A.p);
     int lw_p = 0;
     ck(cusolverDnDpotrf_bufferSize(c.sol, CUBLAS_FILL_MODE_UPPER, N, P.U.p, N, &lw_p), "potrf_bufferSize");
     SolverWork sw(c, lw_p);
@@ -502,6 +587,11 @@ void pencil_rhs(Ctx &c, const PencilTridiag &P, double *Y, long long m) {
     const double one = 1.0;
     ProfSpan sp;
     sp.begin("pencil_rhs", c.st, 0);
+    if (P.k) {  // rows of Y without their components along the null vectors
+        T a = alloc(c, {m, P.k}, false);
+        gemm(c, false, true, m, P.k, P.n, 1.0, Y, P.n, P.N.p, P.n, 0.0, a.p, P.k);
+        gemm(c, false, false, m, P.n, P.k, -1.0, a.p, P.k, P.N.p, P.n, 1.0, Y, P.n);
+    }
     ck(cublasDtrsm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT, N, Mc, &one,
                    P.U.p, N, Y, N),
        "trsm");

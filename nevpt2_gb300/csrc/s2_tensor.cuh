@@ -144,11 +144,18 @@ void symmetrize_upper(Ctx &c, const double *A, long long n, double *out);
 // off-diagonal e[n-1].  U, Q (reflectors + tau) stay in the struct, which
 // then maps right-hand sides into T's basis.  False if S is not positive
 // definite.
+// A metric with exact null vectors (those of a spin eigenfunction) and every other
+// eigenvalue above the threshold is deflated: with N its null vectors (rows, k of
+// them) and P = 1 - N^T N the pencil is P K P + N^T N, S + N^T N, whose null part is
+// a block of its own, and right-hand sides are projected by P.
 struct PencilTridiag {
     T U, A, d, e, tau;  // U: column-major upper factor; A: reflectors of Q
-    long long n = 0;
+    T N;                // null vectors of the metric [k, n]
+    long long n = 0, k = 0;
 };
-bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, PencilTridiag &P);
+// False, with nothing kept, unless every eigenvalue of S is above thr or null
+// (|w| <= 1e-12 of the largest; at most 48 of them).
+bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, double thr, PencilTridiag &P);
 // Upper triangle of A (column-major, symmetric) <- that of U^-T A U^-1.
 void reduce_to_standard(Ctx &c, double *A, const double *U, long long n);
 // Householder tridiagonalisation of the symmetric A (column-major; both

@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "../../include/nvpt2.h"
+#include "band.cuh"
 #include "s2_tensor.cuh"
 
 extern "C" unsigned nvpt_context_wait_limit(const nvpt_context *ctx);
@@ -652,7 +653,8 @@ class PencilFork {
         } else {
             cudaStreamSynchronize(a.st);
         }
-        for (T *t : {&pt_.U, &pt_.A, &pt_.d, &pt_.e, &pt_.tau, &pt_.N}) t->st = c_.st;
+        for (T *t : {&pt_.U, &pt_.A, &pt_.d, &pt_.e, &pt_.tau, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm})
+            t->st = c_.st;
         a.split = false;
         a.oz_err = nullptr;
         a.sm_share = 1;
@@ -872,7 +874,12 @@ class Runner {
         const long long L = (long long)shift.size(), n = PT.n;
         T sg = upload(c, shift);
         T a = alloc(c, {2 + 8}, true);
-        if (L > 0 && n > 0) {
+        if (L > 0 && n > 0 && PT.band) {
+            ProfSpan sp;
+            sp.begin("pencil_solve", c.st, 0);
+            band_resolvent(c, PT.AB.p, n, Yt.p, Yt.sh[1], L, nother < 0 ? M - 1 : nother, sg.p, a.p, nd, dcol0, rho, xout);
+            sp.end();
+        } else if (L > 0 && n > 0) {
             const size_t smem = sizeof(double) * 6 * (size_t)n;
             // one limit for every caller: pencils of different orders are
             // solved concurrently on other host threads

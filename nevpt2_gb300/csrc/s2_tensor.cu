@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "band.cuh"
 #include "ozaki.cuh"
 
 namespace nvpt {
@@ -416,7 +417,7 @@ namespace {
 __global__ void k_mirror_block(double *A, long long ld, int kb) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)kb * kb) return;
-    const int i = (int)(t % kb), j = (int)(t / kb);
+    const long long i = t % kb, j = t / kb;
     if (i > j) A[i + j * ld] = A[j + i * ld];
 }
 }  // namespace
@@ -560,9 +561,6 @@ bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, doubl
         gemm(c, true, false, n, n, k, 1.0, P.N.p, n, Q.p, n, 1.0, P.A.p, n);
         gemm(c, true, false, n, n, k, 1.0, Q.p, n, P.N.p, n, 1.0, P.A.p, n);
     }
-    P.d = alloc(c, {n}, false);
-    P.e = alloc(c, {n}, true);
-    P.tau = alloc(c, {n}, true);
     int lw_p = 0;
     ck(cusolverDnDpotrf_bufferSize(c.sol, CUBLAS_FILL_MODE_UPPER, N, P.U.p, N, &lw_p), "potrf_bufferSize");
     SolverWork sw(c, lw_p);
@@ -575,9 +573,25 @@ bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, doubl
     reduce_to_standard(c, P.A.p, P.U.p, n);
     sp.end();
     sp.begin("pencil_sytrd", c.st, 0);
-    const int trc = sytrd_lower(c, P.A.p, n, P.d.p, P.e.p, P.tau.p, true, std::min(4, std::max(1, c.sm_share)));
+    int trc;
+    P.band = n >= kPencilBandMin;
+    if (P.band) {
+        const int np = band_panels(n);
+        P.V = alloc(c, {band_rows(n), kBand}, false);
+        P.Tm = alloc(c, {np, kBand, kBand}, false);
+        P.AB = alloc(c, {kBand + 1, n}, false);
+        k_mirror_block<<<nblk(n * n), TPB, 0, c.st>>>(P.A.p, n, N);
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        trc = band_reduce(c, P.A.p, n, P.V.p, P.Tm.p, P.AB.p);
+        P.A.release();
+    } else {
+        P.d = alloc(c, {n}, false);
+        P.e = alloc(c, {n}, true);
+        P.tau = alloc(c, {n}, true);
+        trc = sytrd_lower(c, P.A.p, n, P.d.p, P.e.p, P.tau.p, true, std::min(4, std::max(1, c.sm_share)));
+    }
     sp.end();
-    if (trc != 0) throw Error(4, "tridiagonalisation: a grid barrier timed out");
+    if (trc != 0) throw Error(4, "pencil reduction: a grid barrier timed out");
     return true;
 }
 
@@ -595,6 +609,11 @@ void pencil_rhs(Ctx &c, const PencilTridiag &P, double *Y, long long m) {
     ck(cublasDtrsm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT, N, Mc, &one,
                    P.U.p, N, Y, N),
        "trsm");
+    if (P.band) {
+        band_apply(c, P.n, P.V.p, P.Tm.p, Y, m, true);
+        sp.end();
+        return;
+    }
     int lw = 0;
     ck(cusolverDnDormtr_bufferSize(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, N, Mc, P.A.p, N,
                                    P.tau.p, Y, N, &lw),
@@ -614,19 +633,24 @@ void pencil_back(Ctx &c, const PencilTridiag &P, double *X, long long m) {
     const double one = 1.0;
     ProfSpan sp;
     sp.begin("pencil_rhs", c.st, 0);
-    int lw = 0;
-    ck(cusolverDnDormtr_bufferSize(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, N, Mc, P.A.p, N,
-                                   P.tau.p, X, N, &lw),
-       "ormtr_bufferSize");
-    SolverWork sw(c, lw);
-    ck(cusolverDnDormtr(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, N, Mc, P.A.p, N, P.tau.p, X, N,
-                        sw.w, lw, sw.info),
-       "ormtr");
+    int st = 0;
+    if (P.band) {
+        band_apply(c, P.n, P.V.p, P.Tm.p, X, m, false);
+    } else {
+        int lw = 0;
+        ck(cusolverDnDormtr_bufferSize(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, N, Mc, P.A.p, N,
+                                       P.tau.p, X, N, &lw),
+           "ormtr_bufferSize");
+        SolverWork sw(c, lw);
+        ck(cusolverDnDormtr(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, N, Mc, P.A.p, N, P.tau.p, X,
+                            N, sw.w, lw, sw.info),
+           "ormtr");
+        st = sw.status();
+    }
     ck(cublasDtrsm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, N, Mc, &one,
                    P.U.p, N, X, N),
        "trsm");
     sp.end();
-    const int st = sw.status();
     if (st != 0) throw Error(2, "ormtr failed, info=" + std::to_string(st));
 }
 

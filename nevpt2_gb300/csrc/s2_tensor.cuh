@@ -148,8 +148,13 @@ void symmetrize_upper(Ctx &c, const double *A, long long n, double *out);
 // eigenvalue above the threshold is deflated: with N its null vectors (rows, k of
 // them) and P = 1 - N^T N the pencil is P K P + N^T N, S + N^T N, whose null part is
 // a block of its own, and right-hand sides are projected by P.
+// Orders of at least kPencilBandMin keep K~ = Q B Q^T in band form (band.cu: AB, V,
+// Tm) instead of the tridiagonal one.
+constexpr long long kPencilBandMin = 512;
 struct PencilTridiag {
     T U, A, d, e, tau;  // U: column-major upper factor; A: reflectors of Q
+    T AB, V, Tm;
+    bool band = false;
     T N;                // null vectors of the metric [k, n]
     long long n = 0, k = 0;
 };

@@ -28,6 +28,7 @@
 #include <cstdlib>
 
 #include "../../include/nvpt2.h"
+#include "grid_bar.cuh"
 #include "s2_tensor.cuh"
 
 namespace nvpt {
@@ -47,49 +48,6 @@ int sm_share(int share) {
     }();
     return v ? v : share;
 }
-constexpr unsigned kBarSpin = 1u << 22;  // polls (with back-off) before a barrier gives up
-
-struct Bar {
-    unsigned count, gen;
-    int err;
-};
-
-// Grid-wide barrier (all CTAs co-resident: cooperative launch).  Arrival is
-// an acq_rel add on the counter; the last CTA resets it and publishes the
-// next generation with a release store; the others poll the generation with
-// acquire loads.  Returns false if the wait timed out or another CTA
-// reported an error.
-__device__ bool grid_bar(Bar *b, unsigned nblk, unsigned &gen, unsigned limit) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const unsigned g = gen;
-        unsigned old;
-        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(&b->count) : "memory");
-        if (old == nblk - 1) {
-            asm volatile("st.relaxed.gpu.global.u32 [%0], 0;" ::"l"(&b->count) : "memory");
-            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&b->gen), "r"(g + 1) : "memory");
-        } else {
-            unsigned spins = 0, cur;
-            for (;;) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(&b->gen) : "memory");
-                if (cur != g) break;
-                if (++spins > limit || *(volatile int *)&b->err) {
-                    atomicExch(&b->err, 1);
-                    ok = 0;
-                    break;
-                }
-                if (spins > 64) __nanosleep(32);
-            }
-        }
-        gen = g + 1;
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
 __device__ __forceinline__ double block_sum(double v, double *red) {
     for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;

@@ -646,11 +646,10 @@ static int unfold_d(nvpt_context *ctx, int which, double *dst, int64_t ld, int64
     NV_TRY(check_nact(ctx, nact, 1));
     if (nentries < 0 || !dst || (nentries > 0 && (!labels || !values)) || ld < 1)
         return fail(ctx, NVPT_EINVAL, "permute_rdm: bad arguments");
-    const int64_t n = nact, W = n * (n + 1) * (n + 2) * (n + 3) / 24;
-    const int64_t slots = which == 4 ? W * n * n * n * n : n * n * n * n * n * n;
-    unsigned long long *owner = nullptr;
+    const int64_t n = nact;
+    void *owner = nullptr;
     int *bad = nullptr;
-    NV_TRY(cuda_check(ctx, cudaMallocAsync((void **)&owner, sizeof(unsigned long long) * slots, st), "permute_rdm"));
+    NV_TRY(cuda_check(ctx, cudaMallocAsync(&owner, unfold_scratch(which, (int)n, nentries), st), "permute_rdm"));
     if (cudaMallocAsync((void **)&bad, sizeof(int), st) != cudaSuccess) {
         cudaFreeAsync(owner, st);
         return fail(ctx, NVPT_ENOMEM, "permute_rdm: device allocation failed");

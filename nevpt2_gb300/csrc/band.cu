@@ -31,28 +31,36 @@ constexpr int NB = kBand;      // panel width = half bandwidth
 constexpr int TB = 256;        // threads per CTA
 constexpr int LP = NB + 1;     // padded row of a panel in shared memory
 
+constexpr int kQrMost = 39;  // CTAs of a panel: with the pivot row, at most 5 messages a thread
+constexpr unsigned long long kNoMsg = ~0ull;
+
 struct QrArgs {
     double *A;            // column-major n x n; panel columns j0 .. j0 + NB - 1, rows r0 .. n - 1
     long long n;
     int j0, m;            // m = n - r0 panel rows
     int chunk;            // rows per CTA (CTA 0 holds the pivot rows)
     double *V, *T, *G;    // V [m][NB] row-major, T [NB][NB] row-major; G [NB][NB] is zeroed for k_band_g
-    double *acc;          // [3][2 NB]: column sums and pivot rows, triple-buffered; zero on entry
-    Bar *bar;
-    unsigned spin;
+    unsigned long long *msg;  // [NB][CTAs + 1][NB], all kNoMsg on entry
+    int *err;
+    unsigned spin;        // polls before a wait gives up
 };
 
-// Householder QR of one panel, its rows in the shared memory of a few CTAs.  A
-// column costs one grid barrier: lane k of a warp holds entry k of a row, so the
-// sums a^T p_k over the rows below the pivot give, for k >= c, the reflector's
-// norm and the products it is applied with and, for k < c, the products with the
-// earlier reflectors that T needs.
+// Householder QR of one panel, its rows in the shared memory of a few CTAs.  Lane k
+// of a warp holds entry k of a row, so the sums a^T p_k over the rows below the
+// pivot give, for k >= c, the reflector's norm and the products it is applied with
+// and, for k < c, the products with the earlier reflectors that T needs.
+// Bound by latency: a column is one exchange of those sums between the CTAs.  Each
+// CTA stores its share where every other one polls for it (a word that is not
+// kNoMsg has arrived: one trip instead of the sums, fence, counter and flag of a
+// grid barrier, and the order of the additions is fixed); one warp turns the sums
+// into the reflector (a square root and two divisions in all eight would fill the
+// FP64 pipe for 2 us) and the update of a row also takes its share of the next
+// column's sums.  Order 2744: 7.3 -> 5.4 us a column.
 __global__ void __launch_bounds__(TB, 1) k_band_qr(QrArgs a) {
     extern __shared__ double P[];  // [chunk][LP]
-    __shared__ double red[TB / 32][NB], s_d[NB], s_p[NB], Gs[NB][NB + 1], tau_s[NB];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r0 = a.j0 + NB;
+    __shared__ double red[TB / 32][NB], red2[TB / 32][NB], s_p[NB], s_w[NB], Gs[NB][NB + 1], tau_s[NB], s_beta, s_scal;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r0 = a.j0 + NB, ctas = gridDim.x;
     const int i0 = blockIdx.x * a.chunk, rows = max(0, min(a.chunk, a.m - i0)), nref = min(NB, a.m);
-    unsigned gen = *(volatile unsigned *)&a.bar->gen;
     if (blockIdx.x == 0)
         for (int i = tid; i < NB * NB; i += TB) a.G[i] = 0.0;
     for (int i = tid; i < rows * NB; i += TB) {
@@ -60,53 +68,90 @@ __global__ void __launch_bounds__(TB, 1) k_band_qr(QrArgs a) {
         P[row * LP + k] = a.A[(r0 + i0 + row) + (a.j0 + k) * a.n];
     }
     __syncthreads();
+    double s = 0.0;
+    for (int row = warp; row < rows; row += TB / 32) {
+        const double p = P[row * LP + lane], x = __shfl_sync(0xffffffffu, p, 0);
+        if (i0 + row > 0) s = fma(x, p, s);
+    }
     for (int c = 0; c < nref; ++c) {
-        double *acc = a.acc + (c % 3) * 2 * NB, *accz = a.acc + ((c + 2) % 3) * 2 * NB;
-        double s = 0.0;
-        for (int row = warp; row < rows; row += TB / 32) {
-            const double p = P[row * LP + lane], x = __shfl_sync(0xffffffffu, p, c);
-            if (i0 + row > c) s = fma(x, p, s);
-        }
+        unsigned long long *msg = a.msg + (long long)c * (ctas + 1) * NB;
         red[warp][lane] = s;
         __syncthreads();
         if (warp == 0) {
             double t = 0.0;
+#pragma unroll
             for (int w = 0; w < TB / 32; ++w) t += red[w][lane];
-            atomicAdd(acc + lane, t);
-            if (blockIdx.x == 0) __stcg(acc + NB + lane, P[c * LP + lane]);
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(msg + blockIdx.x * NB + lane),
+                         "l"(__double_as_longlong(t)) : "memory");
+        } else if (warp == 1 && blockIdx.x == 0) {
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(msg + ctas * NB + lane),
+                         "l"(__double_as_longlong(P[c * LP + lane])) : "memory");
         }
-        if (!grid_bar(a.bar, gridDim.x, gen, a.spin)) return;
-        // this buffer's sums were last read before this barrier and are next added to after the coming one
-        if (blockIdx.x == 0 && tid < 2 * NB) __stcg(accz + tid, 0.0);
+        unsigned long long v[5];
+        int ok = 1;
+        for (unsigned spins = 0;;) {
+            bool all = true;
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                const int b = warp + q * (TB / 32);
+                v[q] = 0;
+                if (b <= ctas)
+                    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[q]) : "l"(msg + b * NB + lane) : "memory");
+            }
+#pragma unroll
+            for (int q = 0; q < 5; ++q) all = all && v[q] != kNoMsg;
+            if (all) break;
+            if (++spins > a.spin || (spins % 64 == 0 && *(volatile int *)a.err)) {
+                atomicExch(a.err, 1);
+                ok = 0;
+                break;
+            }
+        }
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            const int b = warp + q * (TB / 32);
+            if (b < ctas) t += __longlong_as_double(v[q]);
+            if (b == ctas) s_p[lane] = __longlong_as_double(v[q]);
+        }
+        red2[warp][lane] = t;
+        if (!__syncthreads_and(ok)) return;
         if (warp == 0) {
-            s_d[lane] = __ldcg(acc + lane);
-            s_p[lane] = __ldcg(acc + NB + lane);
+            double d = 0.0;
+#pragma unroll
+            for (int w = 0; w < TB / 32; ++w) d += red2[w][lane];
+            const double x2 = __shfl_sync(0xffffffffu, d, c), alpha = s_p[c];
+            double tau = 0.0, beta = alpha, scal = 0.0;
+            if (x2 != 0.0) {
+                beta = -copysign(sqrt(fma(alpha, alpha, x2)), alpha);
+                tau = (beta - alpha) / beta;
+                scal = 1.0 / (alpha - beta);
+            }
+            const double dot = fma(scal, d, s_p[lane]);  // v_c . p_k
+            s_w[lane] = lane > c ? tau * dot : 0.0;
+            if (lane == 0) {
+                s_beta = beta;
+                s_scal = scal;
+                tau_s[c] = tau;
+            }
+            Gs[lane][c] = dot;  // k < c: v_k . v_c
         }
         __syncthreads();
-        const double alpha = s_p[c], x2 = s_d[c];
-        double tau = 0.0, beta = alpha, scal = 0.0;
-        if (x2 != 0.0) {
-            beta = -copysign(sqrt(alpha * alpha + x2), alpha);
-            tau = (beta - alpha) / beta;
-            scal = 1.0 / (alpha - beta);
-        }
-        const double dot = s_p[lane] + scal * s_d[lane];  // v_c . p_k
-        if (blockIdx.x == 0 && warp == 0) {
-            Gs[lane][c] = dot;  // k < c: v_k . v_c
-            if (lane == 0) tau_s[c] = tau;
-        }
-        const double w = lane > c ? tau * dot : 0.0;
+        const double w = s_w[lane], scal = s_scal, beta = s_beta;
+        s = 0.0;
         for (int row = warp; row < rows; row += TB / 32) {
             const int i = i0 + row;
+            if (i < c) continue;
             double p = P[row * LP + lane];
             const double v = i == c ? 1.0 : scal * __shfl_sync(0xffffffffu, p, c);
-            if (i < c) continue;
             p = fma(-v, w, p);
             if (lane == c) p = i == c ? beta : v;
             P[row * LP + lane] = p;
+            const double x = __shfl_sync(0xffffffffu, p, (c + 1) & 31);
+            if (i > c + 1) s = fma(x, p, s);
         }
-        __syncthreads();
     }
+    __syncthreads();
     // R into A, V with its unit diagonal
     for (int i = tid; i < rows * NB; i += TB) {
         const int k = i % NB, row = i / NB, gi = i0 + row;
@@ -353,23 +398,30 @@ __device__ __forceinline__ void block_add2(double v, double *dst) {
 
 constexpr int UW = 2 * NB + 2;  // stored row of U: 1 / pivot, 2 NB entries right of it, the reduced right-hand side
 constexpr int WC = 128;         // circular column window (2 NB + 2 columns in use)
+constexpr int SL = NB + 2;      // slots: the NB + 1 rows that a column reaches and the row that comes in
 // The type-0 PC sums of one label (a CTA) from (B + sig)^-1 y: elimination with
 // partial pivoting over the NB + 1 rows a column reaches, kept in slots of shared
-// memory (a pivot is not moved: its slot takes the next row of B), rows of U
-// streamed out, then the back substitution by one warp.  Outputs as
-// k_tridiag_resolvent.  Bound by the FP64 pipe of one SM (2 NB^2 FMAs a column).
+// memory (a row is not moved: its slot is refilled once it was the pivot), rows of U
+// streamed out, then the back substitution by one warp.  The pivot is the largest
+// by the leading 32 bits.  Outputs as k_tridiag_resolvent.
+// Bound by the FP64 pipe of the label's SM (2 NB^2 FMAs, 66 warp instructions of 16
+// clocks, a column).  Warp 0 runs one column ahead of the others (its update,
+// pivot, reciprocal and multipliers, so that the chain of the search is hidden
+// behind the other columns' updates and its division done once), warp 7 moves the
+// rows in and out, so a column is one block barrier.  Order 2744, with the other
+// classes running: 4.6 -> 1.8 us a
+// column.
 __global__ void __launch_bounds__(TB) k_band_resolvent(const double *__restrict__ AB, long long n, const double *Y,
                                                        long long ncol, long long L, long long l0, int nother,
                                                        const double *sig, double *U, double *acc, int nd,
                                                        long long dcol0, double *rho, double *xout) {
     extern __shared__ double x[];  // solution, n
-    __shared__ double Wn[NB + 1][WC + 1], ys[NB + 1];
+    __shared__ double Wn[SL][WC + 1], ys[SL], fs[2][SL], s_inv[2];
+    __shared__ int s_piv[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long l = l0 + blockIdx.x;
     const double s = sig[l];
     double *Ul = U + (long long)blockIdx.x * n * UW;
-    for (int e = tid; e < (NB + 1) * (WC + 1); e += TB) Wn[0][e] = 0.0;
-    __syncthreads();
     // element t of row r: column r - NB + t
     auto band = [&](long long r, int t) {
         const long long c = r - NB + t;
@@ -377,65 +429,108 @@ __global__ void __launch_bounds__(TB) k_band_resolvent(const double *__restrict_
         const int k = t < NB ? NB - t : t - NB;
         return AB[k * n + (c < r ? c : r)] + (k == 0 ? s : 0.0);
     };
+    for (int e = tid; e < SL * (WC + 1); e += TB) Wn[0][e] = 0.0;
+    __syncthreads();
     for (int e = tid; e < (NB + 1) * (2 * NB + 1); e += TB) {
         const int r = e / (2 * NB + 1), t = e % (2 * NB + 1), c = r - NB + t;
         if (c >= 0 && r < n) Wn[r][c & (WC - 1)] = band(r, t);
     }
-    if (tid <= NB) ys[tid] = tid < n ? Y[tid * ncol + l] : 0.0;
+    if (tid < SL) ys[tid] = tid <= NB && tid < n ? Y[tid * ncol + l] : 0.0;
     __syncthreads();
-    int live = (int)min((long long)(NB + 1), n);  // slots 0 .. live - 1 hold rows (all slots but at the end)
-    unsigned long long dead = 0;                  // slots whose row is used up and not replaced
-    for (int e = live; e <= NB; ++e) dead |= 1ull << e;
-    for (long long j = 0; j < n; ++j) {
-        const int cj = (int)(j & (WC - 1));
-        const long long rn = j + NB + 1;
-        double next = 0.0, ynext = 0.0;  // the row that takes the pivot's slot
-        if (tid <= 2 * NB) next = band(rn, tid);
-        else if (tid == 2 * NB + 1 && rn < n) ynext = Y[rn * ncol + l];
-        // the pivot: every warp finds the same one
-        double best = (dead >> lane & 1) ? -1.0 : fabs(Wn[lane][cj]);
-        int p = lane;
-        if (lane == 0 && !(dead >> NB & 1)) {
-            const double b = fabs(Wn[NB][cj]);
-            if (b > best) { best = b; p = NB; }
+    // slots without a row: the one that is filled next (free) and, at the end, used-up ones
+    int free_slot = NB + 1;
+    unsigned long long none = ~0ull << min((long long)(NB + 1), n);
+    double f0 = 0.0, f1 = 0.0;  // warp 0: the multipliers of slots lane and 32 + lane
+    // warp 0: pivot, reciprocal and multipliers of column j from its entries v0, v1 in the slots
+    auto select = [&](long long j, double v0, double v1, unsigned long long off) {
+        unsigned k0 = off >> lane & 1 ? 0u : ((unsigned)__double2hiint(v0) & 0x7fffffffu) + 1u;
+        unsigned k1 = lane >= SL - 32 || (off >> (32 + lane) & 1) ? 0u : ((unsigned)__double2hiint(v1) & 0x7fffffffu) + 1u;
+        const unsigned top = __reduce_max_sync(0xffffffffu, max(k0, k1));
+        const int from = __ffs(__ballot_sync(0xffffffffu, max(k0, k1) == top)) - 1;
+        const double pv = __shfl_sync(0xffffffffu, k1 > k0 ? v1 : v0, from);
+        const int slot = __shfl_sync(0xffffffffu, k1 > k0 ? 32 + lane : lane, from);
+        const double inv = 1.0 / pv;
+        f0 = v0 * inv;
+        f1 = v1 * inv;
+        const int b = (int)(j & 1);
+        fs[b][lane] = f0;
+        if (lane < SL - 32) fs[b][32 + lane] = f1;
+        if (lane == 0) {
+            s_piv[b] = slot;
+            s_inv[b] = inv;
         }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const double b = __shfl_xor_sync(0xffffffffu, best, o);
-            const int q = __shfl_xor_sync(0xffffffffu, p, o);
-            if (b > best || (b == best && q < p)) { best = b; p = q; }
-        }
-        const double inv = 1.0 / Wn[p][cj], yp = ys[p];
-        const int c0 = (cj + 1 + lane) & (WC - 1), c1 = (cj + 1 + NB + lane) & (WC - 1), cz = (cj + 1 + 2 * NB) & (WC - 1);
-        const double p0 = Wn[p][c0], p1 = Wn[p][c1];
+    };
+    if (warp == 0) select(0, Wn[lane][0], lane < SL - 32 ? Wn[32 + lane][0] : 0.0, none);
+    // rows that come in, PF columns ahead: warp 7 whole rows, warp 0 their first entries
+    constexpr int PF = 4;
+    double a0[PF], a1[PF], a2[PF];
+    auto fetch = [&](long long j, int q) {
+        const long long r = j + NB + 1;
         if (warp == 7) {
-            Ul[j * UW + 1 + lane] = p0;
-            Ul[j * UW + 1 + NB + lane] = p1;
-            if (lane == 0) Ul[j * UW] = inv;
-            if (lane == 1) Ul[j * UW + 2 * NB + 1] = yp;
+            a0[q] = band(r, lane);
+            a1[q] = band(r, NB + lane);
+            a2[q] = lane == 0 ? band(r, 2 * NB) : lane == 1 && r < n ? Y[r * ncol + l] : 0.0;
+        } else if (warp == 0) {
+            a0[q] = band(r, 0);
         }
-        for (int q = warp; q <= NB; q += TB / 32) {
-            if (q == p || (dead >> q & 1)) continue;
-            const double f = Wn[q][cj] * inv;
-            Wn[q][c0] = fma(-f, p0, Wn[q][c0]);
-            Wn[q][c1] = fma(-f, p1, Wn[q][c1]);
-            if (lane == 0) {
-                ys[q] = fma(-f, yp, ys[q]);
-                Wn[q][cz] = 0.0;  // a column that enters the window
+    };
+#pragma unroll
+    for (int q = 0; q < PF; ++q) fetch(q, q);
+    __syncthreads();
+    for (long long jb = 0; jb < n; jb += PF) {
+#pragma unroll
+        for (int q = 0; q < PF; ++q) {
+            const long long j = jb + q;
+            if (j >= n) break;
+            const int b = (int)(j & 1), p = s_piv[b], in = free_slot, c1 = (int)((j + 1) & (WC - 1));
+            const bool more = j + NB + 1 < n;
+            const unsigned long long off = none | 1ull << p;  // slots not updated
+            unsigned long long next = off;                    // slots without a row after this column
+            if (more) next &= ~(1ull << in);
+            if (warp == 0) {
+                const double pc = Wn[p][c1];
+                double v0 = off >> lane & 1 ? 0.0 : fma(-f0, pc, Wn[lane][c1]), v1 = 0.0;
+                if (lane < SL - 32 && !(off >> (32 + lane) & 1)) v1 = fma(-f1, pc, Wn[32 + lane][c1]);
+                if (more && lane == in) v0 = a0[q];
+                if (more && 32 + lane == in) v1 = a0[q];
+                if (j + 1 < n) select(j + 1, v0, v1, next);
+            } else if (warp < 7) {
+                // columns j + 2 .. j + 65; the last one enters the window
+                const int ca = (int)((j + 2 + lane) & (WC - 1)), cb = (int)((j + 2 + NB + lane) & (WC - 1));
+                const double pa = Wn[p][ca], pb = Wn[p][cb];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    const int r = warp - 1 + 6 * k;
+                    if (r < SL && !(off >> r & 1)) {
+                        const double f = fs[b][r];
+                        Wn[r][ca] = fma(-f, pa, Wn[r][ca]);
+                        Wn[r][cb] = lane == 31 ? 0.0 : fma(-f, pb, Wn[r][cb]);
+                    }
+                }
+            } else {
+                const double yp = ys[p];
+                double *u = Ul + j * UW;
+                u[1 + lane] = Wn[p][(int)((j + 1 + lane) & (WC - 1))];
+                u[1 + NB + lane] = Wn[p][(int)((j + 1 + NB + lane) & (WC - 1))];
+                if (lane == 0) u[0] = s_inv[b];
+                if (lane == 1) u[2 * NB + 1] = yp;
+                if (!(off >> lane & 1)) ys[lane] = fma(-fs[b][lane], yp, ys[lane]);
+                if (lane < SL - 32 && !(off >> (32 + lane) & 1)) ys[32 + lane] = fma(-fs[b][32 + lane], yp, ys[32 + lane]);
+                if (more) {
+                    Wn[in][(int)((j + 1 + lane) & (WC - 1))] = a0[q];
+                    Wn[in][(int)((j + 1 + NB + lane) & (WC - 1))] = a1[q];
+                    if (lane == 0) Wn[in][(int)((j + 1 + 2 * NB) & (WC - 1))] = a2[q];
+                    if (lane == 1) ys[in] = a2[q];
+                }
             }
+            fetch(j + PF, q);
+            none = next;
+            free_slot = p;
+            __syncthreads();
         }
-        __syncthreads();
-        if (rn < n) {
-            if (tid <= 2 * NB) Wn[p][(int)((j + 1 + tid) & (WC - 1))] = next;
-            else if (tid == 2 * NB + 1) ys[p] = ynext;
-        } else {
-            dead |= 1ull << p;
-        }
-        __syncthreads();
     }
     // back substitution: a warp, two entries of a row per lane, rows prefetched
     if (warp == 0) {
-        constexpr int PF = 4;
         double u0[PF], u1[PF], dv[PF], yv[PF];
         auto load = [&](long long j, int q) {
             const double *u = Ul + max(j, 0ll) * UW;
@@ -491,9 +586,8 @@ long long band_rows(long long n) {  // rows of all panels
 int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *AB) {
     const int np = band_panels(n);
     T W = alloc(c, {n, NB}, false), G = alloc(c, {NB, NB}, false);
-    T ctl = alloc(c, {2 + 6 * NB}, true);  // Bar, column sums
-    Bar *bar = (Bar *)ctl.p;
-    double *acc = ctl.p + 2;
+    T msg = alloc(c, {NB, kQrMost + 1, NB}, false), ctl = alloc(c, {1}, true);
+    int *err = (int *)ctl.p;
     int sms = 0, dev = 0;
     ck(cudaGetDevice(&dev), "cudaGetDevice");
     ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr");
@@ -506,12 +600,12 @@ int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *A
         const int j0 = p * NB, r0 = j0 + NB, m = (int)n - r0;
         double *t = Tm + (long long)p * NB * NB;
         // 64 to 128 panel rows per CTA: the column's latency falls with its rows, and rises with the CTAs
-        const int G0 = std::max(1, std::min(sms / 4, m / 64));
+        const int G0 = std::max(1, std::min(std::min(sms / 4, kQrMost), m / 64));
         const int chunk = std::max(NB, (m + G0 - 1) / G0), ctas = (m + chunk - 1) / chunk;
         const size_t smem = sizeof(double) * (size_t)chunk * LP;
         if ((long long)smem > lim) throw Error(1, "band: order too large for the panel's shared memory");
-        if (p) ck(cudaMemsetAsync(acc, 0, sizeof(double) * 6 * NB, c.st), "memset");
-        QrArgs q{A, n, j0, m, chunk, v, t, G.p, acc, bar, c.wait_limit ? c.wait_limit : kBarSpin};
+        ck(cudaMemsetAsync(msg.p, 0xff, sizeof(double) * NB * (ctas + 1) * NB, c.st), "memset");
+        QrArgs q{A, n, j0, m, chunk, v, t, G.p, (unsigned long long *)msg.p, err, c.wait_limit ? c.wait_limit : kBarSpin};
         void *args[] = {&q};
         ck(cudaLaunchCooperativeKernel((const void *)k_band_qr, dim3(ctas), dim3(TB), args, smem, c.st),
            "cooperative launch");
@@ -528,10 +622,10 @@ int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *A
     k_band_extract<<<(unsigned)((n * (NB + 1) + 255) / 256), 256, 0, c.st>>>(A, n, AB);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     ck(cudaGetLastError(), "band reduction");
-    int h[3] = {0, 0, 0};
-    ck(cudaMemcpyAsync(h, ctl.p, sizeof(int) * 3, cudaMemcpyDeviceToHost, c.st), "barrier state");
+    int h = 0;
+    ck(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, c.st), "wait state");
     ck(cudaStreamSynchronize(c.st), "band sync");
-    return h[2] ? 4 : 0;
+    return h ? 4 : 0;
 }
 
 void band_apply(Ctx &c, long long n, const double *V, const double *Tm, double *Y, long long m, bool forward) {

@@ -119,8 +119,33 @@ struct IjklState {
     }
 };
 
+namespace {
+// A context's staging block of the host-pointer calls: device memory and its pinned
+// host image, made by the first such call and kept for the context's life.
+struct Pack {
+    static constexpr size_t kBytes = 1u << 20, kMost = 128u << 10;  // in all, and of one array
+    std::mutex mu;
+    char *dev = nullptr, *host = nullptr;
+    bool ready(int device) {
+        int cur = -1;
+        if (cudaGetDevice(&cur) != cudaSuccess || cur != device) return false;
+        if (dev) return true;
+        if (cudaMalloc((void **)&dev, kBytes) != cudaSuccess) dev = nullptr;
+        else if (cudaHostAlloc((void **)&host, kBytes, cudaHostAllocDefault) != cudaSuccess) release();
+        if (!dev) cudaGetLastError();  // the arrays are copied by themselves
+        return dev != nullptr;
+    }
+    void release() {
+        cudaFree(dev);
+        cudaFreeHost(host);
+        dev = host = nullptr;
+    }
+};
+}  // namespace
+
 struct nvpt_context {
     int device = 0;
+    Pack pack;
     int precision = NVPT_PRECISION_FP64;
     cudaStream_t stream = nullptr;
     std::string err;
@@ -180,50 +205,98 @@ int64_t ipow(int64_t b, int e) {
 int64_t f_len(int64_t nact, int64_t ncore) { return (ncore + nact) * (ncore + nact + 1) / 2; }
 
 // Stream-ordered device staging area for one host-pointer call.
-struct Stage {
+class Stage {
     nvpt_context *ctx;
     cudaStream_t st;
     std::vector<void *> bufs;
-    int status = NVPT_OK;
-    Stage(nvpt_context *c) : ctx(c), st(c->stream) {}
+    // Small arrays share the context's staging block: packed on the host, they take
+    // one copy each way (a copy of a few KB costs 5 to 10 us of latency whatever its
+    // size).  Larger ones, and a call that finds the block in use by another thread,
+    // are copied by themselves.
+    struct Back {
+        double *h;
+        size_t off, bytes;
+    };
+    int status_ = NVPT_OK;  // read through commit(), which nothing may leave out
+    std::unique_lock<std::mutex> lock;
+    size_t used = 0, sent = 0;
+    std::vector<Back> back;
+
+  public:
+    explicit Stage(nvpt_context *c) : ctx(c), st(c->stream), lock(c->pack.mu, std::try_to_lock) {
+        if (lock.owns_lock() && !c->pack.ready(c->device)) lock.unlock();
+    }
     ~Stage() {
         for (void *p : bufs) cudaFreeAsync(p, st);
         cudaStreamSynchronize(st);
     }
-    double *alloc(int64_t count) {
-        if (status != NVPT_OK) return nullptr;
-        void *p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, sizeof(double) * (size_t)(count > 0 ? count : 1), st);
-        if (e != cudaSuccess) { status = cuda_check(ctx, e, "cudaMallocAsync"); return nullptr; }
-        bufs.push_back(p);
-        return (double *)p;
-    }
-    double *up(const double *h, int64_t count) {
-        double *d = alloc(count);
-        if (!d) return nullptr;
-        cudaError_t e = cudaMemcpyAsync(d, h, sizeof(double) * (size_t)count, cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) { status = cuda_check(ctx, e, "H2D copy"); return nullptr; }
-        return d;
-    }
-    void *up_bytes(const void *h, size_t bytes) {
-        if (status != NVPT_OK) return nullptr;
-        void *p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, bytes > 0 ? bytes : 1, st);
-        if (e != cudaSuccess) { status = cuda_check(ctx, e, "cudaMallocAsync"); return nullptr; }
-        bufs.push_back(p);
-        e = cudaMemcpyAsync(p, h, bytes, cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) { status = cuda_check(ctx, e, "H2D copy"); return nullptr; }
+    // a piece of the staging block, or null
+    char *piece(size_t bytes) {
+        if (!lock.owns_lock() || bytes > Pack::kMost || used + bytes > Pack::kBytes) return nullptr;
+        char *p = ctx->pack.dev + used;
+        used += (bytes + 255) / 256 * 256;
         return p;
     }
+    void *alloc_bytes(size_t bytes) {
+        if (status_ != NVPT_OK) return nullptr;
+        void *p = piece(bytes);
+        if (p) return p;
+        cudaError_t e = cudaMallocAsync(&p, bytes > 0 ? bytes : 1, st);
+        if (e != cudaSuccess) { status_ = cuda_check(ctx, e, "cudaMallocAsync"); return nullptr; }
+        bufs.push_back(p);
+        return p;
+    }
+    bool packed(const void *p) const {
+        return lock.owns_lock() && (const char *)p >= ctx->pack.dev && (const char *)p < ctx->pack.dev + Pack::kBytes;
+    }
+    double *alloc(int64_t count) { return (double *)alloc_bytes(sizeof(double) * (size_t)(count > 0 ? count : 0)); }
+    void *up_bytes(const void *h, size_t bytes) {
+        void *p = alloc_bytes(bytes);
+        if (!p) return nullptr;
+        if (packed(p) && h) {
+            const size_t off = (char *)p - ctx->pack.dev;
+            std::memcpy(ctx->pack.host + off, h, bytes);
+            sent = off + bytes;
+            return p;
+        }
+        cudaError_t e = cudaMemcpyAsync(p, h, bytes, cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess) { status_ = cuda_check(ctx, e, "H2D copy"); return nullptr; }
+        return p;
+    }
+    double *up(const double *h, int64_t count) { return (double *)up_bytes(h, sizeof(double) * (size_t)count); }
+    // Sends the packed inputs, before the first kernel; the staging's status so far.
+    int commit() {
+        if (status_ == NVPT_OK && sent) {
+            cudaError_t e = cudaMemcpyAsync(ctx->pack.dev, ctx->pack.host, sent, cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess) status_ = cuda_check(ctx, e, "H2D copy");
+        }
+        return status_;
+    }
     int down(double *h, const double *d, int64_t count) {
-        if (status != NVPT_OK) return status;
+        if (status_ != NVPT_OK) return status_;
+        if (packed(d) && h) {
+            back.push_back({h, (size_t)((const char *)d - ctx->pack.dev), sizeof(double) * (size_t)count});
+            return status_;
+        }
         cudaError_t e = cudaMemcpyAsync(h, d, sizeof(double) * (size_t)count, cudaMemcpyDeviceToHost, st);
-        if (e != cudaSuccess) status = cuda_check(ctx, e, "D2H copy");
-        return status;
+        if (e != cudaSuccess) status_ = cuda_check(ctx, e, "D2H copy");
+        return status_;
     }
     int finish() {
-        if (status != NVPT_OK) return status;
-        return cuda_check(ctx, cudaStreamSynchronize(st), "stream synchronize");
+        if (status_ != NVPT_OK) return status_;
+        size_t lo = Pack::kBytes, hi = 0;
+        for (const Back &b : back) {
+            lo = std::min(lo, b.off);
+            hi = std::max(hi, b.off + b.bytes);
+        }
+        if (lo < hi) {
+            cudaError_t e = cudaMemcpyAsync(ctx->pack.host + lo, ctx->pack.dev + lo, hi - lo, cudaMemcpyDeviceToHost, st);
+            if (e != cudaSuccess) return status_ = cuda_check(ctx, e, "D2H copy");
+        }
+        int rc = cuda_check(ctx, cudaStreamSynchronize(st), "stream synchronize");
+        if (rc == NVPT_OK)
+            for (const Back &b : back) std::memcpy(b.h, ctx->pack.host + b.off, b.bytes);
+        return rc;
     }
 };
 
@@ -264,6 +337,7 @@ int nvpt_destroy(nvpt_context *ctx) {
     if (!ctx) return NVPT_EINVAL;
     cudaStreamSynchronize(ctx->stream);
     ctx->ijkl.release();
+    ctx->pack.release();
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return NVPT_OK;
@@ -538,8 +612,8 @@ int nvpt_ai_twoint(nvpt_context *ctx, int64_t count, const int64_t *ijkl, double
     Stage sg(ctx);
     const int64_t *d_q = (const int64_t *)sg.up_bytes(ijkl, sizeof(int64_t) * 4 * (size_t)count);
     double *d_o = sg.alloc(count);
-    NV_TRY(sg.status);
-    launch_ai_twoint(T, count, d_q, d_o, sg.st);
+    NV_TRY(sg.commit());
+    launch_ai_twoint(T, count, d_q, d_o, ctx->stream);
     NV_TRY(after_launch(ctx, "ai_twoint"));
     sg.down(out, d_o, count);
     return sg.finish();
@@ -563,8 +637,8 @@ int nvpt_get_aj_atwo_twoint(nvpt_context *ctx, double *atwo, int64_t nact, int64
     const int64_t npair = norb * (norb + 1) / 2;
     Stage sg(ctx);
     double *d_one = sg.up(oneint, npair), *d_aj = sg.alloc(npair), *d_atwo = sg.alloc(ipow(nact, 4));
-    NV_TRY(sg.status);
-    NV_TRY(nvpt_get_aj_atwo_twoint_d(ctx, d_atwo, nact, ncore, norb, d_aj, d_one, sg.st));
+    NV_TRY(sg.commit());
+    NV_TRY(nvpt_get_aj_atwo_twoint_d(ctx, d_atwo, nact, ncore, norb, d_aj, d_one, ctx->stream));
     sg.down(atwo, d_atwo, ipow(nact, 4));
     sg.down(aj, d_aj, npair);
     return sg.finish();
@@ -819,7 +893,7 @@ int nvpt_bro3(nvpt_context *ctx, const double *ro4, double *daaa, int64_t nact, 
     Stage S(ctx);
     const double *d_ro4 = S.up(ro4, W * n4 * metat);
     double *d_out = S.alloc(n6 * metat);
-    if (S.status) return S.status;
+    if (int rc = S.commit()) return rc;
     NV_TRY(nvpt_bro3_d(ctx, d_ro4, d_out, nact, nele, metat, nullptr));
     S.down(daaa, d_out, n6 * metat);
     return S.finish();
@@ -831,7 +905,7 @@ int nvpt_bro2(nvpt_context *ctx, const double *daaa, double *taa, int64_t nact, 
     Stage S(ctx);
     const double *d_in = S.up(daaa, n6 * metat);
     double *d_out = S.alloc(n4 * metat);
-    if (S.status) return S.status;
+    if (int rc = S.commit()) return rc;
     NV_TRY(nvpt_bro2_d(ctx, d_in, d_out, nact, nele, metat, nullptr));
     S.down(taa, d_out, n4 * metat);
     return S.finish();
@@ -843,7 +917,7 @@ int nvpt_bro1(nvpt_context *ctx, const double *taa, double *dal, int64_t nact, i
     Stage S(ctx);
     const double *d_in = S.up(taa, n4 * metat);
     double *d_out = S.alloc(n2 * metat);
-    if (S.status) return S.status;
+    if (int rc = S.commit()) return rc;
     NV_TRY(nvpt_bro1_d(ctx, d_in, d_out, nact, nele, metat, nullptr));
     S.down(dal, d_out, n2 * metat);
     return S.finish();
@@ -859,7 +933,7 @@ int nvpt_get_aj_atwo(nvpt_context *ctx, double *atwo, int64_t nact, int64_t ncor
     const double *d_L = S.up(chol, npair * nchovec);
     double *d_atwo = S.alloc(ipow(nact, 4));
     double *d_aj = S.alloc(npair);
-    if (S.status) return S.status;
+    if (int rc = S.commit()) return rc;
     NV_TRY(nvpt_get_aj_atwo_d(ctx, d_atwo, nact, ncore, norb, d_aj, d_one, d_L, nchovec, nullptr));
     S.down(atwo, d_atwo, ipow(nact, 4));
     S.down(aj, d_aj, npair);
@@ -879,7 +953,7 @@ int nvpt_koop_matrices_ctl(nvpt_context *ctx, int64_t metat, int64_t nact, int64
     const double *d_aj = S.up(aj, nf);
     double *o_ip1 = S.alloc(n2 * M), *o_ea1 = S.alloc(n2 * M), *o_h = S.alloc(n4 * M), *o_ip2 = S.alloc(n4 * M);
     double *o_ea2 = S.alloc(n4 * M), *o_a = S.alloc(n4 * M), *o_d = S.alloc(n4 * M), *o_f = S.alloc(n2 * M);
-    if (S.status) return S.status;
+    if (int rc = S.commit()) return rc;
     NV_TRY(nvpt_koop_matrices_ctl_d(ctx, metat, nact, ncore, d_atwo, d3, d2, d1, d_f, d_aj, o_ip1, o_ea1, o_h, o_ip2,
                                     o_ea2, o_a, o_d, o_f, nullptr));
     S.down(ipko1, o_ip1, n2 * M); S.down(eako1, o_ea1, n2 * M); S.down(hrdm2, o_h, n4 * M);
@@ -901,7 +975,7 @@ int nvpt_bamat(nvpt_context *ctx, double *amat, double *atmat, const double *atw
     double *d_f = S.up(f, nf);
     const double *d_aj = S.up(aj, nf);
     double *o_a = S.alloc(n6 * M), *o_at = S.alloc(n6 * M);
-    if (S.status) return S.status;
+    if (int rc = S.commit()) return rc;
     NV_TRY(nvpt_bamat_d(ctx, o_a, o_at, d_atwo, d_ro4, d3, d2, d1, nact, ncore, d_f, d_aj, norb, metat, nsym, nullptr));
     S.down(amat, o_a, n6 * M); S.down(atmat, o_at, n6 * M); S.down(f, d_f, nf);
     return S.finish();
@@ -918,7 +992,7 @@ static int unfold_host(nvpt_context *ctx, int which, double *dst, int64_t ld, in
     const int32_t *l = nentries ? (const int32_t *)S.up_bytes(labels, sizeof(int32_t) * (which == 4 ? 8 : 6) * nentries)
                                 : nullptr;
     const double *v = nentries ? S.up(values, nentries) : nullptr;
-    if (S.status) return S.status;
+    if (int rc = S.commit()) return rc;
     NV_TRY(unfold_d(ctx, which, d, ld, nact, l, v, nentries, trans, ctx->stream));
     S.down(dst, d, count);
     return S.finish();
@@ -947,7 +1021,7 @@ static int bcd_host(nvpt_context *ctx, int which, const double *atwo, double *x,
     double *d_f = S.up(f, nf);
     const double *d_aj = S.up(aj, nf);
     double *o = S.alloc(nout), *ot = S.alloc(nout);
-    if (S.status) return S.status;
+    if (int rc = S.commit()) return rc;
     int rc;
     if (which == 1) rc = nvpt_bbmat_d(ctx, d_atwo, o, ot, d3, d2, d1, nact, ncore, d_f, d_aj, metat, nullptr);
     else if (which == 2) rc = nvpt_bcmat_d(ctx, d_atwo, o, ot, d3, d2, d1, nact, ncore, d_f, d_aj, metat, nullptr);

@@ -613,6 +613,7 @@ class PencilFork {
         a.sm_share = c_.sm_share;
         a.wait_limit = c_.wait_limit;
         a.all_pc_resolvent = c_.all_pc_resolvent;
+        a.arena = c_.arena;
         try {
             ck(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming), "cudaEventCreate");
             ck(cudaEventCreateWithFlags(&done_, cudaEventDisableTiming), "cudaEventCreate");
@@ -660,6 +661,7 @@ class PencilFork {
         a.sm_share = 1;
         a.wait_limit = 0;
         a.all_pc_resolvent = false;
+        a.arena = nullptr;
         CtxPool::release(aux_, dev_);
         if (ready_) cudaEventDestroy(ready_);
         if (done_) cudaEventDestroy(done_);
@@ -1936,6 +1938,7 @@ struct ClassStreams {
             x.sm_share = 1;
             x.wait_limit = 0;
             x.all_pc_resolvent = false;
+            x.arena = nullptr;
         }
         CtxPool::release(c, dev);
     }
@@ -1954,18 +1957,31 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
         err = "qdnevpt: empty class mask";
         return NVPT_EINVAL;
     }
-    Ctx c{st, nullptr, nullptr};
-    ck(cublasCreate(&c.blas), "cublasCreate");
-    ck(cublasSetStream(c.blas, st), "cublasSetStream");
-    ck(cusolverDnCreate(&c.sol), "cusolverDnCreate");
-    ck(cusolverDnSetStream(c.sol, st), "cusolverDnSetStream");
+    // The handles of a pooled context, on the caller's stream (creating and destroying
+    // a pair costs 6 ms).
     struct Handles {
-        Ctx &c;
-        ~Handles() {
-            cublasDestroy(c.blas);
-            cusolverDnDestroy(c.sol);
+        std::vector<Ctx> lent;
+        cudaStream_t st;
+        int dev = 0;
+        explicit Handles(cudaStream_t s) : st(s) {
+            ck(cudaGetDevice(&dev), "cudaGetDevice");
+            lent = CtxPool::acquire(1, dev);
+            bind(st);
         }
-    } guard{c};
+        void bind(cudaStream_t s) {
+            ck(cublasSetStream(lent[0].blas, s), "cublasSetStream");
+            ck(cusolverDnSetStream(lent[0].sol, s), "cusolverDnSetStream");
+        }
+        ~Handles() {
+            cudaStreamSynchronize(st);  // their workspace is free again
+            cublasSetStream(lent[0].blas, lent[0].st);
+            cusolverDnSetStream(lent[0].sol, lent[0].st);
+            CtxPool::release(lent, dev);
+        }
+    } guard(st);
+    Arena arena(st);
+    Ctx c{st, guard.lent[0].blas, guard.lent[0].sol};
+    c.arena = &arena;
     // split precision: the stage's large products run as Ozaki digit products
     c.split = nvpt_get_precision(ctx) == NVPT_PRECISION_SPLIT;
     T ozerr;
@@ -2079,6 +2095,7 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
             pc_.sm_share = pc && pencils >= 4 ? 4 : 1;
             pc_.wait_limit = nvpt_context_wait_limit(ctx);
             pc_.all_pc_resolvent = nvpt_context_pc_route(ctx) == 1;
+            pc_.arena = &arena;
         }
     ck(cudaEventRecord(ps.prep, c.st), "event");  // B and h ready
     std::vector<std::unique_ptr<Runner>> SR(M);

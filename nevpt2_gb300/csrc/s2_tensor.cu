@@ -159,7 +159,13 @@ T alloc_v(Ctx &c, const std::vector<long long> &shape, bool zero) {
     t.nd = (int)shape.size();
     for (int i = 0; i < t.nd; ++i) t.sh[i] = shape[i];
     long long n = t.size();
-    ck(cudaMallocAsync((void **)&t.p, sizeof(double) * (size_t)(n > 0 ? n : 1), c.st), "cudaMallocAsync");
+    const size_t bytes = sizeof(double) * (size_t)(n > 0 ? n : 1);
+    if (c.arena && bytes <= Arena::kMost) {
+        t.p = (double *)c.arena->take(bytes, c.st, t.cls);
+        t.arena = c.arena;
+    } else {
+        ck(cudaMallocAsync((void **)&t.p, bytes, c.st), "cudaMallocAsync");
+    }
     if (zero) ck(cudaMemsetAsync(t.p, 0, sizeof(double) * (size_t)(n > 0 ? n : 1), c.st), "memset");
     return t;
 }
@@ -270,6 +276,26 @@ void symmetrize_upper(Ctx &c, const double *A, long long n, double *out) {
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
+namespace {
+// cuSOLVER workspace of `count` doubles + info word, stream-ordered.
+struct SolverWork {
+    Ctx &c;
+    T buf, inf;
+    double *w = nullptr;
+    int *info = nullptr;
+    SolverWork(Ctx &cc, int count) : c(cc), buf(alloc(cc, {std::max(count, 1)}, false)), inf(alloc(cc, {1}, false)) {
+        w = buf.p;
+        info = (int *)inf.p;
+    }
+    int status() {
+        int h = -1;
+        ck(cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, c.st), "info copy");
+        ck(cudaStreamSynchronize(c.st), "solver sync");
+        return h;
+    }
+};
+}  // namespace
+
 void eigh_upper(Ctx &c, const double *A, long long n, double *w, double *V) {
     if (n == 0) return;
     // Symmetric copy, so that the triangle cuSOLVER reads is the reference's upper one.
@@ -278,18 +304,11 @@ void eigh_upper(Ctx &c, const double *A, long long n, double *w, double *V) {
     ck(cusolverDnDsyevd_bufferSize(c.sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, (int)n, V, (int)n, w,
                                    &lwork),
        "syevd_bufferSize");
-    double *work = nullptr;
-    int *info = nullptr;
-    ck(cudaMallocAsync((void **)&work, sizeof(double) * (size_t)lwork, c.st), "cudaMallocAsync");
-    ck(cudaMallocAsync((void **)&info, sizeof(int), c.st), "cudaMallocAsync");
-    ck(cusolverDnDsyevd(c.sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, (int)n, V, (int)n, w, work, lwork,
-                        info),
+    SolverWork sw(c, lwork);
+    ck(cusolverDnDsyevd(c.sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, (int)n, V, (int)n, w, sw.w, lwork,
+                        sw.info),
        "syevd");
-    int hinfo = 0;
-    ck(cudaMemcpyAsync(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost, c.st), "info copy");
-    ck(cudaStreamSynchronize(c.st), "syevd sync");
-    cudaFreeAsync(work, c.st);
-    cudaFreeAsync(info, c.st);
+    const int hinfo = sw.status();
     if (hinfo != 0) throw Error(2, "syevd failed, info=" + std::to_string(hinfo));
     // The symmetric input makes row-/column-major identical; cuSOLVER stores
     // eigenvector k as column k (column-major) = row k of the row-major array.
@@ -343,73 +362,32 @@ int raise_dynamic_smem(const void *kernel) {
 
 bool metric_above(Ctx &c, const double *A, long long n, double thr) {
     if (n == 0) return true;
-    double *M = nullptr, *work = nullptr;
-    int *info = nullptr;
-    ck(cudaMallocAsync((void **)&M, sizeof(double) * (size_t)(n * n), c.st), "cudaMallocAsync");
-    symmetrize_upper(c, A, n, M);
-    k_add_diag<<<nblk(n), TPB, 0, c.st>>>(M, n, -thr);
+    T M = alloc(c, {n, n}, false);
+    symmetrize_upper(c, A, n, M.p);
+    k_add_diag<<<nblk(n), TPB, 0, c.st>>>(M.p, n, -thr);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     int lwork = 0;
-    ck(cusolverDnDpotrf_bufferSize(c.sol, CUBLAS_FILL_MODE_UPPER, (int)n, M, (int)n, &lwork), "potrf_bufferSize");
-    ck(cudaMallocAsync((void **)&work, sizeof(double) * (size_t)(lwork > 0 ? lwork : 1), c.st), "cudaMallocAsync");
-    ck(cudaMallocAsync((void **)&info, sizeof(int), c.st), "cudaMallocAsync");
-    ck(cusolverDnDpotrf(c.sol, CUBLAS_FILL_MODE_UPPER, (int)n, M, (int)n, work, lwork, info), "potrf");
-    int hinfo = -1;
-    ck(cudaMemcpyAsync(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost, c.st), "info copy");
-    ck(cudaStreamSynchronize(c.st), "potrf sync");
-    cudaFreeAsync(work, c.st);
-    cudaFreeAsync(info, c.st);
-    cudaFreeAsync(M, c.st);
-    return hinfo == 0;
+    ck(cusolverDnDpotrf_bufferSize(c.sol, CUBLAS_FILL_MODE_UPPER, (int)n, M.p, (int)n, &lwork), "potrf_bufferSize");
+    SolverWork sw(c, lwork);
+    ck(cusolverDnDpotrf(c.sol, CUBLAS_FILL_MODE_UPPER, (int)n, M.p, (int)n, sw.w, lwork, sw.info), "potrf");
+    return sw.status() == 0;
 }
 
 bool sygvd_upper(Ctx &c, const double *K, const double *S, long long n, double *w, double *V) {
     if (n == 0) return true;
-    double *B = nullptr, *work = nullptr;
-    int *info = nullptr;
+    T B = alloc(c, {n, n}, false);
     symmetrize_upper(c, K, n, V);
-    ck(cudaMallocAsync((void **)&B, sizeof(double) * (size_t)(n * n), c.st), "cudaMallocAsync");
-    symmetrize_upper(c, S, n, B);
+    symmetrize_upper(c, S, n, B.p);
     int lwork = 0;
     ck(cusolverDnDsygvd_bufferSize(c.sol, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER,
-                                   (int)n, V, (int)n, B, (int)n, w, &lwork),
+                                   (int)n, V, (int)n, B.p, (int)n, w, &lwork),
        "sygvd_bufferSize");
-    ck(cudaMallocAsync((void **)&work, sizeof(double) * (size_t)(lwork > 0 ? lwork : 1), c.st), "cudaMallocAsync");
-    ck(cudaMallocAsync((void **)&info, sizeof(int), c.st), "cudaMallocAsync");
+    SolverWork sw(c, lwork);
     ck(cusolverDnDsygvd(c.sol, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, (int)n, V,
-                        (int)n, B, (int)n, w, work, lwork, info),
+                        (int)n, B.p, (int)n, w, sw.w, lwork, sw.info),
        "sygvd");
-    int hinfo = -1;
-    ck(cudaMemcpyAsync(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost, c.st), "info copy");
-    ck(cudaStreamSynchronize(c.st), "sygvd sync");
-    cudaFreeAsync(work, c.st);
-    cudaFreeAsync(info, c.st);
-    cudaFreeAsync(B, c.st);
-    return hinfo == 0;
+    return sw.status() == 0;
 }
-
-namespace {
-// cuSOLVER workspace of `count` doubles + info word, stream-ordered.
-struct SolverWork {
-    Ctx &c;
-    double *w = nullptr;
-    int *info = nullptr;
-    SolverWork(Ctx &cc, int count) : c(cc) {
-        ck(cudaMallocAsync((void **)&w, sizeof(double) * (size_t)(count > 0 ? count : 1), c.st), "cudaMallocAsync");
-        ck(cudaMallocAsync((void **)&info, sizeof(int), c.st), "cudaMallocAsync");
-    }
-    int status() {
-        int h = -1;
-        ck(cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, c.st), "info copy");
-        ck(cudaStreamSynchronize(c.st), "solver sync");
-        return h;
-    }
-    ~SolverWork() {
-        cudaFreeAsync(w, c.st);
-        cudaFreeAsync(info, c.st);
-    }
-};
-}  // namespace
 
 namespace {
 // Mirror the upper triangle of the kb x kb diagonal block at A (column-major,

@@ -15,6 +15,8 @@
 #include <cusolverDn.h>
 
 #include <array>
+#include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -39,21 +41,87 @@ inline void ck(cusolverStatus_t e, const char *what) {
     if (e != CUSOLVER_STATUS_SUCCESS) throw Error(2, std::string(what) + ": cuSOLVER status " + std::to_string((int)e));
 }
 
-// Owning device tensor (stream-ordered allocation), or a non-owning view of
-// one (T::view) that never frees.
+// Small device blocks of one call (at most kMost bytes), carved from slabs and kept in
+// per-stream free lists: a block given back on a stream is only taken again on that
+// stream, so its reuse is ordered like that of a stream-ordered free.  The concurrent
+// tasks of a call made thousands of driver allocations, each behind the driver's lock;
+// these are a few hundred nanoseconds of host time.  Slabs go back when the call ends.
+class Arena {
+  public:
+    static constexpr size_t kMost = 1u << 20, kSlab = 4u << 20;
+    // home: where the slabs are freed, once every other stream's work has been waited for
+    explicit Arena(cudaStream_t home) : home_(home) {}
+    Arena(const Arena &) = delete;
+    Arena &operator=(const Arena &) = delete;
+    ~Arena() {
+        cudaStreamSynchronize(home_);
+        for (void *p : slabs_) cudaFreeAsync(p, home_);
+    }
+    // classes of 256 bytes * {4, 5, 6, 7} / 4 * 2^k; cls receives the block's
+    void *take(size_t bytes, cudaStream_t st, int &cls) {
+        size_t size = 256;
+        cls = 0;
+        while (size < bytes) {
+            ++cls;
+            size = (size_t)(64 * (4 + cls % 4)) << (cls / 4);
+        }
+        size = (size + 255) / 256 * 256;
+        std::lock_guard<std::mutex> g(mu_);
+        Lane &l = lanes_[st];
+        if ((size_t)cls >= l.free.size()) l.free.resize(cls + 1);
+        if (!l.free[cls].empty()) {
+            void *p = l.free[cls].back();
+            l.free[cls].pop_back();
+            return p;
+        }
+        if (l.left < size) {
+            void *p = nullptr;
+            ck(cudaMallocAsync(&p, kSlab, st), "cudaMallocAsync");
+            slabs_.push_back(p);
+            l.cur = (char *)p;
+            l.left = kSlab;
+        }
+        void *p = l.cur;
+        l.cur += size;
+        l.left -= size;
+        return p;
+    }
+    void give(void *p, int cls, cudaStream_t st) {
+        std::lock_guard<std::mutex> g(mu_);
+        Lane &l = lanes_[st];
+        if ((size_t)cls >= l.free.size()) l.free.resize(cls + 1);
+        l.free[cls].push_back(p);
+    }
+
+  private:
+    struct Lane {
+        char *cur = nullptr;
+        size_t left = 0;
+        std::vector<std::vector<void *>> free;
+    };
+    cudaStream_t home_;
+    std::mutex mu_;
+    std::map<cudaStream_t, Lane> lanes_;
+    std::vector<void *> slabs_;
+};
+
+// Owning device tensor (stream-ordered allocation, or a block of an arena), or a
+// non-owning view of one (T::view) that never frees.
 struct T {
     double *p = nullptr;
     int nd = 0;
     std::array<long long, 6> sh{{1, 1, 1, 1, 1, 1}};
     cudaStream_t st = nullptr;
     bool own = true;
+    Arena *arena = nullptr;  // whose block of class cls this is
+    int cls = 0;
     T() = default;
     T(const T &) = delete;
     T &operator=(const T &) = delete;
     T(T &&o) noexcept { *this = std::move(o); }
     T &operator=(T &&o) noexcept {
         release();
-        p = o.p; nd = o.nd; sh = o.sh; st = o.st; own = o.own;
+        p = o.p; nd = o.nd; sh = o.sh; st = o.st; own = o.own; arena = o.arena; cls = o.cls;
         o.p = nullptr;
         return *this;
     }
@@ -64,7 +132,10 @@ struct T {
         return v;
     }
     void release() {
-        if (p && own) cudaFreeAsync(p, st);
+        if (p && own) {
+            if (arena) arena->give(p, cls, st);
+            else cudaFreeAsync(p, st);
+        }
         p = nullptr;
     }
     long long size() const {
@@ -92,6 +163,7 @@ struct Ctx {
     // Resolvents (no eigenvectors) for every PC class whose metric keeps all
     // its eigenvalues, not only the order-n^3 pencils of the (+-1') classes.
     bool all_pc_resolvent = false;
+    Arena *arena = nullptr;  // small allocations of the call, if any
 };
 
 T alloc(Ctx &c, std::initializer_list<long long> shape, bool zero = true);

@@ -403,14 +403,13 @@ constexpr int SL = NB + 2;      // slots: the NB + 1 rows that a column reaches 
 // partial pivoting over the NB + 1 rows a column reaches, kept in slots of shared
 // memory (a row is not moved: its slot is refilled once it was the pivot), rows of U
 // streamed out, then the back substitution by one warp.  The pivot is the largest
-// by the leading 32 bits.  Outputs as k_tridiag_resolvent.
+// by the leading 32 bits.
 // Bound by the FP64 pipe of the label's SM (2 NB^2 FMAs, 66 warp instructions of 16
 // clocks, a column).  Warp 0 runs one column ahead of the others (its update,
 // pivot, reciprocal and multipliers, so that the chain of the search is hidden
 // behind the other columns' updates and its division done once), warp 7 moves the
 // rows in and out, so a column is one block barrier.  Order 2744, with the other
-// classes running: 4.6 -> 1.8 us a
-// column.
+// classes running: 4.6 -> 1.8 us a column.
 __global__ void __launch_bounds__(TB) k_band_resolvent(const double *__restrict__ AB, long long n, const double *Y,
                                                        long long ncol, long long L, long long l0, int nother,
                                                        const double *sig, double *U, double *acc, int nd,

@@ -158,90 +158,6 @@ __global__ void k_pc_finish(const double *R, const double *Rp, const double *Rj,
     for (int j = 0; j < nother && j < 8; ++j) block_add(offs[j], acc + 2 + j);
 }
 
-// PC sums of one class from the tridiagonal form of its pencil: for label l
-// (one CTA each) with shift sig[l], x = (T + sig I)^-1 y_l by Gaussian
-// elimination with partial pivoting on the tridiagonal T (d[n], e[n-1]),
-// then
-//   acc[0] -= y_l . x,   acc[1] += x . x,   acc[2 + k] -= y_{k+1,l} . x,
-// which are the type-0 sums of k_pc_finish over the eigenpairs of T
-// (sum_mu r_mu^2 / (w_mu + sig) = y^T (T + sig)^-1 y with r = G^T y).
-// Y is row-major [n][ncol], column k L + l holding block k (0: own state,
-// k > 0: the other states) of label l.  The CTA stages d, e and y_l in
-// shared memory; one thread runs the elimination and the back substitution
-// there (every step a shared-memory access, no global latency), then all
-// threads form the dot products.  Shared memory: 6 n doubles.
-// With nd > 0 the kernel also forms rho[l nd + k] = -x . Y[:, dcol0 + k] for
-// k < nd: the first-order density of the label against nd extra right-hand
-// sides transformed with the labels' (sum_mu r_mu v_mu,k / (w_mu + sig) =
-// z^T (K + sig S)^-1 g_k with v = C^T g).  xout, when given, receives the
-// solution x of each label, row-major [n][L].
-__global__ void k_tridiag_resolvent(const double *d, const double *e, long long n, const double *Y, long long ncol,
-                                    long long L, int nother, const double *sig, double *acc, int nd,
-                                    long long dcol0, double *rho, double *xout) {
-    extern __shared__ double sm[];
-    double *sd = sm, *se = sm + n, *wb = sm + 2 * n, *wc = sm + 3 * n, *wd = sm + 4 * n, *wy = sm + 5 * n;
-    const long long l = blockIdx.x;
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        sd[i] = d[i];
-        se[i] = i + 1 < n ? e[i] : 0.0;
-        wy[i] = Y[i * ncol + l];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double s = sig[l];
-        // row i: diagonal b, super-diagonal c; the fill of a row exchange goes to wd
-        double b = sd[0] + s, cc = se[0], y = wy[0];
-        for (long long i = 0; i + 1 < n; ++i) {
-            const double a1 = se[i];                        // row i+1, column i
-            const double b1 = sd[i + 1] + s;                // row i+1, column i+1
-            const double c1 = i + 2 < n ? se[i + 1] : 0.0;  // row i+1, column i+2
-            const double y1 = wy[i + 1];
-            if (fabs(b) >= fabs(a1)) {  // keep row i as pivot row
-                const double f = a1 / b;
-                wb[i] = b; wc[i] = cc; wd[i] = 0.0; wy[i] = y;
-                b = b1 - f * cc;
-                cc = c1;
-                y = y1 - f * y;
-            } else {                    // interchange rows i and i+1
-                const double f = b / a1;
-                wb[i] = a1; wc[i] = b1; wd[i] = c1; wy[i] = y1;
-                b = cc - f * b1;
-                cc = -f * c1;
-                y = y - f * y1;
-            }
-        }
-        wb[n - 1] = b;
-        // back substitution, x over wy
-        double x2 = 0.0, x1 = y / b;
-        wy[n - 1] = x1;
-        for (long long i = n - 2; i >= 0; --i) {
-            const double x = (wy[i] - wc[i] * x1 - wd[i] * x2) / wb[i];
-            wy[i] = x;
-            x2 = x1;
-            x1 = x;
-        }
-    }
-    __syncthreads();
-    if (xout)
-        for (long long i = threadIdx.x; i < n; i += blockDim.x) xout[i * L + l] = wy[i];
-    double en = 0.0, ps = 0.0;
-    double offs[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        const double x = wy[i];
-        en -= Y[i * ncol + l] * x;
-        ps += x * x;
-        for (int k = 0; k < nother && k < 8; ++k) offs[k] -= Y[i * ncol + (k + 1) * L + l] * x;
-    }
-    block_add(en, acc + 0);
-    block_add(ps, acc + 1);
-    for (int j = 0; j < nother && j < 8; ++j) block_add(offs[j], acc + 2 + j);
-    for (int k = 0; k < nd; ++k) {
-        double r = 0.0;
-        for (long long i = threadIdx.x; i < n; i += blockDim.x) r -= Y[i * ncol + dcol0 + k] * wy[i];
-        block_add(r, rho + l * nd + k);
-    }
-}
-
 // First-order density of a PC class on its eigenpairs: rho[l, k] =
 // -sum_mu R[l, mu] V[k, mu] / (w_mu + base_l), one thread per (l, k).
 __global__ void k_rho_pc(const double *R, const double *V, const double *w, const double *base, long long L,
@@ -610,7 +526,6 @@ class PencilFork {
         Ctx &a = aux_[0];
         a.split = c_.split;
         a.oz_err = c_.oz_err;
-        a.sm_share = c_.sm_share;
         a.wait_limit = c_.wait_limit;
         a.all_pc_resolvent = c_.all_pc_resolvent;
         a.arena = c_.arena;
@@ -654,11 +569,9 @@ class PencilFork {
         } else {
             cudaStreamSynchronize(a.st);
         }
-        for (T *t : {&pt_.U, &pt_.A, &pt_.d, &pt_.e, &pt_.tau, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm})
-            t->st = c_.st;
+        for (T *t : {&pt_.W, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm}) t->st = c_.st;
         a.split = false;
         a.oz_err = nullptr;
-        a.sm_share = 1;
         a.wait_limit = 0;
         a.all_pc_resolvent = false;
         a.arena = nullptr;
@@ -876,24 +789,11 @@ class Runner {
         const long long L = (long long)shift.size(), n = PT.n;
         T sg = upload(c, shift);
         T a = alloc(c, {2 + 8}, true);
-        if (L > 0 && n > 0 && PT.band) {
+        if (L > 0 && n > 0) {
             ProfSpan sp;
             sp.begin("pencil_solve", c.st, 0);
             band_resolvent(c, PT.AB.p, n, Yt.p, Yt.sh[1], L, nother < 0 ? M - 1 : nother, sg.p, a.p, nd, dcol0, rho, xout);
             sp.end();
-        } else if (L > 0 && n > 0) {
-            const size_t smem = sizeof(double) * 6 * (size_t)n;
-            // one limit for every caller: pencils of different orders are
-            // solved concurrently on other host threads
-            const int lim = raise_dynamic_smem((const void *)k_tridiag_resolvent);
-            if ((long long)smem > lim) throw Error(NVPT_EINVAL, "resolvent: pencil order above the shared-memory limit");
-            ProfSpan sp;
-            sp.begin("pencil_solve", c.st, 0);
-            k_tridiag_resolvent<<<(unsigned)L, 128, smem, c.st>>>(PT.d.p, PT.e.p, n, Yt.p, Yt.sh[1], L,
-                                                                   nother < 0 ? M - 1 : nother, sg.p, a.p, nd, dcol0,
-                                                                   rho, xout);
-            sp.end();
-            LAUNCHED();
         }
         return download(c, a.p, 2 + 8);
     }
@@ -1935,7 +1835,6 @@ struct ClassStreams {
         for (auto &x : c) {
             x.split = false;
             x.oz_err = nullptr;
-            x.sm_share = 1;
             x.wait_limit = 0;
             x.all_pc_resolvent = false;
             x.arena = nullptr;
@@ -2085,14 +1984,10 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
     int dev = 0;
     ck(cudaGetDevice(&dev), "cudaGetDevice");
     ClassStreams ps((size_t)M), cs((size_t)M * nj);
-    // order-n^3 pencils in flight at once: one per state and (+-1') class
-    const int pencils = M * (((m & 64u) ? 1 : 0) + ((m & 32u) ? 1 : 0));
     for (auto *pool : {&ps, &cs})
         for (auto &pc_ : pool->c) {
             pc_.split = c.split;
             pc_.oz_err = c.oz_err;
-            // measured: 8 pencils (4 states) fastest on quarters; 2 pencils on the whole GPU each
-            pc_.sm_share = pc && pencils >= 4 ? 4 : 1;
             pc_.wait_limit = nvpt_context_wait_limit(ctx);
             pc_.all_pc_resolvent = nvpt_context_pc_route(ctx) == 1;
             pc_.arena = &arena;

@@ -6,6 +6,7 @@
 
 #include "band.cuh"
 #include "ozaki.cuh"
+#include "spd.cuh"
 
 namespace nvpt {
 namespace s2 {
@@ -390,63 +391,6 @@ bool sygvd_upper(Ctx &c, const double *K, const double *S, long long n, double *
 }
 
 namespace {
-// Mirror the upper triangle of the kb x kb diagonal block at A (column-major,
-// ld) into its lower triangle.
-__global__ void k_mirror_block(double *A, long long ld, int kb) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)kb * kb) return;
-    const long long i = t % kb, j = t / kb;
-    if (i > j) A[i + j * ld] = A[j + i * ld];
-}
-}  // namespace
-
-// Upper triangle of A (column-major n x n, symmetric on entry) <- the upper
-// triangle of U^-T A U^-1, U upper triangular: the blocked right-looking
-// reduction of a symmetric-definite pencil to standard form (n^3 flops, half
-// of two full triangular solves).  Per diagonal block k of width kb, with the
-// trailing blocks 12 (kb x m) and 22:
-//   A11 <- U11^-T A11 U11^-1
-//   A12 <- U11^-T A12 - 1/2 A11 U12
-//   A22 <- A22 - A12^T U12 - U12^T A12          (upper triangle)
-//   A12 <- (A12 - 1/2 A11 U12) U22^-1
-// after which A22 is reduced in turn.  The lower triangle is left stale.
-void reduce_to_standard(Ctx &c, double *A, const double *U, long long n) {
-    constexpr int NB = 256;
-    const double one = 1.0, mhalf = -0.5, mone = -1.0;
-    for (long long k = 0; k < n; k += NB) {
-        const int kb = (int)std::min<long long>(NB, n - k), m = (int)(n - k - kb);
-        double *A11 = A + k + k * n;
-        const double *U11 = U + k + k * n;
-        k_mirror_block<<<nblk((long long)kb * kb), TPB, 0, c.st>>>(A11, n, kb);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        ck(cublasDtrsm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT, kb, kb,
-                       &one, U11, (int)n, A11, (int)n),
-           "trsm");
-        ck(cublasDtrsm(c.blas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, kb, kb,
-                       &one, U11, (int)n, A11, (int)n),
-           "trsm");
-        if (m == 0) break;
-        double *A12 = A + k + (k + kb) * n, *A22 = A + (k + kb) + (k + kb) * n;
-        const double *U12 = U + k + (k + kb) * n, *U22 = U + (k + kb) + (k + kb) * n;
-        ck(cublasDtrsm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT, kb, m,
-                       &one, U11, (int)n, A12, (int)n),
-           "trsm");
-        ck(cublasDsymm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, kb, m, &mhalf, A11, (int)n, U12, (int)n, &one,
-                       A12, (int)n),
-           "symm");
-        ck(cublasDsyr2k(c.blas, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, m, kb, &mone, A12, (int)n, U12, (int)n, &one, A22,
-                        (int)n),
-           "syr2k");
-        ck(cublasDsymm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, kb, m, &mhalf, A11, (int)n, U12, (int)n, &one,
-                       A12, (int)n),
-           "symm");
-        ck(cublasDtrsm(c.blas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, kb, m,
-                       &one, U22, (int)n, A12, (int)n),
-           "trsm");
-    }
-}
-
-namespace {
 // Deterministic start vectors of the inverse iteration, in [-0.5, 0.5).
 __global__ void k_start_block(double *X, long long count) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -464,34 +408,35 @@ __global__ void k_start_block(double *X, long long count) {
 // False if the metric is not of this kind.
 bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long long &k) {
     const long long b = std::min<long long>(64, n);
+    Ctx f = c;
+    f.split = false;
     k = 0;
     T L = alloc(c, {n, n}, false), X = alloc(c, {b, n}, false), Y = alloc(c, {b, n}, false);
     T w = alloc(c, {b}, false), H = alloc(c, {b, b}, false), V = alloc(c, {b, b}, false);
+    const long long ld = spd_ld(n);
+    T W = alloc(c, {ld, ld}, false);
     ck(cudaMemcpyAsync(L.p, S, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.st), "copy");
     std::vector<double> dg(n);
     ck(cudaMemcpy2DAsync(dg.data(), sizeof(double), S, sizeof(double) * (n + 1), sizeof(double), n,
                          cudaMemcpyDeviceToHost, c.st), "diagonal");
     ck(cudaStreamSynchronize(c.st), "sync");
-    double top = 0.0;
+    double top = 0.0, tr = 0.0;
     for (double x : dg) top = std::max(top, x);
     if (!(top > 0.0)) return false;
     k_add_diag<<<nblk(n), TPB, 0, c.st>>>(L.p, n, 1e-9 * top);
     k_start_block<<<nblk(b * n), TPB, 0, c.st>>>(X.p, b * n);
     g_launches.fetch_add(2, std::memory_order_relaxed);
-    const int Ni = (int)n, bi = (int)b;
-    int lw = 0;
-    ck(cusolverDnDpotrf_bufferSize(c.sol, CUBLAS_FILL_MODE_UPPER, Ni, L.p, Ni, &lw), "potrf_bufferSize");
-    SolverWork sw(c, lw);
-    ck(cusolverDnDpotrf(c.sol, CUBLAS_FILL_MODE_UPPER, Ni, L.p, Ni, sw.w, lw, sw.info), "potrf");
-    if (sw.status() != 0) return false;
+    if (!spd_inverse_factor(c, L.p, n, W.p, tr)) return false;
     // rows of X are the columns of a column-major [n, b]: solve, then orthonormalise by QR
+    const int Ni = (int)n, bi = (int)b;
     T tau = alloc(c, {b}, false);
     int lq = 0, lg = 0;
     ck(cusolverDnDgeqrf_bufferSize(c.sol, Ni, bi, X.p, Ni, &lq), "geqrf_bufferSize");
     ck(cusolverDnDorgqr_bufferSize(c.sol, Ni, bi, bi, X.p, Ni, tau.p, &lg), "orgqr_bufferSize");
     SolverWork qw(c, std::max(lq, lg));
     for (int it = 0; it < 3; ++it) {
-        ck(cusolverDnDpotrs(c.sol, CUBLAS_FILL_MODE_UPPER, Ni, bi, L.p, Ni, X.p, Ni, sw.info), "potrs");
+        gemm(f, false, true, b, n, n, 1.0, X.p, n, W.p, ld, 0.0, Y.p, n);
+        gemm(f, false, false, b, n, n, 1.0, Y.p, n, W.p, ld, 0.0, X.p, n);
         ck(cusolverDnDgeqrf(c.sol, Ni, bi, X.p, Ni, tau.p, qw.w, lq, qw.info), "geqrf");
         ck(cusolverDnDorgqr(c.sol, Ni, bi, bi, X.p, Ni, tau.p, qw.w, lg, qw.info), "orgqr");
     }
@@ -517,119 +462,87 @@ bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, doubl
     P.n = n;
     P.k = 0;
     if (n == 0) return true;
-    const int N = (int)n;
-    P.U = alloc(c, {n, n}, false);
-    P.A = alloc(c, {n, n}, false);
-    symmetrize_upper(c, S, n, P.U.p);
-    symmetrize_upper(c, K, n, P.A.p);
-    if (!metric_above(c, S, n, thr)) {
-        if (!metric_null(c, P.U.p, n, thr, P.N, P.k)) return false;
+    const long long ld = spd_ld(n);
+    P.W = alloc(c, {ld, ld}, false);
+    ProfSpan sp;
+    // every eigenvalue above thr: by tr S^-1 >= 1 / the smallest, or else by S - thr
+    auto factor = [&](const double *M) {
+        double tr = 0.0;
+        sp.begin("pencil_potrf", c.st, 0);
+        const bool ok = spd_inverse_factor(c, M, n, P.W.p, tr);
+        sp.end();
+        return ok && ((thr >= 0.0 && tr * thr <= 0.999) || metric_above(c, M, n, thr));
+    };
+    T S2, K2;
+    const double *Kp = K;
+    if (!factor(S)) {
+        S2 = alloc(c, {n, n}, false);
+        symmetrize_upper(c, S, n, S2.p);
+        if (!metric_null(c, S2.p, n, thr, P.N, P.k)) return false;
         const long long k = P.k;
         // S + N^T N, then every eigenvalue has to be above the threshold
-        gemm(c, true, false, n, n, k, 1.0, P.N.p, n, P.N.p, n, 1.0, P.U.p, n);
-        if (!metric_above(c, P.U.p, n, thr)) return false;
+        gemm(c, true, false, n, n, k, 1.0, P.N.p, n, P.N.p, n, 1.0, S2.p, n);
+        if (!factor(S2.p)) return false;
         // P K P + N^T N = K - N^T G - G^T N + N^T (1 + G N^T) N with G = N K
+        K2 = alloc(c, {n, n}, false);
+        symmetrize_upper(c, K, n, K2.p);
         T G = alloc(c, {k, n}, false), M = alloc(c, {k, k}, false), Q = alloc(c, {k, n}, false);
-        gemm(c, false, false, k, n, n, 1.0, P.N.p, n, P.A.p, n, 0.0, G.p, n);
+        gemm(c, false, false, k, n, n, 1.0, P.N.p, n, K2.p, n, 0.0, G.p, n);
         gemm(c, false, true, k, k, n, 1.0, G.p, n, P.N.p, n, 0.0, M.p, k);
         k_add_diag<<<nblk(k), TPB, 0, c.st>>>(M.p, k, 1.0);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         gemm(c, false, false, k, n, k, 0.5, M.p, k, P.N.p, n, 0.0, Q.p, n);
         axpby(c, k * n, 1.0, Q.p, -1.0, G.p, Q.p);  // Q = (1 + G N^T) N / 2 - G
-        gemm(c, true, false, n, n, k, 1.0, P.N.p, n, Q.p, n, 1.0, P.A.p, n);
-        gemm(c, true, false, n, n, k, 1.0, Q.p, n, P.N.p, n, 1.0, P.A.p, n);
+        gemm(c, true, false, n, n, k, 1.0, P.N.p, n, Q.p, n, 1.0, K2.p, n);
+        gemm(c, true, false, n, n, k, 1.0, Q.p, n, P.N.p, n, 1.0, K2.p, n);
+        Kp = K2.p;
     }
-    int lw_p = 0;
-    ck(cusolverDnDpotrf_bufferSize(c.sol, CUBLAS_FILL_MODE_UPPER, N, P.U.p, N, &lw_p), "potrf_bufferSize");
-    SolverWork sw(c, lw_p);
-    ProfSpan sp;
-    sp.begin("pencil_potrf", c.st, 0);
-    ck(cusolverDnDpotrf(c.sol, CUBLAS_FILL_MODE_UPPER, N, P.U.p, N, sw.w, lw_p, sw.info), "potrf");
-    sp.end();
-    if (sw.status() != 0) return false;
+    S2.release();
+    T A = alloc(c, {n, n}, false);
     sp.begin("pencil_reduce", c.st, 0);
-    reduce_to_standard(c, P.A.p, P.U.p, n);
+    spd_congruence(c, P.W.p, Kp, n, A.p);
     sp.end();
+    K2.release();
     sp.begin("pencil_sytrd", c.st, 0);
-    int trc;
-    P.band = n >= kPencilBandMin;
-    if (P.band) {
-        const int np = band_panels(n);
-        P.V = alloc(c, {band_rows(n), kBand}, false);
-        P.Tm = alloc(c, {np, kBand, kBand}, false);
-        P.AB = alloc(c, {kBand + 1, n}, false);
-        k_mirror_block<<<nblk(n * n), TPB, 0, c.st>>>(P.A.p, n, N);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        trc = band_reduce(c, P.A.p, n, P.V.p, P.Tm.p, P.AB.p);
-        P.A.release();
-    } else {
-        P.d = alloc(c, {n}, false);
-        P.e = alloc(c, {n}, true);
-        P.tau = alloc(c, {n}, true);
-        trc = sytrd_lower(c, P.A.p, n, P.d.p, P.e.p, P.tau.p, true, std::min(4, std::max(1, c.sm_share)));
-    }
+    const int np = band_panels(n);
+    P.V = alloc(c, {band_rows(n), kBand}, false);
+    P.Tm = alloc(c, {np, kBand, kBand}, false);
+    P.AB = alloc(c, {kBand + 1, n}, false);
+    const int rc = band_reduce(c, A.p, n, P.V.p, P.Tm.p, P.AB.p);
     sp.end();
-    if (trc != 0) throw Error(4, "pencil reduction: a grid barrier timed out");
+    if (rc != 0) throw Error(4, "pencil reduction: a grid barrier timed out");
     return true;
 }
 
 void pencil_rhs(Ctx &c, const PencilTridiag &P, double *Y, long long m) {
     if (P.n == 0 || m == 0) return;
-    const int N = (int)P.n, Mc = (int)m;
-    const double one = 1.0;
     ProfSpan sp;
     sp.begin("pencil_rhs", c.st, 0);
-    if (P.k) {  // rows of Y without their components along the null vectors
+    Ctx f = c;
+    f.split = false;
+    T Z = alloc(c, {m, P.n}, false);
+    ck(cudaMemcpyAsync(Z.p, Y, sizeof(double) * m * P.n, cudaMemcpyDeviceToDevice, c.st), "copy");
+    if (P.k) {  // rows without their components along the null vectors
         T a = alloc(c, {m, P.k}, false);
         gemm(c, false, true, m, P.k, P.n, 1.0, Y, P.n, P.N.p, P.n, 0.0, a.p, P.k);
-        gemm(c, false, false, m, P.n, P.k, -1.0, a.p, P.k, P.N.p, P.n, 1.0, Y, P.n);
+        gemm(c, false, false, m, P.n, P.k, -1.0, a.p, P.k, P.N.p, P.n, 1.0, Z.p, P.n);
     }
-    ck(cublasDtrsm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT, N, Mc, &one,
-                   P.U.p, N, Y, N),
-       "trsm");
-    if (P.band) {
-        band_apply(c, P.n, P.V.p, P.Tm.p, Y, m, true);
-        sp.end();
-        return;
-    }
-    int lw = 0;
-    ck(cusolverDnDormtr_bufferSize(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, N, Mc, P.A.p, N,
-                                   P.tau.p, Y, N, &lw),
-       "ormtr_bufferSize");
-    SolverWork sw(c, lw);
-    ck(cusolverDnDormtr(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, N, Mc, P.A.p, N, P.tau.p, Y, N,
-                        sw.w, lw, sw.info),
-       "ormtr");
+    gemm(f, false, true, m, P.n, P.n, 1.0, Z.p, P.n, P.W.p, spd_ld(P.n), 0.0, Y, P.n);
+    band_apply(c, P.n, P.V.p, P.Tm.p, Y, m, true);
     sp.end();
-    const int st = sw.status();
-    if (st != 0) throw Error(2, "ormtr failed, info=" + std::to_string(st));
 }
 
 void pencil_back(Ctx &c, const PencilTridiag &P, double *X, long long m) {
     if (P.n == 0 || m == 0) return;
-    const int N = (int)P.n, Mc = (int)m;
-    const double one = 1.0;
     ProfSpan sp;
     sp.begin("pencil_rhs", c.st, 0);
-    int st = 0;
-    if (P.band) {
-        band_apply(c, P.n, P.V.p, P.Tm.p, X, m, false);
-    } else {
-        int lw = 0;
-        ck(cusolverDnDormtr_bufferSize(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, N, Mc, P.A.p, N,
-                                       P.tau.p, X, N, &lw),
-           "ormtr_bufferSize");
-        SolverWork sw(c, lw);
-        ck(cusolverDnDormtr(c.sol, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, N, Mc, P.A.p, N, P.tau.p, X,
-                            N, sw.w, lw, sw.info),
-           "ormtr");
-        st = sw.status();
-    }
-    ck(cublasDtrsm(c.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, N, Mc, &one,
-                   P.U.p, N, X, N),
-       "trsm");
+    Ctx f = c;
+    f.split = false;
+    band_apply(c, P.n, P.V.p, P.Tm.p, X, m, false);
+    T Z = alloc(c, {m, P.n}, false);
+    ck(cudaMemcpyAsync(Z.p, X, sizeof(double) * m * P.n, cudaMemcpyDeviceToDevice, c.st), "copy");
+    gemm(f, false, false, m, P.n, P.n, 1.0, Z.p, P.n, P.W.p, spd_ld(P.n), 0.0, X, P.n);
     sp.end();
-    if (st != 0) throw Error(2, "ormtr failed, info=" + std::to_string(st));
 }
 
 void build_ee2L(Ctx &c, const double *taa, const double *dal, int n, double *out) {

@@ -6,8 +6,8 @@
 // qdnevpt-local normal-ordered products (src/qdnevpt.F:6448-6519), dense
 // GEMMs (cuBLAS FP64, or split-precision digit products on the tensor cores
 // in split mode), symmetric eigendecompositions (cuSOLVER syevd) and, for
-// the order-n^3 pencils, Cholesky + reduction to standard form + the device
-// tridiagonalisation (tridiag.cu).  All work of one context is enqueued on
+// the order-n^3 pencils, the reduction to standard form (spd.cu) and to a band
+// (band.cu).  All work of one context is enqueued on
 // its stream; allocations are stream-ordered.
 #pragma once
 #include <cublas_v2.h>
@@ -154,9 +154,6 @@ struct Ctx {
     // products on the tensor cores; a pipeline timeout sets *oz_err.
     bool split = false;
     int *oz_err = nullptr;
-    // Order-n^3 pencils tridiagonalised at the same time on other streams:
-    // each takes 1/sm_share of the SMs (at most 4), so that they overlap.
-    int sm_share = 1;
     // Polls a device-side wait (grid barrier) makes before it gives up and
     // the call reports NVPT_ETIMEDOUT; 0 = the built-in limit.
     unsigned wait_limit = 0;
@@ -210,43 +207,31 @@ bool sygvd_upper(Ctx &c, const double *K, const double *S, long long n, double *
 // Symmetric copy: out = triu(A) + triu(A,1)^T.
 void symmetrize_upper(Ctx &c, const double *A, long long n, double *out);
 
-// The pencil K v = w S v in tridiagonal form, without its eigenvectors:
-// S = U^T U (Cholesky of the symmetric view of S), K~ = U^-T K U^-1 (K's
-// symmetric view), K~ = Q T Q^T (Householder).  T: diagonal d[n],
-// off-diagonal e[n-1].  U, Q (reflectors + tau) stay in the struct, which
-// then maps right-hand sides into T's basis.  False if S is not positive
-// definite.
+// The pencil K v = w S v in band form, without its eigenvectors: S = L L^T (its
+// symmetric view), W = L^-1, W K W^T = Q B Q^T (K's symmetric view; Householder).
+// W and Q stay in the struct, which then maps right-hand sides into B's basis.
 // A metric with exact null vectors (those of a spin eigenfunction) and every other
 // eigenvalue above the threshold is deflated: with N its null vectors (rows, k of
 // them) and P = 1 - N^T N the pencil is P K P + N^T N, S + N^T N, whose null part is
 // a block of its own, and right-hand sides are projected by P.
-// Orders of at least kPencilBandMin keep K~ = Q B Q^T in band form (band.cu: AB, V,
-// Tm) instead of the tridiagonal one.
-constexpr long long kPencilBandMin = 512;
 struct PencilTridiag {
-    T U, A, d, e, tau;  // U: column-major upper factor; A: reflectors of Q
-    T AB, V, Tm;
-    bool band = false;
-    T N;                // null vectors of the metric [k, n]
+    T W;           // inverse Cholesky factor of the metric (spd.cuh)
+    T AB, V, Tm;   // W K W^T = Q B Q^T (band.cuh)
+    T N;           // null vectors of the metric [k, n]
     long long n = 0, k = 0;
 };
 // False, with nothing kept, unless every eigenvalue of S is above thr or null
 // (|w| <= 1e-12 of the largest; at most 48 of them).
 bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, double thr, PencilTridiag &P);
-// Upper triangle of A (column-major, symmetric) <- that of U^-T A U^-1.
-void reduce_to_standard(Ctx &c, double *A, const double *U, long long n);
-// Householder tridiagonalisation of the symmetric A (column-major; both
-// triangles valid, or only the upper one with upper_valid) in the output
-// form of dsytrd('L'): d[n], e[n-1], tau[n-1], reflectors below the
-// subdiagonal of A (tridiag.cu); the panel kernels use 1/share of the SMs.
-// 0, or 4 if a grid barrier timed out.
-int sytrd_lower(Ctx &c, double *A, long long n, double *d, double *e, double *tau, bool upper_valid,
-                int share = 1);
-// Y <- Q^T U^-T Y for Y column-major [n, m] (= row-major [m, n]): each row
-// z of the row-major view becomes y with z^T (K + s S)^-1 z = y^T (T + s)^-1 y.
+// Householder tridiagonalisation of the symmetric A (column-major, both triangles
+// valid) in the output form of dsytrd('L'): d[n], e[n-1], tau[n-1], reflectors below
+// the subdiagonal of A (tridiag.cu).  0, or 4 if a grid barrier timed out.
+int sytrd_lower(Ctx &c, double *A, long long n, double *d, double *e, double *tau);
+// Y <- Q^T W Y for Y column-major [n, m] (= row-major [m, n]): each row
+// z of the row-major view becomes y with z^T (K + s S)^-1 z = y^T (B + s)^-1 y.
 void pencil_rhs(Ctx &c, const PencilTridiag &P, double *Y, long long m);
-// The inverse map of m vectors of the tridiagonal basis (columns of a
-// column-major [n, m] X, in place): X <- U^-1 Q X.
+// The inverse map of m vectors of the band's basis (columns of a
+// column-major [n, m] X, in place): X <- W^T Q X.
 void pencil_back(Ctx &c, const PencilTridiag &P, double *X, long long m);
 
 // Accessor builders (C-ordered n-index tensors of one state or pair).

@@ -1,0 +1,339 @@
+// Reduction of the order-n^3 pencils K v = w S v to standard form through the
+// inverse Cholesky factor W = L^-1 of S = L L^T: K~ = W K W^T.
+//
+// FP64 runs at 2 FMAs a clock and SM here, so an O(n^3) step is bound by that pipe
+// wherever it is a product of tiles, and by latency wherever it is a triangular
+// solve.  Everything below is therefore a 64 x 64 tile product; the only serial
+// part is the factorisation of a diagonal block.  All matrices are padded to whole
+// 64-blocks (identity in S, zero in K), so no tile has a ragged edge.
+//   factor   for each block column k: k_spd_panel   L21 = A21 W11^T, W[k, :] = W11 R[k, :]
+//                                     k_spd_step    A22 -= L21 L21^T, R[i, :] -= L21 W[k, :],
+//                                                   and the next diagonal block's L11, W11
+//            (R, the identity under elimination, ends as W; n^3/3 + n^3/3 flops)
+//   product  k_spd_n    N = W M, K = M + M^T with M lower triangular   (n^3/3)
+//   product  k_spd_k    K~ = N W^T + W N^T, the lower tiles mirrored  (2n^3/3)
+// W also gives tr S^-1 = |W|^2, which bounds the smallest metric eigenvalue (no second
+// factorisation of S - thr in the common case), and takes right-hand sides by products.
+// Order 2744 (with the library's two factorisations, triangular solves and rank-2k
+// updates before): 90 -> 38 ms.
+#include <algorithm>
+#include <cstring>
+
+#include "spd.cuh"
+
+namespace nvpt {
+namespace s2 {
+namespace {
+
+constexpr int B = 64;    // block
+constexpr int KS = 16;   // slab of a tile product
+constexpr int LS = B + 2;
+constexpr int TP = 256;
+
+struct Slab {
+    double a[KS][LS], b[KS][LS];
+};
+
+// acc += A B^T (BT: B [64][ldb], k along the rows) or A B (B [K][ldb]) for the 64 x K
+// tile A [64][lda]; K a multiple of KS.  Thread (ty, tx) holds rows {2ty, 2ty+1, 32+2ty,
+// 33+2ty} and columns {2tx, ...}; the next slab's loads are issued before the FMAs.
+template <bool BT>
+__device__ __forceinline__ void tile(double (&acc)[4][4], const double *A, long long lda, const double *Bm, long long ldb,
+                                     int K, Slab &s) {
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const double *pa = A + (tid >> 2) * lda + (tid & 3) * 4;
+    const double *pb = BT ? Bm + (tid >> 2) * ldb + (tid & 3) * 4 : Bm + (long long)(tid >> 4) * ldb + (tid & 15) * 4;
+    double2 ra0, ra1, rb0, rb1;
+    auto fetch = [&]() {
+        ra0 = *reinterpret_cast<const double2 *>(pa);
+        ra1 = *reinterpret_cast<const double2 *>(pa + 2);
+        rb0 = *reinterpret_cast<const double2 *>(pb);
+        rb1 = *reinterpret_cast<const double2 *>(pb + 2);
+        pa += KS;
+        pb += BT ? KS : KS * ldb;
+    };
+    fetch();
+    for (int k0 = 0; k0 < K; k0 += KS) {
+        __syncthreads();
+        {
+            const int r = tid >> 2, k = (tid & 3) * 4;
+            s.a[k][r] = ra0.x; s.a[k + 1][r] = ra0.y; s.a[k + 2][r] = ra1.x; s.a[k + 3][r] = ra1.y;
+            if (BT) {
+                s.b[k][r] = rb0.x; s.b[k + 1][r] = rb0.y; s.b[k + 2][r] = rb1.x; s.b[k + 3][r] = rb1.y;
+            } else {
+                *reinterpret_cast<double2 *>(&s.b[tid >> 4][(tid & 15) * 4]) = rb0;
+                *reinterpret_cast<double2 *>(&s.b[tid >> 4][(tid & 15) * 4 + 2]) = rb1;
+            }
+        }
+        __syncthreads();
+        if (k0 + KS < K) fetch();
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+            const double2 a0 = *reinterpret_cast<const double2 *>(&s.a[k][2 * ty]);
+            const double2 a1 = *reinterpret_cast<const double2 *>(&s.a[k][32 + 2 * ty]);
+            const double2 b0 = *reinterpret_cast<const double2 *>(&s.b[k][2 * tx]);
+            const double2 b1 = *reinterpret_cast<const double2 *>(&s.b[k][32 + 2 * tx]);
+            const double a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
+        }
+    }
+}
+
+__device__ __forceinline__ int own(int t, int p) { return (p >> 1) * 32 + 2 * t + (p & 1); }
+
+// row r and position in it of the triangle's element x (row r has r + 1 of them)
+__device__ __forceinline__ void triangle(int x, int &r, int &at) {
+    r = (int)((sqrtf(8.0f * x + 1.0f) - 1.0f) * 0.5f);
+    while ((r + 1) * (r + 2) / 2 <= x) ++r;
+    while (r * (r + 1) / 2 > x) --r;
+    at = x - r * (r + 1) / 2;
+}
+
+// L11 and its inverse of the 64 x 64 block D (lower triangle, in shared memory): the
+// elimination of [D | I], one column at a time; W11 is stored, L11 is not needed.
+// *bad is raised on a pivot that is not positive.
+struct Diag {
+    double d[B][B + 1], v[B][B + 1], r[B];
+};
+__device__ void factor_block(Diag &s, double *W, long long ld, int *bad) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int e = tid; e < B * B; e += TP) s.v[e / B][e % B] = e / B == e % B ? 1.0 : 0.0;
+    for (int c = 0; c < B; ++c) {
+        __syncthreads();
+        if (warp == 0) {
+            double d = s.d[c][c];
+            if (!(d > 0.0)) {
+                if (lane == 0) atomicExch(bad, 1);
+                d = 1.0;
+            }
+            const double r = 1.0 / sqrt(d);
+            if (lane == 0) s.r[c] = r;
+            for (int i = c + 1 + lane; i < B; i += 32) s.d[i][c] *= r;
+        }
+        __syncthreads();
+        const double r = s.r[c];
+        for (int i = c + 1 + warp; i < B; i += TP / 32) {
+            const double f = s.d[i][c];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = lane + 32 * h;
+                if (32 * h > i) break;
+                if (j <= c) s.v[i][j] = fma(-f * r, s.v[c][j], s.v[i][j]);
+                else if (j <= i) s.d[i][j] = fma(-f, s.d[j][c], s.d[i][j]);
+            }
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < B * B; e += TP) W[(e / B) * ld + e % B] = s.v[e / B][e % B] * s.r[e / B];
+}
+
+// L (lower) <- S, W <- 0, padding as in the identity.
+__global__ void k_spd_load(const double *__restrict__ S, int n, long long ld, double *L, double *W) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ld * ld) return;
+    const int j = (int)(t / ld), i = (int)(t % ld);  // i along the rows of S: its upper triangle is read in order
+    W[t] = 0.0;
+    if (j <= i) L[i * ld + j] = j < n && i < n ? S[(long long)j * n + i] : i == j ? 1.0 : 0.0;
+}
+
+// M (lower, half the diagonal, zeros above) of K = M + M^T.
+__global__ void k_spd_half(const double *__restrict__ K, int n, long long ld, double *M) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ld * ld) return;
+    const int j = (int)(t / ld), i = (int)(t % ld);
+    const double v = j < n && i < n && j <= i ? K[(long long)j * n + i] : 0.0;
+    M[i * ld + j] = i == j ? 0.5 * v : v;
+}
+
+__global__ void __launch_bounds__(TP) k_spd_first(double *L, long long ld, double *W, int *bad) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    Diag &s = *reinterpret_cast<Diag *>(smem);
+    for (int e = threadIdx.x; e < B * B; e += TP) s.d[e / B][e % B] = e % B <= e / B ? L[(e / B) * ld + e % B] : 0.0;
+    factor_block(s, W, ld, bad);
+}
+
+// 16 rows of L21 = A21 W11^T, or 16 columns of W[k, :] = W11 R[k, :], a CTA (in place).
+__global__ void __launch_bounds__(TP) k_spd_panel(double *L, double *W, long long ld, int k, int nb, const int *bad) {
+    __shared__ double w[B][B + 1], x[16][B + 1];
+    if (*bad) return;
+    const int tid = threadIdx.x, below = 4 * (nb - 1 - k);
+    const double *W11 = W + (long long)k * B * ld + k * B;
+    const bool rows = (int)blockIdx.x < below;
+    double *P = rows ? L + ((long long)(k + 1) * B + 16 * blockIdx.x) * ld + k * B
+                     : W + (long long)k * B * ld + 16 * ((int)blockIdx.x - below);
+    for (int e = tid; e < B * B; e += TP) w[e / B][e % B] = W11[(e / B) * ld + e % B];
+    for (int e = tid; e < 16 * B; e += TP) {
+        if (rows) x[e / B][e % B] = P[(e / B) * ld + e % B];
+        else x[e % 16][e / 16] = P[(e / 16) * ld + e % 16];
+    }
+    __syncthreads();
+    // out[r][c] = sum_q x[r][q] w[c][q], the same for both
+    const int r = tid >> 4, c0 = tid & 15;
+    double acc[4] = {};
+#pragma unroll 8
+    for (int q = 0; q < B; ++q) {
+        const double xv = x[r][q];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) acc[p] = fma(xv, w[c0 + 16 * p][q], acc[p]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < 4; ++p) x[r][c0 + 16 * p] = acc[p];
+    __syncthreads();
+    for (int e = tid; e < 16 * B; e += TP) {
+        if (rows) P[(e / B) * ld + e % B] = x[e / B][e % B];
+        else P[(e / 16) * ld + e % 16] = x[e % 16][e / 16];
+    }
+}
+
+// Tile 0: the next diagonal block, which is then factored while the other tiles run;
+// then the rest of A22's lower tiles and the tiles of R below row k.
+__global__ void __launch_bounds__(TP) k_spd_step(double *L, double *W, long long ld, int k, int nb, int *bad) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    if (__syncthreads_or(*(volatile int *)bad)) return;  // W is not used then
+    const int t = nb - 1 - k, tri = t * (t + 1) / 2, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    Slab &s = *reinterpret_cast<Slab *>(smem);
+    double acc[4][4] = {};
+    double *C;
+    int i, j;
+    if ((int)blockIdx.x < tri) {
+        triangle(blockIdx.x, i, j);
+        i += k + 1;
+        j += k + 1;
+        tile<true>(acc, L + (long long)i * B * ld + k * B, ld, L + (long long)j * B * ld + k * B, ld, B, s);
+        C = L + (long long)i * B * ld + j * B;
+    } else {
+        const int x = blockIdx.x - tri;
+        i = k + 1 + x / (k + 1);
+        j = x % (k + 1);
+        tile<false>(acc, L + (long long)i * B * ld + k * B, ld, W + (long long)k * B * ld + j * B, ld, B, s);
+        C = W + (long long)i * B * ld + j * B;
+    }
+    if (blockIdx.x == 0) {
+        __syncthreads();
+        Diag &d = *reinterpret_cast<Diag *>(smem);
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int a = own(ty, p), b = own(tx, q);
+                d.d[a][b] = b <= a ? C[a * ld + b] - acc[p][q] : 0.0;
+            }
+        factor_block(d, W + (long long)(k + 1) * B * ld + (k + 1) * B, ld, bad);
+        return;
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            double2 *c2 = reinterpret_cast<double2 *>(C + own(ty, p) * ld + 32 * q + 2 * tx);
+            double2 v = *c2;
+            v.x -= acc[p][2 * q];
+            v.y -= acc[p][2 * q + 1];
+            *c2 = v;
+        }
+}
+
+__global__ void __launch_bounds__(TP) k_spd_norm(const double *__restrict__ W, int n, long long ld, double *out) {
+    __shared__ double red[TP / 32];
+    double v = 0.0;
+    const int i = blockIdx.x;
+    for (int j = threadIdx.x; j <= i; j += TP) {
+        const double w = W[i * ld + j];
+        v = fma(w, w, v);
+    }
+    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < TP / 32; ++w) v += red[w];
+        atomicAdd(out, v);
+    }
+}
+
+// N = W M: tile (i, j) is the sum over the blocks j .. i; the longest first.
+__global__ void __launch_bounds__(TP) k_spd_n(const double *__restrict__ W, const double *__restrict__ M, long long ld,
+                                              int nb, double *N) {
+    __shared__ __align__(16) Slab s;
+    int r, j;
+    triangle(blockIdx.x, r, j);
+    const int i = j + nb - 1 - r, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double acc[4][4] = {};
+    tile<false>(acc, W + (long long)i * B * ld + j * B, ld, M + (long long)j * B * ld + j * B, ld, (i - j + 1) * B, s);
+    double *C = N + (long long)i * B * ld + j * B;
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            *reinterpret_cast<double2 *>(C + own(ty, p) * ld + 32 * q + 2 * tx) = make_double2(acc[p][2 * q], acc[p][2 * q + 1]);
+}
+
+// K~ = N W^T + W N^T: tile (i, j <= i) sums over the blocks 0 .. j; the longest first.
+__global__ void __launch_bounds__(TP) k_spd_k(const double *__restrict__ W, const double *__restrict__ N, long long ld,
+                                              int nb, int n, double *out) {
+    __shared__ __align__(16) Slab s;
+    int r, x;
+    triangle(blockIdx.x, r, x);
+    const int j = nb - 1 - r, i = j + x, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double acc[4][4] = {};
+    const long long ro = (long long)i * B * ld, co = (long long)j * B * ld;
+    tile<true>(acc, N + ro, ld, W + co, ld, (j + 1) * B, s);
+    tile<true>(acc, W + ro, ld, N + co, ld, (j + 1) * B, s);
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int a = i * B + own(ty, p), b = j * B + own(tx, q);
+            if (a < n && b <= a) {
+                out[(long long)a * n + b] = acc[p][q];
+                out[(long long)b * n + a] = acc[p][q];
+            }
+        }
+}
+
+unsigned blocks(long long count) { return (unsigned)((count + TP - 1) / TP); }
+
+}  // namespace
+
+bool spd_inverse_factor(Ctx &c, const double *S, long long n, double *W, double &inv_trace) {
+    const long long ld = spd_ld(n);
+    const int nb = (int)(ld / B);
+    T L = alloc(c, {ld, ld}, false), stat = alloc(c, {2}, true);  // |W|^2, bad pivot
+    int *bad = (int *)(stat.p + 1);
+    raise_dynamic_smem((const void *)k_spd_first);
+    raise_dynamic_smem((const void *)k_spd_step);
+    k_spd_load<<<blocks(ld * ld), TP, 0, c.st>>>(S, (int)n, ld, L.p, W);
+    k_spd_first<<<1, TP, sizeof(Diag), c.st>>>(L.p, ld, W, bad);
+    for (int k = 0; k < nb; ++k) {
+        const int t = nb - 1 - k;
+        if (t + k) k_spd_panel<<<4 * (t + k), TP, 0, c.st>>>(L.p, W, ld, k, nb, bad);
+        if (t) k_spd_step<<<t * (t + 1) / 2 + t * (k + 1), TP, sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, bad);
+    }
+    k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, (int)n, ld, stat.p);
+    g_launches.fetch_add(2 * nb + 2, std::memory_order_relaxed);
+    ck(cudaGetLastError(), "inverse factor");
+    double h[2];
+    ck(cudaMemcpyAsync(h, stat.p, sizeof(h), cudaMemcpyDeviceToHost, c.st), "status copy");
+    ck(cudaStreamSynchronize(c.st), "inverse factor sync");
+    inv_trace = h[0];
+    int failed;
+    memcpy(&failed, h + 1, sizeof(int));
+    return failed == 0;
+}
+
+void spd_congruence(Ctx &c, const double *W, const double *K, long long n, double *out) {
+    const long long ld = spd_ld(n);
+    const int nb = (int)(ld / B);
+    T M = alloc(c, {ld, ld}, false), N = alloc(c, {ld, ld}, false);
+    k_spd_half<<<blocks(ld * ld), TP, 0, c.st>>>(K, (int)n, ld, M.p);
+    k_spd_n<<<nb * (nb + 1) / 2, TP, 0, c.st>>>(W, M.p, ld, nb, N.p);
+    k_spd_k<<<nb * (nb + 1) / 2, TP, 0, c.st>>>(W, N.p, ld, nb, (int)n, out);
+    g_launches.fetch_add(3, std::memory_order_relaxed);
+    ck(cudaGetLastError(), "congruence");
+}
+
+}  // namespace s2
+}  // namespace nvpt

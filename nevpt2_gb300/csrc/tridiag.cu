@@ -1,5 +1,4 @@
-// Householder tridiagonalisation of a symmetric FP64 matrix (the PC pencils
-// of the order-n^3 classes), in the output form of LAPACK dsytrd('L'):
+// Householder tridiagonalisation of a symmetric FP64 matrix, in the output form of LAPACK dsytrd('L'):
 // d, e, tau and the reflectors below the subdiagonal of A, so that cuSOLVER's
 // ormtr applies Q.
 //
@@ -39,14 +38,14 @@ namespace {
 constexpr int NBP = 32;        // panel width
 constexpr int TT = 256;        // threads per CTA
 constexpr int PARTS = 2 + 2 * NBP;  // column sums: |x|^2, w.v, (W^T a, V^T a)[NBP]
-// NVPT_SYTRD_SHARE (1..16) overrides the caller's SM split, for tuning on other parts.
-int sm_share(int share) {
+// NVPT_SYTRD_SHARE (1..16): 1/share of the SMs, for tuning on other parts.
+int sm_share() {
     static const int v = [] {
         const char *e = std::getenv("NVPT_SYTRD_SHARE");
         const int x = e ? std::atoi(e) : 0;
-        return (x >= 1 && x <= 16) ? x : 0;
+        return (x >= 1 && x <= 16) ? x : 1;
     }();
-    return v ? v : share;
+    return v;
 }
 __device__ __forceinline__ double block_sum(double v, double *red) {
     for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -243,24 +242,12 @@ __global__ void k_mirror_trailing(double *A, long long n, long long k) {
     if (i < jc) A[i + jc * n] = A[jc + i * n];
 }
 
-// Upper triangle -> lower (column-major): the full symmetric matrix.
-__global__ void k_mirror_to_lower(double *A, long long n) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * n) return;
-    const long long i = t % n, jc = t / n;
-    if (i > jc) A[i + jc * n] = A[jc + i * n];
-}
-
 }  // namespace
 
-int sytrd_lower(Ctx &c, double *A, long long n, double *d, double *e, double *tau, bool upper_valid, int share) {
+int sytrd_lower(Ctx &c, double *A, long long n, double *d, double *e, double *tau) {
     if (n <= 0) return 0;
     constexpr int TPB = 256;
     auto nb = [](long long x) { return (unsigned)((x + TPB - 1) / TPB); };
-    if (upper_valid) {
-        k_mirror_to_lower<<<nb(n * n), TPB, 0, c.st>>>(A, n);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-    }
     int dev = 0, sms = 0, per = 0;
     ck(cudaGetDevice(&dev), "cudaGetDevice");
     ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr");
@@ -272,11 +259,7 @@ int sytrd_lower(Ctx &c, double *A, long long n, double *d, double *e, double *ta
         throw Error(1, "sytrd: order too large for the shared-memory column");
     ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sytrd_panel, TT, vbytes), "occupancy");
     if (per < 1) throw Error(2, "sytrd panel kernel cannot be resident");
-    // 1/share of the SMs per tridiagonalisation: the pencils of a QD step
-    // reach this point together on their own streams and then share the GPU
-    // -- the per-column barrier latency of one overlaps the FP64 products of
-    // the others.
-    const unsigned G = (unsigned)std::max(1, sms / std::max(1, sm_share(share)));
+    const unsigned G = (unsigned)std::max(1, sms / sm_share());
     T V = alloc(c, {NBP, n}, false), W = alloc(c, {NBP, n}, false), y = alloc(c, {n}, false);
     T accs = alloc(c, {2, PARTS}, true);  // zero: the first column of every panel has parity 0
     T barw = alloc(c, {2}, true);  // Bar (12 bytes) in 16 zeroed bytes
@@ -328,7 +311,7 @@ extern "C" int nvpt_sytrd_d(nvpt_context *ctx, int64_t n, double *A, double *d, 
         ck(cublasSetStream(blas.h, st), "cublasSetStream");
         Ctx c{st, blas.h, nullptr};
         c.wait_limit = nvpt_context_wait_limit(ctx);
-        const int rc = sytrd_lower(c, A, n, d, e, tau, false);
+        const int rc = sytrd_lower(c, A, n, d, e, tau);
         if (rc) {
             nvpt_context_error_set(ctx, "sytrd: a grid barrier timed out");
             return NVPT_ETIMEDOUT;

@@ -290,8 +290,8 @@ int nvpt_get_precision(nvpt_context *ctx);
 int nvpt_set_profiling(nvpt_context *ctx, int on);
 int nvpt_profile_read(nvpt_context *ctx, const char *tag, double *ms, int64_t *launches, int64_t *bytes);
 
-/* Polls a device-side wait (the grid barriers of the order-n^3 pencil
- * tridiagonalisation, in nvpt_sytrd_d and nvpt_qdnevpt) makes before it
+/* Polls a device-side wait (between the blocks of a tridiagonalisation or band
+ * reduction, in nvpt_sytrd_d and nvpt_qdnevpt) makes before it
  * gives up on ctx; 0 (the default) restores the built-in limit of 2^22
  * polls with back-off (about 0.4 s).  A wait that gives up makes the kernel
  * return, and the call returns NVPT_ETIMEDOUT with the context still usable.
@@ -299,15 +299,11 @@ int nvpt_profile_read(nvpt_context *ctx, const char *tag, double *ms, int64_t *l
 int nvpt_set_wait_limit(nvpt_context *ctx, int64_t polls);
 
 /* Route of the PC classes in nvpt_qdnevpt (no counterpart in the reference,
- * which always diagonalises).  mode 0 (default): the order-n^3 metrics of
- * the (+-1') classes (order >= 512) are evaluated as resolvents of the pencil
- * K v = w S v when every metric eigenvalue is kept; the other classes follow
- * the reference's eigenpair sequence.  mode 1: every PC class whose metric
- * keeps all eigenvalues (the (+-2), (0') and (+-1') metrics of any order)
- * takes the resolvent route -- closer to the exact sums on near-singular
- * denominators, and slower: the small pencils add FP64 triangular solves on
- * every label and grid-synchronised tridiagonalisations that compete with
- * the large ones. */
+ * which always diagonalises).  A class whose metric keeps every eigenvalue but
+ * exact zeros is evaluated as resolvents of its pencil K v = w S v; a metric that
+ * drops other eigenvalues follows the reference's eigenpair sequence.  Both modes,
+ * 0 (the default) and 1, do this; they differed while the resolvents of the small
+ * pencils were the slower form. */
 int nvpt_set_pc_route(nvpt_context *ctx, int mode);
 
 /* Autotuning of launch parameters (no counterpart in the reference).  With

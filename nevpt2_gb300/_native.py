@@ -165,8 +165,8 @@ class Context:
         self.call("nvpt_set_autotune", 1 if on else 0)
 
     def pc_route(self, mode: int) -> None:
-        """nvpt_set_pc_route: 0 = resolvents for the order-n^3 (+-1') pencils
-        only (default), 1 = for every PC class whose metric is kept whole."""
+        """nvpt_set_pc_route: 0 (default) and 1 take the same route, resolvents for
+        every PC class whose metric is kept whole."""
         self.call("nvpt_set_pc_route", int(mode))
 
     def autotune_report(self) -> dict:

@@ -21,7 +21,7 @@ CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 GENCODE = "-gencode=arch=compute_103a,code=sm_103a"
 
-CUDA_SOURCES = ["capi.cu", "koop_kernels.cu", "koop_sym.cu", "bamat.cu", "bamat_gemm.cu", "bamat_sym.cu", "s2_tensor.cu", "tridiag.cu", "band.cu", "spd.cu", "qdnevpt.cu", "ozaki.cu", "ozaki_wide.cu", "rdm_unfold.cu", "ijkl_sym.cu", "tuner.cu", "container.cpp", "rdm_build.cu"]
+CUDA_SOURCES = ["capi.cu", "koop_kernels.cu", "koop_sym.cu", "bamat.cu", "bamat_gemm.cu", "bamat_sym.cu", "s2_tensor.cu", "tridiag.cu", "band.cu", "tri.cu", "spd.cu", "qdnevpt.cu", "ozaki.cu", "ozaki_wide.cu", "rdm_unfold.cu", "ijkl_sym.cu", "tuner.cu", "container.cpp", "rdm_build.cu"]
 CUDA_HEADERS = ["eexx.cuh", "nvpt2_internal.h", "bamat_sym.cuh", "koop_sym.cuh", "sym_check.cuh", "s2_tensor.cuh", "band.cuh", "spd.cuh", "grid_bar.cuh", "ozaki.cuh", "oz_ptx.cuh", "tuner.h"]
 
 

@@ -337,7 +337,7 @@ __global__ void k_band_extract(const double *__restrict__ A, long long n, double
 
 // One column of Y (column-major, ld n) per CTA: Y <- Q^T Y (forward) or Q Y, the
 // column in shared memory, panel after panel.
-__global__ void __launch_bounds__(TB) k_band_apply(long long n, int npanel, const double *__restrict__ V,
+__global__ void __launch_bounds__(TB) k_wy_apply(long long n, int npanel, int first, const double *__restrict__ V,
                                                    const double *__restrict__ Tm, double *Y, int forward) {
     extern __shared__ double y[];
     __shared__ double red[TB / 32][NB], t_s[NB], s_s[NB];
@@ -346,9 +346,9 @@ __global__ void __launch_bounds__(TB) k_band_apply(long long n, int npanel, cons
     for (long long i = tid; i < n; i += TB) y[i] = col[i];
     __syncthreads();
     for (int q = 0; q < npanel; ++q) {
-        const int p = forward ? q : npanel - 1 - q, r0 = (p + 1) * NB, m = (int)n - r0;
-        // panels are packed one after another: rows n - NB (1 + p') for p' < p before this one
-        const double *v = V + ((long long)p * n - (long long)NB * p * (p + 1) / 2) * NB, *T = Tm + (long long)p * NB * NB;
+        const int p = forward ? q : npanel - 1 - q, r0 = p * NB + first, m = (int)n - r0;
+        // panels are packed one after another: n - first - NB p' rows for each p' < p before this one
+        const double *v = V + (p * (n - first) - (long long)NB * p * (p - 1) / 2) * NB, *T = Tm + (long long)p * NB * NB;
         double s = 0.0;
         for (int i = warp; i < m; i += TB / 32) s = fma(v[(long long)i * NB + lane], y[r0 + i], s);
         red[warp][lane] = s;
@@ -577,13 +577,8 @@ __global__ void __launch_bounds__(TB) k_band_resolvent(const double *__restrict_
 
 }  // namespace
 
-long long band_rows(long long n) {  // rows of all panels
-    const long long np = band_panels(n);
-    return np * n - kBand * np * (np + 1) / 2;
-}
-
 int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *AB) {
-    const int np = band_panels(n);
+    const int np = wy_panels(n, NB);
     T W = alloc(c, {n, NB}, false), G = alloc(c, {NB, NB}, false);
     T msg = alloc(c, {NB, kQrMost + 1, NB}, false), ctl = alloc(c, {1}, true);
     int *err = (int *)ctl.p;
@@ -627,15 +622,15 @@ int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *A
     return h ? 4 : 0;
 }
 
-void band_apply(Ctx &c, long long n, const double *V, const double *Tm, double *Y, long long m, bool forward) {
-    const int np = band_panels(n);
+void wy_apply(Ctx &c, long long n, int first, const double *V, const double *Tm, double *Y, long long m, bool forward) {
+    const int np = wy_panels(n, first);
     if (np == 0 || m == 0) return;
     const size_t smem = sizeof(double) * (size_t)n;
-    if ((long long)smem > raise_dynamic_smem((const void *)k_band_apply))
-        throw Error(NVPT_EINVAL, "band: order above the shared-memory limit");
-    k_band_apply<<<(unsigned)m, TB, smem, c.st>>>(n, np, V, Tm, Y, forward ? 1 : 0);
+    if ((long long)smem > raise_dynamic_smem((const void *)k_wy_apply))
+        throw Error(NVPT_EINVAL, "reflectors: order above the shared-memory limit");
+    k_wy_apply<<<(unsigned)m, TB, smem, c.st>>>(n, np, first, V, Tm, Y, forward ? 1 : 0);
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    ck(cudaGetLastError(), "band apply");
+    ck(cudaGetLastError(), "reflectors");
 }
 
 void band_resolvent(Ctx &c, const double *AB, long long n, const double *Y, long long ncol, long long L, int nother,

@@ -152,7 +152,6 @@ struct nvpt_context {
     long long launches_at_create = 0;
     IjklState ijkl;
     unsigned wait_limit = 0;  // nvpt_set_wait_limit (0 = built-in)
-    int pc_route = 0;         // nvpt_set_pc_route
 };
 
 namespace {
@@ -379,12 +378,9 @@ int nvpt_set_wait_limit(nvpt_context *ctx, int64_t polls) {
     return NVPT_OK;
 }
 
-int nvpt_context_pc_route(const nvpt_context *ctx) { return ctx ? ctx->pc_route : 0; }
-
 int nvpt_set_pc_route(nvpt_context *ctx, int mode) {
     if (!ctx || mode < 0 || mode > 1) return NVPT_EINVAL;
-    ctx->pc_route = mode;
-    return NVPT_OK;
+    return NVPT_OK;  // both modes take the same route
 }
 
 int64_t nvpt_launch_count(const nvpt_context *ctx) { return ctx ? g_launches.load() - ctx->launches_at_create : 0; }

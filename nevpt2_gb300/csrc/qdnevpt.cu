@@ -30,7 +30,6 @@
 #include "s2_tensor.cuh"
 
 extern "C" unsigned nvpt_context_wait_limit(const nvpt_context *ctx);
-extern "C" int nvpt_context_pc_route(const nvpt_context *ctx);
 
 namespace nvpt {
 namespace s2 {
@@ -249,27 +248,8 @@ struct PcResult {
 };
 
 // src/qdnevpt.F:1963-2033 and siblings: the PC metric sequence.
-// Metrics of at least this order take the generalised-eigenproblem route
-// when every metric eigenvalue is above the threshold.
-constexpr long long kPcCholMin = 512;
-
 PcResult pc_transform(Ctx &c, const T &S, const T &K, long long nd, double thr) {
     PcResult r;
-    if (nd >= kPcCholMin && metric_above(c, S.p, nd, thr)) {
-        // Every eigenvalue of S is kept (nnew = nd), so the orthonormalised
-        // Koopmans eigenproblem X^T K X y = w y, X = U w_S^-1/2, is the pencil
-        // K v = w S v with v = X y: same eigenvalues and, up to rotations
-        // inside degenerate eigenspaces, the same PC coefficients C = X Y.
-        // One Cholesky-based solve replaces the metric eigensolve and the
-        // three order-nd GEMMs around it.
-        T w = alloc(c, {nd}, false), V = alloc(c, {nd, nd}, false);
-        if (sygvd_upper(c, K.p, S.p, nd, w.p, V.p)) {
-            r.nnew = (int)nd;
-            r.w = std::move(w);
-            r.C = permuted(c, V, {1, 0});  // C[i][mu] = V[mu][i]
-            return r;
-        }
-    }
     T w = alloc(c, {nd}, false), V = alloc(c, {nd, nd}, false);
     eigh_upper(c, S.p, nd, w.p, V.p);
     std::vector<double> wh(nd);
@@ -527,7 +507,6 @@ class PencilFork {
         a.split = c_.split;
         a.oz_err = c_.oz_err;
         a.wait_limit = c_.wait_limit;
-        a.all_pc_resolvent = c_.all_pc_resolvent;
         a.arena = c_.arena;
         try {
             ck(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming), "cudaEventCreate");
@@ -569,11 +548,10 @@ class PencilFork {
         } else {
             cudaStreamSynchronize(a.st);
         }
-        for (T *t : {&pt_.W, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm}) t->st = c_.st;
+        for (T *t : {&pt_.W, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm, &pt_.d, &pt_.e}) t->st = c_.st;
         a.split = false;
         a.oz_err = nullptr;
         a.wait_limit = 0;
-        a.all_pc_resolvent = false;
         a.arena = nullptr;
         CtxPool::release(aux_, dev_);
         if (ready_) cudaEventDestroy(ready_);
@@ -792,7 +770,11 @@ class Runner {
         if (L > 0 && n > 0) {
             ProfSpan sp;
             sp.begin("pencil_solve", c.st, 0);
-            band_resolvent(c, PT.AB.p, n, Yt.p, Yt.sh[1], L, nother < 0 ? M - 1 : nother, sg.p, a.p, nd, dcol0, rho, xout);
+            if (nother < 0) nother = M - 1;
+            if (n <= kTriMost)
+                tri_resolvent(c, PT.d.p, PT.e.p, n, Yt.p, Yt.sh[1], L, nother, sg.p, a.p, nd, dcol0, rho, xout);
+            else
+                band_resolvent(c, PT.AB.p, n, Yt.p, Yt.sh[1], L, nother, sg.p, a.p, nd, dcol0, rho, xout);
             sp.end();
         }
         return download(c, a.p, 2 + 8);
@@ -806,7 +788,7 @@ class Runner {
     bool pc_resolvent(const T &S, const T &K, long long nd, long long L, int nnew_slot,
                       const std::vector<double> &shift, std::vector<double> &e2, double &psi2,
                       const std::function<void(double *)> &fill) {
-        if (nd == 0 || L == 0 || !c.all_pc_resolvent) return false;
+        if (nd == 0 || L == 0) return false;
         PencilTridiag PT;
         if (!pencil_tridiag(c, K.p, S.p, nd, thr, PT)) return false;
         acc.nnew[nnew_slot + 10 * s] = (int)(nd - PT.k);
@@ -1421,7 +1403,7 @@ class Runner {
                 for (int r = 0; r < nv; ++r) acc.rhoir[i + (size_t)nc * (r + (size_t)nv * s)] += rl[(size_t)i * nv + r];
         };
         PencilTridiag PT;
-        if (c.all_pc_resolvent && pencil_tridiag(c, K.p, S.p, n2, thr, PT)) {
+        if (pencil_tridiag(c, K.p, S.p, n2, thr, PT)) {
             // every metric eigenvalue is kept: resolvents of the pencil (as in
             // the (+-1') classes) on the numerators before the PC basis change,
             //   z = [di A1 + 2 h g1 | -dj A1 + dk A2 - h g1]   (R = z C),
@@ -1578,7 +1560,7 @@ class Runner {
             S = view2(permuted(c, W3, {3, 4, 5, 0, 1, 2}), n3, n3);  // [(a,b,c),(ap,bp,cp)]
             K = view2(permuted(c, A, {3, 4, 5, 0, 1, 2}), n3, n3);
             // the pencil's reduction overlaps the SC work below
-            if (n3 >= kPcCholMin || c.all_pc_resolvent) fork.reset(new PencilFork(c, S, K, n3, thr, PT));
+            fork.reset(new PencilFork(c, S, K, n3, thr, PT));
             Yown = alloc(c, {L, (long long)n3}, false);
             gemm(c, false, false, L, n3, n3, 1.0, Vd.p, n3, S.p, n3, 0.0, Yown.p, n3);
         }
@@ -1836,7 +1818,6 @@ struct ClassStreams {
             x.split = false;
             x.oz_err = nullptr;
             x.wait_limit = 0;
-            x.all_pc_resolvent = false;
             x.arena = nullptr;
         }
         CtxPool::release(c, dev);
@@ -1989,7 +1970,6 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
             pc_.split = c.split;
             pc_.oz_err = c.oz_err;
             pc_.wait_limit = nvpt_context_wait_limit(ctx);
-            pc_.all_pc_resolvent = nvpt_context_pc_route(ctx) == 1;
             pc_.arena = &arena;
         }
     ck(cudaEventRecord(ps.prep, c.st), "event");  // B and h ready

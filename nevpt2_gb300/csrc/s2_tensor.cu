@@ -374,23 +374,32 @@ bool metric_above(Ctx &c, const double *A, long long n, double thr) {
     return sw.status() == 0;
 }
 
-bool sygvd_upper(Ctx &c, const double *K, const double *S, long long n, double *w, double *V) {
-    if (n == 0) return true;
-    T B = alloc(c, {n, n}, false);
-    symmetrize_upper(c, K, n, V);
-    symmetrize_upper(c, S, n, B.p);
-    int lwork = 0;
-    ck(cusolverDnDsygvd_bufferSize(c.sol, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER,
-                                   (int)n, V, (int)n, B.p, (int)n, w, &lwork),
-       "sygvd_bufferSize");
-    SolverWork sw(c, lwork);
-    ck(cusolverDnDsygvd(c.sol, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, (int)n, V,
-                        (int)n, B.p, (int)n, w, sw.w, lwork, sw.info),
-       "sygvd");
-    return sw.status() == 0;
+namespace {
+// A += rel * (largest diagonal element) on the diagonal; that element into *top.
+__global__ void k_shift_diag(double *A, long long n, double rel, double *top) {
+    __shared__ double red[TPB];
+    double m = 0.0;
+    for (long long i = threadIdx.x; i < n; i += TPB) m = fmax(m, A[i * n + i]);
+    red[threadIdx.x] = m;
+    __syncthreads();
+    for (int t = 0; t < TPB; ++t) m = fmax(m, red[t]);
+    for (long long i = threadIdx.x; i < n; i += TPB) A[i * n + i] += rel * m;
+    if (threadIdx.x == 0) *top = m;
 }
 
-namespace {
+// *out += |X[r] . Y[r]|, a row a block.
+__global__ void k_dot_abs(const double *X, const double *Y, long long n, double *out) {
+    __shared__ double red[TPB];
+    double v = 0.0;
+    for (long long i = threadIdx.x; i < n; i += TPB) v = fma(X[blockIdx.x * n + i], Y[blockIdx.x * n + i], v);
+    red[threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int t = 1; t < TPB; ++t) v += red[t];
+        atomicAdd(out, fabs(v));
+    }
+}
+
 // Deterministic start vectors of the inverse iteration, in [-0.5, 0.5).
 __global__ void k_start_block(double *X, long long count) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -402,58 +411,57 @@ __global__ void k_start_block(double *X, long long count) {
 }
 
 // The null vectors of the positive semidefinite S (full storage), if its
-// eigenvalues below thr are all null: N [k, n] orthonormal rows.  Block inverse
-// iteration on S + delta, delta = 1e-9 of the largest diagonal element: a null
-// vector gains a factor w / delta on the kept ones in each of the three steps.
-// False if the metric is not of this kind.
+// eigenvalues below thr are all null: N [k, n] orthonormal rows.  With delta = 1e-9 of
+// the largest diagonal element, delta tr (S + delta)^-1 counts them (a kept eigenvalue
+// w adds delta / w); block inverse iteration on S + delta from k random vectors then
+// gains a factor w / delta in each of three steps, with the block orthonormalised
+// through the inverse factor of its Gram matrix.  False if the metric is not of this
+// kind.  All products and one factorisation of order n: the QR factorisations of a
+// wider block that this replaces took 5 ms at order 216, latency for the most part.
 bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long long &k) {
-    const long long b = std::min<long long>(64, n);
     Ctx f = c;
     f.split = false;
     k = 0;
-    T L = alloc(c, {n, n}, false), X = alloc(c, {b, n}, false), Y = alloc(c, {b, n}, false);
-    T w = alloc(c, {b}, false), H = alloc(c, {b, b}, false), V = alloc(c, {b, b}, false);
     const long long ld = spd_ld(n);
-    T W = alloc(c, {ld, ld}, false);
+    T L = alloc(c, {n, n}, false), W = alloc(c, {ld, ld}, false), top = alloc(c, {1}, true);
     ck(cudaMemcpyAsync(L.p, S, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.st), "copy");
-    std::vector<double> dg(n);
-    ck(cudaMemcpy2DAsync(dg.data(), sizeof(double), S, sizeof(double) * (n + 1), sizeof(double), n,
-                         cudaMemcpyDeviceToHost, c.st), "diagonal");
-    ck(cudaStreamSynchronize(c.st), "sync");
-    double top = 0.0, tr = 0.0;
-    for (double x : dg) top = std::max(top, x);
-    if (!(top > 0.0)) return false;
-    k_add_diag<<<nblk(n), TPB, 0, c.st>>>(L.p, n, 1e-9 * top);
-    k_start_block<<<nblk(b * n), TPB, 0, c.st>>>(X.p, b * n);
-    g_launches.fetch_add(2, std::memory_order_relaxed);
-    if (!spd_inverse_factor(c, L.p, n, W.p, tr)) return false;
-    // rows of X are the columns of a column-major [n, b]: solve, then orthonormalise by QR
-    const int Ni = (int)n, bi = (int)b;
-    T tau = alloc(c, {b}, false);
-    int lq = 0, lg = 0;
-    ck(cusolverDnDgeqrf_bufferSize(c.sol, Ni, bi, X.p, Ni, &lq), "geqrf_bufferSize");
-    ck(cusolverDnDorgqr_bufferSize(c.sol, Ni, bi, bi, X.p, Ni, tau.p, &lg), "orgqr_bufferSize");
-    SolverWork qw(c, std::max(lq, lg));
+    k_shift_diag<<<1, TPB, 0, c.st>>>(L.p, n, 1e-9, top.p);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    double tr = 0.0, st[2], big = 0.0;
+    ck(cudaMemcpyAsync(&big, top.p, sizeof(double), cudaMemcpyDeviceToHost, c.st), "diagonal");
+    if (!spd_inverse_factor(c, L.p, n, W.p, tr) || !(big > 0.0)) return false;  // synchronises
+    const double count = tr * 1e-9 * big;
+    if (!(count < (double)n)) return false;
+    k = std::llround(count);
+    if (k < 1 || 2 * k > n || std::fabs(count - (double)k) > 0.1) return false;
+    T X = alloc(c, {k, n}, false), Y = alloc(c, {k, n}, false), G = alloc(c, {k, k}, false);
+    const long long lk = spd_ld(k);
+    T R = alloc(c, {lk, lk}, false), stat = alloc(c, {2}, true);
+    k_start_block<<<nblk(k * n), TPB, 0, c.st>>>(X.p, k * n);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    auto orthonormalise = [&]() {
+        gemm(f, false, true, k, k, n, 1.0, X.p, n, X.p, n, 0.0, G.p, k);
+        spd_inverse_factor_async(c, G.p, k, R.p, stat.p);
+        gemm(f, false, false, k, n, k, 1.0, R.p, lk, X.p, n, 0.0, Y.p, n);
+        std::swap(X, Y);
+    };
     for (int it = 0; it < 3; ++it) {
-        gemm(f, false, true, b, n, n, 1.0, X.p, n, W.p, ld, 0.0, Y.p, n);
-        gemm(f, false, false, b, n, n, 1.0, Y.p, n, W.p, ld, 0.0, X.p, n);
-        ck(cusolverDnDgeqrf(c.sol, Ni, bi, X.p, Ni, tau.p, qw.w, lq, qw.info), "geqrf");
-        ck(cusolverDnDorgqr(c.sol, Ni, bi, bi, X.p, Ni, tau.p, qw.w, lg, qw.info), "orgqr");
+        gemm(f, false, true, k, n, n, 1.0, X.p, n, W.p, ld, 0.0, Y.p, n);
+        gemm(f, false, false, k, n, n, 1.0, Y.p, n, W.p, ld, 0.0, X.p, n);
+        orthonormalise();
     }
-    std::vector<double> wh(b);
-    // Rayleigh-Ritz in the block
-    gemm(c, false, false, b, n, n, 1.0, X.p, n, S, n, 0.0, Y.p, n);
-    gemm(c, false, true, b, b, n, 1.0, Y.p, n, X.p, n, 0.0, H.p, b);
-    eigh_upper(c, H.p, b, w.p, V.p);
-    ck(cudaMemcpyAsync(wh.data(), w.p, sizeof(double) * b, cudaMemcpyDeviceToHost, c.st), "w copy");
+    orthonormalise();
+    // the Rayleigh quotients, none negative but for rounding: their sum bounds each
+    gemm(f, false, false, k, n, n, 1.0, X.p, n, S, n, 0.0, Y.p, n);
+    ck(cudaMemsetAsync(top.p, 0, sizeof(double), c.st), "memset");
+    k_dot_abs<<<(unsigned)k, TPB, 0, c.st>>>(X.p, Y.p, n, top.p);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    double w = 0.0;
+    ck(cudaMemcpyAsync(&w, top.p, sizeof(double), cudaMemcpyDeviceToHost, c.st), "quotients");
+    ck(cudaMemcpyAsync(st, stat.p, sizeof(st), cudaMemcpyDeviceToHost, c.st), "status");
     ck(cudaStreamSynchronize(c.st), "sync");
-    while (k < b && !(wh[k] >= thr)) {
-        if (!(std::fabs(wh[k]) <= 1e-12 * top)) return false;
-        ++k;
-    }
-    if (k == 0 || k > 48) return false;
-    N = alloc(c, {k, n}, false);
-    gemm(c, false, false, k, n, b, 1.0, V.p, b, X.p, n, 0.0, N.p, n);
+    if (spd_failed(st) || !(w <= 1e-12 * big)) return false;
+    N = std::move(X);
     return true;
 }
 }  // namespace
@@ -504,13 +512,21 @@ bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, doubl
     sp.end();
     K2.release();
     sp.begin("pencil_sytrd", c.st, 0);
-    const int np = band_panels(n);
-    P.V = alloc(c, {band_rows(n), kBand}, false);
-    P.Tm = alloc(c, {np, kBand, kBand}, false);
-    P.AB = alloc(c, {kBand + 1, n}, false);
-    const int rc = band_reduce(c, A.p, n, P.V.p, P.Tm.p, P.AB.p);
+    const bool tri = n <= kTriMost;
+    const int first = tri ? 1 : kBand;
+    P.V = alloc(c, {wy_rows(n, first), kBand}, false);
+    P.Tm = alloc(c, {wy_panels(n, first), kBand, kBand}, false);
+    int rc;
+    if (tri) {
+        P.d = alloc(c, {n}, false);
+        P.e = alloc(c, {n}, false);
+        rc = tri_reduce(c, A.p, n, P.d.p, P.e.p, P.V.p, P.Tm.p);
+    } else {
+        P.AB = alloc(c, {kBand + 1, n}, false);
+        rc = band_reduce(c, A.p, n, P.V.p, P.Tm.p, P.AB.p);
+    }
     sp.end();
-    if (rc != 0) throw Error(4, "pencil reduction: a grid barrier timed out");
+    if (rc != 0) throw Error(4, "pencil reduction: a device wait timed out");
     return true;
 }
 
@@ -528,7 +544,7 @@ void pencil_rhs(Ctx &c, const PencilTridiag &P, double *Y, long long m) {
         gemm(c, false, false, m, P.n, P.k, -1.0, a.p, P.k, P.N.p, P.n, 1.0, Z.p, P.n);
     }
     gemm(f, false, true, m, P.n, P.n, 1.0, Z.p, P.n, P.W.p, spd_ld(P.n), 0.0, Y, P.n);
-    band_apply(c, P.n, P.V.p, P.Tm.p, Y, m, true);
+    wy_apply(c, P.n, P.n <= kTriMost ? 1 : kBand, P.V.p, P.Tm.p, Y, m, true);
     sp.end();
 }
 
@@ -538,7 +554,7 @@ void pencil_back(Ctx &c, const PencilTridiag &P, double *X, long long m) {
     sp.begin("pencil_rhs", c.st, 0);
     Ctx f = c;
     f.split = false;
-    band_apply(c, P.n, P.V.p, P.Tm.p, X, m, false);
+    wy_apply(c, P.n, P.n <= kTriMost ? 1 : kBand, P.V.p, P.Tm.p, X, m, false);
     T Z = alloc(c, {m, P.n}, false);
     ck(cudaMemcpyAsync(Z.p, X, sizeof(double) * m * P.n, cudaMemcpyDeviceToDevice, c.st), "copy");
     gemm(f, false, false, m, P.n, P.n, 1.0, Z.p, P.n, P.W.p, spd_ld(P.n), 0.0, X, P.n);

@@ -157,9 +157,6 @@ struct Ctx {
     // Polls a device-side wait (grid barrier) makes before it gives up and
     // the call reports NVPT_ETIMEDOUT; 0 = the built-in limit.
     unsigned wait_limit = 0;
-    // Resolvents (no eigenvectors) for every PC class whose metric keeps all
-    // its eigenvalues, not only the order-n^3 pencils of the (+-1') classes.
-    bool all_pc_resolvent = false;
     Arena *arena = nullptr;  // small allocations of the call, if any
 };
 
@@ -200,10 +197,6 @@ bool metric_above(Ctx &c, const double *A, long long n, double thr);
 // is the same for every caller, so host threads launching the kernel with
 // different sizes concurrently cannot undercut one another's launches.
 int raise_dynamic_smem(const void *kernel);
-// Generalised symmetric-definite eigenproblem K v = w S v (upper triangles;
-// cusolverDnDsygvd): w ascending, V[k][i] = component i of eigenvector k,
-// eigenvectors S-orthonormal.  False if S is not positive definite.
-bool sygvd_upper(Ctx &c, const double *K, const double *S, long long n, double *w, double *V);
 // Symmetric copy: out = triu(A) + triu(A,1)^T.
 void symmetrize_upper(Ctx &c, const double *A, long long n, double *out);
 
@@ -216,7 +209,9 @@ void symmetrize_upper(Ctx &c, const double *A, long long n, double *out);
 // a block of its own, and right-hand sides are projected by P.
 struct PencilTridiag {
     T W;           // inverse Cholesky factor of the metric (spd.cuh)
-    T AB, V, Tm;   // W K W^T = Q B Q^T (band.cuh)
+    T V, Tm;       // W K W^T = Q B Q^T (band.cuh)
+    T AB;          // B as a band, orders above kTriMost
+    T d, e;        // B tridiagonal, the others
     T N;           // null vectors of the metric [k, n]
     long long n = 0, k = 0;
 };

@@ -298,11 +298,11 @@ unsigned blocks(long long count) { return (unsigned)((count + TP - 1) / TP); }
 
 }  // namespace
 
-bool spd_inverse_factor(Ctx &c, const double *S, long long n, double *W, double &inv_trace) {
+void spd_inverse_factor_async(Ctx &c, const double *S, long long n, double *W, double *stat) {
     const long long ld = spd_ld(n);
     const int nb = (int)(ld / B);
-    T L = alloc(c, {ld, ld}, false), stat = alloc(c, {2}, true);  // |W|^2, bad pivot
-    int *bad = (int *)(stat.p + 1);
+    T L = alloc(c, {ld, ld}, false);
+    int *bad = (int *)(stat + 1);
     raise_dynamic_smem((const void *)k_spd_first);
     raise_dynamic_smem((const void *)k_spd_step);
     k_spd_load<<<blocks(ld * ld), TP, 0, c.st>>>(S, (int)n, ld, L.p, W);
@@ -312,16 +312,25 @@ bool spd_inverse_factor(Ctx &c, const double *S, long long n, double *W, double 
         if (t + k) k_spd_panel<<<4 * (t + k), TP, 0, c.st>>>(L.p, W, ld, k, nb, bad);
         if (t) k_spd_step<<<t * (t + 1) / 2 + t * (k + 1), TP, sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, bad);
     }
-    k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, (int)n, ld, stat.p);
+    k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, (int)n, ld, stat);
     g_launches.fetch_add(2 * nb + 2, std::memory_order_relaxed);
     ck(cudaGetLastError(), "inverse factor");
+}
+
+bool spd_failed(const double *stat_on_host) {
+    int failed;
+    memcpy(&failed, stat_on_host + 1, sizeof(int));
+    return failed != 0;
+}
+
+bool spd_inverse_factor(Ctx &c, const double *S, long long n, double *W, double &inv_trace) {
+    T stat = alloc(c, {2}, true);  // |W|^2, bad pivot
+    spd_inverse_factor_async(c, S, n, W, stat.p);
     double h[2];
     ck(cudaMemcpyAsync(h, stat.p, sizeof(h), cudaMemcpyDeviceToHost, c.st), "status copy");
     ck(cudaStreamSynchronize(c.st), "inverse factor sync");
     inv_trace = h[0];
-    int failed;
-    memcpy(&failed, h + 1, sizeof(int));
-    return failed == 0;
+    return !spd_failed(h);
 }
 
 void spd_congruence(Ctx &c, const double *W, const double *K, long long n, double *out) {

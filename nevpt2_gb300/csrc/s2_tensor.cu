@@ -411,11 +411,11 @@ __global__ void k_start_block(double *X, long long count) {
 }
 
 // The null vectors of the positive semidefinite S (full storage), if its
-// eigenvalues below thr are all null: N [k, n] orthonormal rows.  With delta = 1e-9 of
+// eigenvalues below thr are all null: N [k, n] orthonormal rows.  With delta = 1e-11 of
 // the largest diagonal element, delta tr (S + delta)^-1 counts them (a kept eigenvalue
-// w adds delta / w); block inverse iteration on S + delta from k random vectors then
-// gains a factor w / delta in each of three steps, with the block orthonormalised
-// through the inverse factor of its Gram matrix.  False if the metric is not of this
+// w adds delta / w); two steps of inverse iteration on S + delta from k random vectors
+// gain a factor w / delta each, and the block is orthonormalised through the inverse
+// factor of its Gram matrix, twice.  False if the metric is not of this
 // kind.  All products and one factorisation of order n: the QR factorisations of a
 // wider block that this replaces took 5 ms at order 216, latency for the most part.
 bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long long &k) {
@@ -425,12 +425,12 @@ bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long lo
     const long long ld = spd_ld(n);
     T L = alloc(c, {n, n}, false), W = alloc(c, {ld, ld}, false), top = alloc(c, {1}, true);
     ck(cudaMemcpyAsync(L.p, S, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.st), "copy");
-    k_shift_diag<<<1, TPB, 0, c.st>>>(L.p, n, 1e-9, top.p);
+    k_shift_diag<<<1, TPB, 0, c.st>>>(L.p, n, 1e-11, top.p);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     double tr = 0.0, st[2], big = 0.0;
     ck(cudaMemcpyAsync(&big, top.p, sizeof(double), cudaMemcpyDeviceToHost, c.st), "diagonal");
     if (!spd_inverse_factor(c, L.p, n, W.p, tr) || !(big > 0.0)) return false;  // synchronises
-    const double count = tr * 1e-9 * big;
+    const double count = tr * 1e-11 * big;
     if (!(count < (double)n)) return false;
     k = std::llround(count);
     if (k < 1 || 2 * k > n || std::fabs(count - (double)k) > 0.1) return false;
@@ -439,18 +439,16 @@ bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long lo
     T R = alloc(c, {lk, lk}, false), stat = alloc(c, {2}, true);
     k_start_block<<<nblk(k * n), TPB, 0, c.st>>>(X.p, k * n);
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    auto orthonormalise = [&]() {
-        gemm(f, false, true, k, k, n, 1.0, X.p, n, X.p, n, 0.0, G.p, k);
-        spd_inverse_factor_async(c, G.p, k, R.p, stat.p);
-        gemm(f, false, false, k, n, k, 1.0, R.p, lk, X.p, n, 0.0, Y.p, n);
-        std::swap(X, Y);
-    };
-    for (int it = 0; it < 3; ++it) {
+    for (int it = 0; it < 2; ++it) {
         gemm(f, false, true, k, n, n, 1.0, X.p, n, W.p, ld, 0.0, Y.p, n);
         gemm(f, false, false, k, n, n, 1.0, Y.p, n, W.p, ld, 0.0, X.p, n);
-        orthonormalise();
     }
-    orthonormalise();
+    for (int it = 0; it < 2; ++it) {
+        gemm(f, false, true, k, k, n, 1.0, X.p, n, X.p, n, 0.0, G.p, k);
+        spd_inverse_factor_async(c, G.p, k, R.p, stat.p, false);
+        gemm(f, false, false, k, n, k, 1.0, R.p, lk, X.p, n, 0.0, Y.p, n);
+        std::swap(X, Y);
+    }
     // the Rayleigh quotients, none negative but for rounding: their sum bounds each
     gemm(f, false, false, k, n, n, 1.0, X.p, n, S, n, 0.0, Y.p, n);
     ck(cudaMemsetAsync(top.p, 0, sizeof(double), c.st), "memset");

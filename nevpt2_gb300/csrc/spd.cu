@@ -92,42 +92,68 @@ __device__ __forceinline__ void triangle(int x, int &r, int &at) {
     at = x - r * (r + 1) / 2;
 }
 
-// L11 and its inverse of the 64 x 64 block D (lower triangle, in shared memory): the
-// elimination of [D | I], one column at a time; W11 is stored, L11 is not needed.
-// *bad is raised on a pivot that is not positive.
+// W11 = L11^-1 of the 64 x 64 block D, live rows of it (identity below): in place, the
+// columns already eliminated hold the inverse of the unit-lower factor, the others the
+// reduced block, so that a column is one FMA for each element of the rows below,
+//   M[i][j] -= m_i src[j],  m_i = M[i][c] / M[c][c],  src = (M[c][j < c], 1, M[j > c][c]).
+// Warp 0 runs a column ahead (its entries, reciprocal and multipliers), so the division
+// and its chain are hidden behind the other warps' rows and a column is one barrier;
+// the square roots come last, all rows at once.  *bad is raised on a pivot that is not
+// positive.  A whole block: 125 us (a square root, two barriers and two kinds of
+// element a column) -> 63 us.
 struct Diag {
-    double d[B][B + 1], v[B][B + 1], r[B];
+    double m[B][B + 1], col[2][B], mul[2][B], d[B];
 };
-__device__ void factor_block(Diag &s, double *W, long long ld, int *bad) {
+__device__ void factor_block(Diag &s, double *W, long long ld, int live, int *bad) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int e = tid; e < B * B; e += TP) s.v[e / B][e % B] = e / B == e % B ? 1.0 : 0.0;
-    for (int c = 0; c < B; ++c) {
-        __syncthreads();
-        if (warp == 0) {
-            double d = s.d[c][c];
-            if (!(d > 0.0)) {
-                if (lane == 0) atomicExch(bad, 1);
-                d = 1.0;
-            }
-            const double r = 1.0 / sqrt(d);
-            if (lane == 0) s.r[c] = r;
-            for (int i = c + 1 + lane; i < B; i += 32) s.d[i][c] *= r;
+    // warp 0: column c's entries v0, v1 (rows lane, 32 + lane), their multipliers
+    auto column = [&](int c, double v0, double v1) {
+        const int b = c & 1;
+        double d = __shfl_sync(0xffffffffu, c < 32 ? v0 : v1, c & 31);
+        if (!(d > 0.0)) {
+            if (lane == 0) atomicExch(bad, 1);
+            d = 1.0;
         }
-        __syncthreads();
-        const double r = s.r[c];
-        for (int i = c + 1 + warp; i < B; i += TP / 32) {
-            const double f = s.d[i][c];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = lane + 32 * h;
-                if (32 * h > i) break;
-                if (j <= c) s.v[i][j] = fma(-f * r, s.v[c][j], s.v[i][j]);
-                else if (j <= i) s.d[i][j] = fma(-f, s.d[j][c], s.d[i][j]);
-            }
-        }
-    }
+        const double inv = 1.0 / d;
+        s.col[b][lane] = v0;
+        s.col[b][32 + lane] = v1;
+        s.mul[b][lane] = v0 * inv;
+        s.mul[b][32 + lane] = v1 * inv;
+        if (lane == 0) s.d[c] = d;
+    };
     __syncthreads();
-    for (int e = tid; e < B * B; e += TP) W[(e / B) * ld + e % B] = s.v[e / B][e % B] * s.r[e / B];
+    if (warp == 0) column(0, s.m[lane][0], s.m[32 + lane][0]);
+    __syncthreads();
+    for (int c = 0; c < live; ++c) {
+        const int b = c & 1;
+        if (warp == 0) {
+            if (c + 1 < live) {
+                const double x = s.col[b][c + 1];
+                double v0 = 0.0, v1 = 0.0;
+                if (lane > c) v0 = fma(-s.mul[b][lane], x, s.m[lane][c + 1]);
+                if (32 + lane > c) v1 = fma(-s.mul[b][32 + lane], x, s.m[32 + lane][c + 1]);
+                column(c + 1, v0, v1);
+            }
+        } else {
+            // warp 0 reads column c + 1 as it was: it is not written here, the next column's
+            // entries are in col
+            const double s0 = lane < c ? s.m[c][lane] : lane == c ? 1.0 : s.col[b][lane];
+            const double s1 = 32 + lane < c ? s.m[c][32 + lane] : 32 + lane == c ? 1.0 : s.col[b][32 + lane];
+            for (int i = c + warp; i < live; i += TP / 32 - 1) {
+                const double f = -s.mul[b][i];
+                if (lane <= i && lane != c + 1) s.m[i][lane] = fma(f, s0, lane == c ? 0.0 : s.m[i][lane]);
+                if (i >= 32 && 32 + lane <= i && 32 + lane != c + 1)
+                    s.m[i][32 + lane] = fma(f, s1, 32 + lane == c ? 0.0 : s.m[i][32 + lane]);
+            }
+        }
+        __syncthreads();
+    }
+    if (tid < B) s.d[tid] = tid < live ? 1.0 / sqrt(s.d[tid]) : 1.0;
+    __syncthreads();
+    for (int e = tid; e < B * B; e += TP) {
+        const int i = e / B, j = e % B;
+        W[i * ld + j] = i == j ? s.d[i] : j < i && i < live ? s.m[i][j] * s.d[i] : 0.0;
+    }
 }
 
 // L (lower) <- S, W <- 0, padding as in the identity.
@@ -148,11 +174,11 @@ __global__ void k_spd_half(const double *__restrict__ K, int n, long long ld, do
     M[i * ld + j] = i == j ? 0.5 * v : v;
 }
 
-__global__ void __launch_bounds__(TP) k_spd_first(double *L, long long ld, double *W, int *bad) {
+__global__ void __launch_bounds__(TP) k_spd_first(double *L, long long ld, double *W, int n, int *bad) {
     extern __shared__ __align__(16) unsigned char smem[];
     Diag &s = *reinterpret_cast<Diag *>(smem);
-    for (int e = threadIdx.x; e < B * B; e += TP) s.d[e / B][e % B] = e % B <= e / B ? L[(e / B) * ld + e % B] : 0.0;
-    factor_block(s, W, ld, bad);
+    for (int e = threadIdx.x; e < B * B; e += TP) s.m[e / B][e % B] = e % B <= e / B ? L[(e / B) * ld + e % B] : 0.0;
+    factor_block(s, W, ld, min(B, n), bad);
 }
 
 // 16 rows of L21 = A21 W11^T, or 16 columns of W[k, :] = W11 R[k, :], a CTA (in place).
@@ -191,7 +217,7 @@ __global__ void __launch_bounds__(TP) k_spd_panel(double *L, double *W, long lon
 
 // Tile 0: the next diagonal block, which is then factored while the other tiles run;
 // then the rest of A22's lower tiles and the tiles of R below row k.
-__global__ void __launch_bounds__(TP) k_spd_step(double *L, double *W, long long ld, int k, int nb, int *bad) {
+__global__ void __launch_bounds__(TP) k_spd_step(double *L, double *W, long long ld, int k, int nb, int n, int *bad) {
     extern __shared__ __align__(16) unsigned char smem[];
     if (__syncthreads_or(*(volatile int *)bad)) return;  // W is not used then
     const int t = nb - 1 - k, tri = t * (t + 1) / 2, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -220,9 +246,9 @@ __global__ void __launch_bounds__(TP) k_spd_step(double *L, double *W, long long
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int a = own(ty, p), b = own(tx, q);
-                d.d[a][b] = b <= a ? C[a * ld + b] - acc[p][q] : 0.0;
+                d.m[a][b] = b <= a ? C[a * ld + b] - acc[p][q] : 0.0;
             }
-        factor_block(d, W + (long long)(k + 1) * B * ld + (k + 1) * B, ld, bad);
+        factor_block(d, W + (long long)(k + 1) * B * ld + (k + 1) * B, ld, min(B, n - (k + 1) * B), bad);
         return;
     }
 #pragma unroll
@@ -256,13 +282,13 @@ __global__ void __launch_bounds__(TP) k_spd_norm(const double *__restrict__ W, i
 
 // N = W M: tile (i, j) is the sum over the blocks j .. i; the longest first.
 __global__ void __launch_bounds__(TP) k_spd_n(const double *__restrict__ W, const double *__restrict__ M, long long ld,
-                                              int nb, double *N) {
+                                              int nb, int n, double *N) {
     __shared__ __align__(16) Slab s;
     int r, j;
     triangle(blockIdx.x, r, j);
     const int i = j + nb - 1 - r, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     double acc[4][4] = {};
-    tile<false>(acc, W + (long long)i * B * ld + j * B, ld, M + (long long)j * B * ld + j * B, ld, (i - j + 1) * B, s);
+    tile<false>(acc, W + (long long)i * B * ld + j * B, ld, M + (long long)j * B * ld + j * B, ld, min((i - j + 1) * B, (n + KS - 1) / KS * KS - j * B), s);
     double *C = N + (long long)i * B * ld + j * B;
 #pragma unroll
     for (int p = 0; p < 4; ++p)
@@ -280,8 +306,9 @@ __global__ void __launch_bounds__(TP) k_spd_k(const double *__restrict__ W, cons
     const int j = nb - 1 - r, i = j + x, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     double acc[4][4] = {};
     const long long ro = (long long)i * B * ld, co = (long long)j * B * ld;
-    tile<true>(acc, N + ro, ld, W + co, ld, (j + 1) * B, s);
-    tile<true>(acc, W + ro, ld, N + co, ld, (j + 1) * B, s);
+    const int K = min((j + 1) * B, (n + KS - 1) / KS * KS);  // M has only zeros in the padding
+    tile<true>(acc, N + ro, ld, W + co, ld, K, s);
+    tile<true>(acc, W + ro, ld, N + co, ld, K, s);
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
@@ -298,7 +325,7 @@ unsigned blocks(long long count) { return (unsigned)((count + TP - 1) / TP); }
 
 }  // namespace
 
-void spd_inverse_factor_async(Ctx &c, const double *S, long long n, double *W, double *stat) {
+void spd_inverse_factor_async(Ctx &c, const double *S, long long n, double *W, double *stat, bool trace) {
     const long long ld = spd_ld(n);
     const int nb = (int)(ld / B);
     T L = alloc(c, {ld, ld}, false);
@@ -306,14 +333,14 @@ void spd_inverse_factor_async(Ctx &c, const double *S, long long n, double *W, d
     raise_dynamic_smem((const void *)k_spd_first);
     raise_dynamic_smem((const void *)k_spd_step);
     k_spd_load<<<blocks(ld * ld), TP, 0, c.st>>>(S, (int)n, ld, L.p, W);
-    k_spd_first<<<1, TP, sizeof(Diag), c.st>>>(L.p, ld, W, bad);
+    k_spd_first<<<1, TP, sizeof(Diag), c.st>>>(L.p, ld, W, (int)n, bad);
     for (int k = 0; k < nb; ++k) {
         const int t = nb - 1 - k;
         if (t + k) k_spd_panel<<<4 * (t + k), TP, 0, c.st>>>(L.p, W, ld, k, nb, bad);
-        if (t) k_spd_step<<<t * (t + 1) / 2 + t * (k + 1), TP, sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, bad);
+        if (t) k_spd_step<<<t * (t + 1) / 2 + t * (k + 1), TP, sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, (int)n, bad);
     }
-    k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, (int)n, ld, stat);
-    g_launches.fetch_add(2 * nb + 2, std::memory_order_relaxed);
+    if (trace) k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, (int)n, ld, stat);
+    g_launches.fetch_add(2 * nb + (trace ? 2 : 1), std::memory_order_relaxed);
     ck(cudaGetLastError(), "inverse factor");
 }
 
@@ -325,7 +352,7 @@ bool spd_failed(const double *stat_on_host) {
 
 bool spd_inverse_factor(Ctx &c, const double *S, long long n, double *W, double &inv_trace) {
     T stat = alloc(c, {2}, true);  // |W|^2, bad pivot
-    spd_inverse_factor_async(c, S, n, W, stat.p);
+    spd_inverse_factor_async(c, S, n, W, stat.p, true);
     double h[2];
     ck(cudaMemcpyAsync(h, stat.p, sizeof(h), cudaMemcpyDeviceToHost, c.st), "status copy");
     ck(cudaStreamSynchronize(c.st), "inverse factor sync");
@@ -338,7 +365,7 @@ void spd_congruence(Ctx &c, const double *W, const double *K, long long n, doubl
     const int nb = (int)(ld / B);
     T M = alloc(c, {ld, ld}, false), N = alloc(c, {ld, ld}, false);
     k_spd_half<<<blocks(ld * ld), TP, 0, c.st>>>(K, (int)n, ld, M.p);
-    k_spd_n<<<nb * (nb + 1) / 2, TP, 0, c.st>>>(W, M.p, ld, nb, N.p);
+    k_spd_n<<<nb * (nb + 1) / 2, TP, 0, c.st>>>(W, M.p, ld, nb, (int)n, N.p);
     k_spd_k<<<nb * (nb + 1) / 2, TP, 0, c.st>>>(W, N.p, ld, nb, (int)n, out);
     g_launches.fetch_add(3, std::memory_order_relaxed);
     ck(cudaGetLastError(), "congruence");

@@ -301,7 +301,11 @@ __global__ void __launch_bounds__(256) k_sym_x(Rdm r, int s, int bc, int pr0, co
 // two summed indices, lo the one with stride M, so the tile loads need no
 // intermediate matrix.  64 x 64 tiles, 4 x 4 per thread; bound by the FP64 pipe
 // (n = 16: 13.8 ms for 1.6e10 flops, 1.14 TFLOP/s).
-constexpr int kN8 = 64, kN8K = 16;
+constexpr int kN8K = 16;
+// 64 x 64 tiles from this many on, 32 x 32 below (n <= 7): a tile is 17 us of one SM's FP64
+// pipe for each 16 of its n^2 products, whether the other SMs have one or not.  32 / 64,
+// us: n = 4 9 / 24, n = 6 29 / 57, n = 7 54 / 74.
+constexpr unsigned kN8Tiles = 128;
 // Offset of a row of Gamma3 (in units of M) and the stride of its slow summed index.
 __device__ __forceinline__ ll n8_row(int n, int kind, ll row) {
     const ll n1 = n, n2 = n1 * n, n3 = n2 * n, n4 = n2 * n2, n5 = n4 * n;
@@ -323,9 +327,11 @@ __device__ __forceinline__ double n8_pair2(const Rdm &r, int s, ll row) {
     unpair((int)(row / (n * n)), p, p2);
     return r.d2[s + (ll)r.M * (p + n * (p2 + n * ((row / n) % n + n * (row % n))))];
 }
+template <int kN8>
 __global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__restrict__ I4,
                                                 const double *__restrict__ IJ, double *out, const int *flag) {
     if (*flag) return;
+    constexpr int P = kN8 / 16;  // rows and columns of a thread
     __shared__ double As[kN8K][kN8 + 1], Bs[kN8K][kN8];
     const int n = r.n, np = n * (n + 1) / 2, kind = blockIdx.z;
     const ll M = r.M, n2 = (ll)n * n, rows = np * n2;
@@ -337,48 +343,48 @@ __global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__re
     double *C = out + kind * rows * n2;
     const ll hi = M * n8_hi(n, kind);
     const int tid = threadIdx.x, lk = tid & 15, lr = tid >> 4;
-    const double *base[4];
+    const double *base[P];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < P; ++i) {
         const ll row = min(r0 + lr + 16 * i, rows - 1);
         base[i] = r.d3 + s + M * n8_row(n, kind, row);
     }
-    double acc[4][4] = {};
-    const int tc = (tid & 15) * 4, tr = (tid >> 4) * 4;
+    double acc[P][P] = {};
+    const int tc = (tid & 15) * P, tr = (tid >> 4) * P;
     const int K = (int)n2;
     for (int k0 = 0; k0 < K; k0 += kN8K) {
         const int k = k0 + lk;
         const ll ko = (k / n) * hi + (k % n) * M;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) As[lk][lr + 16 * i] = k < K ? base[i][ko] : 0.0;
+        for (int i = 0; i < P; ++i) As[lk][lr + 16 * i] = k < K ? base[i][ko] : 0.0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int kk = (tid >> 6) + 4 * i, c = tid & 63;
+        for (int i = 0; i < P; ++i) {
+            const int kk = tid / kN8 + 256 / kN8 * i, c = tid % kN8;
             Bs[kk][c] = (k0 + kk < K && c0 + c < N) ? Bm[(ll)(k0 + kk) * N + c0 + c] : 0.0;
         }
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < kN8K; ++kk) {
-            double a[4], b[4];
+            double a[P], b[P];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < P; ++i) {
                 a[i] = As[kk][tr + i];
                 b[i] = Bs[kk][tc + i];
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < P; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < P; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < P; ++i) {
         const ll row = r0 + tr + i;
         if (row >= rows) break;
         const double w = kind == 3 ? n8_pair2(r, s, row) : 0.0;  // J += Gamma2[(p,q), (p',r)] g(x,y)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < P; ++j) {
             const int col = c0 + tc + j;
             if (col >= N) break;
             double v = acc[i][j];
@@ -443,21 +449,24 @@ struct SymView {
     __device__ __forceinline__ ll i4(int a, int b, int c, int d) const { return ((ll)(a * n + b) * n + c) * n + d; }
 };
 
-// n^6 sums over two indices, one thread per n^4 element:
+// n^6 sums over two indices, kSmallLanes threads per n^4 element (a chain of n^2 steps and
+// an idle chip at small n otherwise; n = 8: 32 -> 10 us, n = 16: 174 -> 156):
 //   G1[p,q,c,a] = sum_e J[(p,q),(e,c);e,a]         G3[p,q,r,x] = sum_e J[(p,e),(q,r);x,e]
 //   Q1[p,t,x,y] = sum Gamma2[(p,f),(t,e)] (xf|ye)  J2 as above
 //   JW = J2 + sum Gamma2[(p,f),(e,q)] (xf|ey)      Z[p,c,q,b] = 2 J2 - sum Gamma2[(p,c),(e,f)] (qf|be)
+constexpr int kSmallLanes = 4;
 __global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double *G3, double *Q1, double *JW,
                                                   double *J2, double *Z, const int *flag) {
     if (*flag) return;
-    const int n = v.n;
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= v.n2 * v.n2) return;
-    const int d = (int)(t % n), c = (int)((t / n) % n), b = (int)((t / v.n2) % n), a = (int)(t / (v.n2 * n));
-    double g1 = 0.0, g3 = 0.0, q1 = 0.0, w2 = 0.0, j2 = v.d1(a, b) * v.g[c * n + d], y2 = 0.0;
-    for (int e = 0; e < n; ++e) {
+    const int n = v.n, e0 = threadIdx.x % kSmallLanes;
+    const ll t = ((ll)blockIdx.x * blockDim.x + threadIdx.x) / kSmallLanes;
+    const ll u = t < v.n2 * v.n2 ? t : 0;
+    const int d = (int)(u % n), c = (int)((u / n) % n), b = (int)((u / v.n2) % n), a = (int)(u / (v.n2 * n));
+    double g1 = 0.0, g3 = 0.0, q1 = 0.0, w2 = 0.0, j2 = e0 ? 0.0 : v.d1(a, b) * v.g[c * n + d], y2 = 0.0;
+    for (int e = e0; e < n; e += kSmallLanes) {
         g1 += v.jj(a, b, e, c, e, d);
         g3 += v.jj(a, e, b, c, d, e);
+#pragma unroll 4
         for (int f = 0; f < n; ++f) {
             const double x = v.ai(c, f, d, e);
             q1 = fma(v.d2(a, b, f, e), x, q1);
@@ -466,6 +475,12 @@ __global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double 
             j2 = fma(v.d2(a, e, b, f), v.ai(e, f, c, d), j2);
         }
     }
+    auto sum = [](double x) {
+        for (int o = kSmallLanes / 2; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    };
+    g1 = sum(g1); g3 = sum(g3); q1 = sum(q1); w2 = sum(w2); j2 = sum(j2); y2 = sum(y2);
+    if (e0 || t >= v.n2 * v.n2) return;
     G1[t] = g1; G3[t] = g3; Q1[t] = q1; JW[t] = j2 + w2; J2[t] = j2; Z[t] = 2.0 * j2 - y2;
 }
 
@@ -476,7 +491,9 @@ __global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double 
 // element) keep ap in registers, so that five of their six factors are loaded
 // once for all of them.  n = 16: 5.8 ms (one element per thread, ap across the
 // warp: 24.7 ms).
-constexpr int kOutAp = 4;
+// Up to kOutSmall orbitals in blocks of 64 threads, to spread over the SMs: 64 / 256 threads,
+// us: n = 4 22 / 27, n = 6 24 / 32, n = 7 33 / 35, n = 8 73 / 63.
+constexpr int kOutAp = 4, kOutSmall = 7;
 __global__ void __launch_bounds__(256) k_sym_out(SymView v, double *amat, double *atmat, const int *flag) {
     if (*flag) return;
     const int n = v.n;
@@ -625,9 +642,10 @@ void launch_sym_ops(const double *atwo, const double *f, int ncore, int n, const
 namespace {
 void sym_finish(const SymView &v, const SymScratch &S, double *amat, double *atmat, const int *fl, cudaStream_t st) {
     const ll n = v.n, n4 = n * n * n * n;
-    k_sym_small<<<(unsigned)((n4 + 63) / 64), 64, 0, st>>>(v, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, fl);
-    const dim3 go((unsigned)((n4 * n + 255) / 256), (unsigned)((n + kOutAp - 1) / kOutAp));
-    k_sym_out<<<go, 256, 0, st>>>(v, amat, atmat, fl);
+    k_sym_small<<<(unsigned)((kSmallLanes * n4 + 63) / 64), 64, 0, st>>>(v, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, fl);
+    const int tb = n <= kOutSmall ? 64 : 256;
+    const dim3 go((unsigned)((n4 * n + tb - 1) / tb), (unsigned)((n + kOutAp - 1) / kOutAp));
+    k_sym_out<<<go, tb, 0, st>>>(v, amat, atmat, fl);
     g_launches.fetch_add(2, std::memory_order_relaxed);
 }
 void sym_unpack(const Rdm &r, int s, const SymScratch &S, int *flag, cudaStream_t st) {
@@ -647,8 +665,11 @@ int launch_sym_state(const Rdm &r, int s, const double *atwo, const SymScratch &
     const int n = r.n, np = n * (n + 1) / 2, *fl = flag + s;
     const ll n2 = (ll)n * n, rows = np * n2;
     sym_unpack(r, s, S, flag, st);
-    const dim3 g8((unsigned)((rows + kN8 - 1) / kN8), (unsigned)((n2 + kN8 - 1) / kN8), 4);
-    k_sym_n8<<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
+    // tiles of 64 unless they leave SMs idle
+    auto grid = [&](int t) { return dim3((unsigned)((rows + t - 1) / t), (unsigned)((n2 + t - 1) / t), 4); };
+    const dim3 g8 = grid(64);
+    if (g8.x * g8.y * g8.z >= kN8Tiles) k_sym_n8<64><<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
+    else k_sym_n8<32><<<grid(32), 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
     const FShape fs = f_shape(n);
     const FKernel fk = f_kernel(fs.rpt);
     const int smem = (fs.bc * n * (np | 1) + np * n) * (int)sizeof(double);

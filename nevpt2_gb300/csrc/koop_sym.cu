@@ -66,9 +66,11 @@ __global__ void __launch_bounds__(256) k_ks_prep(Rdm r, const double *__restrict
 
 // blockIdx.x < nf: F3 of a tile of R rows (p,q,c), all columns a: K = n np + n, the
 // rows of Gamma3 affine in (d, f, e) with e the fastest index, two loads per K for
-// the symmetric pair (d,f).  The other blocks: the n^6 sums, a thread per element.
+// the symmetric pair (d,f).  The other blocks: the n^6 sums, one or four threads per element
+// (n = 8, the whole kernel: 31 -> 16 us with four).
 // blockIdx.y: the state.
 constexpr int kKsRpt = 4;
+template <int kSumLanes>
 __global__ void __launch_bounds__(256) k_ks_sums(Rdm r, const double *__restrict__ atwo, KsScratch S, int nf,
                                                  int R, int kc, const int *flag) {
     extern __shared__ double sm[];
@@ -77,15 +79,19 @@ __global__ void __launch_bounds__(256) k_ks_sums(Rdm r, const double *__restrict
     const ll M = r.M, n1 = n, n2 = n1 * n, n3 = n2 * n, n4 = n3 * n, n5 = n4 * n;
     const int np = n * (n + 1) / 2;
     if (blockIdx.x >= nf) {
-        const ll t = (ll)(blockIdx.x - nf) * blockDim.x + tid;
-        if (t >= n4) return;
-        const int d = (int)(t % n), c = (int)((t / n) % n), b = (int)((t / n2) % n), a = (int)(t / n3);
+        // kSumLanes threads an element, e over them
+        const ll t = ((ll)(blockIdx.x - nf) * 256 + tid) / kSumLanes;
+        const int e0 = tid % kSumLanes;
+        const bool in = t < n4;
+        const ll u = in ? t : 0;
+        const int d = (int)(u % n), c = (int)((u / n) % n), b = (int)((u / n2) % n), a = (int)(u / n3);
         auto d2 = [&](int i, int j, int k, int l) { return r.d2[s + M * (i + n * (j + n * (k + n * l)))]; };
         auto d1 = [&](int i, int j) { return r.d1[s + M * (i + n * j)]; };
         const double h = S.B[(ll)np * n2 + c * n + d];
-        double j2 = d1(a, b) * h, w2 = 0.0, q1 = 0.0, x2 = 0.0, t1 = 0.0;
-        for (int e = 0; e < n; ++e) {
+        double j2 = e0 ? 0.0 : d1(a, b) * h, w2 = 0.0, q1 = 0.0, x2 = 0.0, t1 = 0.0;
+        for (int e = e0; e < n; e += kSumLanes) {
             t1 = fma(d1(a, e), AT(b, c, d, e), t1);
+#pragma unroll 4
             for (int f = 0; f < n; ++f) {
                 const double x = AT(c, f, d, e);
                 j2 = fma(d2(a, e, b, f), AT(e, f, c, d), j2);
@@ -94,16 +100,24 @@ __global__ void __launch_bounds__(256) k_ks_sums(Rdm r, const double *__restrict
                 x2 = fma(d2(a, f, b, e), x, x2);
             }
         }
-        S.arr(s, kJ2)[t] = j2;
-        S.arr(s, kW2)[t] = w2;
-        S.arr(s, kQ1)[t] = q1;
-        S.arr(s, kX2)[t] = x2;
-        S.arr(s, kT1)[t] = t1;
-        if (t < n2) {  // a = b = 0
-            double y = -2.0 * h;
-            for (int e = 0; e < n; ++e)
+        auto sum = [](double v) {
+            for (int o = kSumLanes / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            return v;
+        };
+        j2 = sum(j2); w2 = sum(w2); q1 = sum(q1); x2 = sum(x2); t1 = sum(t1);
+        if (in && e0 == 0) {
+            S.arr(s, kJ2)[t] = j2;
+            S.arr(s, kW2)[t] = w2;
+            S.arr(s, kQ1)[t] = q1;
+            S.arr(s, kX2)[t] = x2;
+            S.arr(s, kT1)[t] = t1;
+        }
+        if (__any_sync(0xffffffffu, t < n2)) {  // a = b = 0
+            double y = e0 ? 0.0 : -2.0 * h;
+            for (int e = e0; e < n; e += kSumLanes)
                 for (int f = 0; f < n; ++f) y += d1(e, f) * (AT(c, f, d, e) - 2.0 * AT(e, f, c, d));
-            S.arr(s, kY)[t] = y;
+            y = sum(y);
+            if (t < n2 && e0 == 0) S.arr(s, kY)[t] = y;
         }
         return;
     }
@@ -240,6 +254,11 @@ __global__ void __launch_bounds__(256) k_ks_out(Rdm r, const double *__restrict_
 
 }  // namespace
 
+// Four threads an element of the n^6 sums up to this many elements, one above: four fill
+// the chip, and read Gamma2 across its stride.  The kernel with four / one thread, us:
+// n = 8 16 / 31, n = 11 51 / 79, n = 13 140 / 150, n = 13 with two states 305 / 238.
+constexpr ll kSumLanesMost = 32768;
+
 int launch_koop_sym(const Rdm &r, const double *atwo, const double *aj, int ncore, int kind, double *const out[5],
                     int *flag, cudaStream_t st) {
     const int n = r.n, np = n * (n + 1) / 2;
@@ -262,7 +281,10 @@ int launch_koop_sym(const Rdm &r, const double *atwo, const double *aj, int ncor
     const int R = (int)std::max<ll>(std::min<ll>(most, n3 * ns / 304), std::min(4, most));
     const int kc = std::max(32, std::min(256, 2048 / R)), nf = (int)((n3 + R - 1) / R);
     const size_t smem = sizeof(double) * (size_t)std::max(kc * (R | 1) + kc * n, R * n);
-    k_ks_sums<<<dim3((unsigned)(nf + (n4 + 255) / 256), ns), 256, smem, st>>>(r, atwo, S, nf, R, kc, flag);
+    const int lanes = n4 * ns <= kSumLanesMost ? 4 : 1;
+    const dim3 g((unsigned)(nf + (lanes * n4 + 255) / 256), ns);
+    if (lanes == 4) k_ks_sums<4><<<g, 256, smem, st>>>(r, atwo, S, nf, R, kc, flag);
+    else k_ks_sums<1><<<g, 256, smem, st>>>(r, atwo, S, nf, R, kc, flag);
     k_ks_out<<<dim3((unsigned)((n4 + 255) / 256), ns), 256, 0, st>>>(r, atwo, S, kind, o, flag);
     g_launches.fetch_add(3, std::memory_order_relaxed);
     cudaFreeAsync(w, st);

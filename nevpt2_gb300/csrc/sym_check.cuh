@@ -20,16 +20,20 @@ __device__ __forceinline__ void unpair(int p, int &i, int &j) {  // p = pidx(i, 
     j = p - pidx(i, 0);
 }
 
+// Scales are compared by their leading 32 bits: comparisons of doubles run on the FP64
+// pipe (16 clocks a warp), and every block takes its own scale.
+__device__ __forceinline__ unsigned abs_hi(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
+
 // Tolerance of the RDM checks of state s (0-based): all threads of the block.
 __device__ __forceinline__ double rdm_tolerance(const Rdm &r, int s) {
-    __shared__ double red[8];
-    double m = 0.0;
-    for (int i = threadIdx.x; i < r.n * r.n; i += blockDim.x) m = fmax(m, fabs(r.d1[s + (ll)r.M * i]));
-    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    __shared__ unsigned red[8];
+    unsigned m = 0;
+    for (int i = threadIdx.x; i < r.n * r.n; i += blockDim.x) m = max(m, abs_hi(r.d1[s + (ll)r.M * i]));
+    m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-    return kSymTol * m;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = max(m, red[w]);
+    return kSymTol * __hiloint2double((int)m, 0);
 }
 __device__ __forceinline__ bool sym_differ(double x, double y, double tol) { return !(fabs(x - y) <= tol); }
 
@@ -62,9 +66,9 @@ __device__ __forceinline__ bool rdm_asymmetric(const Rdm &r, int s, ll t, double
 // Element (i,j,k,l) of the integrals against its images.
 __device__ __forceinline__ bool integral_asymmetric(const double *atwo, int n, int i, int j, int k, int l) {
     auto at = [&](int a, int b, int c, int d) { return atwo[a + n * (b + n * (c + (ll)n * d))]; };
-    double scale = 0.0;
-    for (int q = 0; q < n; ++q) scale = fmax(scale, fabs(at(q, q, q, q)));
-    const double v = at(i, j, k, l), tol = kSymTol * scale;
+    unsigned scale = 0;
+    for (int q = 0; q < n; ++q) scale = max(scale, abs_hi(at(q, q, q, q)));
+    const double v = at(i, j, k, l), tol = kSymTol * __hiloint2double((int)scale, 0);
     return sym_differ(v, at(j, i, k, l), tol) || sym_differ(v, at(k, l, i, j), tol);
 }
 

@@ -267,63 +267,63 @@ __global__ void __launch_bounds__(TB) k_band_w(int m, const double *__restrict__
     }
 }
 
-// A22 -= V W^T + W V^T, 64 x 64 tiles of the lower triangle, each also written
-// to its mirror image (the matrix stays in full storage).
+// A22 -= V W^T + W V^T, 32 x 32 tiles of the lower triangle, each also written to its
+// mirror image (the matrix stays in full storage).  Bound by the FP64 pipe; tiles of 64
+// left SMs idle in the last wave of each panel.  Order 2744, all panels: 15.4 -> 12.3 ms
+// (2/3 n^3 flops, 12.1 ms at the FP64 rate).
 __global__ void __launch_bounds__(TB) k_band_update(double *__restrict__ A, long long n, int r0, int m,
                                                     const double *__restrict__ V, const double *__restrict__ W) {
-    __shared__ double Ls[64][LP], Rs[64][LP];
+    __shared__ double Ls[2][32][LP], Rs[2][32][LP];
     // tile (I >= J) of the triangle
     int I = (int)((sqrtf(8.0f * blockIdx.x + 1.0f) - 1.0f) * 0.5f);
     while ((I + 1) * (I + 2) / 2 <= (int)blockIdx.x) ++I;
     while (I * (I + 1) / 2 > (int)blockIdx.x) --I;
-    const int J = blockIdx.x - I * (I + 1) / 2, i0 = I * 64, jq = J * 64, tid = threadIdx.x;
+    const int i0 = I * 32, j0 = (blockIdx.x - I * (I + 1) / 2) * 32, tid = threadIdx.x;
     const int tr = tid & 15, tc = tid >> 4;
-    double acc[4][4] = {};
-    for (int half = 0; half < 2; ++half) {
-        const double *L = half ? W : V, *Rr = half ? V : W;
-        for (int e = tid; e < 64 * NB; e += TB) {
-            const int i = e / NB, k = e % NB;
-            Ls[i][k] = i0 + i < m ? L[(long long)(i0 + i) * NB + k] : 0.0;
-            Rs[i][k] = jq + i < m ? Rr[(long long)(jq + i) * NB + k] : 0.0;
+    for (int e = tid; e < 32 * NB; e += TB) {
+        const int r = e / NB, k = e % NB;
+        const bool li = i0 + r < m, lj = j0 + r < m;
+        const long long a = (long long)(i0 + r) * NB + k, b = (long long)(j0 + r) * NB + k;
+        Ls[0][r][k] = li ? V[a] : 0.0;
+        Ls[1][r][k] = li ? W[a] : 0.0;
+        Rs[0][r][k] = lj ? W[b] : 0.0;
+        Rs[1][r][k] = lj ? V[b] : 0.0;
+    }
+    // the old tile arrives meanwhile
+    double old[2][2], acc[2][2] = {};
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = i0 + tr + 16 * p, j = j0 + tc + 16 * q;
+            old[p][q] = i < m && j < m ? A[(r0 + i) + (r0 + j) * n] : 0.0;
         }
-        __syncthreads();
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
 #pragma unroll 8
         for (int k = 0; k < NB; ++k) {
-            double l[4], r[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                l[q] = Ls[tr + 16 * q][k];
-                r[q] = Rs[tc + 16 * q][k];
-            }
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[p][q] = fma(l[p], r[q], acc[p][q]);
+            const double l0 = Ls[h][tr][k], l1 = Ls[h][tr + 16][k], r0_ = Rs[h][tc][k], r1 = Rs[h][tc + 16][k];
+            acc[0][0] = fma(l0, r0_, acc[0][0]);
+            acc[0][1] = fma(l0, r1, acc[0][1]);
+            acc[1][0] = fma(l1, r0_, acc[1][0]);
+            acc[1][1] = fma(l1, r1, acc[1][1]);
         }
-        __syncthreads();
-    }
+    __syncthreads();
     // the new tile, through shared memory for the mirror image
-    double *S = &Ls[0][0];  // [64][33] halves: 64 x 32 at a time
-    for (int h = 0; h < 2; ++h) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                const int i = i0 + tr + 16 * p, jl = tc + 16 * q, j = jq + 32 * h + jl;
-                double v = 0.0;
-                if (i < m && j < m && i >= j) {
-                    double *x = A + (r0 + i) + (r0 + j) * n;
-                    v = *x - acc[p][2 * h + q];
-                    *x = v;
-                }
-                S[(tr + 16 * p) * LP + jl] = v;
-            }
-        __syncthreads();
-        for (int e = tid; e < 64 * 32; e += TB) {
-            const int jl = e & 31, i = i0 + (e >> 5), j = jq + 32 * h + jl;
-            if (i < m && j < m && i > j) A[(r0 + j) + (r0 + i) * n] = S[(e >> 5) * LP + jl];
+        for (int q = 0; q < 2; ++q) {
+            const int i = i0 + tr + 16 * p, j = j0 + tc + 16 * q;
+            const double v = old[p][q] - acc[p][q];
+            if (i < m && j < m && i >= j) A[(r0 + i) + (r0 + j) * n] = v;
+            Ls[0][tr + 16 * p][tc + 16 * q] = v;
         }
-        __syncthreads();
+    __syncthreads();
+    for (int e = tid; e < 32 * 32; e += TB) {
+        const int j = j0 + (e & 31), i = i0 + (e >> 5);
+        if (i < m && j < m && i > j) A[(r0 + j) + (r0 + i) * n] = Ls[0][e >> 5][e & 31];
     }
 }
 
@@ -586,8 +586,9 @@ int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *A
     ck(cudaGetDevice(&dev), "cudaGetDevice");
     ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr");
     const int lim = raise_dynamic_smem((const void *)k_band_qr);
-    // shares of A22 V: enough CTAs for the chip, at least 128 of K each
-    const int most = (int)std::max<long long>(1, std::min<long long>(8, n / 128));
+    // shares of A22 V: eight CTAs an SM, so that the last one costs little, at least 64 of K each
+    // (two an SM: 15.7 ms for all panels of order 2744, eight: 12.6)
+    const int most = (int)std::max<long long>(1, std::min<long long>(16, n / 64));
     T Zp = alloc(c, {most, n, NB}, false);
     double *v = V;
     for (int p = 0; p < np; ++p) {
@@ -603,13 +604,12 @@ int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *A
         void *args[] = {&q};
         ck(cudaLaunchCooperativeKernel((const void *)k_band_qr, dim3(ctas), dim3(TB), args, smem, c.st),
            "cooperative launch");
-        const int tiles = (m + 31) / 32, splits = std::max(1, std::min(most, std::min((2 * sms + tiles - 1) / tiles, m / 128)));
+        const int tiles = (m + 31) / 32, splits = std::max(1, std::min(most, std::min((8 * sms + tiles / 2) / tiles, m / 64)));
         const int per = ((m + splits - 1) / splits + 31) / 32 * 32, ns = (m + per - 1) / per;
         k_band_z<<<dim3(tiles, ns), TB, 0, c.st>>>(A, n, r0, m, per, v, Zp.p);
         k_band_g<<<(m + kGRows - 1) / kGRows, TB, 0, c.st>>>(m, ns, v, Zp.p, G.p);
         k_band_w<<<(m + kGRows - 1) / kGRows, TB, 0, c.st>>>(m, v, Zp.p, t, G.p, W.p);
-        const int t64 = (m + 63) / 64;
-        k_band_update<<<t64 * (t64 + 1) / 2, TB, 0, c.st>>>(A, n, r0, m, v, W.p);
+        k_band_update<<<tiles * (tiles + 1) / 2, TB, 0, c.st>>>(A, n, r0, m, v, W.p);
         g_launches.fetch_add(5, std::memory_order_relaxed);
         v += (long long)m * NB;
     }

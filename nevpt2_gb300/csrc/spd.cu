@@ -15,7 +15,7 @@
 // W also gives tr S^-1 = |W|^2, which bounds the smallest metric eigenvalue (no second
 // factorisation of S - thr in the common case), and takes right-hand sides by products.
 // Order 2744 (with the library's two factorisations, triangular solves and rank-2k
-// updates before): 90 -> 38 ms.
+// updates before): 90 -> 36 ms.
 #include <algorithm>
 #include <cstring>
 
@@ -34,14 +34,16 @@ struct Slab {
     double a[KS][LS], b[KS][LS];
 };
 
-// acc += A B^T (BT: B [64][ldb], k along the rows) or A B (B [K][ldb]) for the 64 x K
-// tile A [64][lda]; K a multiple of KS.  Thread (ty, tx) holds rows {2ty, 2ty+1, 32+2ty,
-// 33+2ty} and columns {2tx, ...}; the next slab's loads are issued before the FMAs.
-template <bool BT>
-__device__ __forceinline__ void tile(double (&acc)[4][4], const double *A, long long lda, const double *Bm, long long ldb,
+// acc += A B^T (BT: B [64][ldb], k along the rows) or A B (B [K][ldb]) for the 16 R x K
+// tile A [16 R][lda]; K a multiple of KS.  Thread (ty, tx) holds rows {2ty, 2ty+1} (R = 4:
+// and {32+2ty, 33+2ty}) and columns {2tx, 2tx+1, 32+2tx, 33+2tx}; the next slab's loads are
+// issued before the FMAs.
+template <bool BT, int R>
+__device__ __forceinline__ void tile(double (&acc)[R][4], const double *A, long long lda, const double *Bm, long long ldb,
                                      int K, Slab &s) {
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const double *pa = A + (tid >> 2) * lda + (tid & 3) * 4;
+    const bool la = R == 4 || tid < 128;
+    const double *pa = A + (la ? tid >> 2 : 0) * lda + (tid & 3) * 4;
     const double *pb = BT ? Bm + (tid >> 2) * ldb + (tid & 3) * 4 : Bm + (long long)(tid >> 4) * ldb + (tid & 15) * 4;
     double2 ra0, ra1, rb0, rb1;
     auto fetch = [&]() {
@@ -57,7 +59,9 @@ __device__ __forceinline__ void tile(double (&acc)[4][4], const double *A, long 
         __syncthreads();
         {
             const int r = tid >> 2, k = (tid & 3) * 4;
-            s.a[k][r] = ra0.x; s.a[k + 1][r] = ra0.y; s.a[k + 2][r] = ra1.x; s.a[k + 3][r] = ra1.y;
+            if (la) {
+                s.a[k][r] = ra0.x; s.a[k + 1][r] = ra0.y; s.a[k + 2][r] = ra1.x; s.a[k + 3][r] = ra1.y;
+            }
             if (BT) {
                 s.b[k][r] = rb0.x; s.b[k + 1][r] = rb0.y; s.b[k + 2][r] = rb1.x; s.b[k + 3][r] = rb1.y;
             } else {
@@ -70,12 +74,12 @@ __device__ __forceinline__ void tile(double (&acc)[4][4], const double *A, long 
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
             const double2 a0 = *reinterpret_cast<const double2 *>(&s.a[k][2 * ty]);
-            const double2 a1 = *reinterpret_cast<const double2 *>(&s.a[k][32 + 2 * ty]);
+            const double2 a1 = R == 4 ? *reinterpret_cast<const double2 *>(&s.a[k][32 + 2 * ty]) : a0;
             const double2 b0 = *reinterpret_cast<const double2 *>(&s.b[k][2 * tx]);
             const double2 b1 = *reinterpret_cast<const double2 *>(&s.b[k][32 + 2 * tx]);
             const double a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
+            for (int p = 0; p < R; ++p)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
         }
@@ -215,30 +219,19 @@ __global__ void __launch_bounds__(TP) k_spd_panel(double *L, double *W, long lon
     }
 }
 
-// Tile 0: the next diagonal block, which is then factored while the other tiles run;
-// then the rest of A22's lower tiles and the tiles of R below row k.
+// Block 0: the next diagonal block, which is then factored while the other tiles run;
+// then the rest of A22's lower tiles and the tiles of R below row k, a half (32 rows) a
+// block, so that the last wave leaves less of the chip idle (order 2744, all steps: 15.9 ->
+// 13.3 ms).
 __global__ void __launch_bounds__(TP) k_spd_step(double *L, double *W, long long ld, int k, int nb, int n, int *bad) {
     extern __shared__ __align__(16) unsigned char smem[];
     if (__syncthreads_or(*(volatile int *)bad)) return;  // W is not used then
     const int t = nb - 1 - k, tri = t * (t + 1) / 2, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     Slab &s = *reinterpret_cast<Slab *>(smem);
-    double acc[4][4] = {};
-    double *C;
-    int i, j;
-    if ((int)blockIdx.x < tri) {
-        triangle(blockIdx.x, i, j);
-        i += k + 1;
-        j += k + 1;
-        tile<true>(acc, L + (long long)i * B * ld + k * B, ld, L + (long long)j * B * ld + k * B, ld, B, s);
-        C = L + (long long)i * B * ld + j * B;
-    } else {
-        const int x = blockIdx.x - tri;
-        i = k + 1 + x / (k + 1);
-        j = x % (k + 1);
-        tile<false>(acc, L + (long long)i * B * ld + k * B, ld, W + (long long)k * B * ld + j * B, ld, B, s);
-        C = W + (long long)i * B * ld + j * B;
-    }
     if (blockIdx.x == 0) {
+        const double *P = L + (long long)(k + 1) * B * ld + k * B, *C = P + B;
+        double acc[4][4] = {};
+        tile<true, 4>(acc, P, ld, P, ld, B, s);
         __syncthreads();
         Diag &d = *reinterpret_cast<Diag *>(smem);
 #pragma unroll
@@ -251,11 +244,27 @@ __global__ void __launch_bounds__(TP) k_spd_step(double *L, double *W, long long
         factor_block(d, W + (long long)(k + 1) * B * ld + (k + 1) * B, ld, min(B, n - (k + 1) * B), bad);
         return;
     }
+    const int x = ((int)blockIdx.x + 1) / 2, half = ((int)blockIdx.x + 1) % 2 * 32;  // tile x >= 1
+    double acc[2][4] = {};
+    double *C;
+    int i, j;
+    if (x < tri) {
+        triangle(x, i, j);
+        i += k + 1;
+        j += k + 1;
+        tile<true, 2>(acc, L + ((long long)i * B + half) * ld + k * B, ld, L + (long long)j * B * ld + k * B, ld, B, s);
+        C = L + ((long long)i * B + half) * ld + j * B;
+    } else {
+        i = k + 1 + (x - tri) / (k + 1);
+        j = (x - tri) % (k + 1);
+        tile<false, 2>(acc, L + ((long long)i * B + half) * ld + k * B, ld, W + (long long)k * B * ld + j * B, ld, B, s);
+        C = W + ((long long)i * B + half) * ld + j * B;
+    }
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            double2 *c2 = reinterpret_cast<double2 *>(C + own(ty, p) * ld + 32 * q + 2 * tx);
+            double2 *c2 = reinterpret_cast<double2 *>(C + (2 * ty + p) * ld + 32 * q + 2 * tx);
             double2 v = *c2;
             v.x -= acc[p][2 * q];
             v.y -= acc[p][2 * q + 1];
@@ -288,7 +297,7 @@ __global__ void __launch_bounds__(TP) k_spd_n(const double *__restrict__ W, cons
     triangle(blockIdx.x, r, j);
     const int i = j + nb - 1 - r, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     double acc[4][4] = {};
-    tile<false>(acc, W + (long long)i * B * ld + j * B, ld, M + (long long)j * B * ld + j * B, ld, min((i - j + 1) * B, (n + KS - 1) / KS * KS - j * B), s);
+    tile<false, 4>(acc, W + (long long)i * B * ld + j * B, ld, M + (long long)j * B * ld + j * B, ld, min((i - j + 1) * B, (n + KS - 1) / KS * KS - j * B), s);
     double *C = N + (long long)i * B * ld + j * B;
 #pragma unroll
     for (int p = 0; p < 4; ++p)
@@ -307,8 +316,8 @@ __global__ void __launch_bounds__(TP) k_spd_k(const double *__restrict__ W, cons
     double acc[4][4] = {};
     const long long ro = (long long)i * B * ld, co = (long long)j * B * ld;
     const int K = min((j + 1) * B, (n + KS - 1) / KS * KS);  // M has only zeros in the padding
-    tile<true>(acc, N + ro, ld, W + co, ld, K, s);
-    tile<true>(acc, W + ro, ld, N + co, ld, K, s);
+    tile<true, 4>(acc, N + ro, ld, W + co, ld, K, s);
+    tile<true, 4>(acc, W + ro, ld, N + co, ld, K, s);
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
@@ -337,7 +346,7 @@ void spd_inverse_factor_async(Ctx &c, const double *S, long long n, double *W, d
     for (int k = 0; k < nb; ++k) {
         const int t = nb - 1 - k;
         if (t + k) k_spd_panel<<<4 * (t + k), TP, 0, c.st>>>(L.p, W, ld, k, nb, bad);
-        if (t) k_spd_step<<<t * (t + 1) / 2 + t * (k + 1), TP, sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, (int)n, bad);
+        if (t) k_spd_step<<<2 * (t * (t + 1) / 2 + t * (k + 1)) - 1, TP, sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, (int)n, bad);
     }
     if (trace) k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, (int)n, ld, stat);
     g_launches.fetch_add(2 * nb + (trace ? 2 : 1), std::memory_order_relaxed);

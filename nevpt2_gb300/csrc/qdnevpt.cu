@@ -495,23 +495,24 @@ class CtxPool {
 // The reduction of one pencil K v = w S v on a helper stream and host thread:
 // the Cholesky check of the metric, its factorisation, the reduction to
 // standard form and the tridiagonalisation need only S and K, so they overlap
-// the caller's work on its own stream.  join() waits for them, orders the
-// caller's stream after the helper's and hands the pencil's buffers to the
-// caller's stream (where they are used and freed from then on).
+// the caller's work on its own stream.  join(to) waits for them, orders the
+// stream of `to` after the helper's and hands the pencil's buffers to it (where
+// they are used and freed from then on).
 class PencilFork {
   public:
-    PencilFork(Ctx &caller, const T &S, const T &K, long long n, double thr, PencilTridiag &pt) : c_(caller), pt_(pt) {
+    PencilFork(Ctx &caller, const T &S, const T &K, long long n, double thr, PencilTridiag &pt)
+        : c_(&caller), pt_(pt) {
         ck(cudaGetDevice(&dev_), "cudaGetDevice");
         aux_ = CtxPool::acquire(1, dev_);
         Ctx &a = aux_[0];
-        a.split = c_.split;
-        a.oz_err = c_.oz_err;
-        a.wait_limit = c_.wait_limit;
-        a.arena = c_.arena;
+        a.split = c_->split;
+        a.oz_err = c_->oz_err;
+        a.wait_limit = c_->wait_limit;
+        a.arena = c_->arena;
         try {
             ck(cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming), "cudaEventCreate");
             ck(cudaEventCreateWithFlags(&done_, cudaEventDisableTiming), "cudaEventCreate");
-            ck(cudaEventRecord(ready_, c_.st), "cudaEventRecord");
+            ck(cudaEventRecord(ready_, c_->st), "cudaEventRecord");
             ck(cudaStreamWaitEvent(a.st, ready_, 0), "cudaStreamWaitEvent");
         } catch (...) {  // no thread yet: hand the helper context back before failing
             finish();
@@ -530,7 +531,8 @@ class PencilFork {
     PencilFork(const PencilFork &) = delete;
     PencilFork &operator=(const PencilFork &) = delete;
     // true when the metric kept every eigenvalue and the pencil is reduced
-    bool join() {
+    bool join(Ctx &to) {
+        c_ = &to;
         finish();
         if (err_) std::rethrow_exception(err_);
         return ok_;
@@ -544,11 +546,11 @@ class PencilFork {
         Ctx &a = aux_[0];
         if (done_) {
             cudaEventRecord(done_, a.st);
-            cudaStreamWaitEvent(c_.st, done_, 0);
+            cudaStreamWaitEvent(c_->st, done_, 0);
         } else {
             cudaStreamSynchronize(a.st);
         }
-        for (T *t : {&pt_.W, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm, &pt_.d, &pt_.e}) t->st = c_.st;
+        for (T *t : {&pt_.W, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm, &pt_.d, &pt_.e}) t->st = c_->st;
         a.split = false;
         a.oz_err = nullptr;
         a.wait_limit = 0;
@@ -558,7 +560,7 @@ class PencilFork {
         if (done_) cudaEventDestroy(done_);
         ready_ = done_ = nullptr;
     }
-    Ctx &c_;
+    Ctx *c_;
     PencilTridiag &pt_;
     int dev_ = 0;
     std::vector<Ctx> aux_;
@@ -566,6 +568,32 @@ class PencilFork {
     std::thread th_;
     std::exception_ptr err_;
     bool ok_ = false;
+};
+
+// The order-n^3 pencil of a (+-1') class of one state.  It depends on the RDMs and
+// Koopmans matrices alone, so the reduction of a single state's -- the longest chain of a
+// call -- is started before the orbitals and integrals are prepared (early / within the
+// class: CAS(6) 11.0 / 14.6 ms, CAS(12) split 62 / 74, CAS(14) 190 / 204).  With more states
+// their pencils would hold up the preparation instead (CAS(6), three states: 34.5 / 32 ms).
+struct Pencil1p {
+    T S, K;
+    PencilTridiag PT;
+    std::unique_ptr<PencilFork> fork;
+    void start(Ctx &c, const StateData &D, int n, bool minus, double thr) {
+        const int n3 = n * n * n;
+        T E2 = alloc(c, {n, n, n, n}, false), E3 = alloc(c, {n, n, n, n, n, n}, false);
+        build_ee2L(c, D.g2.p, D.g1.p, n, E2.p);
+        build_eee2L(c, D.g3.p, D.g2.p, D.g1.p, n, E3.p);
+        if (!minus) {
+            T E3t = alloc(c, {n, n, n, n, n, n}, false);
+            build_eee2tL(c, E3.p, E2.p, n, E3t.p);
+            E3 = std::move(E3t);
+        }
+        // W3 = eee2(t)(cp,ap,bp,b,a,c) transposed: [(a,b,c),(ap,bp,cp)]
+        S = view2(permuted(c, E3, {4, 3, 5, 1, 2, 0}), n3, n3);
+        K = view2(permuted(c, minus ? D.aIP : D.aEA, {3, 4, 5, 0, 1, 2}), n3, n3);
+        fork.reset(new PencilFork(c, S, K, n3, thr, PT));
+    }
 };
 
 class Runner {
@@ -584,6 +612,7 @@ class Runner {
     std::vector<double> eps;
     T Rcc, Rca, Rcv, Raa, Rav, hcv, hca, hav;
     T Jcc;  // [Q] sum_j Rcc[x,j,j]
+    Pencil1p *pencil[2] = {nullptr, nullptr};  // of (+1'), (-1'), perhaps under way
 
     Runner(Ctx &cc, int nc_, int na_, int nv_, int M_, long long Q_, double thr_, const unsigned char *fro,
            std::vector<StateData> &sd_, std::vector<PairData> &pd_, Accum &a)
@@ -599,6 +628,7 @@ class Runner {
         Rcc = T::view(b.Rcc); Rca = T::view(b.Rca); Rcv = T::view(b.Rcv); Raa = T::view(b.Raa);
         Rav = T::view(b.Rav); hcv = T::view(b.hcv); hca = T::view(b.hca); hav = T::view(b.hav);
         Jcc = T::view(b.Jcc);
+        for (int k = 0; k < 2; ++k) pencil[k] = b.pencil[k];
     }
 
     bool frozen(int orb) const { return fro_h && fro_h[orb]; }
@@ -1525,20 +1555,25 @@ class Runner {
         zero_rows(Vd, fm);
         zero_rows(H, fm);
         // accessor tensors of this state
-        T E2 = alloc(c, {n, n, n, n}, false), E3 = alloc(c, {n, n, n, n, n, n}, false);
+        T E2 = alloc(c, {n, n, n, n}, false), W2 = alloc(c, {n, n, n, n}, false), W3;
         build_ee2L(c, D.g2.p, D.g1.p, n, E2.p);
-        build_eee2L(c, D.g3.p, D.g2.p, D.g1.p, n, E3.p);
-        T W2 = alloc(c, {n, n, n, n}, false), W3 = alloc(c, {n, n, n, n, n, n}, false);
+        if (!pc) {
+            T E3 = alloc(c, {n, n, n, n, n, n}, false);
+            build_eee2L(c, D.g3.p, D.g2.p, D.g1.p, n, E3.p);
+            if (!minus) {
+                T E3t = alloc(c, {n, n, n, n, n, n}, false);
+                build_eee2tL(c, E3.p, E2.p, n, E3t.p);
+                E3 = std::move(E3t);
+            }
+            W3 = permuted(c, E3, {1, 2, 0, 4, 3, 5});  // eee2(t)(cp,ap,bp,b,a,c)
+        }
         T rho = copy_of(c, D.g1.p, {n, n});  // [ap, a]
         if (minus) {
-            permute(c, E2.p, {n, n, n, n}, {1, 2, 0, 3}, W2.p);           // ee2(cp,ap,bp,a)
-            permute(c, E3.p, {n, n, n, n, n, n}, {1, 2, 0, 4, 3, 5}, W3.p);  // eee2(cp,ap,bp,b,a,c)
+            permute(c, E2.p, {n, n, n, n}, {1, 2, 0, 3}, W2.p);  // ee2(cp,ap,bp,a)
         } else {
-            T E2tr = alloc(c, {n, n, n, n}, false), E3t = alloc(c, {n, n, n, n, n, n}, false);
+            T E2tr = alloc(c, {n, n, n, n}, false);
             build_ee2trL(c, E2.p, D.g1.p, n, E2tr.p);
-            build_eee2tL(c, E3.p, E2.p, n, E3t.p);
             permute(c, E2tr.p, {n, n, n, n}, {1, 2, 0, 3}, W2.p);
-            permute(c, E3t.p, {n, n, n, n, n, n}, {1, 2, 0, 4, 3, 5}, W3.p);
             std::vector<double> I2(n * n, 0.0);
             for (int a = 0; a < n; ++a) I2[a * n + a] = 2.0;
             T Id = upload(c, I2);
@@ -1552,17 +1587,13 @@ class Runner {
         // dp'W3 dp = diag(Vd S Vd^T) with the metric S = W3^T (the diagonal of
         // a quadratic form does not see the transpose); another state j:
         // Vd W3o_j is Vd S_j, S_j the transition metric of its numerators.
-        T S, K, Yown;
+        T Yown;
         std::map<int, T> yoth;
-        PencilTridiag PT;
-        std::unique_ptr<PencilFork> fork;
+        Pencil1p *pen = pencil[minus];
         if (pc) {
-            S = view2(permuted(c, W3, {3, 4, 5, 0, 1, 2}), n3, n3);  // [(a,b,c),(ap,bp,cp)]
-            K = view2(permuted(c, A, {3, 4, 5, 0, 1, 2}), n3, n3);
-            // the pencil's reduction overlaps the SC work below
-            fork.reset(new PencilFork(c, S, K, n3, thr, PT));
+            if (!pen->fork) pen->start(c, D, n, minus, thr);  // overlaps the SC work below
             Yown = alloc(c, {L, (long long)n3}, false);
-            gemm(c, false, false, L, n3, n3, 1.0, Vd.p, n3, S.p, n3, 0.0, Yown.p, n3);
+            gemm(c, false, false, L, n3, n3, 1.0, Vd.p, n3, pen->S.p, n3, 0.0, Yown.p, n3);
         }
         // dumm = h'rho h + 2 dp'W2 h + dp'W3 dp ; dumk = h'Dm h + dp'Bc h + dp'A dp
         // (y3pre: Vd W3 or a product with the same diagonal form; y3keep: keep Vd W3)
@@ -1686,7 +1717,13 @@ class Runner {
                     else acc.rhoid[l + (size_t)nc * (d + (size_t)na * s)] += v;
                 }
         };
-        if (fork && fork->join()) {
+        PencilTridiag &PT = pen->PT;
+        const bool reduced = pen->fork->join(c);
+        struct Release {  // the form's buffers, on this stream
+            PencilTridiag &p;
+            ~Release() { p = PencilTridiag{}; }
+        } release{PT};
+        if (reduced) {
             // Every metric eigenvalue but exact zeros is kept: the PC sums over
             // the eigenpairs of K v = w S v are resolvents of the pencil,
             //   sum_mu r_mu^2 / (w_mu + s) = z^T (K + s S)^-1 z,
@@ -1742,7 +1779,7 @@ class Runner {
             pc_accum(e2, psi2, resolvent_sums(PT, Yt, pb, nd, (long long)M * L, rho.p));
             if (nd) store_rho(download(c, rho.p, L * nd));
         } else {
-            PcResult P = pc_transform(c, S, K, n3, thr);
+            PcResult P = pc_transform(c, pen->S, pen->K, n3, thr);
             acc.nnew[(minus ? 7 : 6) + 10 * s] = P.nnew;
             // R[l, mu] = sum_x Z[l, x] C[x, mu]: the order-n3 products S C and
             // W2t C of the reference are reassociated onto the L rows.
@@ -1862,6 +1899,7 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
     Arena arena(st);
     Ctx c{st, guard.lent[0].blas, guard.lent[0].sol};
     c.arena = &arena;
+    c.wait_limit = nvpt_context_wait_limit(ctx);
     // split precision: the stage's large products run as Ozaki digit products
     c.split = nvpt_get_precision(ctx) == NVPT_PRECISION_SPLIT;
     T ozerr;
@@ -1917,6 +1955,7 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
             }
         }
     }
+    std::vector<std::array<Pencil1p, 2>> pencils(M);
     std::vector<PairData> pd(P);
     if (P > 0) {
         T T1 = S(in->trdm1, P * n2), T2 = S(in->trdm2, P * n4), T3 = S(in->trdm3, P * n6);
@@ -1972,7 +2011,11 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
             pc_.wait_limit = nvpt_context_wait_limit(ctx);
             pc_.arena = &arena;
         }
-    ck(cudaEventRecord(ps.prep, c.st), "event");  // B and h ready
+    if (pc && M == 1) {  // the longest chains first: see Pencil1p
+        if ((m & 64u) && nv) pencils[0][1].start(c, sd[0], n, true, in->thr_lindep);
+        if ((m & 32u) && nc) pencils[0][0].start(c, sd[0], n, false, in->thr_lindep);
+    }
+    ck(cudaEventRecord(ps.prep, c.st), "event");  // B and h ready, and the pencils' metrics
     std::vector<std::unique_ptr<Runner>> SR(M);
     {
         std::vector<std::exception_ptr> fail(M);
@@ -1981,6 +2024,7 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
                 ck(cudaSetDevice(dev), "cudaSetDevice");
                 ck(cudaStreamWaitEvent(ps.c[st_].st, ps.prep, 0), "wait");
                 SR[st_].reset(new Runner(R, ps.c[st_], acc));
+                for (int k = 0; k < 2; ++k) SR[st_]->pencil[k] = &pencils[st_][k];
                 ProfSpan span;
                 span.begin("s2_prepare", ps.c[st_].st, 0);
                 SR[st_]->prepare_state(st_);
@@ -2032,6 +2076,7 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
         for (size_t idx = 0; idx < nt; ++idx) acc.merge(local[idx]);
     }
     SR.clear();
+    pencils.clear();
     ck(cudaStreamSynchronize(c.st), "qdnevpt sync");
     if (c.split) {
         int h = 0;

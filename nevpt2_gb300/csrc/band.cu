@@ -41,7 +41,7 @@ struct QrArgs {
     int chunk;            // rows per CTA (CTA 0 holds the pivot rows)
     double *V, *T, *G;    // V [m][NB] row-major, T [NB][NB] row-major; G [NB][NB] is zeroed for k_band_g
     unsigned long long *msg;  // [NB][CTAs + 1][NB], all kNoMsg on entry
-    int *err;
+    int *err;             // raised once a wait gave up
     unsigned spin;        // polls before a wait gives up
 };
 
@@ -230,9 +230,11 @@ __global__ void __launch_bounds__(TB) k_band_g(int m, int splits, const double *
     }
 }
 
-// W = (Z - 1/2 V N) T with N = T^T G, 16 rows per CTA.
+// W = (Z - 1/2 V N) T with N = T^T G, 16 rows per CTA; the messages are reset for the next panel.
 __global__ void __launch_bounds__(TB) k_band_w(int m, const double *__restrict__ V, const double *__restrict__ Z,
-                                               const double *__restrict__ Tm, const double *__restrict__ G, double *W) {
+                                               const double *__restrict__ Tm, const double *__restrict__ G, double *W,
+                                               unsigned long long *msg, int words) {
+    for (int i = blockIdx.x * TB + threadIdx.x; i < words; i += gridDim.x * TB) msg[i] = kNoMsg;
     __shared__ double ts[NB][NB], gs[NB][NB], ns[NB][NB], vs[kGRows][NB], us[kGRows][NB];
     const int tid = threadIdx.x, i0 = blockIdx.x * kGRows;
     for (int e = tid; e < NB * NB; e += TB) {
@@ -599,7 +601,7 @@ int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *A
         const int chunk = std::max(NB, (m + G0 - 1) / G0), ctas = (m + chunk - 1) / chunk;
         const size_t smem = sizeof(double) * (size_t)chunk * LP;
         if ((long long)smem > lim) throw Error(1, "band: order too large for the panel's shared memory");
-        ck(cudaMemsetAsync(msg.p, 0xff, sizeof(double) * NB * (ctas + 1) * NB, c.st), "memset");
+        if (!p) ck(cudaMemsetAsync(msg.p, 0xff, sizeof(double) * NB * (ctas + 1) * NB, c.st), "memset");
         QrArgs q{A, n, j0, m, chunk, v, t, G.p, (unsigned long long *)msg.p, err, c.wait_limit ? c.wait_limit : kBarSpin};
         void *args[] = {&q};
         ck(cudaLaunchCooperativeKernel((const void *)k_band_qr, dim3(ctas), dim3(TB), args, smem, c.st),
@@ -608,7 +610,8 @@ int band_reduce(Ctx &c, double *A, long long n, double *V, double *Tm, double *A
         const int per = ((m + splits - 1) / splits + 31) / 32 * 32, ns = (m + per - 1) / per;
         k_band_z<<<dim3(tiles, ns), TB, 0, c.st>>>(A, n, r0, m, per, v, Zp.p);
         k_band_g<<<(m + kGRows - 1) / kGRows, TB, 0, c.st>>>(m, ns, v, Zp.p, G.p);
-        k_band_w<<<(m + kGRows - 1) / kGRows, TB, 0, c.st>>>(m, v, Zp.p, t, G.p, W.p);
+        k_band_w<<<(m + kGRows - 1) / kGRows, TB, 0, c.st>>>(m, v, Zp.p, t, G.p, W.p,
+                                                           (unsigned long long *)msg.p, NB * (ctas + 1) * NB);
         k_band_update<<<tiles * (tiles + 1) / 2, TB, 0, c.st>>>(A, n, r0, m, v, W.p);
         g_launches.fetch_add(5, std::memory_order_relaxed);
         v += (long long)m * NB;

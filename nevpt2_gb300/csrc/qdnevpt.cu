@@ -350,7 +350,7 @@ __global__ void k_zero_rows(double *A, long long L, long long m, const unsigned 
 // q[L] = sum V1[L,u] X[u,v] V2[L,v]
 T bilin(Ctx &c, const T &V1, const double *X, long long m, const T &V2, double alpha = 1.0) {
     long long L = V1.sh[0];
-    T q = alloc(c, {L}, true);
+    T q = alloc(c, {L}, false);
     if (L == 0) return q;
     T Y = alloc(c, {L, m}, false);
     gemm(c, false, false, L, m, m, 1.0, V1.p, m, X, m, 0.0, Y.p, m);

@@ -351,13 +351,20 @@ void gram(Ctx &c, const double *X, long long Q, long long m, double *out) {
 }
 
 int raise_dynamic_smem(const void *kernel) {
-    cudaFuncAttributes fa{};
-    ck(cudaFuncGetAttributes(&fa, kernel), "cudaFuncGetAttributes");
     int dev = 0, optin = 0;
     ck(cudaGetDevice(&dev), "cudaGetDevice");
+    // once per device and kernel: three driver calls otherwise, in front of most launches
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, int> known;
+    std::lock_guard<std::mutex> g(mu);
+    const auto it = known.find({dev, kernel});
+    if (it != known.end()) return it->second;
+    cudaFuncAttributes fa{};
+    ck(cudaFuncGetAttributes(&fa, kernel), "cudaFuncGetAttributes");
     ck(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "attr");
     const int lim = optin - (int)fa.sharedSizeBytes;
     ck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim), "smem attr");
+    known[{dev, kernel}] = lim;
     return lim;
 }
 

@@ -160,13 +160,23 @@ __device__ void factor_block(Diag &s, double *W, long long ld, int live, int *ba
     }
 }
 
-// L (lower) <- S, W <- 0, padding as in the identity.
-__global__ void k_spd_load(const double *__restrict__ S, int n, long long ld, double *L, double *W) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// L (lower) <- S, W <- 0, padding as in the identity; block 0: W11 of the first diagonal
+// block, while the others copy.
+__global__ void __launch_bounds__(TP) k_spd_load(const double *__restrict__ S, int n, long long ld, double *L, double *W,
+                                                 int *bad) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    auto at = [&](int i, int j) { return j < n && i < n ? S[(long long)j * n + i] : i == j ? 1.0 : 0.0; };
+    if (blockIdx.x == 0) {
+        Diag &s = *reinterpret_cast<Diag *>(smem);
+        for (int e = threadIdx.x; e < B * B; e += TP) s.m[e % B][e / B] = e / B <= e % B ? at(e % B, e / B) : 0.0;
+        factor_block(s, W, ld, min(B, n), bad);
+        return;
+    }
+    const long long t = (long long)(blockIdx.x - 1) * TP + threadIdx.x;
     if (t >= ld * ld) return;
     const int j = (int)(t / ld), i = (int)(t % ld);  // i along the rows of S: its upper triangle is read in order
-    W[t] = 0.0;
-    if (j <= i) L[i * ld + j] = j < n && i < n ? S[(long long)j * n + i] : i == j ? 1.0 : 0.0;
+    if (i >= B || j >= B) W[t] = 0.0;
+    if (j <= i) L[i * ld + j] = at(i, j);
 }
 
 // M (lower, half the diagonal, zeros above) of K = M + M^T.
@@ -176,13 +186,6 @@ __global__ void k_spd_half(const double *__restrict__ K, int n, long long ld, do
     const int j = (int)(t / ld), i = (int)(t % ld);
     const double v = j < n && i < n && j <= i ? K[(long long)j * n + i] : 0.0;
     M[i * ld + j] = i == j ? 0.5 * v : v;
-}
-
-__global__ void __launch_bounds__(TP) k_spd_first(double *L, long long ld, double *W, int n, int *bad) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    Diag &s = *reinterpret_cast<Diag *>(smem);
-    for (int e = threadIdx.x; e < B * B; e += TP) s.m[e / B][e % B] = e % B <= e / B ? L[(e / B) * ld + e % B] : 0.0;
-    factor_block(s, W, ld, min(B, n), bad);
 }
 
 // 16 rows of L21 = A21 W11^T, or 16 columns of W[k, :] = W11 R[k, :], a CTA (in place).
@@ -339,17 +342,16 @@ void spd_inverse_factor_async(Ctx &c, const double *S, long long n, double *W, d
     const int nb = (int)(ld / B);
     T L = alloc(c, {ld, ld}, false);
     int *bad = (int *)(stat + 1);
-    raise_dynamic_smem((const void *)k_spd_first);
+    raise_dynamic_smem((const void *)k_spd_load);
     raise_dynamic_smem((const void *)k_spd_step);
-    k_spd_load<<<blocks(ld * ld), TP, 0, c.st>>>(S, (int)n, ld, L.p, W);
-    k_spd_first<<<1, TP, sizeof(Diag), c.st>>>(L.p, ld, W, (int)n, bad);
+    k_spd_load<<<1 + blocks(ld * ld), TP, sizeof(Diag), c.st>>>(S, (int)n, ld, L.p, W, bad);
     for (int k = 0; k < nb; ++k) {
         const int t = nb - 1 - k;
         if (t + k) k_spd_panel<<<4 * (t + k), TP, 0, c.st>>>(L.p, W, ld, k, nb, bad);
         if (t) k_spd_step<<<2 * (t * (t + 1) / 2 + t * (k + 1)) - 1, TP, sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, (int)n, bad);
     }
     if (trace) k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, (int)n, ld, stat);
-    g_launches.fetch_add(2 * nb + (trace ? 2 : 1), std::memory_order_relaxed);
+    g_launches.fetch_add(2 * nb - 1 + (trace ? 1 : 0), std::memory_order_relaxed);
     ck(cudaGetLastError(), "inverse factor");
 }
 

@@ -22,9 +22,9 @@ constexpr unsigned long long kNoMsg = ~0ull;
 struct TriArgs {
     const double *A;  // n x n, both triangles
     int n;
-    double *d, *e, *tau, *V;   // V: panels as in band_apply with first = 1, zero on entry
+    double *d, *e, *tau, *V;   // V: panels as in wy_apply with first = 1
     unsigned long long *msg;   // [n][2][n], all kNoMsg on entry
-    int *err;
+    int *err;                  // 0 once a wait gave up
     unsigned spin;
 };
 
@@ -49,6 +49,9 @@ __global__ void __launch_bounds__(TB, 1) k_tri_reduce(TriArgs a) {
         x[k] = a.A[k];
         vo[k] = w[k] = 0.0;
     }
+    for (int i = b; i < n; i += G)  // own rows of V: zero where no reflector reaches
+        for (int p = warp; p * NB + 1 <= i && p * NB + 2 < n; p += TB / 32)
+            a.V[panel_at(n, p) + (long long)(i - p * NB - 1) * NB + lane] = 0.0;
     __syncthreads();
     // sum over the block, in warp 0
     auto total = [&](double s) {
@@ -122,8 +125,8 @@ __global__ void __launch_bounds__(TB, 1) k_tri_reduce(TriArgs a) {
 #pragma unroll
             for (int q = 0; q < 2; ++q) all = all && m0[q] != kNoMsg && m1[q] != kNoMsg;
             if (all) break;
-            if (++spins > a.spin || (spins % 64 == 0 && *(volatile int *)a.err)) {
-                atomicExch(a.err, 1);
+            if (++spins > a.spin || (spins % 64 == 0 && !*(volatile int *)a.err)) {
+                atomicExch(a.err, 0);
                 ok = 0;
                 break;
             }
@@ -277,10 +280,10 @@ int tri_reduce(Ctx &c, const double *A, long long n, double *d, double *e, doubl
     const size_t smem = sizeof(double) * (size_t)(5 + rows) * n;
     if ((long long)smem > raise_dynamic_smem((const void *)k_tri_reduce))
         throw Error(NVPT_EINVAL, "tridiagonal form: order above the shared-memory limit");
-    T tau = alloc(c, {n}, true), msg = alloc(c, {n, 2, n}, false), ctl = alloc(c, {1}, true);
-    ck(cudaMemsetAsync(msg.p, 0xff, sizeof(double) * 2 * n * n, c.st), "memset");
-    ck(cudaMemsetAsync(V, 0, sizeof(double) * wy_rows(n, 1) * NB, c.st), "memset");
-    TriArgs a{A, ni, d, e, tau.p, V, (unsigned long long *)msg.p, (int *)ctl.p, c.wait_limit ? c.wait_limit : kBarSpin};
+    T tau = alloc(c, {n}, false), msg = alloc(c, {2 * n * n + 1}, false);  // the messages, the error word
+    ck(cudaMemsetAsync(msg.p, 0xff, sizeof(double) * (2 * n * n + 1), c.st), "memset");
+    int *err = (int *)(msg.p + 2 * n * n);
+    TriArgs a{A, ni, d, e, tau.p, V, (unsigned long long *)msg.p, err, c.wait_limit ? c.wait_limit : kBarSpin};
     void *args[] = {&a};
     ck(cudaLaunchCooperativeKernel((const void *)k_tri_reduce, dim3(G), dim3(TB), args, smem, c.st),
        "cooperative launch");
@@ -288,9 +291,9 @@ int tri_reduce(Ctx &c, const double *A, long long n, double *d, double *e, doubl
     g_launches.fetch_add(2, std::memory_order_relaxed);
     ck(cudaGetLastError(), "tridiagonal reduction");
     int h = 0;
-    ck(cudaMemcpyAsync(&h, ctl.p, sizeof(int), cudaMemcpyDeviceToHost, c.st), "wait state");
+    ck(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, c.st), "wait state");
     ck(cudaStreamSynchronize(c.st), "tridiagonal sync");
-    return h ? 4 : 0;
+    return h ? 0 : 4;
 }
 
 void tri_resolvent(Ctx &c, const double *d, const double *e, long long n, const double *Y, long long ncol, long long L,

@@ -656,13 +656,13 @@ def run_ours(args):
     if rank != 0:
         dist.destroy_process_group() if ws > 1 else None
         return
-    # roofline (FP64 path): bamat as FP64 contractions (slab unpack + cuBLAS
-    # DGEMMs); algorithmic flops of the reference loop 12n^9 + 16n^8 + 12n^7
-    # per state, against the FP64 DGEMM rate measured in this run.
+    # roofline (FP64 path): bamat as one n^9 contraction over pairs of orbitals,
+    # four n^8 ones and the n^7 sums of its output; the reference loop's
+    # 12n^9 + 16n^8 + 12n^7 flops per state are given beside it.  Against the
+    # FP64 DGEMM rate measured in this run.
     alg_flops = M * (12 * n**9 + 16 * n**8 + 12 * n**7)
-    # what the dense reformulation executes: four n^3-deep products per slab
-    # (8 n^9) and the n^8 lower-order GEMMs (4 n^8)
-    exec_flops = M * (8 * n**9 + 4 * n**8)
+    pairs = n * (n + 1) // 2
+    exec_flops = M * (2 * pairs * (pairs + 1) * n**5 + 6 * pairs * n**6 + 2 * pairs**2 * n**4 + 12 * n**7)
     peak64 = fp64_peak(dev)
     achieved = alg_flops / (bamat_ms * 1e-3) / 1e12
     achieved_exec = exec_flops / (bamat_ms * 1e-3) / 1e12
@@ -700,16 +700,16 @@ def run_ours(args):
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded CI vector, exact RDMs, random DF integrals)",
             "config": workload_desc(p), "gpu_launches": int(launches),
             "e2e": {"value": e2e, "unit": "s/state", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
-            "roofline": {"kernel": "bamat (k_bamat_slabs_t + k_dgemm_skinny + k_rest_*)", "bound": "fp64 pipe",
-                         "achieved": achieved, "peak": peak64, "unit": "TFLOP/s", "frac": achieved / peak64,
-                         "achieved_executed": achieved_exec, "frac_executed": achieved_exec / peak64,
-                         "note": "achieved counts the reference loop's 12n^9+16n^8+12n^7 flops per state; the dense "
-                                 "reformulation executes 8n^9+4n^8 (achieved_executed, frac_executed)",
+            "roofline": {"kernel": "bamat (k_sym_unpack + k_sym_n8 + k_sym_f + k_sym_small + k_sym_out)", "bound": "fp64 pipe",
+                         "achieved": achieved_exec, "peak": peak64, "unit": "TFLOP/s", "frac": achieved_exec / peak64,
+                         "reference_loop_rate": achieved,
+                         "note": "achieved counts the flops executed: 2 p (p + 1) n^5 + 6 p n^6 + 2 p^2 n^4 + 12 n^7 "
+                                 "per state, p = n (n + 1) / 2; reference_loop_rate the reference loop's 12n^9 + "
+                                 "16n^8 + 12n^7 in the same time",
                          "traffic": bamat_traffic(n, M),
-                         "traffic_source": "DRAM bytes per step of the bamat kernels, scaled from ncu captures at "
-                                           "CAS(10,10) (k_bamat_slabs_t 73 MB read + 459 MB written, k_dgemm_skinny "
-                                           "517 + 6 MB per batch of 16 slabs) by (n/10)^6 per batch and M n^2/16 "
-                                           "batches per step",
+                         "traffic_source": "DRAM bytes per step of k_sym_n8, k_sym_f and k_sym_out, scaled from the "
+                                           "ncu capture at CAS(12) (profiles/bamat_sym_cas12.md) by the packed 4-RDM "
+                                           "(n/12)^8",
                          "precision": "fp64",
                          "peak_source": "FP64 DGEMM rate measured live in this run (cuBLAS 4096^3)",
                          "kernel_ms": bamat_ms, "alg_flops": alg_flops},
@@ -921,12 +921,10 @@ def run_batch(args):
 
 
 def bamat_traffic(n: int, M: int) -> float:
-    """DRAM bytes of the FP64 bamat kernels per step, from the ncu captures
-    of one batch of 16 slabs at n = 10 (slab production: 73 MB read, 459 MB
-    written; slab products: 517 MB read, 6 MB written); both scale with the
-    slab size n^6, and a step runs M n^2 / 16 batches."""
-    per_batch_n10 = (73 + 459 + 517 + 6) * 1e6
-    return per_batch_n10 * (n / 10) ** 6 * M * n * n / 16
+    """DRAM bytes of the FP64 bamat kernels per step, from the ncu capture of
+    one state at n = 12 (read + written: k_sym_n8 23, k_sym_f 591,
+    k_sym_out 140 MB), scaled with the unpacked 4-RDM."""
+    return 754e6 * (n / 12) ** 8 * M
 
 
 def live_ro4_entries(n: int) -> int:

@@ -284,9 +284,9 @@ int nvpt_get_precision(nvpt_context *ctx);
  * "s2_class_-1", "s2_class_+2", "s2_class_-2", "s2_class_0p",
  * "s2_class_+1p", "s2_class_-1p" (one class of one state, on its stream);
  * "pencil_potrf", "pencil_reduce", "pencil_sytrd", "pencil_rhs",
- * "pencil_solve" (the steps of one order-n^3 PC pencil: metric Cholesky,
- * reduction to standard form, tridiagonalisation, right-hand sides and the
- * per-label tridiagonal solves). */
+ * "pencil_solve" (the steps of one PC pencil: inverse Cholesky factor of the
+ * metric, standard form, band or tridiagonal form, right-hand sides and the
+ * labels' eliminations). */
 int nvpt_set_profiling(nvpt_context *ctx, int on);
 int nvpt_profile_read(nvpt_context *ctx, const char *tag, double *ms, int64_t *launches, int64_t *bytes);
 
@@ -311,10 +311,9 @@ int nvpt_set_pc_route(nvpt_context *ctx, int mode);
  * every candidate of its parameter with CUDA events on the call's stream
  * (synchronising that stream once) and keeps the fastest; later launches of
  * that shape use the kept choice whether tuning is on or not (on = 0 stops
- * tuning new shapes, on = 2 forgets every choice).  Tuned today: the tile
- * height of the FP64 bamat slab products (64 or 128 rows) and the raster
- * group of the general split-precision product (4 .. 32 row tiles sharing a
- * column tile).  Candidates only reorder independent output tiles, so the
+ * tuning new shapes, on = 2 forgets every choice).  Tuned today: the
+ * raster group of the general split-precision product (4 .. 32 row tiles
+ * sharing a column tile).  Candidates only reorder independent output tiles, so the
  * results do not depend on the choice.  Choices are per device and shared by
  * the contexts of a process.  nvpt_autotune_report writes them as JSON
  * (choice and the timed milliseconds per candidate) into buf (len bytes,

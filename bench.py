@@ -657,12 +657,12 @@ def run_ours(args):
         dist.destroy_process_group() if ws > 1 else None
         return
     # roofline (FP64 path): bamat as one n^9 contraction over pairs of orbitals,
-    # four n^8 ones and the n^7 sums of its output; the reference loop's
+    # four n^8 ones and one n^7 one; the reference loop's
     # 12n^9 + 16n^8 + 12n^7 flops per state are given beside it.  Against the
     # FP64 DGEMM rate measured in this run.
     alg_flops = M * (12 * n**9 + 16 * n**8 + 12 * n**7)
     pairs = n * (n + 1) // 2
-    exec_flops = M * (2 * pairs * (pairs + 1) * n**5 + 6 * pairs * n**6 + 2 * pairs**2 * n**4 + 12 * n**7)
+    exec_flops = M * (2 * pairs * (pairs + 1) * n**5 + 6 * pairs * n**6 + 2 * pairs**2 * n**4 + 2 * pairs * n**5)
     peak64 = fp64_peak(dev)
     achieved = alg_flops / (bamat_ms * 1e-3) / 1e12
     achieved_exec = exec_flops / (bamat_ms * 1e-3) / 1e12
@@ -700,10 +700,10 @@ def run_ours(args):
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded CI vector, exact RDMs, random DF integrals)",
             "config": workload_desc(p), "gpu_launches": int(launches),
             "e2e": {"value": e2e, "unit": "s/state", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
-            "roofline": {"kernel": "bamat (k_sym_unpack + k_sym_n8 + k_sym_f + k_sym_small + k_sym_out)", "bound": "fp64 pipe",
+            "roofline": {"kernel": "bamat (k_sym_unpack + k_sym_n8 + k_sym_f + k_sym_small + k_sym_t3 + k_sym_out)", "bound": "fp64 pipe",
                          "achieved": achieved_exec, "peak": peak64, "unit": "TFLOP/s", "frac": achieved_exec / peak64,
                          "reference_loop_rate": achieved,
-                         "note": "achieved counts the flops executed: 2 p (p + 1) n^5 + 6 p n^6 + 2 p^2 n^4 + 12 n^7 "
+                         "note": "achieved counts the flops executed: 2 p (p + 1) n^5 + 6 p n^6 + 2 p^2 n^4 + 2 p n^5 "
                                  "per state, p = n (n + 1) / 2; reference_loop_rate the reference loop's 12n^9 + "
                                  "16n^8 + 12n^7 in the same time",
                          "traffic": bamat_traffic(n, M),
@@ -922,9 +922,9 @@ def run_batch(args):
 
 def bamat_traffic(n: int, M: int) -> float:
     """DRAM bytes of the FP64 bamat kernels per step, from the ncu capture of
-    one state at n = 12 (read + written: k_sym_n8 23, k_sym_f 591,
-    k_sym_out 140 MB), scaled with the unpacked 4-RDM."""
-    return 754e6 * (n / 12) ** 8 * M
+    one state at n = 12 (read + written: k_sym_n8 23, k_sym_f 588,
+    k_sym_out 556 MB), scaled with the unpacked 4-RDM."""
+    return 1167e6 * (n / 12) ** 8 * M
 
 
 def live_ro4_entries(n: int) -> int:

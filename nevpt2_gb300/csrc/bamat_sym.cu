@@ -81,7 +81,6 @@ __global__ void __launch_bounds__(256) k_sym_ops(const double *atwo, const doubl
     if (i >= j) S.Bf[((ll)k * np + pidx(i, j)) * n + l] = v;  // [(e, df), a] = (df|ea)
     S.I4[((ll)j * n + l) * n2 + (ll)i * n + k] = v;           // [(f, e), (x, y)] = (xf|ye)
     if (k >= l) S.IJ[((ll)j * n + i) * np + pidx(k, l)] = v;  // [(f, d), (x y)] = (df|xy)
-    S.Lb[t] = 2.0 * AT(l, k, j, i) - AT(i, k, j, l);          // [i][j][k][l] = 2 (lk|ji) - (ik|jl)
     if (t < n2) {                                             // (x, y) = (k, l)
         double kk = 0.0;
         for (int z = 0; z < n; ++z) kk += AT(k, z, z, l);
@@ -413,7 +412,7 @@ struct SymView {
     Rdm r;
     int s, n;
     ll n2, rows;  // rows of one n^8 block
-    const double *F, *N8, *G1, *G3, *Q1, *JW, *J2, *Z, *atwo, *Lb, *g;
+    const double *F, *N8, *G1, *G3, *Q1, *JW, *J2, *Z, *atwo, *g, *T3;
 
     __device__ __forceinline__ double d1(int a, int b) const { return r.d1[s + (ll)r.M * (a + n * b)]; }
     __device__ __forceinline__ double d2(int a, int b, int c, int d) const {
@@ -446,8 +445,51 @@ struct SymView {
         const int np = n * (n + 1) / 2;
         return p >= p2 ? A[row3(p, p2, q, q2) * np + pmx(x, y)] : A[row3(p2, p, q2, q) * np + pmx(x, y)];
     }
+    __device__ __forceinline__ double t3(int x1, int x2, int x3, int p, int q, int r) const {
+        return T3[(((ll)(x1 * n + x2) * n + x3) * (n * (n + 1) / 2) + pmx(q, r)) * n + p];
+    }
     __device__ __forceinline__ ll i4(int a, int b, int c, int d) const { return ((ll)(a * n + b) * n + c) * n + d; }
 };
+
+// T3[x1,x2,x3; (q r), p] = sum_d Gamma2[(x1,d),(x2,x3)] (pd|qr): every n^7 sum of the
+// output is an element of it.  Rows (x1,x2,x3), columns (pair, p), K = n in one slab;
+// 64 x 64 tiles, bound by the FP64 pipe (n^7/2 FMAs; n = 16: 243 us, n = 8: 13).
+__global__ void __launch_bounds__(256) k_sym_t3(Rdm r, int s, const double *__restrict__ atwo, double *T3, const int *flag) {
+    if (*flag) return;
+    __shared__ double As[16][65], Bs[16][64];
+    const int n = r.n, np = n * (n + 1) / 2, n3 = n * n * n, cols = np * n, tid = threadIdx.x;
+    const int r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
+    for (int e = tid; e < 64 * n; e += 256) {
+        const int d = e % n, row = min(r0 + e / n, n3 - 1), x3 = row % n, x2 = (row / n) % n, x1 = row / (n * n);
+        As[d][e / n] = r.d2[s + (ll)r.M * (d + n * (x3 + n * (x1 + n * x2)))];
+    }
+    for (int e = tid; e < 64 * n; e += 256) {
+        const int d = e / 64, col = min(c0 + e % 64, cols - 1), p = col % n;
+        int q, t;
+        unpair(col / n, q, t);
+        Bs[d][e % 64] = AT(p, d, q, t);
+    }
+    __syncthreads();
+    const int tc = (tid & 15) * 4, tr = (tid >> 4) * 4;
+    double acc[4][4] = {};
+    for (int k = 0; k < n; ++k) {
+        double a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            a[i] = As[k][tr + i];
+            b[i] = Bs[k][tc + i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (r0 + tr + i < n3 && c0 + tc + j < cols) T3[(ll)(r0 + tr + i) * cols + c0 + tc + j] = acc[i][j];
+}
 
 // n^6 sums over two indices, kSmallLanes threads per n^4 element (a chain of n^2 steps and
 // an idle chip at small n otherwise; n = 8: 32 -> 10 us, n = 16: 174 -> 156):
@@ -484,88 +526,67 @@ __global__ void __launch_bounds__(64) k_sym_small(SymView v, double *G1, double 
     G1[t] = g1; G3[t] = g3; Q1[t] = q1; JW[t] = j2 + w2; J2[t] = j2; Z[t] = 2.0 * j2 - y2;
 }
 
-// amat/atmat(s, ap,bp,cp,a,b,c): a thread owns (a, c, b, bp, cp), a fastest,
-// and kOutAp values of ap.  With a and c across a warp most gathers of F and the
-// n^8 tensors (whose last indices are a, c or b) use whole sectors.  The sums
-// over one index (Gamma2 with the integrals: the FP64 work, 6 n FMAs per
-// element) keep ap in registers, so that five of their six factors are loaded
-// once for all of them.  n = 16: 5.8 ms (one element per thread, ap across the
-// warp: 24.7 ms).
-// Up to kOutSmall orbitals in blocks of 64 threads, to spread over the SMs: 64 / 256 threads,
-// us: n = 4 22 / 27, n = 6 24 / 32, n = 7 33 / 35, n = 8 73 / 63.
-constexpr int kOutAp = 4, kOutSmall = 7;
-__global__ void __launch_bounds__(256) k_sym_out(SymView v, double *amat, double *atmat, const int *flag) {
+// amat/atmat(s, ap,bp,cp,a,b,c), a thread an element, a fastest, then c, so that most
+// gathers of F and the n^8 tensors (whose last indices are a, c or b) share sectors.
+// Bound by the FP64 pipe (some 35 additions an element, with the Kronecker deltas more in
+// most warps).  Blocks of 64 spread the small spaces over the SMs and cost the large ones
+// nothing.  With the n^7 sums formed here (6 n FMAs an element) 27 / 63 / 5850 us at n =
+// 4 / 8 / 16, now 8 / 33 / 1990 and k_sym_t3.
+constexpr int kOutTb = 64;
+__global__ void __launch_bounds__(kOutTb) k_sym_out(SymView v, double *amat, double *atmat, const int *flag) {
     if (*flag) return;
     const int n = v.n;
     const ll n5 = v.n2 * v.n2 * n;
-    const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+    const ll t = (ll)blockIdx.x * kOutTb + threadIdx.x;
     if (t >= n5) return;
     ll x = t;
     const int a = (int)(x % n); x /= n;
     const int c = (int)(x % n); x /= n;
     const int b = (int)(x % n); x /= n;
     const int bp = (int)(x % n); x /= n;
-    const int cp = (int)x;
-    const int ap0 = blockIdx.y * kOutAp;
-    double sum[kOutAp] = {};
-    for (int d = 0; d < n; ++d) {
-        const double m1 = 2.0 * v.ai(d, a, b, bp) - v.ai(bp, a, b, d), m2 = v.d2(d, c, cp, a), m3 = v.d2(d, c, cp, b);
-        const double m4 = v.d2(d, c, b, cp), m5 = v.d2(d, cp, c, bp), m6 = v.d2(d, cp, bp, c);
-#pragma unroll
-        for (int i = 0; i < kOutAp; ++i) {
-            const int ap = min(ap0 + i, n - 1);
-            double y = fma(m1, v.d2(ap, c, cp, d), sum[i]);                     // Gamma2[(cp,ap),(d,c)] [2 (da|b bp) - (bp a|bd)]
-            y = fma(m2, v.Lb[ap + n * (d + n * (b + n * bp))], y);              // Gamma2[(cp,d),(a,c)] [2 (ap d|b bp) - (bp d|b ap)]
-            y = fma(-m3, v.ai(ap, d, bp, a), y);                                // Gamma2[(cp,d),(b,c)] (ap d|bp a)
-            y = fma(-m4, v.ai(ap, a, bp, d), y);                                // Gamma2[(cp,c),(b,d)] (bp d|ap a)
-            y = fma(-m5, v.ai(ap, b, a, d), y);                                 // Gamma2[(cp,bp),(d,c)] (da|b ap)
-            sum[i] = fma(-m6, v.ai(ap, a, b, d), y);                            // Gamma2[(cp,c),(d,bp)] (ap a|bd)
-        }
-    }
+    const int cp = (int)x, ap = blockIdx.y;
     const double d1 = v.d1(cp, c);
-#pragma unroll
-    for (int i = 0; i < kOutAp; ++i) {
-        const int ap = ap0 + i;
-        if (ap >= n) break;
-        double A = v.f4(cp, ap, bp, b, c, a) - v.f4(ap, cp, b, bp, a, c) - v.f4(ap, cp, c, a, bp, b);
-        double T = v.f4(ap, cp, bp, b, a, c) - v.f4(cp, ap, b, bp, c, a) - v.f4(cp, ap, a, c, bp, b);
-        A += v.wca(cp, bp, b, c, ap, a) + v.jj(cp, c, bp, b, ap, a) - v.waa(cp, bp, b, a, ap, c) -
-             v.waa(bp, cp, ap, a, b, c) - v.waa(cp, a, c, bp, ap, b);
-        T += v.waa(cp, b, bp, a, ap, c) + v.waa(b, cp, ap, a, bp, c) - v.waa(c, ap, cp, bp, a, b) -
-             v.wca(cp, b, bp, c, ap, a) - v.wca(b, cp, ap, c, bp, a) - v.wca(cp, a, c, bp, ap, b);
-        T += 2.0 * v.jj(cp, ap, a, c, b, bp) - v.jj(cp, c, b, bp, ap, a) - v.jj(cp, ap, b, c, bp, a) -
-             v.jj(cp, bp, a, c, ap, b) - v.kx(cp, ap, a, c, b, bp);
-        T += sum[i] + d1 * (2.0 * v.ai(ap, a, b, bp) - v.ai(bp, a, b, ap));
-        // Kronecker deltas
-        auto q2 = [&]() {  // sum_e J2[cp,e;c,e]
-            double q = 0.0;
-            for (int e = 0; e < n; ++e) q += v.J2[v.i4(cp, e, c, e)];
-            return q;
-        };
-        if (ap == bp) {
-            A += v.G1[v.i4(cp, b, c, a)] - v.G1[v.i4(b, cp, a, c)] - v.G3[v.i4(cp, a, c, b)] - v.Q1[v.i4(cp, a, b, c)];
-            if (a == b) A -= q2();
-        }
-        if (ap == a) {
-            A -= v.G3[v.i4(cp, bp, b, c)] + v.G3[v.i4(bp, cp, c, b)] + v.Q1[v.i4(bp, cp, b, c)];
-            T += v.G3[v.i4(cp, b, bp, c)] + v.Q1[v.i4(b, cp, bp, c)] - v.G1[v.i4(cp, c, bp, b)] + v.Z[v.i4(cp, c, bp, b)];
-        }
-        if (a == b) A -= v.G3[v.i4(bp, cp, ap, c)] + v.Q1[v.i4(cp, bp, ap, c)];
-        if (ap == b) {
-            T += v.G1[v.i4(bp, cp, a, c)] - v.G1[v.i4(cp, bp, c, a)] - v.JW[v.i4(cp, c, bp, a)] + v.Q1[v.i4(cp, a, bp, c)];
-            if (bp == a) T += q2();
-        }
-        if (bp == a)
-            T += v.G3[v.i4(b, cp, ap, c)] + v.Q1[v.i4(cp, b, ap, c)] - v.G1[v.i4(cp, ap, c, b)] - v.JW[v.i4(cp, c, ap, b)];
-        if (b == bp) {
-            T += 2.0 * (v.G1[v.i4(cp, ap, c, a)] + v.JW[v.i4(cp, c, ap, a)] - v.G3[v.i4(a, cp, ap, c)] -
-                        v.Q1[v.i4(cp, a, ap, c)]);
-            if (a == ap) T -= 2.0 * q2();
-        }
-        const ll o = v.s + (ll)v.r.M * (ap + n * (bp + n * (cp + n * (a + (ll)n * (b + n * c)))));
-        amat[o] = A;
-        atmat[o] = T;
+    double A = v.f4(cp, ap, bp, b, c, a) - v.f4(ap, cp, b, bp, a, c) - v.f4(ap, cp, c, a, bp, b);
+    double T = v.f4(ap, cp, bp, b, a, c) - v.f4(cp, ap, b, bp, c, a) - v.f4(cp, ap, a, c, bp, b);
+    A += v.wca(cp, bp, b, c, ap, a) + v.jj(cp, c, bp, b, ap, a) - v.waa(cp, bp, b, a, ap, c) -
+         v.waa(bp, cp, ap, a, b, c) - v.waa(cp, a, c, bp, ap, b);
+    T += v.waa(cp, b, bp, a, ap, c) + v.waa(b, cp, ap, a, bp, c) - v.waa(c, ap, cp, bp, a, b) -
+         v.wca(cp, b, bp, c, ap, a) - v.wca(b, cp, ap, c, bp, a) - v.wca(cp, a, c, bp, ap, b);
+    T += 2.0 * v.jj(cp, ap, a, c, b, bp) - v.jj(cp, c, b, bp, ap, a) - v.jj(cp, ap, b, c, bp, a) -
+         v.jj(cp, bp, a, c, ap, b) - v.kx(cp, ap, a, c, b, bp);
+    T += 2.0 * (v.t3(c, ap, cp, a, b, bp) + v.t3(cp, a, c, ap, b, bp)) - v.t3(c, ap, cp, b, bp, a) -
+         v.t3(cp, a, c, bp, b, ap) - v.t3(cp, b, c, ap, bp, a) - v.t3(b, cp, c, bp, ap, a) -
+         v.t3(c, bp, cp, a, ap, b) - v.t3(bp, c, cp, b, ap, a);
+    T += d1 * (2.0 * v.ai(ap, a, b, bp) - v.ai(bp, a, b, ap));
+    // Kronecker deltas
+    auto q2 = [&]() {  // sum_e J2[cp,e;c,e]
+        double q = 0.0;
+        for (int e = 0; e < n; ++e) q += v.J2[v.i4(cp, e, c, e)];
+        return q;
+    };
+    if (ap == bp) {
+        A += v.G1[v.i4(cp, b, c, a)] - v.G1[v.i4(b, cp, a, c)] - v.G3[v.i4(cp, a, c, b)] - v.Q1[v.i4(cp, a, b, c)];
+        if (a == b) A -= q2();
     }
+    if (ap == a) {
+        A -= v.G3[v.i4(cp, bp, b, c)] + v.G3[v.i4(bp, cp, c, b)] + v.Q1[v.i4(bp, cp, b, c)];
+        T += v.G3[v.i4(cp, b, bp, c)] + v.Q1[v.i4(b, cp, bp, c)] - v.G1[v.i4(cp, c, bp, b)] + v.Z[v.i4(cp, c, bp, b)];
+    }
+    if (a == b) A -= v.G3[v.i4(bp, cp, ap, c)] + v.Q1[v.i4(cp, bp, ap, c)];
+    if (ap == b) {
+        T += v.G1[v.i4(bp, cp, a, c)] - v.G1[v.i4(cp, bp, c, a)] - v.JW[v.i4(cp, c, bp, a)] + v.Q1[v.i4(cp, a, bp, c)];
+        if (bp == a) T += q2();
+    }
+    if (bp == a)
+        T += v.G3[v.i4(b, cp, ap, c)] + v.Q1[v.i4(cp, b, ap, c)] - v.G1[v.i4(cp, ap, c, b)] - v.JW[v.i4(cp, c, ap, b)];
+    if (b == bp) {
+        T += 2.0 * (v.G1[v.i4(cp, ap, c, a)] + v.JW[v.i4(cp, c, ap, a)] - v.G3[v.i4(a, cp, ap, c)] -
+                    v.Q1[v.i4(cp, a, ap, c)]);
+        if (a == ap) T -= 2.0 * q2();
+    }
+    const ll o = v.s + (ll)v.r.M * (ap + n * (bp + n * (cp + n * (a + (ll)n * (b + n * c)))));
+    amat[o] = A;
+    atmat[o] = T;
 }
 #undef AT
 
@@ -609,7 +630,7 @@ FKernel f_kernel(int rpt) {
 ll SymScratch::doubles(int n) {
     const ll n2 = (ll)n * n, n4 = n2 * n2, np = n * (n + 1) / 2;
     const ll W = (ll)n * (n + 1) * (n + 2) * (n + 3) / 24;
-    return W * n4 + 4 * np * n4 + np * np * n2 + 8 * n4 + 2 * np * n2 + np + 2 * n2 + W / 2 + 1;
+    return W * n4 + 4 * np * n4 + np * np * n2 + 7 * n4 + 2 * np * n2 + np + 2 * n2 + W / 2 + 1;
 }
 
 SymScratch::SymScratch(int n, double *w) {
@@ -627,7 +648,6 @@ SymScratch::SymScratch(int n, double *w) {
     Bf = take((np + 1) * n2);
     I4 = take(n4);
     IJ = take((n2 + 1) * np);
-    Lb = take(n4);
     g = take(n2);
     key = (int *)take(W / 2 + 1);
 }
@@ -643,10 +663,11 @@ namespace {
 void sym_finish(const SymView &v, const SymScratch &S, double *amat, double *atmat, const int *fl, cudaStream_t st) {
     const ll n = v.n, n4 = n * n * n * n;
     k_sym_small<<<(unsigned)((kSmallLanes * n4 + 63) / 64), 64, 0, st>>>(v, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, fl);
-    const int tb = n <= kOutSmall ? 64 : 256;
-    const dim3 go((unsigned)((n4 * n + tb - 1) / tb), (unsigned)((n + kOutAp - 1) / kOutAp));
-    k_sym_out<<<go, tb, 0, st>>>(v, amat, atmat, fl);
-    g_launches.fetch_add(2, std::memory_order_relaxed);
+    const dim3 gt((unsigned)((n * n * n + 63) / 64), (unsigned)((n * n * (n + 1) / 2 + 63) / 64));
+    k_sym_t3<<<gt, 256, 0, st>>>(v.r, v.s, v.atwo, S.H, fl);
+    const dim3 go((unsigned)((n4 * n + kOutTb - 1) / kOutTb), (unsigned)n);
+    k_sym_out<<<go, kOutTb, 0, st>>>(v, amat, atmat, fl);
+    g_launches.fetch_add(3, std::memory_order_relaxed);
 }
 void sym_unpack(const Rdm &r, int s, const SymScratch &S, int *flag, cudaStream_t st) {
     const ll n = r.n, n4 = n * n * n * n;
@@ -656,7 +677,7 @@ void sym_unpack(const Rdm &r, int s, const SymScratch &S, int *flag, cudaStream_
 }
 SymView sym_view(const Rdm &r, int s, const double *atwo, const SymScratch &S) {
     const ll n2 = (ll)r.n * r.n;
-    return SymView{r, s, r.n, n2, r.n * (r.n + 1) / 2 * n2, S.F, S.N8, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, atwo, S.Lb, S.g};
+    return SymView{r, s, r.n, n2, r.n * (r.n + 1) / 2 * n2, S.F, S.N8, S.G1, S.G3, S.Q1, S.JW, S.J2, S.Z, atwo, S.g, S.H};
 }
 }  // namespace
 

@@ -11,9 +11,9 @@ constexpr int kSymMaxRpt = 6;  // rows per thread of the n^9 product
 
 // Views into one scratch block of doubles(n) doubles, reused for every state.
 struct SymScratch {
-    double *H, *F, *N8;                       // unpacked 4-RDM [W][n^4]; F; the four n^8 tensors
+    double *H, *F, *N8;                       // unpacked 4-RDM [W][n^4], then T3; F; the four n^8 tensors
     double *G1, *G3, *Q1, *JW, *J2, *Z;       // n^4 sums
-    double *Bf, *I4, *IJ, *Lb, *g;            // integral operands, f + K/2
+    double *Bf, *I4, *IJ, *g;                 // integral operands, f + K/2
     int *key;                                 // packed key quadruples [W]
     SymScratch(int n, double *w);
     static ll doubles(int n);

@@ -298,19 +298,44 @@ __global__ void __launch_bounds__(256) k_sym_x(Rdm r, int s, int bc, int pr0, co
 // q, r): Wca and Waa have p' their second creator (s or t) and (q,r) the free
 // pair, Kx and J the pairs (p,q), (p',r).  The rows of Gamma3 are affine in the
 // two summed indices, lo the one with stride M, so the tile loads need no
-// intermediate matrix.  64 x 64 tiles, 4 x 4 per thread; bound by the FP64 pipe
-// (n = 16: 13.8 ms for 1.6e10 flops, 1.14 TFLOP/s).
-constexpr int kN8K = 16;
-// 64 x 64 tiles from this many on, 32 x 32 below (n <= 7): a tile is 17 us of one SM's FP64
-// pipe for each 16 of its n^2 products, whether the other SMs have one or not.  32 / 64,
-// us: n = 4 9 / 24, n = 6 29 / 57, n = 7 54 / 74.
-constexpr unsigned kN8Tiles = 128;
+// intermediate matrix.  Bound by the FP64 pipe (n = 16: 10.5 ms for 1.23e10 flops, 1.17
+// TFLOP/s).  32 x 32 tiles, 2 x 2 per thread: a tile of 64 is four times as long and leaves
+// SMs idle in the last wave and columns in the last tile; 32 / 64, us: n = 4 9 / 22, n = 8
+// 70 / 73, n = 9 175 / 298, n = 12 1230 / 1590, n = 14 4420 / 4990, n = 16 10540 / 10960.
+constexpr int kN8 = 32, kN8K = 16;
+// Kx and J keep their value under the exchange of creators and annihilators (Kx with x, y
+// exchanged), so their rows are pairs of pairs: (p >= p') of index ua >= ub of (q,r), and q,
+// r in either order, about half of the others' np n^2.
+__host__ __device__ __forceinline__ ll n8_rows(int n, int kind) {
+    const ll np = n * (n + 1) / 2;
+    return kind < 2 ? np * n * n : np * (np + 1);
+}
+__host__ __device__ __forceinline__ ll n8_at(int n, int kind) {  // first element of a kind's results, and rows x n^2
+    const ll n2 = (ll)n * n;
+    return (kind < 3 ? kind * n8_rows(n, 0) : 2 * n8_rows(n, 0) + n8_rows(n, 2)) * n2;
+}
+__device__ __forceinline__ void n8_labels(int n, int kind, ll row, int &p, int &p2, int &q1, int &q2) {
+    if (kind < 2) {
+        q2 = (int)(row % n);
+        q1 = (int)((row / n) % n);
+        unpair((int)(row / (n * n)), p, p2);
+    } else {
+        int ua, ub;
+        unpair((int)(row >> 1), ua, ub);
+        unpair(ua, p, p2);
+        unpair(ub, q1, q2);
+        if (row & 1) {
+            const int t = q1;
+            q1 = q2;
+            q2 = t;
+        }
+    }
+}
 // Offset of a row of Gamma3 (in units of M) and the stride of its slow summed index.
 __device__ __forceinline__ ll n8_row(int n, int kind, ll row) {
     const ll n1 = n, n2 = n1 * n, n3 = n2 * n, n4 = n2 * n2, n5 = n4 * n;
-    const int q2 = (int)(row % n), q1 = (int)((row / n) % n);
-    int p, p2;
-    unpair((int)(row / n2), p, p2);
+    int p, p2, q1, q2;
+    n8_labels(n, kind, row, p, p2, q1, q2);
     if (kind == 0) return n1 * p + n2 * q1 + n3 * p2 + n5 * q2;       // (e,s), (p,f), (q,r)
     if (kind == 1) return n2 * q2 + n3 * p2 + n4 * p + n5 * q1;       // (e,t), (f,p), (r,q): exchanged
     if (kind == 2) return n1 * q1 + n2 * q2 + n4 * p + n5 * p2;       // (e,d), (q,p), (r,p'): exchanged
@@ -319,27 +344,26 @@ __device__ __forceinline__ ll n8_row(int n, int kind, ll row) {
 __device__ __forceinline__ ll n8_hi(int n, int kind) {
     return kind == 0 ? (ll)n * n * n * n : kind == 1 ? (ll)n : (ll)n * n * n;
 }
-// Gamma2 factor of row ((p >= p'), q, r) of J
+// Gamma2 factor of a row of J
 __device__ __forceinline__ double n8_pair2(const Rdm &r, int s, ll row) {
     const int n = r.n;
-    int p, p2;
-    unpair((int)(row / (n * n)), p, p2);
-    return r.d2[s + (ll)r.M * (p + n * (p2 + n * ((row / n) % n + n * (row % n))))];
+    int p, p2, q1, q2;
+    n8_labels(n, 3, row, p, p2, q1, q2);
+    return r.d2[s + (ll)r.M * (p + n * (p2 + n * (q1 + n * q2)))];
 }
-template <int kN8>
 __global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__restrict__ I4,
                                                 const double *__restrict__ IJ, double *out, const int *flag) {
     if (*flag) return;
     constexpr int P = kN8 / 16;  // rows and columns of a thread
     __shared__ double As[kN8K][kN8 + 1], Bs[kN8K][kN8];
     const int n = r.n, np = n * (n + 1) / 2, kind = blockIdx.z;
-    const ll M = r.M, n2 = (ll)n * n, rows = np * n2;
+    const ll M = r.M, n2 = (ll)n * n, rows = n8_rows(n, kind);
     const int N = kind == 3 ? np : (int)n2;
     const int c0 = blockIdx.y * kN8;
-    if (c0 >= N) return;
     const ll r0 = (ll)blockIdx.x * kN8;
+    if (c0 >= N || r0 >= rows) return;
     const double *Bm = kind == 3 ? IJ : I4;
-    double *C = out + kind * rows * n2;
+    double *C = out + n8_at(n, kind);
     const ll hi = M * n8_hi(n, kind);
     const int tid = threadIdx.x, lk = tid & 15, lr = tid >> 4;
     const double *base[P];
@@ -398,12 +422,11 @@ __global__ void __launch_bounds__(256) k_sym_n8(Rdm r, int s, const double *__re
 __global__ void __launch_bounds__(256) k_sym_rows(Rdm r, int s, double *__restrict__ R, const int *flag) {
     if (*flag) return;
     const int n = r.n, kind = blockIdx.y, n2 = n * n, K = kind == 3 ? n2 + 1 : n2;
-    const ll rows = (ll)(n * (n + 1) / 2) * n2;
     const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= rows * K) return;
+    if (t >= n8_rows(n, kind) * K) return;
     const ll row = t / K;
     const int k = (int)(t % K);
-    R[kind * rows * n2 + t] = k == n2 ? n8_pair2(r, s, row)
+    R[n8_at(n, kind) + t] = k == n2 ? n8_pair2(r, s, row)
                                       : r.d3[s + (ll)r.M * (n8_row(n, kind, row) + (k / n) * n8_hi(n, kind) + k % n)];
 }
 
@@ -436,14 +459,23 @@ struct SymView {
         const double *A = N8 + rows * n2;
         return p >= t ? A[row3(p, t, q, q2) * n2 + x * n + y] : A[row3(t, p, q, q2) * n2 + y * n + x];
     }
+    // row of ((p,q), (p2,q2)) in Kx and J; tr: of its transpose
+    __device__ __forceinline__ ll rowk(int p, int q, int p2, int q2, bool &tr) const {
+        int ua = pmx(p, p2), ub = pmx(q, q2);
+        tr = ua < ub;
+        const bool flip = tr ? q < q2 : p < p2, less = tr ? p < p2 : q < q2;  // of the leading pair, of the other
+        const int up = tr ? ub : ua, lo = tr ? ua : ub;
+        return (ll)pidx(up, lo) * 2 + (flip != less ? 1 : 0);
+    }
     __device__ __forceinline__ double kx(int p, int q, int p2, int q2, int x, int y) const {
-        const double *A = N8 + 2 * rows * n2;
-        return p >= p2 ? A[row3(p, p2, q, q2) * n2 + x * n + y] : A[row3(p2, p, q2, q) * n2 + x * n + y];
+        bool tr;
+        const ll row = rowk(p, q, p2, q2, tr);
+        return N8[n8_at(n, 2) + row * n2 + (tr ? y * n + x : x * n + y)];
     }
     __device__ __forceinline__ double jj(int p, int q, int p2, int q2, int x, int y) const {
-        const double *A = N8 + 3 * rows * n2;
-        const int np = n * (n + 1) / 2;
-        return p >= p2 ? A[row3(p, p2, q, q2) * np + pmx(x, y)] : A[row3(p2, p, q2, q) * np + pmx(x, y)];
+        bool tr;
+        const ll row = rowk(p, q, p2, q2, tr);
+        return N8[n8_at(n, 3) + row * (n * (n + 1) / 2) + pmx(x, y)];
     }
     __device__ __forceinline__ double t3(int x1, int x2, int x3, int p, int q, int r) const {
         return T3[(((ll)(x1 * n + x2) * n + x3) * (n * (n + 1) / 2) + pmx(q, r)) * n + p];
@@ -630,7 +662,7 @@ FKernel f_kernel(int rpt) {
 ll SymScratch::doubles(int n) {
     const ll n2 = (ll)n * n, n4 = n2 * n2, np = n * (n + 1) / 2;
     const ll W = (ll)n * (n + 1) * (n + 2) * (n + 3) / 24;
-    return W * n4 + 4 * np * n4 + np * np * n2 + 7 * n4 + 2 * np * n2 + np + 2 * n2 + W / 2 + 1;
+    return W * n4 + np * n4 + n8_at(n, 3) + n8_rows(n, 3) * np + 7 * n4 + 2 * np * n2 + np + 2 * n2 + W / 2 + 1;
 }
 
 SymScratch::SymScratch(int n, double *w) {
@@ -643,7 +675,7 @@ SymScratch::SymScratch(int n, double *w) {
     };
     H = take(W * n4);
     F = take(np * n4);
-    N8 = take(3 * np * n4 + np * np * n2);
+    N8 = take(n8_at(n, 3) + n8_rows(n, 3) * np);
     for (double **p : {&G1, &G3, &Q1, &JW, &J2, &Z}) *p = take(n4);
     Bf = take((np + 1) * n2);
     I4 = take(n4);
@@ -684,13 +716,10 @@ SymView sym_view(const Rdm &r, int s, const double *atwo, const SymScratch &S) {
 int launch_sym_state(const Rdm &r, int s, const double *atwo, const SymScratch &S, double *amat, double *atmat,
                      int *flag, cudaStream_t st) {
     const int n = r.n, np = n * (n + 1) / 2, *fl = flag + s;
-    const ll n2 = (ll)n * n, rows = np * n2;
+    const ll n2 = (ll)n * n, rows = std::max(n8_rows(n, 0), n8_rows(n, 2));
     sym_unpack(r, s, S, flag, st);
-    // tiles of 64 unless they leave SMs idle
-    auto grid = [&](int t) { return dim3((unsigned)((rows + t - 1) / t), (unsigned)((n2 + t - 1) / t), 4); };
-    const dim3 g8 = grid(64);
-    if (g8.x * g8.y * g8.z >= kN8Tiles) k_sym_n8<64><<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
-    else k_sym_n8<32><<<grid(32), 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
+    const dim3 g8((unsigned)((rows + kN8 - 1) / kN8), (unsigned)((n2 + kN8 - 1) / kN8), 4);
+    k_sym_n8<<<g8, 256, 0, st>>>(r, s, S.I4, S.IJ, S.N8, fl);
     const FShape fs = f_shape(n);
     const FKernel fk = f_kernel(fs.rpt);
     const int smem = (fs.bc * n * (np | 1) + np * n) * (int)sizeof(double);
@@ -706,7 +735,7 @@ int launch_sym_state(const Rdm &r, int s, const double *atwo, const SymScratch &
 int launch_sym_state_split(const Rdm &r, int s, const double *atwo, const SymScratch &S, double *rows_buf,
                            void *oz_work, int *oz_err, double *amat, double *atmat, int *flag, cudaStream_t st) {
     const int n = r.n, np = n * (n + 1) / 2, *fl = flag + s;
-    const ll n2 = (ll)n * n, n3 = n2 * n, rows = np * n2;
+    const ll n2 = (ll)n * n, n3 = n2 * n, rows = std::max(n8_rows(n, 0), n8_rows(n, 2));
     const oz::Gate gate{fl, false};
     sym_unpack(r, s, S, flag, st);
     // F: the operand rows of some creator pairs at a time, then their digit product
@@ -730,15 +759,15 @@ int launch_sym_state_split(const Rdm &r, int s, const double *atwo, const SymScr
     k_sym_rows<<<gr, 256, 0, st>>>(r, s, rows_buf, fl);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     oz::WideGemm g;
-    g.m = 3 * rows; g.n = n2; g.K = (int)n2;
+    g.m = n8_at(n, 3) / n2; g.n = n2; g.K = (int)n2;
     g.A = rows_buf; g.a_r = n2; g.a_k = 1;
     g.B = S.I4; g.b_c = 1; g.b_k = n2;
     g.C = S.N8; g.ldc = n2;
     if (oz::oz_gemm_wide(g, oz_work, oz_err, st)) return 1;
-    g.m = rows; g.n = np; g.K = (int)n2 + 1;
-    g.A = rows_buf + 3 * rows * n2; g.a_r = n2 + 1;
+    g.m = n8_rows(n, 3); g.n = np; g.K = (int)n2 + 1;
+    g.A = rows_buf + n8_at(n, 3); g.a_r = n2 + 1;
     g.B = S.IJ; g.b_k = np;
-    g.C = S.N8 + 3 * rows * n2; g.ldc = np;
+    g.C = S.N8 + n8_at(n, 3); g.ldc = np;
     if (oz::oz_gemm_wide(g, oz_work, oz_err, st)) return 1;
     sym_finish(sym_view(r, s, atwo, S), S, amat, atmat, fl, st);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
@@ -748,13 +777,13 @@ int sym_split_pairs(int n) { return std::max(1, std::min(n * (n + 1) / 2, 65536 
 
 ll sym_split_rows_doubles(int n) {
     const ll n2 = (ll)n * n, np = n * (n + 1) / 2, xr = sym_split_pairs(n) * n2 * n;
-    return std::max(xr * (n * (np + 1) + 1), np * n2 * (4 * n2 + 1));
+    return std::max(xr * (n * (np + 1) + 1), n8_at(n, 3) + n8_rows(n, 3) * (n2 + 1));
 }
 
 size_t sym_split_oz_bytes(int n) {
     const ll n2 = (ll)n * n, np = n * (n + 1) / 2;
     return std::max({oz::OzPlan(1, sym_split_pairs(n) * n2 * n, n * (int)(np + 1), n).bytes(),
-                     oz::oz_wide_bytes(3 * np * n2, n2, (int)n2), oz::oz_wide_bytes(np * n2, np, (int)n2 + 1)});
+                     oz::oz_wide_bytes(n8_at(n, 3) / n2, n2, (int)n2), oz::oz_wide_bytes(n8_rows(n, 3), np, (int)n2 + 1)});
 }
 
 }  // namespace nvpt

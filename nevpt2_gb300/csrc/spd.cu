@@ -292,40 +292,45 @@ __global__ void __launch_bounds__(TP) k_spd_norm(const double *__restrict__ W, i
     }
 }
 
-// N = W M: tile (i, j) is the sum over the blocks j .. i; the longest first.
+// N = W M: tile (i, j) is the sum over the blocks j .. i, a half (32 rows) a block, the
+// longest first.
 __global__ void __launch_bounds__(TP) k_spd_n(const double *__restrict__ W, const double *__restrict__ M, long long ld,
                                               int nb, int n, double *N) {
     __shared__ __align__(16) Slab s;
     int r, j;
-    triangle(blockIdx.x, r, j);
+    triangle(blockIdx.x / 2, r, j);
     const int i = j + nb - 1 - r, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4] = {};
-    tile<false, 4>(acc, W + (long long)i * B * ld + j * B, ld, M + (long long)j * B * ld + j * B, ld, min((i - j + 1) * B, (n + KS - 1) / KS * KS - j * B), s);
-    double *C = N + (long long)i * B * ld + j * B;
+    const long long ro = ((long long)i * B + blockIdx.x % 2 * 32) * ld + j * B;
+    double acc[2][4] = {};
+    tile<false, 2>(acc, W + ro, ld, M + (long long)j * B * ld + j * B, ld,
+                   min((i - j + 1) * B, (n + KS - 1) / KS * KS - j * B), s);
+    double *C = N + ro;
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
         for (int q = 0; q < 2; ++q)
-            *reinterpret_cast<double2 *>(C + own(ty, p) * ld + 32 * q + 2 * tx) = make_double2(acc[p][2 * q], acc[p][2 * q + 1]);
+            *reinterpret_cast<double2 *>(C + (2 * ty + p) * ld + 32 * q + 2 * tx) = make_double2(acc[p][2 * q], acc[p][2 * q + 1]);
 }
 
-// K~ = N W^T + W N^T: tile (i, j <= i) sums over the blocks 0 .. j; the longest first.
+// K~ = N W^T + W N^T: tile (i, j <= i) sums over the blocks 0 .. j, a half (32 rows) a block,
+// the longest first (order 2744 13.2 -> 13.0 ms; order 1000 1.33 ms, where the longest whole
+// tile is 32 block products of 67 us).
 __global__ void __launch_bounds__(TP) k_spd_k(const double *__restrict__ W, const double *__restrict__ N, long long ld,
                                               int nb, int n, double *out) {
     __shared__ __align__(16) Slab s;
     int r, x;
-    triangle(blockIdx.x, r, x);
-    const int j = nb - 1 - r, i = j + x, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4] = {};
-    const long long ro = (long long)i * B * ld, co = (long long)j * B * ld;
+    triangle(blockIdx.x / 2, r, x);
+    const int j = nb - 1 - r, i0 = (j + x) * B + blockIdx.x % 2 * 32, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double acc[2][4] = {};
+    const long long ro = i0 * ld, co = (long long)j * B * ld;
     const int K = min((j + 1) * B, (n + KS - 1) / KS * KS);  // M has only zeros in the padding
-    tile<true, 4>(acc, N + ro, ld, W + co, ld, K, s);
-    tile<true, 4>(acc, W + ro, ld, N + co, ld, K, s);
+    tile<true, 2>(acc, N + ro, ld, W + co, ld, K, s);
+    tile<true, 2>(acc, W + ro, ld, N + co, ld, K, s);
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int a = i * B + own(ty, p), b = j * B + own(tx, q);
+            const int a = i0 + 2 * ty + p, b = j * B + own(tx, q);
             if (a < n && b <= a) {
                 out[(long long)a * n + b] = acc[p][q];
                 out[(long long)b * n + a] = acc[p][q];
@@ -376,8 +381,8 @@ void spd_congruence(Ctx &c, const double *W, const double *K, long long n, doubl
     const int nb = (int)(ld / B);
     T M = alloc(c, {ld, ld}, false), N = alloc(c, {ld, ld}, false);
     k_spd_half<<<blocks(ld * ld), TP, 0, c.st>>>(K, (int)n, ld, M.p);
-    k_spd_n<<<nb * (nb + 1) / 2, TP, 0, c.st>>>(W, M.p, ld, nb, (int)n, N.p);
-    k_spd_k<<<nb * (nb + 1) / 2, TP, 0, c.st>>>(W, N.p, ld, nb, (int)n, out);
+    k_spd_n<<<nb * (nb + 1), TP, 0, c.st>>>(W, M.p, ld, nb, (int)n, N.p);
+    k_spd_k<<<nb * (nb + 1), TP, 0, c.st>>>(W, N.p, ld, nb, (int)n, out);
     g_launches.fetch_add(3, std::memory_order_relaxed);
     ck(cudaGetLastError(), "congruence");
 }

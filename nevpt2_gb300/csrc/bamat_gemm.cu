@@ -562,7 +562,8 @@ __global__ void k_slab_list(int n, int *cp, int *ap);
 
 // Split mode takes the digit products from this many active orbitals on; the
 // FP64 products are the faster and the more exact below (one state, FP64 / digits:
-// n = 10 1.68 / 1.81 ms, n = 11 3.32 / 3.07, n = 14 22.6 / 14.4, n = 16 60.4 / 37.3).
+// n = 10 1.42 / 1.69 ms, n = 11 2.75 / 2.74, n = 12 5.4 / 4.5, n = 14 19.4 / 12.8, n = 16
+// 52.6 / 32.4).
 constexpr int kSplitMinNact = 11;
 constexpr unsigned kSlabCtas = 152 * 16;  // CTAs of a slab launch: one wave or so, looping
 

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256) k_sym_ops(const double *atwo, const doubl
 // annihilators of higher rank than K (where the packed form keeps the
 // exchanged element).  Reads are coalesced along K, writes along l1.  The
 // blocks from nub on check Gamma1..3.  Bound by HBM (16 W n^4 bytes) and by the
-// gathers of the completed half; n = 16: 3.9 ms.
+// gathers of the completed half; n = 16: 3.0 ms.
 __global__ void __launch_bounds__(256) k_sym_unpack(Rdm r, int s, const int *key, unsigned nub, double *H, int *flag) {
     const int n = r.n;
     const ll n2 = (ll)n * n, n3 = n2 * n, n4 = n2 * n2, W = r.W;

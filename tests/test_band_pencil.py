@@ -1,6 +1,6 @@
-"""The order-n^3 pencils in band form (half bandwidth 32) against the oracle's
-eigenvector sequence: 512 = 16 * 32, the smallest order that takes this form, and
-729 = 22 * 32 + 25, whose last panel is ragged.
+"""The order-n^3 pencils on both sides of the change of form against the oracle's
+eigenvector sequence: 512, the largest order in tridiagonal form, and 729 = 22 * 32 +
+25 in band form (half bandwidth 32), whose last panel is ragged.
 Energies, norms, cross terms of several states, and the densities, whose
 solutions are mapped back through the reflectors.  Tolerances as for the other
 resolvent tests: 1e-9 relative, 1e-10 (densities) and 1e-9 (energies) absolute."""

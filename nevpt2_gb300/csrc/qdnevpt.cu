@@ -1955,7 +1955,6 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
             }
         }
     }
-    std::vector<std::array<Pencil1p, 2>> pencils(M);
     std::vector<PairData> pd(P);
     if (P > 0) {
         T T1 = S(in->trdm1, P * n2), T2 = S(in->trdm2, P * n4), T3 = S(in->trdm3, P * n6);
@@ -2011,6 +2010,9 @@ int run_qdnevpt(nvpt_context *ctx, cudaStream_t st, const nvpt_qdnevpt_in *in, n
             pc_.wait_limit = nvpt_context_wait_limit(ctx);
             pc_.arena = &arena;
         }
+    // After ps and cs, and so destroyed before them: the fork of a class that failed
+    // before its join still points to that class's context.
+    std::vector<std::array<Pencil1p, 2>> pencils(M);
     if (pc && M == 1) {  // the longest chains first: see Pencil1p
         if ((m & 64u) && nv) pencils[0][1].start(c, sd[0], n, true, in->thr_lindep);
         if ((m & 32u) && nc) pencils[0][0].start(c, sd[0], n, false, in->thr_lindep);

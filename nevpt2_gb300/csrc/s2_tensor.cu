@@ -422,7 +422,9 @@ __global__ void k_start_block(double *X, long long count) {
 // the largest diagonal element, delta tr (S + delta)^-1 counts them (a kept eigenvalue
 // w adds delta / w); two steps of inverse iteration on S + delta from k random vectors
 // gain a factor w / delta each, and the block is orthonormalised through the inverse
-// factor of its Gram matrix, twice.  False if the metric is not of this
+// factor of its Gram matrix, twice.  Null means that the Rayleigh quotients of the block
+// add up to at most 1e-12 of that element; a threshold below this line may keep such an
+// eigenvalue, and its pencil is not deflated.  False if the metric is not of this
 // kind.  All products and one factorisation of order n: the QR factorisations of a
 // wider block that this replaces took 5 ms at order 216, latency for the most part.
 bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long long &k) {
@@ -437,6 +439,8 @@ bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long lo
     double tr = 0.0, st[2], big = 0.0;
     ck(cudaMemcpyAsync(&big, top.p, sizeof(double), cudaMemcpyDeviceToHost, c.st), "diagonal");
     if (!spd_inverse_factor(c, L.p, n, W.p, tr) || !(big > 0.0)) return false;  // synchronises
+    const double null = 1e-12 * big;
+    if (!(thr >= null)) return false;
     const double count = tr * 1e-11 * big;
     if (!(count < (double)n)) return false;
     k = std::llround(count);
@@ -465,7 +469,7 @@ bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long lo
     ck(cudaMemcpyAsync(&w, top.p, sizeof(double), cudaMemcpyDeviceToHost, c.st), "quotients");
     ck(cudaMemcpyAsync(st, stat.p, sizeof(st), cudaMemcpyDeviceToHost, c.st), "status");
     ck(cudaStreamSynchronize(c.st), "sync");
-    if (spd_failed(st) || !(w <= 1e-12 * big)) return false;
+    if (spd_failed(st) || !(w <= null)) return false;
     N = std::move(X);
     return true;
 }

@@ -215,8 +215,9 @@ struct PencilTridiag {
     T N;           // null vectors of the metric [k, n]
     long long n = 0, k = 0;
 };
-// False, with nothing kept, unless every eigenvalue of S is above thr or null
-// (|w| <= 1e-12 of the largest; at most 48 of them).
+// False, with nothing kept, unless every eigenvalue of S is above thr or null; the null
+// ones are at most half of them, their Rayleigh quotients add up to at most 1e-12 of the
+// largest diagonal element, and thr is not below that.
 bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, double thr, PencilTridiag &P);
 // Householder tridiagonalisation of the symmetric A (column-major, both triangles
 // valid) in the output form of dsytrd('L'): d[n], e[n-1], tau[n-1], reflectors below

@@ -32,7 +32,6 @@ constexpr int TB = 256;        // threads per CTA
 constexpr int LP = NB + 1;     // padded row of a panel in shared memory
 
 constexpr int kQrMost = 39;  // CTAs of a panel: with the pivot row, at most 5 messages a thread
-constexpr unsigned long long kNoMsg = ~0ull;
 
 struct QrArgs {
     double *A;            // column-major n x n; panel columns j0 .. j0 + NB - 1, rows r0 .. n - 1
@@ -81,11 +80,9 @@ __global__ void __launch_bounds__(TB, 1) k_band_qr(QrArgs a) {
             double t = 0.0;
 #pragma unroll
             for (int w = 0; w < TB / 32; ++w) t += red[w][lane];
-            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(msg + blockIdx.x * NB + lane),
-                         "l"(__double_as_longlong(t)) : "memory");
+            send_word(msg + blockIdx.x * NB + lane, t);
         } else if (warp == 1 && blockIdx.x == 0) {
-            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(msg + ctas * NB + lane),
-                         "l"(__double_as_longlong(P[c * LP + lane])) : "memory");
+            send_word(msg + ctas * NB + lane, P[c * LP + lane]);
         }
         unsigned long long v[5];
         int ok = 1;

@@ -1,5 +1,5 @@
-// Grid-wide barrier of cooperative kernels (all CTAs co-resident), with a bounded
-// wait.
+// Waits between the CTAs of cooperative kernels (all co-resident), bounded: a grid-wide
+// barrier, and words that arrive where they are polled for.
 #pragma once
 
 namespace nvpt {
@@ -45,6 +45,16 @@ __device__ __forceinline__ bool grid_bar(Bar *b, unsigned nblk, unsigned &gen, u
     }
     __syncthreads();
     return s_ok != 0;
+}
+
+// A double as a word that its reader polls for: kNoMsg until it has arrived.  A NaN of
+// these very bits (payloads pass through FP64 arithmetic, and memory filled with 0xff
+// bytes is one) becomes another NaN, or its readers would wait for good.
+constexpr unsigned long long kNoMsg = ~0ull;
+__device__ __forceinline__ void send_word(unsigned long long *to, double x) {
+    unsigned long long w = (unsigned long long)__double_as_longlong(x);
+    if (w == kNoMsg) w = 0x7ff8000000000000ull;
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(to), "l"(w) : "memory");
 }
 
 }  // namespace s2

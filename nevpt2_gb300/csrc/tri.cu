@@ -17,7 +17,6 @@ namespace {
 
 constexpr int TB = 256;
 constexpr int NB = kBand;  // reflectors of a panel of Q
-constexpr unsigned long long kNoMsg = ~0ull;
 
 struct TriArgs {
     const double *A;  // n x n, both triangles
@@ -104,9 +103,8 @@ __global__ void __launch_bounds__(TB, 1) k_tri_reduce(TriArgs a) {
             }
             for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
             if (lane == 0) {
-                asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(msg + i), "l"(__double_as_longlong(t)) : "memory");
-                asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(msg + n + i),
-                             "l"(__double_as_longlong(row[j + 1])) : "memory");
+                send_word(msg + i, t);
+                send_word(msg + n + i, row[j + 1]);
                 V[(long long)(i - s0) * NB] = v[i];
             }
         }

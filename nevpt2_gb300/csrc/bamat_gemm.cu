@@ -24,8 +24,6 @@
 #include "ozaki.cuh"
 
 #include <algorithm>
-#include <atomic>
-#include <cstdlib>
 #include <vector>
 
 namespace nvpt {
@@ -69,25 +67,27 @@ __global__ void __launch_bounds__(256) k_bamat_slabs(Rdm r, int s, const int *sl
 // With rmax, the block also folds the magnitudes into the row maxima of the
 // four layouts (bit patterns of non-negative doubles order like integers):
 // rmax[L * nslab n^3 + row] for layout L.
-constexpr int kSlabTileMax = 16 * (16 * 17 + 1);
+// Bound by the gathers of the packed 4-RDM: as many warps in flight as fit, so
+// the shared memory is the size's own, and each of the resident CTAs takes its
+// share of the blocks (a state: n = 9 1.05 ms, n = 13 17.9, n = 16 92.6; 2432 CTAs
+// and a sort in local memory, n = 16: 103).
+__host__ __device__ __forceinline__ int slab_tile(int n) { return n * (n * (n + 1) + 1); }
 __global__ void __launch_bounds__(256) k_bamat_slabs_t(Rdm r, int s, const int *slab_cp, const int *slab_ap,
                                                        int nslab, double *X1, double *X2, double *X3, double *X4,
                                                        unsigned long long *rmax, const int *flag) {
     if (flag && !*flag) return;
-    __shared__ double tile[kSlabTileMax];
-    __shared__ double mwz[256];
+    extern __shared__ double tile[];  // slab_tile(n), and n^2 with rmax
     const int n = r.n, sw = n + 1, sf = n * (n + 1) + 1;
-    const ll n2 = (ll)n * n, n3 = n2 * n, n6 = n3 * n3;
-    for (ll blk = blockIdx.x; blk < nslab * n3; blk += gridDim.x) {
+    const int n2 = n * n, n3 = n2 * n;
+    const ll n6 = (ll)n3 * n3;
+    double *mwz = tile + slab_tile(n);
+    for (int blk = blockIdx.x; blk < nslab * n3; blk += gridDim.x) {
         __syncthreads();
-        ll b = blk;
-        const int d = (int)(b % n); b /= n;
-        const int v = (int)(b % n); b /= n;
-        const int u = (int)(b % n); b /= n;
-        const int sl = (int)b;
+        const int d = blk % n, v = blk / n % n, u = blk / n2 % n, sl = blk / n3;
         const int cp = slab_cp[sl], ap = slab_ap[sl];
+#pragma unroll 2
         for (int i = threadIdx.x; i < n3; i += blockDim.x) {
-            const int z = i % n, w = (i / n) % n, f = i / (int)n2;
+            const int z = i % n, w = (i / n) % n, f = i / n2;
             tile[f * sf + w * sw + z] = r.eeee(cp + 1, ap + 1, u + 1, v + 1, d + 1, f + 1, w + 1, z + 1, s + 1);
         }
         __syncthreads();
@@ -95,17 +95,17 @@ __global__ void __launch_bounds__(256) k_bamat_slabs_t(Rdm r, int s, const int *
         for (int i = threadIdx.x; i < n3; i += blockDim.x) {
             // X1 rows (u,v,z) cols (d,f,w): i = (z, f, w)
             {
-                const int w = i % n, f = (i / n) % n, z = i / (int)n2;
+                const int w = i % n, f = (i / n) % n, z = i / n2;
                 X1[base + (((ll)u * n + v) * n + z) * n3 + ((ll)d * n + f) * n + w] = tile[f * sf + w * sw + z];
             }
             // X2 rows (u,v,w) cols (d,f,z): i = (w, f, z)
             {
-                const int z = i % n, f = (i / n) % n, w = i / (int)n2;
+                const int z = i % n, f = (i / n) % n, w = i / n2;
                 X2[base + (((ll)u * n + v) * n + w) * n3 + ((ll)d * n + f) * n + z] = tile[f * sf + w * sw + z];
             }
             // X3 rows (u,w,z) cols (v,d,f), X4 rows (v,w,z) cols (u,d,f): i = (w, z, f)
             {
-                const int f = i % n, z = (i / n) % n, w = i / (int)n2;
+                const int f = i % n, z = (i / n) % n, w = i / n2;
                 const double x = tile[f * sf + w * sw + z];
                 X3[base + (((ll)u * n + w) * n + z) * n3 + ((ll)v * n + d) * n + f] = x;
                 X4[base + (((ll)v * n + w) * n + z) * n3 + ((ll)u * n + d) * n + f] = x;
@@ -349,14 +349,16 @@ __global__ void k_bamat_assemble(int n, int M, int s, const double *T1, const do
 // C[rows, N] = X[rows, K] B[K, N] with K = n^3 and N = n <= 16: skinny
 // products whose cost is the FP64 pipe alone (2 FMA/clock/SM on GB300; the
 // 8 flops per X byte loaded are far above the HBM balance point), so the
-// kernel only has to keep that pipe busy.  One CTA computes a BM x 16 tile
-// (BM = 32 RPT; columns beyond N are zero in shared memory and never
-// stored); 256 threads, each an RPT x 2 register block; X is staged 32
-// columns at a time, transposed in shared memory (stride BM + 1 doubles) so
-// that a thread's rows at one k are contiguous, with the next chunk's global
-// loads issued before the current chunk's FMAs.  blockIdx.y selects one of up
-// to four products.  The tile height RPT is tuned per shape (tuner.h).
-constexpr int kSkBK = 32;
+// kernel only has to keep that pipe busy.  A CTA computes 64 rows: two warps
+// of rows times two of columns, a thread one row and NC = ceil(N/2) columns,
+// so every scheduler has the same FMAs, odd sizes pay one padded column and
+// the last wave leaves an SM at most 64 rows short.  X is staged 32 columns
+// at a time, transposed in shared memory (stride 65 doubles), with the next
+// chunk's global loads issued before the current chunk's FMAs.  blockIdx.y
+// selects one of the four products.  All products of a state, with 16 columns
+// whatever N, two a thread across each warp / as here: n = 9 5.97 / 3.06 ms, n = 13
+// 93.9 / 79.1, n = 16 442 / 442 (1.25 TFLOP/s).
+constexpr int kSkBK = 32, kSkBM = 64;
 struct SkinnyJobs {
     const double *X[4];
     const double *B[4];
@@ -364,156 +366,59 @@ struct SkinnyJobs {
     const int *flag;  // null, or the launch does nothing while *flag is zero
 };
 
-template <int RPT>
-__global__ void __launch_bounds__(256, 2) k_dgemm_skinny(SkinnyJobs jobs, ll rows, int N, int K) {
+template <int NC>
+__global__ void __launch_bounds__(128) k_dgemm_skinny(SkinnyJobs jobs, ll rows, int N, int K) {
     if (jobs.flag && !*jobs.flag) return;
-    constexpr int BM = 32 * RPT, LD = BM + 1, NX = BM / 8;
+    constexpr int LD = kSkBM + 1, NX = kSkBM * kSkBK / 128, NB = (kSkBK * 2 * NC + 127) / 128;
     __shared__ double Xs[kSkBK * LD];
-    __shared__ __align__(16) double Bs[kSkBK * 16];
+    __shared__ double Bs[kSkBK * 2 * NC];
     // constant indices only (a dynamic index would copy the struct to local memory)
     const int jb = blockIdx.y;
     const double *__restrict__ X = jb == 0 ? jobs.X[0] : jb == 1 ? jobs.X[1] : jb == 2 ? jobs.X[2] : jobs.X[3];
     const double *__restrict__ B = jb == 0 ? jobs.B[0] : jb == 1 ? jobs.B[1] : jb == 2 ? jobs.B[2] : jobs.B[3];
     double *__restrict__ C = jb == 0 ? jobs.C[0] : jb == 1 ? jobs.C[1] : jb == 2 ? jobs.C[2] : jobs.C[3];
     const int tid = threadIdx.x;
-    const ll r0 = (ll)blockIdx.x * BM;
-    // loader mapping: lane = k within the chunk, warp = row (+ 8 i)
+    const ll r0 = (ll)blockIdx.x * kSkBM;
+    // loader mapping: lane = k within the chunk, warp = row (+ 4 i)
     const int lk = tid & 31, lr = tid >> 5;
-    // compute mapping: RPT rows (tr*RPT..) x 2 columns (2 tc, 2 tc + 1)
-    const int tc = tid & 7, tr = tid >> 3;
-    double xr[NX], br[2];
+    // compute mapping: row, and the first of NC columns
+    const int row = tid & (kSkBM - 1), c0 = tid / kSkBM * NC;
+    double xr[NX], br[NB];
     auto load = [&](int k0) {
         const int k = k0 + lk;
 #pragma unroll
         for (int i = 0; i < NX; ++i) {
-            const ll r = r0 + lr + 8 * i;
+            const ll r = r0 + lr + 4 * i;
             xr[i] = (r < rows && k < K) ? X[r * K + k] : 0.0;
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int e = tid + 256 * i, kk = e >> 4, c = e & 15;
-            br[i] = (c < N && k0 + kk < K) ? B[(ll)(k0 + kk) * N + c] : 0.0;
+        for (int i = 0; i < NB; ++i) {
+            const int e = tid + 128 * i, kk = e / (2 * NC), c = e % (2 * NC);
+            br[i] = (kk < kSkBK && c < N && k0 + kk < K) ? B[(ll)(k0 + kk) * N + c] : 0.0;
         }
     };
-    double acc[RPT][2] = {};
+    double acc[NC] = {};
     load(0);
     for (int k0 = 0; k0 < K; k0 += kSkBK) {
 #pragma unroll
-        for (int i = 0; i < NX; ++i) Xs[lk * LD + lr + 8 * i] = xr[i];
+        for (int i = 0; i < NX; ++i) Xs[lk * LD + lr + 4 * i] = xr[i];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) Bs[tid + 256 * i] = br[i];
+        for (int i = 0; i < NB; ++i)
+            if (tid + 128 * i < kSkBK * 2 * NC) Bs[tid + 128 * i] = br[i];
         __syncthreads();
         if (k0 + kSkBK < K) load(k0 + kSkBK);
 #pragma unroll 8
         for (int k = 0; k < kSkBK; ++k) {
-            const double *xs = Xs + k * LD + tr * RPT;
-            const double2 b = *reinterpret_cast<const double2 *>(Bs + k * 16 + 2 * tc);
+            const double x = Xs[k * LD + row];
 #pragma unroll
-            for (int i = 0; i < RPT; ++i) {
-                const double x = xs[i];
-                acc[i][0] = fma(x, b.x, acc[i][0]);
-                acc[i][1] = fma(x, b.y, acc[i][1]);
-            }
+            for (int j = 0; j < NC; ++j) acc[j] = fma(x, Bs[k * 2 * NC + c0 + j], acc[j]);
         }
         __syncthreads();
     }
+    if (r0 + row >= rows) return;
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-        const ll r = r0 + tr * RPT + i;
-        if (r >= rows) continue;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-            if (2 * tc + j < N) C[r * N + 2 * tc + j] = acc[i][j];
-    }
-}
-
-// The same product on the FP64 tensor cores: mma.sync m8n8k4 (DMMA).  CTA
-// tile 128 x 16 as above (X staged transposed, B as [k][16] in shared
-// memory); warp w owns rows 16w .. 16w+15 as two 8-row blocks times two 8-col
-// blocks, four accumulators of two doubles per lane.  Fragments (PTX m8n8k4
-// .f64): A a0 = A[lane/4][lane%4], B b0 = B[lane%4][lane/4], C c0,c1 =
-// C[lane/4][2(lane%4) + {0,1}].
-__global__ void __launch_bounds__(256, 2) k_dgemm_skinny_dmma(SkinnyJobs jobs, ll rows, int N, int K) {
-    if (jobs.flag && !*jobs.flag) return;
-    constexpr int BM = 128, LD = BM + 1, NX = BM / 8;
-    __shared__ double Xs[kSkBK * LD];
-    __shared__ __align__(16) double Bs[kSkBK * 16];
-    const int jb = blockIdx.y;
-    const double *__restrict__ X = jb == 0 ? jobs.X[0] : jb == 1 ? jobs.X[1] : jb == 2 ? jobs.X[2] : jobs.X[3];
-    const double *__restrict__ B = jb == 0 ? jobs.B[0] : jb == 1 ? jobs.B[1] : jb == 2 ? jobs.B[2] : jobs.B[3];
-    double *__restrict__ C = jb == 0 ? jobs.C[0] : jb == 1 ? jobs.C[1] : jb == 2 ? jobs.C[2] : jobs.C[3];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const ll r0 = (ll)blockIdx.x * BM;
-    const int lk = tid & 31, lr = tid >> 5;
-    double xr[NX], br[2];
-    auto load = [&](int k0) {
-        const int k = k0 + lk;
-#pragma unroll
-        for (int i = 0; i < NX; ++i) {
-            const ll r = r0 + lr + 8 * i;
-            xr[i] = (r < rows && k < K) ? X[r * K + k] : 0.0;
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int e = tid + 256 * i, kk = e >> 4, c = e & 15;
-            br[i] = (c < N && k0 + kk < K) ? B[(ll)(k0 + kk) * N + c] : 0.0;
-        }
-    };
-    double acc[2][2][2] = {};  // [m block][n block][c0, c1]
-    const int g = lane >> 2, q = lane & 3;
-    load(0);
-    for (int k0 = 0; k0 < K; k0 += kSkBK) {
-#pragma unroll
-        for (int i = 0; i < NX; ++i) Xs[lk * LD + lr + 8 * i] = xr[i];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) Bs[tid + 256 * i] = br[i];
-        __syncthreads();
-        if (k0 + kSkBK < K) load(k0 + kSkBK);
-#pragma unroll
-        for (int kk = 0; kk < kSkBK; kk += 4) {
-            double a[2], b[2];
-#pragma unroll
-            for (int mb = 0; mb < 2; ++mb) a[mb] = Xs[(kk + q) * LD + warp * 16 + mb * 8 + g];
-#pragma unroll
-            for (int nb = 0; nb < 2; ++nb) b[nb] = Bs[(kk + q) * 16 + nb * 8 + g];
-#pragma unroll
-            for (int mb = 0; mb < 2; ++mb)
-#pragma unroll
-                for (int nb = 0; nb < 2; ++nb)
-                    asm volatile(
-                        "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                        : "+d"(acc[mb][nb][0]), "+d"(acc[mb][nb][1])
-                        : "d"(a[mb]), "d"(b[nb]));
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int mb = 0; mb < 2; ++mb) {
-        const ll r = r0 + warp * 16 + mb * 8 + g;
-        if (r >= rows) continue;
-#pragma unroll
-        for (int nb = 0; nb < 2; ++nb)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int col = nb * 8 + 2 * q + i;
-                if (col < N) C[r * N + col] = acc[mb][nb][i];
-            }
-    }
-}
-
-// variant: 2, 4 = DFMA register blocks of 2 or 4 rows per thread; 1 = DMMA
-static void launch_skinny(int rpt, cudaStream_t st, const SkinnyJobs &j, ll rows, int N, int K) {
-    if (rpt == 1) {
-        dim3 grid((unsigned)((rows + 127) / 128), 4);
-        k_dgemm_skinny_dmma<<<grid, 256, 0, st>>>(j, rows, N, K);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        return;
-    }
-    const ll bm = 32LL * rpt;
-    dim3 grid((unsigned)((rows + bm - 1) / bm), 4);
-    if (rpt == 2) k_dgemm_skinny<2><<<grid, 256, 0, st>>>(j, rows, N, K);
-    else k_dgemm_skinny<4><<<grid, 256, 0, st>>>(j, rows, N, K);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    for (int j = 0; j < NC; ++j)
+        if (c0 + j < N) C[(r0 + row) * N + c0 + j] = acc[j];
 }
 
 static int dgemm_skinny4(cudaStream_t st, ll rows, int N, int K, const double *const X[4], const double *const B[4],
@@ -525,16 +430,17 @@ static int dgemm_skinny4(cudaStream_t st, ll rows, int N, int K, const double *c
         j.B[i] = B[i];
         j.C[i] = C[i];
     }
-    // Four rows per thread while there are few row tiles, two at the largest
-    // shapes (65536 x 4096 x 16: 27.6 ms with two, 28.6 with four, 32.5 on the
-    // FP64 tensor cores); NVPT_SKINNY_VARIANT (1, 2, 4) fixes the variant
-    // (tests of each).
-    static const int forced = [] {
-        const char *e = std::getenv("NVPT_SKINNY_VARIANT");
-        const int v = e ? std::atoi(e) : 0;
-        return (v == 1 || v == 2 || v == 4) ? v : 0;
-    }();
-    launch_skinny(forced ? forced : rows >= 65536 ? 2 : 4, st, j, rows, N, K);
+    const dim3 grid((unsigned)((rows + kSkBM - 1) / kSkBM), 4);
+    switch ((N + 1) / 2) {  // N > 5: the direct kernel takes the smaller sizes
+        case 3: k_dgemm_skinny<3><<<grid, 128, 0, st>>>(j, rows, N, K); break;
+        case 4: k_dgemm_skinny<4><<<grid, 128, 0, st>>>(j, rows, N, K); break;
+        case 5: k_dgemm_skinny<5><<<grid, 128, 0, st>>>(j, rows, N, K); break;
+        case 6: k_dgemm_skinny<6><<<grid, 128, 0, st>>>(j, rows, N, K); break;
+        case 7: k_dgemm_skinny<7><<<grid, 128, 0, st>>>(j, rows, N, K); break;
+        case 8: k_dgemm_skinny<8><<<grid, 128, 0, st>>>(j, rows, N, K); break;
+        default: return 1;
+    }
+    g_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
 }
 
@@ -565,7 +471,15 @@ __global__ void k_slab_list(int n, int *cp, int *ap);
 // n = 10 1.42 / 1.69 ms, n = 11 2.75 / 2.74, n = 12 5.4 / 4.5, n = 14 19.4 / 12.8, n = 16
 // 52.6 / 32.4).
 constexpr int kSplitMinNact = 11;
-constexpr unsigned kSlabCtas = 152 * 16;  // CTAs of a slab launch: one wave or so, looping
+
+// CTAs of k_bamat_slabs_t that are resident at once.
+static int slab_ctas(size_t smem) {
+    int per = 1, sms = 1, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bamat_slabs_t, 256, smem);
+    return std::max(1, sms * per);
+}
 
 // Returns 0 on success, 2 on a failed allocation, 5 if a split-precision
 // product timed out, else a launch failure.
@@ -620,13 +534,15 @@ int launch_bamat(const Rdm &r, const double *atwo, const double *f, int ncore, d
     g_launches.fetch_add(2, std::memory_order_relaxed);
     unsigned long long *rmax = nullptr;  // row maxima of the four slab layouts (split digits)
     if (split && !buf.get(&rmax, sizeof(unsigned long long) * 4 * (size_t)B * n3)) return 2;
+    const size_t smem = sizeof(double) * (size_t)(slab_tile(n) + n2);
+    const int ctas = slab_ctas(smem);
     for (int s = 0; s < M; ++s) {
         for (int s0 = 0; s0 < n2; s0 += B) {
             const int nb = std::min(B, (int)n2 - s0);
             const ll rows = (ll)nb * n3;
             const double *Xs[4] = {X, X + (ll)B * n6, X + 2 * (ll)B * n6, X + 3 * (ll)B * n6}, *As[4] = {A1, A2, A3, A3};
             if (rmax) cudaMemsetAsync(rmax, 0, sizeof(unsigned long long) * 4 * (size_t)rows, st);
-            k_bamat_slabs_t<<<(unsigned)std::min<ll>(rows, kSlabCtas), 256, 0, st>>>(
+            k_bamat_slabs_t<<<(unsigned)std::min<ll>(rows, ctas), 256, smem, st>>>(
                 r, s, slabs + s0, slabs + n2 + s0, nb, X, X + (ll)B * n6, X + 2 * (ll)B * n6, X + 3 * (ll)B * n6, rmax,
                 flag + s);
             g_launches.fetch_add(1, std::memory_order_relaxed);

@@ -100,7 +100,9 @@ __global__ void __launch_bounds__(256) k_sym_ops(const double *atwo, const doubl
 __global__ void __launch_bounds__(256) k_sym_unpack(Rdm r, int s, const int *key, unsigned nub, double *H, int *flag) {
     const int n = r.n;
     const ll n2 = (ll)n * n, n3 = n2 * n, n4 = n2 * n2, W = r.W;
-    const double tol = rdm_tolerance(r, s);
+    bool raised;
+    const double tol = rdm_tolerance(r, s, flag, raised);
+    if (raised) return;  // the state's H is not used
     if (blockIdx.x >= nub) {
         const ll t = (ll)(blockIdx.x - nub) * blockDim.x + threadIdx.x;
         if (t < n3 * n3 && rdm_asymmetric(r, s, t, tol)) flag[s] = 1;

@@ -48,10 +48,12 @@ __host__ __device__ __forceinline__ int ord8_key(int a1, int c1, int e1, int g1,
 #pragma unroll
         for (int j = i + 1; j < 4; ++j)
             if (k[j] > imax) { imax = k[j]; jmax = j; }
-        if (jmax != i) {
-            int t = k[i]; k[i] = k[jmax]; k[jmax] = t;
-            t = p[i]; p[i] = p[jmax]; p[jmax] = t;
-        }
+#pragma unroll
+        for (int j = i + 1; j < 4; ++j)
+            if (jmax == j) {  // static indices: the arrays stay in registers
+                int t = k[i]; k[i] = k[j]; k[j] = t;
+                t = p[i]; p[i] = p[j]; p[j] = t;
+            }
     }
     p0 = p[0]; p1 = p[1]; p2 = p[2]; p3 = p[3];
     return lindice4(k[0], k[1], k[2], k[3]);

@@ -49,10 +49,12 @@ __global__ void __launch_bounds__(256) k_ks_prep(Rdm r, const double *__restrict
                                                  int *flag) {
     const int n = r.n, s = blockIdx.y, np = n * (n + 1) / 2;
     const ll n2 = (ll)n * n, n4 = n2 * n2, n6 = n4 * n2;
-    const double tol = rdm_tolerance(r, s);
+    bool raised;
+    const double tol = rdm_tolerance(r, s, flag, raised);
     const ll t0 = (ll)blockIdx.x * blockDim.x + threadIdx.x, step = (ll)gridDim.x * blockDim.x;
     bool bad = false;
-    for (ll t = t0; t < n6; t += step) bad = rdm_asymmetric(r, s, t, tol) || bad;
+    if (!raised)
+        for (ll t = t0; t < n6; t += step) bad = rdm_asymmetric(r, s, t, tol) || bad;
     if (bad) flag[s] = 1;
     if (blockIdx.y) return;
     for (ll t = t0; t < n4; t += step) {

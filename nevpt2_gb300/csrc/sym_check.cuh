@@ -24,14 +24,16 @@ __device__ __forceinline__ void unpair(int p, int &i, int &j) {  // p = pidx(i, 
 // pipe (16 clocks a warp), and every block takes its own scale.
 __device__ __forceinline__ unsigned abs_hi(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
 
-// Tolerance of the RDM checks of state s (0-based): all threads of the block.
-__device__ __forceinline__ double rdm_tolerance(const Rdm &r, int s) {
+// Tolerance of the RDM checks of state s (0-based): all threads of the block.  raised:
+// whether the state's flag was raised already.
+__device__ __forceinline__ double rdm_tolerance(const Rdm &r, int s, const int *flag, bool &raised) {
+    const bool seen = threadIdx.x == 0 && *(volatile const int *)(flag + s) != 0;
     __shared__ unsigned red[8];
     unsigned m = 0;
     for (int i = threadIdx.x; i < r.n * r.n; i += blockDim.x) m = max(m, abs_hi(r.d1[s + (ll)r.M * i]));
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    __syncthreads();
+    raised = __syncthreads_or(seen);
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = max(m, red[w]);
     return kSymTol * __hiloint2double((int)m, 0);
 }

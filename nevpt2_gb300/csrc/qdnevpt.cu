@@ -244,14 +244,14 @@ T eri(Ctx &c, const T &X, const T &Y) {
 struct PcResult {
     T C;       // [nd, nd]: columns mu < nnew are the PC coefficients, rest zero
     T w;       // [nd] reference layout (first nnew: K~ eigenvalues)
-    int nnew;
+    int nnew = 0;
 };
 
 // src/qdnevpt.F:1963-2033 and siblings: the PC metric sequence.
-PcResult pc_transform(Ctx &c, const T &S, const T &K, long long nd, double thr) {
+PcResult pc_transform(Ctx &c, const double *S, const double *K, long long nd, double thr) {
     PcResult r;
     T w = alloc(c, {nd}, false), V = alloc(c, {nd, nd}, false);
-    eigh_upper(c, S.p, nd, w.p, V.p);
+    eigh_upper(c, S, nd, w.p, V.p);
     std::vector<double> wh(nd);
     ck(cudaMemcpyAsync(wh.data(), w.p, sizeof(double) * nd, cudaMemcpyDeviceToHost, c.st), "w copy");
     ck(cudaStreamSynchronize(c.st), "sync");
@@ -282,7 +282,7 @@ PcResult pc_transform(Ctx &c, const T &S, const T &K, long long nd, double thr) 
         cauxT = std::move(tmp);
     }
     T Ks = alloc(c, {nd, nd}, false);
-    symmetrize_upper(c, K.p, nd, Ks.p);
+    symmetrize_upper(c, K, nd, Ks.p);
     // Y = K caux  (nd x nnew);  Tm = caux^T Y  (nnew x nnew)
     T Y = alloc(c, {nd, nnew}, false);
     gemm(c, false, true, nd, nnew, nd, 1.0, Ks.p, nd, cauxT.p, nd, 0.0, Y.p, nnew);
@@ -492,16 +492,15 @@ class CtxPool {
     std::map<int, std::vector<Ctx>> free_;
 };
 
-// The reduction of one pencil K v = w S v on a helper stream and host thread:
-// the Cholesky check of the metric, its factorisation, the reduction to
-// standard form and the tridiagonalisation need only S and K, so they overlap
-// the caller's work on its own stream.  join(to) waits for them, orders the
-// stream of `to` after the helper's and hands the pencil's buffers to it (where
-// they are used and freed from then on).
+// One pencil K v = w S v on a helper stream and host thread: its reduction, or where the
+// metric drops eigenvalues the eigenpair sequence.  Both need only S and K, so they overlap
+// the caller's work on its own stream.  join(to) waits for them, orders the stream of `to`
+// after the helper's and hands the pencil's buffers to it (where they are used and freed
+// from then on).
 class PencilFork {
   public:
-    PencilFork(Ctx &caller, const T &S, const T &K, long long n, double thr, PencilTridiag &pt)
-        : c_(&caller), pt_(pt) {
+    PencilFork(Ctx &caller, const T &S, const T &K, long long n, double thr, PencilTridiag &pt, PcResult &eig)
+        : c_(&caller), pt_(pt), eig_(eig) {
         ck(cudaGetDevice(&dev_), "cudaGetDevice");
         aux_ = CtxPool::acquire(1, dev_);
         Ctx &a = aux_[0];
@@ -523,6 +522,10 @@ class PencilFork {
             try {
                 ck(cudaSetDevice(dev_), "cudaSetDevice");
                 ok_ = pencil_tridiag(aux_[0], Kp, Sp, n, thr, pt_);
+                if (!ok_) {
+                    pt_ = PencilTridiag{};
+                    eig_ = pc_transform(aux_[0], Sp, Kp, n, thr);
+                }
             } catch (...) {
                 err_ = std::current_exception();
             }
@@ -530,7 +533,8 @@ class PencilFork {
     }
     PencilFork(const PencilFork &) = delete;
     PencilFork &operator=(const PencilFork &) = delete;
-    // true when the metric kept every eigenvalue and the pencil is reduced
+    // true when the metric kept every eigenvalue but null ones and the pencil is reduced, false
+    // when its eigenpairs are there instead
     bool join(Ctx &to) {
         c_ = &to;
         finish();
@@ -550,7 +554,7 @@ class PencilFork {
         } else {
             cudaStreamSynchronize(a.st);
         }
-        for (T *t : {&pt_.W, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm, &pt_.d, &pt_.e}) t->st = c_->st;
+        for (T *t : {&pt_.W, &pt_.N, &pt_.AB, &pt_.V, &pt_.Tm, &pt_.d, &pt_.e, &eig_.C, &eig_.w}) t->st = c_->st;
         a.split = false;
         a.oz_err = nullptr;
         a.wait_limit = 0;
@@ -562,6 +566,7 @@ class PencilFork {
     }
     Ctx *c_;
     PencilTridiag &pt_;
+    PcResult &eig_;
     int dev_ = 0;
     std::vector<Ctx> aux_;
     cudaEvent_t ready_ = nullptr, done_ = nullptr;
@@ -578,6 +583,7 @@ class PencilFork {
 struct Pencil1p {
     T S, K;
     PencilTridiag PT;
+    PcResult eig;
     std::unique_ptr<PencilFork> fork;
     void start(Ctx &c, const StateData &D, int n, bool minus, double thr) {
         const int n3 = n * n * n;
@@ -592,7 +598,7 @@ struct Pencil1p {
         // W3 = eee2(t)(cp,ap,bp,b,a,c) transposed: [(a,b,c),(ap,bp,cp)]
         S = view2(permuted(c, E3, {4, 3, 5, 1, 2, 0}), n3, n3);
         K = view2(permuted(c, minus ? D.aIP : D.aEA, {3, 4, 5, 0, 1, 2}), n3, n3);
-        fork.reset(new PencilFork(c, S, K, n3, thr, PT));
+        fork.reset(new PencilFork(c, S, K, n3, thr, PT, eig));
     }
 };
 
@@ -1011,7 +1017,7 @@ class Runner {
         T S = copy_of(c, ro.p, {n, n});
         T Kk = alloc(c, {n, n}, false);
         axpby(c, (long long)n * n, 0.5, gk_.p, 0.0, nullptr, Kk.p);
-        PcResult P = pc_transform(c, S, Kk, n, thr);
+        PcResult P = pc_transform(c, S.p, Kk.p, n, thr);
         acc.nnew[(plus ? 0 : 1) + 10 * s] = P.nnew;
         // own: s(a,mu) = sum_ap X[ap,a] C[ap,mu]  (X = 2-g1 or g1)
         T sm = matmul(c, ro, true, P.C, false);  // [n, n]
@@ -1204,7 +1210,7 @@ class Runner {
                 }
             });
             if (!res) {
-                PcResult P = pc_transform(c, S, K, n2, thr);
+                PcResult P = pc_transform(c, S.p, K.p, n2, thr);
                 acc.nnew[(plus ? 2 : 4) + 10 * s] = P.nnew;
                 T sm = matmul(c, S, true, P.C, false);  // s(ab,mu) = sum_{pq} D[pq,ab] C[pq,mu]
                 T R = matmul(c, V, false, sm, false);
@@ -1263,7 +1269,7 @@ class Runner {
                 }
             });
             if (!res) {
-                PcResult P = pc_transform(c, Sp, Kp, np, thr);
+                PcResult P = pc_transform(c, Sp.p, Kp.p, np, thr);
                 acc.nnew[(plus ? 3 : 5) + 10 * s] = P.nnew;
                 // s(ab,mu) = sum_{abp} 0.5 Sf[abp, ab] C[abp, mu]
                 T smp = matmul(c, Sp, true, P.C, false);
@@ -1467,7 +1473,7 @@ class Runner {
             if (nrho) store_rho(download(c, rho.p, L));
             return;
         }
-        PcResult P = pc_transform(c, S, K, n2, thr);
+        PcResult P = pc_transform(c, S.p, K.p, n2, thr);
         acc.nnew[8 + 10 * s] = P.nnew;
         // aux: s = val C_top, sp = val C_bot, spp = val2 C_bot (val = Snw as [ab,abp])
         T Ctop = alloc(c, {(long long)nn, n2}, false), Cbot = alloc(c, {(long long)nn, n2}, false);
@@ -1720,9 +1726,12 @@ class Runner {
         PencilTridiag &PT = pen->PT;
         const bool reduced = pen->fork->join(c);
         struct Release {  // the form's buffers, on this stream
-            PencilTridiag &p;
-            ~Release() { p = PencilTridiag{}; }
-        } release{PT};
+            Pencil1p &p;
+            ~Release() {
+                p.PT = PencilTridiag{};
+                p.eig = PcResult{};
+            }
+        } release{*pen};
         if (reduced) {
             // Every metric eigenvalue but exact zeros is kept: the PC sums over
             // the eigenpairs of K v = w S v are resolvents of the pencil,
@@ -1779,7 +1788,7 @@ class Runner {
             pc_accum(e2, psi2, resolvent_sums(PT, Yt, pb, nd, (long long)M * L, rho.p));
             if (nd) store_rho(download(c, rho.p, L * nd));
         } else {
-            PcResult P = pc_transform(c, pen->S, pen->K, n3, thr);
+            const PcResult &P = pen->eig;
             acc.nnew[(minus ? 7 : 6) + 10 * s] = P.nnew;
             // R[l, mu] = sum_x Z[l, x] C[x, mu]: the order-n3 products S C and
             // W2t C of the reference are reassociated onto the L rows.

@@ -436,9 +436,9 @@ bool metric_null(Ctx &c, const double *S, long long n, double thr, T &N, long lo
     ck(cudaMemcpyAsync(L.p, S, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, c.st), "copy");
     k_shift_diag<<<1, TPB, 0, c.st>>>(L.p, n, 1e-11, top.p);
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    double tr = 0.0, st[2], big = 0.0;
+    double tr = 0.0, st[2], big = 0.0, shifted = 0.0;
     ck(cudaMemcpyAsync(&big, top.p, sizeof(double), cudaMemcpyDeviceToHost, c.st), "diagonal");
-    if (!spd_inverse_factor(c, L.p, n, W.p, tr) || !(big > 0.0)) return false;  // synchronises
+    if (!spd_inverse_factor(c, L.p, n, W.p, tr, shifted) || !(big > 0.0)) return false;  // synchronises
     const double null = 1e-12 * big;
     if (!(thr >= null)) return false;
     const double count = tr * 1e-11 * big;
@@ -482,17 +482,23 @@ bool pencil_tridiag(Ctx &c, const double *K, const double *S, long long n, doubl
     const long long ld = spd_ld(n);
     P.W = alloc(c, {ld, ld}, false);
     ProfSpan sp;
-    // every eigenvalue above thr: by tr S^-1 >= 1 / the smallest, or else by S - thr
+    // Every eigenvalue above thr, by the smallest one's bounds 1 / tr S^-1 and n / tr S^-1
+    // where they decide (the factor 2 is for the rounding of tr), else by S - thr.  null:
+    // whether some may be null, which none is while 1 / tr S^-1 is above that line.
+    bool null = false;
     auto factor = [&](const double *M) {
-        double tr = 0.0;
+        double tr = 0.0, top = 0.0;
         sp.begin("pencil_potrf", c.st, 0);
-        const bool ok = spd_inverse_factor(c, M, n, P.W.p, tr);
+        const bool ok = spd_inverse_factor(c, M, n, P.W.p, tr, top);
         sp.end();
-        return ok && ((thr >= 0.0 && tr * thr <= 0.999) || metric_above(c, M, n, thr));
+        null = !ok || !(2e-12 * top * tr < 1.0);
+        if (!ok || tr * thr > 2.0 * n) return false;
+        return (thr >= 0.0 && tr * thr <= 0.999) || metric_above(c, M, n, thr);
     };
     T S2, K2;
     const double *Kp = K;
     if (!factor(S)) {
+        if (!null) return false;
         S2 = alloc(c, {n, n}, false);
         symmetrize_upper(c, S, n, S2.p);
         if (!metric_null(c, S2.p, n, thr, P.N, P.k)) return false;

@@ -275,7 +275,9 @@ __global__ void __launch_bounds__(TP) k_spd_step(double *L, double *W, long long
         }
 }
 
-__global__ void __launch_bounds__(TP) k_spd_norm(const double *__restrict__ W, int n, long long ld, double *out) {
+// out[0] += |row i of W|^2, out[2] = max(out[2], S_ii), a row a block.
+__global__ void __launch_bounds__(TP) k_spd_norm(const double *__restrict__ W, const double *__restrict__ S, int n,
+                                                 long long ld, double *out) {
     __shared__ double red[TP / 32];
     double v = 0.0;
     const int i = blockIdx.x;
@@ -289,6 +291,8 @@ __global__ void __launch_bounds__(TP) k_spd_norm(const double *__restrict__ W, i
     if (threadIdx.x == 0) {
         for (int w = 1; w < TP / 32; ++w) v += red[w];
         atomicAdd(out, v);
+        const double d = S[(long long)i * n + i];  // magnitudes order like their bits
+        if (d > 0.0) atomicMax((unsigned long long *)(out + 2), (unsigned long long)__double_as_longlong(d));
     }
 }
 
@@ -363,7 +367,7 @@ void spd_inverse_factor_async(Ctx &c, const double *S, long long n, double *W, d
         if (t)
             k_spd_step<<<grid, TP, grid <= kStepAlone ? kAloneSmem : sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, (int)n, bad);
     }
-    if (trace) k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, (int)n, ld, stat);
+    if (trace) k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, S, (int)n, ld, stat);
     g_launches.fetch_add(2 * nb - 1 + (trace ? 1 : 0), std::memory_order_relaxed);
     ck(cudaGetLastError(), "inverse factor");
 }
@@ -374,13 +378,14 @@ bool spd_failed(const double *stat_on_host) {
     return failed != 0;
 }
 
-bool spd_inverse_factor(Ctx &c, const double *S, long long n, double *W, double &inv_trace) {
-    T stat = alloc(c, {2}, true);  // |W|^2, bad pivot
+bool spd_inverse_factor(Ctx &c, const double *S, long long n, double *W, double &inv_trace, double &top) {
+    T stat = alloc(c, {3}, true);  // |W|^2, bad pivot, largest diagonal element
     spd_inverse_factor_async(c, S, n, W, stat.p, true);
-    double h[2];
+    double h[3];
     ck(cudaMemcpyAsync(h, stat.p, sizeof(h), cudaMemcpyDeviceToHost, c.st), "status copy");
     ck(cudaStreamSynchronize(c.st), "inverse factor sync");
     inv_trace = h[0];
+    top = h[2];
     return !spd_failed(h);
 }
 

@@ -3,16 +3,17 @@
 //
 // The reference loops over (a,b,c,ap,bp,cp) and scatters part of the EA
 // contribution into the b<->bp transposed element atmat(ap,b,cp,a,bp,c).  Here
-// a group of kLanes threads owns one output element O = (ap,bp,cp,a,b,c) of both
+// a group of LANES threads owns one output element O = (ap,bp,cp,a,b,c) of both
 // amat and atmat: it evaluates the iteration (a,b,c,ap,bp,cp) for amat and for the
 // non-transposed atmat terms, and the mirror iteration (a,bp,c,ap,b,cp) for the
 // transposed atmat terms, so there is no atomic and no race.
 //
 // Bound by latency: a chain of n^3 rounds of gathers a thread, and few threads (n =
-// 4: 4096 elements), so the (d, e) pairs are dealt to kLanes of them.  One state, the
-// call, one thread / four: n = 3 241 / 75 us, n = 4 498 / 192, n = 5 989 / 622.  Blocks
-// of 512 from n = 5 on, or the symmetric states, for which every block returns at
-// once, pay 2 us for their number.
+// 4: 4096 elements), so the (d, e) pairs are dealt to LANES of them: eight below n = 5,
+// where elements are few; four in blocks of TB = 512 at n = 5, or the symmetric
+// states, for which every block returns at once, pay 2 us for the number of blocks.
+// One state, the call, one thread / now: n = 2 97 / 52 us, n = 3 235 / 84, n = 4 502 / 124,
+// n = 5 992 / 621.
 #include "nvpt2_internal.h"
 
 namespace nvpt {
@@ -20,13 +21,12 @@ namespace nvpt {
 #define ATWO(i, j, k, l) atwo[((i)-1) + (ll)n * (((j)-1) + (ll)n * (((k)-1) + (ll)n * ((l)-1)))]
 #define FF(i, j) f[tri_index((i) + ncore, (j) + ncore) - 1]
 
-constexpr int kLanes = 4;
-
-__global__ void __launch_bounds__(512) k_bamat_direct(Rdm r, const double *atwo, const double *f, int ncore,
+template <int LANES, int TB>
+__global__ void __launch_bounds__(TB) k_bamat_direct(Rdm r, const double *atwo, const double *f, int ncore,
                                                       double *amat, double *atmat, const int *flag) {
     const int n = r.n, M = r.M;
-    const ll g = ((ll)blockIdx.x * blockDim.x + threadIdx.x) / kLanes, n6 = (ll)n * n * n * n * n * n;
-    const int lane = threadIdx.x % kLanes;
+    const ll g = ((ll)blockIdx.x * blockDim.x + threadIdx.x) / LANES, n6 = (ll)n * n * n * n * n * n;
+    const int lane = threadIdx.x % LANES;
     const ll t = min(g, n6 - 1);
     ll x = t;
     const int ap = (int)(x % n) + 1; x /= n;
@@ -38,14 +38,14 @@ __global__ void __launch_bounds__(512) k_bamat_direct(Rdm r, const double *atwo,
     for (int s = 1; s <= M; ++s) {
         if (flag && !flag[s - 1]) continue;
         double A = 0.0, At = 0.0;
-        for (int d = lane + 1; d <= n; d += kLanes) {
+        for (int d = lane + 1; d <= n; d += LANES) {
             double fda = FF(d, a), fcd = FF(c, d), fbd = FF(b, d);
             A += fda * r.eee2(cp, ap, bp, b, d, c, s) - fcd * r.eee2(cp, ap, bp, b, a, d, s) -
                  fbd * r.eee2(cp, ap, bp, d, a, c, s);
             At += fda * r.eee2t(cp, ap, bp, b, d, c, s) - fcd * r.eee2t(cp, ap, bp, b, a, d, s) +
                   fbd * r.eee2t(cp, ap, bp, d, a, c, s);
         }
-        for (int q = lane; q < n * n; q += kLanes) {
+        for (int q = lane; q < n * n; q += LANES) {
             const int d = q / n + 1, ie = q % n + 1;
             double dint1 = ATWO(c, ie, d, a), dint2 = ATWO(d, ie, ie, a);
             double dint3 = ATWO(c, d, d, ie), dint4 = ATWO(b, d, d, ie);
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(512) k_bamat_direct(Rdm r, const double *atwo,
                 At += e1t * di1 - e2t * di2;
             }
         }
-        for (int o = kLanes / 2; o; o >>= 1) {
+        for (int o = LANES / 2; o; o >>= 1) {
             A += __shfl_xor_sync(0xffffffffu, A, o);
             At += __shfl_xor_sync(0xffffffffu, At, o);
         }
@@ -94,8 +94,11 @@ __global__ void __launch_bounds__(512) k_bamat_direct(Rdm r, const double *atwo,
 void launch_bamat_direct(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
                          cudaStream_t st, const int *flag) {
     ll n6 = (ll)r.n * r.n * r.n * r.n * r.n * r.n;
-    const int tb = r.n < 5 ? 128 : 512;
-    k_bamat_direct<<<(unsigned)((kLanes * n6 + tb - 1) / tb), tb, 0, st>>>(r, atwo, f, ncore, amat, atmat, flag);
+    auto go = [&](auto k, int lanes, int tb) {
+        k<<<(unsigned)((lanes * n6 + tb - 1) / tb), tb, 0, st>>>(r, atwo, f, ncore, amat, atmat, flag);
+    };
+    if (r.n < 5) go(k_bamat_direct<8, 128>, 8, 128);
+    else go(k_bamat_direct<4, 512>, 4, 512);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 

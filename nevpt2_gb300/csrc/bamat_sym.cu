@@ -625,7 +625,8 @@ __global__ void __launch_bounds__(kOutTb) k_sym_out(SymView v, double *amat, dou
 #undef AT
 
 // Values of b per CTA of k_sym_f and rows per thread: the split with the least
-// idle row slots whose tile leaves two CTAs per SM (at most 72 KB of X).
+// idle row slots whose tile leaves two CTAs per SM (at most 72 KB of X).  Rows per
+// thread: 2 at n = 10 and 12, 5 at n = 13, 4 at n = 14, 1 at the other sizes.
 struct FShape {
     int bc = 1, rpt = 1;
 };
@@ -652,10 +653,8 @@ FKernel f_kernel(int rpt) {
     switch (rpt) {
         case 1: return k_sym_f<1>;
         case 2: return k_sym_f<2>;
-        case 3: return k_sym_f<3>;
         case 4: return k_sym_f<4>;
-        case 5: return k_sym_f<5>;
-        default: return k_sym_f<6>;
+        default: return k_sym_f<5>;
     }
 }
 

@@ -7,7 +7,7 @@
 
 namespace nvpt {
 
-constexpr int kSymMaxRpt = 6;  // rows per thread of the n^9 product
+constexpr int kSymMaxRpt = 5;  // rows per thread of the n^9 product
 
 // Views into one scratch block of doubles(n) doubles, reused for every state.
 struct SymScratch {

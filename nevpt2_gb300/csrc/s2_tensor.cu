@@ -407,7 +407,8 @@ __global__ void k_dot_abs(const double *X, const double *Y, long long n, double 
     }
 }
 
-// Deterministic start vectors of the inverse iteration, in [-0.5, 0.5).
+// Deterministic start vectors of the inverse iteration, in [-0.5, 0.5): the outputs of
+// Steele, Lea and Flood's SplitMix64 generator (OOPSLA 2014) at the element's index.
 __global__ void k_start_block(double *X, long long count) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;

@@ -342,10 +342,11 @@ __global__ void __launch_bounds__(TP) k_spd_k(const double *__restrict__ W, cons
         }
 }
 
-// A step of at most this many blocks is as long as its first one (update and factorisation
-// of the next diagonal block), which is slowed by a block beside it on its SM: these steps
-// ask for so much shared memory that none is (order 512 165 -> 127 us, order 1000 192 -> 146).
-constexpr int kStepAlone = 3 * 152;
+// A step of at most this many blocks an SM is as long as its first one (update and
+// factorisation of the next diagonal block), which is slowed by a block beside it on its SM:
+// these steps ask for so much shared memory that none is (order 512 165 -> 127 us, order 1000
+// 192 -> 146).
+constexpr int kStepAlone = 3;
 constexpr size_t kAloneSmem = 120 * 1024;
 
 unsigned blocks(long long count) { return (unsigned)((count + TP - 1) / TP); }
@@ -359,13 +360,16 @@ void spd_inverse_factor_async(Ctx &c, const double *S, long long n, double *W, d
     int *bad = (int *)(stat + 1);
     raise_dynamic_smem((const void *)k_spd_load);
     raise_dynamic_smem((const void *)k_spd_step);
+    int sms = 0, dev = 0;
+    ck(cudaGetDevice(&dev), "cudaGetDevice");
+    ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr");
     k_spd_load<<<1 + blocks(ld * ld), TP, sizeof(Diag), c.st>>>(S, (int)n, ld, L.p, W, bad);
     for (int k = 0; k < nb; ++k) {
         const int t = nb - 1 - k;
         if (t + k) k_spd_panel<<<4 * (t + k), TP, 0, c.st>>>(L.p, W, ld, k, nb, bad);
         const int grid = 2 * (t * (t + 1) / 2 + t * (k + 1)) - 1;
         if (t)
-            k_spd_step<<<grid, TP, grid <= kStepAlone ? kAloneSmem : sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, (int)n, bad);
+            k_spd_step<<<grid, TP, grid <= kStepAlone * sms ? kAloneSmem : sizeof(Diag), c.st>>>(L.p, W, ld, k, nb, (int)n, bad);
     }
     if (trace) k_spd_norm<<<(unsigned)n, TP, 0, c.st>>>(W, S, (int)n, ld, stat);
     g_launches.fetch_add(2 * nb - 1 + (trace ? 1 : 0), std::memory_order_relaxed);

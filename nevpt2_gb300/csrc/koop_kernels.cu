@@ -367,9 +367,10 @@ __device__ __forceinline__ void koop_contract(const Rdm &r, int s, const double 
     const int n = t.n, R = t.R, lda = R + 1, tid = threadIdx.x, K = n * n * n;
     int s1, s2, s3, sx;
     koop_strides<OP>(n, s1, s2, s3, sx);
-    // threads: column, row group, and -- when one row per thread leaves room -- a share of the k's
+    // threads: column, row group, and -- when one row per thread leaves room -- a share of the k's,
+    // no more shares than k's: they are added up one after another (n = 1: 256 of them took 100 us)
     const int groups = 256 / n, rpt = (R + groups - 1) / groups;
-    const int slices = rpt == 1 ? 256 / (R * n) : 1, per = rpt == 1 ? R * n : 256;
+    const int slices = rpt == 1 ? min(256 / (R * n), K) : 1, per = rpt == 1 ? R * n : 256;
     const int slice = tid / per, q = tid % per, col = q % n, grp = q / n;
     const bool live = slice < slices && grp < groups && (rpt > 1 || grp < R);
     double acc[kKoopRpt] = {};

@@ -471,6 +471,10 @@ __global__ void k_slab_list(int n, int *cp, int *ap);
 // n = 10 1.42 / 1.69 ms, n = 11 2.75 / 2.74, n = 12 5.4 / 4.5, n = 14 19.4 / 12.8, n = 16
 // 52.6 / 32.4).
 constexpr int kSplitMinNact = 11;
+// Up to this many active orbitals the direct kernel takes every state: the symmetric route
+// is nine launches there (symmetric inputs, the call, symmetric route / direct kernel, us:
+// n = 2 59 / 27, n = 3 71 / 54, n = 4 75 / 87; at n = 1 the route had cost the host call 6 us).
+constexpr int kDirectAlone = 3;
 
 // CTAs of k_bamat_slabs_t that are resident at once.
 static int slab_ctas(size_t smem) {
@@ -486,6 +490,10 @@ static int slab_ctas(size_t smem) {
 int launch_bamat(const Rdm &r, const double *atwo, const double *f, int ncore, double *amat, double *atmat,
                  cudaStream_t st, bool split) {
     const int n = r.n, M = r.M;
+    if (n <= kDirectAlone) {
+        launch_bamat_direct(r, atwo, f, ncore, amat, atmat, st, nullptr);
+        return 0;
+    }
     const ll n2 = (ll)n * n, n3 = n2 * n, n4 = n3 * n, n6 = n3 * n3;
     AsyncBuffers buf(st);
     // One contraction per state whose inputs have their physical symmetries

@@ -293,7 +293,7 @@ int nvpt_profile_read(nvpt_context *ctx, const char *tag, double *ms, int64_t *l
 /* Polls a device-side wait (between the blocks of a tridiagonalisation or band
  * reduction, in nvpt_sytrd_d and nvpt_qdnevpt) makes before it
  * gives up on ctx; 0 (the default) restores the built-in limit of 2^22
- * polls with back-off (about 0.4 s).  A wait that gives up makes the kernel
+ * polls (1 to 2 s).  A wait that gives up makes the kernel
  * return, and the call returns NVPT_ETIMEDOUT with the context still usable.
  * No counterpart in the reference; for callers that want a tighter bound. */
 int nvpt_set_wait_limit(nvpt_context *ctx, int64_t polls);

@@ -12,8 +12,8 @@
 // 4: 4096 elements), so the (d, e) pairs are dealt to LANES of them: eight below n = 5,
 // where elements are few; four in blocks of TB = 512 at n = 5, or the symmetric
 // states, for which every block returns at once, pay 2 us for the number of blocks.
-// One state, the call, one thread / now: n = 2 97 / 52 us, n = 3 235 / 84, n = 4 502 / 124,
-// n = 5 992 / 621.
+// One state without the symmetries, the call, one thread / now: n = 2 97 / 27 us, n = 3 235 /
+// 54 (no check ahead any more), n = 4 502 / 124, n = 5 992 / 621.
 #include "nvpt2_internal.h"
 
 namespace nvpt {
